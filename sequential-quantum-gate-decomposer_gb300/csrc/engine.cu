@@ -30,6 +30,8 @@
 #include "../../include/sqg.h"
 #include "gates.cuh"
 #include "handle.h"
+#include "rotgrad.cuh"
+#include "rotplan.h"
 #include "tile.cuh"
 #include "tilekern.cuh"
 
@@ -98,62 +100,44 @@ __global__ void k_prep(const Gate* __restrict__ gates, int L, int P, const doubl
   gm[(long long)b * L + g] = m;
 }
 
-template <bool WRITE_BACK, bool TRACE>
+// Numbers of the plan's operations, one CTA per (CTA of runs, instance).
+__global__ void __launch_bounds__(kRotThreads) k_rot_plan(RotPlan pl, const double* __restrict__ theta,
+                                                          long long theta_stride, RotRec* __restrict__ recs,
+                                                          double2* __restrict__ phases) {
+  const long long b = blockIdx.y;
+  rot_plan_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nops, phases + b * pl.ncta + blockIdx.x);
+}
+
+template <bool WRITE_BACK, bool TRACE, int DIR>
 __global__ void __launch_bounds__(kMaxThreads) k_tile_forward(TileArgs a) {
   extern __shared__ double2 smem[];
-  tile_forward_body<WRITE_BACK, TRACE>(a, blockIdx.y, blockIdx.x, smem);
+  tile_forward_body<WRITE_BACK, TRACE, DIR>(a, blockIdx.y, blockIdx.x, smem);
 }
 
+template <bool CPLX>
 __global__ void __launch_bounds__(kMaxThreads) k_tile_adjoint(TileArgs a) {
   extern __shared__ double2 smem[];
-  tile_adjoint_body(a, blockIdx.y, blockIdx.x, smem);
+  tile_adjoint_body<CPLX>(a, blockIdx.y, blockIdx.x, smem);
 }
 
-// Sums the per-tile partials in a fixed order and applies the cost-variant epilogue of
-// the reference (Optimization_Interface.cpp:677-735 for the cost, :1397-1458 for the
-// gradient components).
-__global__ void k_finish(const double2* __restrict__ ws_tr, const double2* __restrict__ ws_gr, int tiles, int P,
-                         int cols, int variant, double* __restrict__ cost, double* __restrict__ grad) {
-  const int b = blockIdx.x;
-  double2 tr = make_double2(0.0, 0.0);
-  for (int t = 0; t < tiles; t++) {
-    double2 v = ws_tr[(long long)b * tiles + t];
-    tr.x += v.x;
-    tr.y += v.y;
-  }
-  if (blockIdx.y == 0 && threadIdx.x == 0) {
-    double f;
-    if (variant == SQG_FROBENIUS_NORM) {
-      f = 1.0 - tr.x / cols;
-    } else if (variant == SQG_HILBERT_SCHMIDT_TEST) {
-      double d = 1.0 / cols;
-      f = 1.0 - d * d * (tr.x * tr.x + tr.y * tr.y);
-    } else {
-      double d = cols;
-      f = 1.0 - ((tr.x * tr.x + tr.y * tr.y) / d + 1) / (d + 1);
-    }
-    cost[b] = f;
-  }
-  if (!grad) return;
-  const int p = blockIdx.y * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  double2 dt = make_double2(0.0, 0.0);
-  for (int t = 0; t < tiles; t++) {
-    double2 v = ws_gr[((long long)b * tiles + t) * P + p];
-    dt.x += v.x;
-    dt.y += v.y;
-  }
-  double gv;
-  if (variant == SQG_FROBENIUS_NORM) {
-    gv = (1.0 - dt.x / cols) - 1.0;
-  } else if (variant == SQG_HILBERT_SCHMIDT_TEST) {
-    double d = 1.0 / cols;
-    gv = -2.0 * d * d * tr.x * dt.x - 2.0 * d * d * tr.y * dt.y;
-  } else {
-    double d = cols;
-    gv = -2.0 / d / (d + 1) * tr.x * dt.x - 2.0 / d / (d + 1) * tr.y * dt.y;
-  }
-  grad[(long long)b * P + p] = gv;
+// Sums the per-tile partials in a fixed order and writes the cost; W doubles per overlap.
+template <int W>
+__global__ void __launch_bounds__(32 * kSumGroups) k_tile_sum(double2* ws_tr, double* ws_gr, int tiles, int noverlaps,
+                                                              int cols, int variant, double* __restrict__ cost) {
+  const long long b = blockIdx.y;
+  tile_sum_body<W>(blockIdx.x, ws_tr + b * tiles, ws_gr + b * tiles * noverlaps * W, tiles, noverlaps, cols, variant,
+                   cost + b);
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(kRotThreads) k_rot_grad(RotPlan pl, const double* __restrict__ theta,
+                                                          const RotRec* __restrict__ recs,
+                                                          const double2* __restrict__ ws_tr,
+                                                          const double* __restrict__ ws_gr, int tiles, int P, int cols,
+                                                          int variant, double* __restrict__ grad) {
+  const long long b = blockIdx.y;
+  rot_grad_body<CPLX>(pl, blockIdx.x, theta + b * P, recs + b * pl.nops, ws_tr + b * tiles,
+                      ws_gr + b * tiles * pl.noverlaps * (CPLX ? 2 : 1), cols, variant, grad + b * P);
 }
 
 // -------------------------------------------------------------------------------------
@@ -342,106 +326,67 @@ int set_smem(K kernel, size_t bytes) {
   return SQG_OK;
 }
 
+// Workspace of the per-gate kernels: gate matrices and (sin, cos) of every parameter.
 struct PrepLayout {
-  size_t gm_off, sc_off, mg_off, end;
+  size_t gm_off, sc_off, end;
 };
 PrepLayout prep_layout(const sqg_circuit* c, int B, size_t start) {
   PrepLayout l;
   l.gm_off = align_up(start, 256);
   l.sc_off = align_up(l.gm_off + (size_t)B * std::max(c->L, 1) * sizeof(GateMat), 256);
-  l.mg_off = align_up(l.sc_off + (size_t)B * std::max(c->P, 1) * sizeof(double2), 256);
-  l.end = align_up(l.mg_off + (size_t)B * c->Lm * sizeof(GateMat), 256);
+  l.end = align_up(l.sc_off + (size_t)B * std::max(c->P, 1) * sizeof(double2), 256);
   return l;
 }
 
-// Full 2x2 matrix of a single-qubit gate from its GateMat (k_prep's storage: U3 whole, the
-// one-parameter gates as (cos, sin) in u[0]).
-__device__ __forceinline__ void full_matrix(int type, const GateMat& m, double2 u[4]) {
-  const double c = m.u[0].x, s = m.u[0].y;
-  if (type == G_U3) {
-    u[0] = m.u[0]; u[1] = m.u[1]; u[2] = m.u[2]; u[3] = m.u[3];
-  } else if (type == G_RY) {
-    u[0] = make_double2(c, 0.0); u[1] = make_double2(dneg(s), 0.0);
-    u[2] = make_double2(s, 0.0); u[3] = make_double2(c, 0.0);
-  } else if (type == G_RX) {
-    u[0] = make_double2(c, 0.0); u[1] = make_double2(0.0, dneg(s));
-    u[2] = make_double2(0.0, dneg(s)); u[3] = make_double2(c, 0.0);
-  } else {  // G_RZ
-    u[0] = make_double2(c, dneg(s)); u[1] = make_double2(0.0, 0.0);
-    u[2] = make_double2(0.0, 0.0); u[3] = make_double2(c, s);
-  }
+// Workspace of the plan's numbers (at most prep_layout's: no more operations than gates, no
+// more CTAs than parameters).
+struct RotLayout {
+  size_t rec_off, ph_off, end;
+};
+RotLayout rot_layout(const sqg_circuit* c, int B, size_t start) {
+  RotLayout l;
+  l.rec_off = align_up(start, 256);
+  l.ph_off = align_up(l.rec_off + (size_t)B * c->plan.nops * sizeof(RotRec), 256);
+  l.end = align_up(l.ph_off + (size_t)B * c->plan.ncta * sizeof(double2), 256);
+  return l;
 }
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-
-// Gate matrices of the merged forward plan, one thread per (instance, merged gate): a kept
-// gate copies its matrix, a merged run multiplies its members' matrices in circuit order
-// (M = G_k ... G_1).
-__global__ void k_merge(const Gate* __restrict__ gates, const GateMat* __restrict__ gm, int L,
-                        const Gate* __restrict__ mgates, const int* __restrict__ mfirst,
-                        const int* __restrict__ members, int Lm, GateMat* __restrict__ out) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (m >= Lm) return;
-  const GateMat* g = gm + (long long)b * L;
-  const int f = mfirst[m], e = mfirst[m + 1];
-  GateMat r;
-  if (mgates[m].type != G_GEN) {
-    r = g[members[f]];
-  } else {
-    double2 M[4];
-    full_matrix(gates[members[f]].type, g[members[f]], M);
-    for (int k = f + 1; k < e; k++) {
-      double2 G[4], R[4];
-      full_matrix(gates[members[k]].type, g[members[k]], G);
-      R[0] = cmul(G[0], M[0]); R[0].x += cmul(G[1], M[2]).x; R[0].y += cmul(G[1], M[2]).y;
-      R[1] = cmul(G[0], M[1]); R[1].x += cmul(G[1], M[3]).x; R[1].y += cmul(G[1], M[3]).y;
-      R[2] = cmul(G[2], M[0]); R[2].x += cmul(G[3], M[2]).x; R[2].y += cmul(G[3], M[2]).y;
-      R[3] = cmul(G[2], M[1]); R[3].x += cmul(G[3], M[3]).x; R[3].y += cmul(G[3], M[3]).y;
-      M[0] = R[0]; M[1] = R[1]; M[2] = R[2]; M[3] = R[3];
-    }
-    r.u[0] = M[0]; r.u[1] = M[1]; r.u[2] = M[2]; r.u[3] = M[3];
-  }
-  out[(long long)b * Lm + m] = r;
-}
-
-// Forward gate list and matrices of a tile launch: the merged plan when the circuit has one
-// (its matrices computed into the workspace at prep.mg_off), else the gates themselves.
-int forward_plan(const sqg_circuit* c, const PrepLayout& prep, char* ws, int B, const GateMat* gm, TileArgs& a,
-                 cudaStream_t st) {
-  if (c->Lm == 0) {
-    a.gates = c->d_gates;
-    a.L = c->L;
-    a.gm = gm;
-    return SQG_OK;
-  }
-  GateMat* mg = (GateMat*)(ws + prep.mg_off);
-  k_merge<<<dim3((c->Lm + 127) / 128, B), 128, 0, st>>>(c->d_gates, gm, c->L, c->d_mgates, c->d_mfirst,
-                                                         c->d_mmembers, c->Lm, mg);
-  a.gates = c->d_mgates;
-  a.L = c->Lm;
-  a.gm = mg;
-  return cuda_status(cudaGetLastError(), "k_merge");
+// Makes the plan's numbers for B parameter vectors in the workspace and points `a` at them.
+int launch_plan(const sqg_circuit* c, const double* theta, long long theta_stride, int B, const RotLayout& l, char* ws,
+                TileArgs& a, cudaStream_t st) {
+  RotRec* recs = (RotRec*)(ws + l.rec_off);
+  double2* ph = (double2*)(ws + l.ph_off);
+  a.ops = c->plan.ops;
+  a.nops = c->plan.nops;
+  a.noverlaps = c->plan.noverlaps;
+  a.n = c->n;
+  a.N = c->N;
+  a.recs = recs;
+  a.phases = ph;
+  a.nphase = c->plan.ncta;
+  if (c->plan.ncta == 0) return SQG_OK;
+  k_rot_plan<<<dim3(c->plan.ncta, B), kRotThreads, 0, st>>>(c->plan, theta, theta_stride, recs, ph);
+  return cuda_status(cudaGetLastError(), "k_rot_plan");
 }
 
 struct EvalLayout {
-  PrepLayout prep;
+  RotLayout rot;
   size_t tr_off, gr_off, ck_off, end;
   TilePlan plan;
   int nck;
 };
+// The overlaps take two doubles each, whatever the cost variant: FROBENIUS_NORM, which needs
+// only their imaginary parts, uses half of that.
 EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckpt_interval) {
   EvalLayout l;
-  l.prep = prep_layout(c, B, 0);
+  l.rot = rot_layout(c, B, 0);
   l.plan = plan_tiles(c->N, cols, grad, B);
-  l.tr_off = l.prep.end;
+  l.tr_off = l.rot.end;
   l.gr_off = align_up(l.tr_off + (size_t)B * l.plan.tiles * sizeof(double2), 256);
-  size_t gr_bytes = grad ? (size_t)B * l.plan.tiles * std::max(c->P, 1) * sizeof(double2) : 0;
+  size_t gr_bytes = grad ? (size_t)B * l.plan.tiles * std::max(c->plan.noverlaps, 1) * sizeof(double2) : 0;
   l.ck_off = align_up(l.gr_off + gr_bytes, 256);
   l.nck = 0;
-  if (grad && ckpt_interval > 0) l.nck = c->L / ckpt_interval;
+  if (grad && ckpt_interval > 0) l.nck = c->plan.nops / ckpt_interval;
   size_t ck_bytes = (size_t)B * l.plan.tiles * l.nck * (size_t)l.plan.TC * c->N * sizeof(double2);
   l.end = align_up(l.ck_off + ck_bytes, 256);
   return l;
@@ -485,7 +430,8 @@ constexpr int kStateThreads = 256;
 int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
   const int n = c->n, K = std::min(n, kStateK), low = std::min(K, kStateLow);
   c->sK = K;
-  std::vector<Gate> lg(c->h_gates);
+  std::vector<RotOp> lops(c->h_ops);
+  size_t done = 0;  // operations placed in blocks (they follow the order of their anchor gates)
   std::vector<int> hitab, inact;
   std::vector<int> inA(n, 0);
   auto close_block = [&](int g0, int g1) {
@@ -500,10 +446,12 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
     std::sort(A.begin(), A.end());
     std::vector<int> loc(n, -1);
     for (int j = 0; j < (int)A.size(); j++) loc[A[j]] = j;
-    for (int g = g0; g < g1; g++) {
-      lg[g].target = loc[c->h_gates[g].target];
-      if (gate_controlled(c->h_gates[g].type)) lg[g].control = loc[c->h_gates[g].control];
+    const int k0 = (int)done;
+    for (; done < lops.size() && c->h_anchor[done] < g1; done++) {
+      const int t = lops[done].qubits & 255, ctl = lops[done].qubits >> 8;
+      lops[done].qubits = loc[t] | (lops[done].kind <= kOpCry ? loc[ctl] << 8 : 0);
     }
+    (void)g0;
     const int hb = K - low;
     for (int h = 0; h < 128; h++) {
       int off = 0;
@@ -519,7 +467,7 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
         k++;
       }
     for (; k < 32; k++) inact.push_back(0);
-    c->sblocks.push_back({g0, g1});
+    c->sblocks.push_back({k0, (int)done});
     std::fill(inA.begin(), inA.end(), 0);
   };
   int g0 = 0, used = 0;
@@ -578,8 +526,8 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
   }
   if (c->L > 0) close_block(g0, c->L);
   if (c->L == 0) return SQG_OK;
-  cudaError_t e = cudaMalloc(&c->d_lgates, sizeof(Gate) * c->L);
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_lgates, lg.data(), sizeof(Gate) * c->L, cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMalloc(&c->d_lops, sizeof(RotOp) * lops.size());
+  if (e == cudaSuccess) e = cudaMemcpy(c->d_lops, lops.data(), sizeof(RotOp) * lops.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&c->d_hitab, sizeof(int) * hitab.size());
   if (e == cudaSuccess) e = cudaMemcpy(c->d_hitab, hitab.data(), sizeof(int) * hitab.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&c->d_inact, sizeof(int) * inact.size());
@@ -594,9 +542,11 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
 struct StateArgs {
   double2* states;
   long long stride;
-  int n, K, low, g0, g1, L;
-  const Gate* lgates;
-  const GateMat* gm;
+  int n, K, low, k0, k1, nops;
+  const RotOp* lops;
+  const RotRec* recs;     // [B][nops]
+  const double2* phases;  // [B][nphase], multiplied in by this pass; null: by another one
+  int nphase;
   const int* hitab;
   const int* inact;
 };
@@ -604,6 +554,7 @@ struct StateArgs {
 __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   extern __shared__ double2 sv[];
   __shared__ int hit[128];
+  __shared__ StagedOp st[kRotChunk];
   const int b = blockIdx.y;
   const int KK = 1 << a.K, hb = a.K - a.low, lowmask = (1 << a.low) - 1;
   for (int h = threadIdx.x; h < (1 << hb); h += blockDim.x) hit[h] = a.hitab[h];
@@ -613,14 +564,24 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   double2* base = a.states + (long long)b * a.stride + cbase;
   __syncthreads();
   for (int l = threadIdx.x; l < KK; l += blockDim.x) sv[l] = base[(l & lowmask) + hit[l >> a.low]];
-  __syncthreads();
-  const GateMat* gmb = a.gm + (long long)b * a.L;
-  for (int g = a.g0; g < a.g1; g++) {
-    const Gate gt = a.lgates[g];
-    tile_apply(sv, KK, a.K, 1, gt, make_op(gt.type, gmb[g], ORIENT_FWD));
+  const RotRec* recs = a.recs + (long long)b * a.nops;
+  for (int k0 = a.k0; k0 < a.k1; k0 += kRotChunk) {
+    const int kn = min(kRotChunk, a.k1 - k0);
     __syncthreads();
+    stage_ops(st, a.lops, recs, k0, kn);
+    __syncthreads();
+    for (int j = 0; j < kn; j++) {
+      rot_tile<kRotFwd>(sv, KK, a.K, 1, st[j]);
+      __syncthreads();
+    }
   }
-  for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = sv[l];
+  if (a.phases) {
+    double2 p = make_double2(1.0, 0.0);
+    for (int k = 0; k < a.nphase; k++) p = cmul(p, a.phases[(long long)b * a.nphase + k]);
+    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = cmul(p, sv[l]);
+  } else {
+    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = sv[l];
+  }
 }
 
 }  // namespace
@@ -628,58 +589,31 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
 // =====================================================================================
 // C ABI
 // =====================================================================================
-// Merged forward plan: walking the gates in order, single-qubit gates collect per qubit; a
-// two-qubit gate first emits the open runs of its two qubits, then itself; the remaining runs
-// are emitted at the end.  This only moves single-qubit gates past gates on other qubits, with
-// which they commute.  A run becomes one general 2x2 gate (16 FP64 instructions per amplitude
-// pair) when its members cost more (U3 14, RX/RY/RZ 8), otherwise its members stay.  The plan is
-// kept only if it removes work; the adjoint and right-application paths use the gates as given.
-int build_merge_plan(sqg_circuit* c) {
-  const std::vector<Gate>& g = c->h_gates;
-  std::vector<std::vector<int>> open(c->n);
-  std::vector<Gate> mg;
-  std::vector<int> first{0}, members;
-  bool merged = false;
-  auto cost1 = [](int type) { return type == G_U3 ? 14 : 8; };
-  auto emit_one = [&](int i) {
-    mg.push_back(g[i]);
-    members.push_back(i);
-    first.push_back((int)members.size());
-  };
-  auto flush = [&](int q) {
-    std::vector<int>& run = open[q];
-    int sum = 0;
-    for (int i : run) sum += cost1(g[i].type);
-    if (run.size() >= 2 && sum > 16) {
-      mg.push_back(Gate{G_GEN, q, -1, -1});
-      members.insert(members.end(), run.begin(), run.end());
-      first.push_back((int)members.size());
-      merged = true;
-    } else {
-      for (int i : run) emit_one(i);
-    }
-    run.clear();
-  };
-  for (int i = 0; i < c->L; i++) {
-    if (gate_controlled(g[i].type)) {
-      flush(g[i].target);
-      flush(g[i].control);
-      emit_one(i);
-    } else {
-      open[g[i].target].push_back(i);
-    }
-  }
-  for (int q = 0; q < c->n; q++) flush(q);
-  if (!merged) return SQG_OK;
-  c->Lm = (int)mg.size();
-  cudaError_t e = cudaMalloc(&c->d_mgates, sizeof(Gate) * mg.size());
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_mfirst, sizeof(int) * first.size());
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_mmembers, sizeof(int) * members.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_mgates, mg.data(), sizeof(Gate) * mg.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_mfirst, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(c->d_mmembers, members.data(), sizeof(int) * members.size(), cudaMemcpyHostToDevice);
-  return cuda_status(e, "merged forward plan");
+// Makes the rotation plan of the circuit and copies it to the device.
+static int make_rot_plan(sqg_circuit* c) {
+  RotPlanHost h = build_rot_plan(c->n, c->h_gates);
+  c->h_ops = h.ops;
+  c->h_anchor = h.anchor;
+  RotPlan& p = c->plan;
+  p.gates = c->d_gates;
+  p.nops = (int)h.ops.size();
+  p.ncta = (int)h.cta.size() - 1;
+  p.noverlaps = h.noverlaps;
+  const size_t ob = h.ops.size() * sizeof(RotOp), rb = h.runs.size() * sizeof(RotRun), mb = h.members.size() * sizeof(int),
+               cb = h.cta.size() * sizeof(int);
+  std::vector<char> blob(ob + rb + mb + cb);
+  if (ob) memcpy(blob.data(), h.ops.data(), ob);
+  if (rb) memcpy(blob.data() + ob, h.runs.data(), rb);
+  if (mb) memcpy(blob.data() + ob + rb, h.members.data(), mb);
+  memcpy(blob.data() + ob + rb + mb, h.cta.data(), cb);
+  cudaError_t e = cudaMalloc(&c->d_plan, blob.size());
+  if (e == cudaSuccess) e = cudaMemcpy(c->d_plan, blob.data(), blob.size(), cudaMemcpyHostToDevice);
+  char* d = (char*)c->d_plan;
+  p.ops = (const RotOp*)d;
+  p.runs = (const RotRun*)(d + ob);
+  p.members = (const int*)(d + ob + rb);
+  p.cta = (const int*)(d + ob + rb + mb);
+  return cuda_status(e, "rotation plan");
 }
 
 extern "C" {
@@ -747,8 +681,8 @@ int sqg_circuit_create(int qbit_num, const sqg_gate* gates, int gate_num, sqg_ci
       return st;
     }
   }
-  int st = build_state_plan(c);
-  if (!st) st = build_merge_plan(c);
+  int st = make_rot_plan(c);
+  if (!st) st = build_state_plan(c);
   if (st) {
     sqg_circuit_destroy(c);
     return st;
@@ -768,10 +702,10 @@ int sqg_circuit_set_partitions(sqg_circuit* c, const int* part_ends, int nparts)
   int dev = -1;
   cudaGetDevice(&dev);
   if (dev != c->device) return fail(SQG_ERR_INVALID_ARGUMENT, "circuit handle belongs to another device");
-  cudaFree(c->d_lgates);
+  cudaFree(c->d_lops);
   cudaFree(c->d_hitab);
   cudaFree(c->d_inact);
-  c->d_lgates = nullptr;
+  c->d_lops = nullptr;
   c->d_hitab = nullptr;
   c->d_inact = nullptr;
   c->sblocks.clear();
@@ -781,12 +715,10 @@ int sqg_circuit_set_partitions(sqg_circuit* c, const int* part_ends, int nparts)
 int sqg_circuit_destroy(sqg_circuit* c) {
   if (!c) return SQG_OK;
   if (c->d_gates) cudaFree(c->d_gates);
-  if (c->d_lgates) cudaFree(c->d_lgates);
+  if (c->d_lops) cudaFree(c->d_lops);
   if (c->d_hitab) cudaFree(c->d_hitab);
   if (c->d_inact) cudaFree(c->d_inact);
-  if (c->d_mgates) cudaFree(c->d_mgates);
-  if (c->d_mfirst) cudaFree(c->d_mfirst);
-  if (c->d_mmembers) cudaFree(c->d_mmembers);
+  if (c->d_plan) cudaFree(c->d_plan);
   delete c;
   return SQG_OK;
 }
@@ -842,15 +774,10 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   if (!workspace || ws_bytes < l.end) return fail(SQG_ERR_WORKSPACE, "workspace too small: need " + std::to_string(l.end));
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = (char*)workspace;
-  GateMat* gm = (GateMat*)(ws + l.prep.gm_off);
-  double2* sc = (double2*)(ws + l.prep.sc_off);
   double2* wtr = (double2*)(ws + l.tr_off);
-  double2* wgr = (double2*)(ws + l.gr_off);
-  if ((st = launch_prep(c, theta, c->P, B, gm, sc, s))) return st;
+  double* wgr = (double*)(ws + l.gr_off);
   TileArgs a;
-  a.gates = c->d_gates;
-  a.L = c->L; a.P = c->P; a.n = c->n; a.N = c->N;
-  a.gm = gm; a.sc = sc;
+  if ((st = launch_plan(c, theta, c->P, B, l.rot, ws, a, s))) return st;
   a.mtx = (double2*)target;
   a.bstride = target_batch_stride;
   a.rstride = cols;
@@ -859,26 +786,34 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   a.TC = l.plan.TC;
   a.tiles = l.plan.tiles;
   a.trace_offset = off;
-  a.reverse_order = 0;
-  a.orient = ORIENT_FWD;
   a.ws_tr = wtr;
   a.ws_gr = wgr;
   a.ckpt = l.nck > 0 ? (double2*)(ws + l.ck_off) : nullptr;
   a.ckpt_interval = checkpoint_interval;
   a.nck = l.nck;
-  dim3 grid(l.plan.tiles, B);
-  if (with_grad) {
-    if ((st = set_smem(k_tile_adjoint, l.plan.smem))) return st;
-    k_tile_adjoint<<<grid, l.plan.threads, l.plan.smem, s>>>(a);
-  } else {
-    if ((st = forward_plan(c, l.prep, ws, B, gm, a, s))) return st;
-    if ((st = set_smem(k_tile_forward<false, true>, l.plan.smem))) return st;
-    k_tile_forward<false, true><<<grid, l.plan.threads, l.plan.smem, s>>>(a);
+  const dim3 grid(l.plan.tiles, B);
+  if (!with_grad) {
+    if ((st = set_smem(k_tile_forward<false, true, kRotFwd>, l.plan.smem))) return st;
+    k_tile_forward<false, true, kRotFwd><<<grid, l.plan.threads, l.plan.smem, s>>>(a);
+    if ((st = cuda_status(cudaGetLastError(), "tile kernel"))) return st;
+    k_tile_sum<1><<<dim3(1, B), 32 * kSumGroups, 0, s>>>(wtr, nullptr, l.plan.tiles, 0, cols, variant, cost);
+    return cuda_status(cudaGetLastError(), "k_tile_sum");
   }
-  if ((st = cuda_status(cudaGetLastError(), "tile kernel"))) return st;
-  dim3 fgrid(B, with_grad ? (c->P + 127) / 128 : 1);
-  k_finish<<<fgrid, 128, 0, s>>>(wtr, wgr, l.plan.tiles, c->P, cols, variant, cost, with_grad ? grad : nullptr);
-  return cuda_status(cudaGetLastError(), "k_finish");
+  const int nov = c->plan.noverlaps;
+  const dim3 sgrid((nov + 31) / 32, B), ggrid(c->plan.ncta, B);
+  // the other variants multiply the derivative of the trace by the trace: complex overlaps
+  if (variant == SQG_FROBENIUS_NORM) {
+    if ((st = set_smem(k_tile_adjoint<false>, l.plan.smem))) return st;
+    k_tile_adjoint<false><<<grid, l.plan.threads, l.plan.smem, s>>>(a);
+    k_tile_sum<1><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
+    k_rot_grad<false><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
+  } else {
+    if ((st = set_smem(k_tile_adjoint<true>, l.plan.smem))) return st;
+    k_tile_adjoint<true><<<grid, l.plan.threads, l.plan.smem, s>>>(a);
+    k_tile_sum<2><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
+    k_rot_grad<true><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
+  }
+  return cuda_status(cudaGetLastError(), "cost and gradient kernels");
 }
 
 }  // extern "C"
@@ -1001,16 +936,11 @@ int sqg_apply(const sqg_circuit* c, const double* theta, int B, void* mtx, int c
   if (c->L == 0) return SQG_OK;
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = (char*)workspace;
-  GateMat* gm = (GateMat*)(ws + l.gm_off);
-  double2* sc = (double2*)(ws + l.sc_off);
-  if ((st = launch_prep(c, theta, c->P, B, gm, sc, s))) return st;
   if (fused) {
     TilePlan pl = plan_tiles(c->N, cols, false);
     TileArgs a;
     memset(&a, 0, sizeof(a));
-    a.gates = c->d_gates;
-    a.L = c->L; a.P = c->P; a.n = c->n; a.N = c->N;
-    a.gm = gm; a.sc = sc;
+    if ((st = launch_plan(c, theta, c->P, B, rot_layout(c, B, 0), ws, a, s))) return st;
     a.mtx = (double2*)mtx;
     a.bstride = batch_stride;
     a.rstride = stride;
@@ -1018,12 +948,13 @@ int sqg_apply(const sqg_circuit* c, const double* theta, int B, void* mtx, int c
     a.cols = cols;
     a.TC = pl.TC;
     a.tiles = pl.tiles;
-    a.orient = ORIENT_FWD;
-    if ((st = forward_plan(c, l, ws, B, gm, a, s))) return st;
-    if ((st = set_smem(k_tile_forward<true, false>, pl.smem))) return st;
-    k_tile_forward<true, false><<<dim3(pl.tiles, B), pl.threads, pl.smem, s>>>(a);
+    if ((st = set_smem(k_tile_forward<true, false, kRotFwd>, pl.smem))) return st;
+    k_tile_forward<true, false, kRotFwd><<<dim3(pl.tiles, B), pl.threads, pl.smem, s>>>(a);
     return cuda_status(cudaGetLastError(), "k_tile_forward");
   }
+  GateMat* gm = (GateMat*)(ws + l.gm_off);
+  double2* sc = (double2*)(ws + l.sc_off);
+  if ((st = launch_prep(c, theta, c->P, B, gm, sc, s))) return st;
   // unfused: one pass over the matrix per gate
   for (int b = 0; b < B; b++) {
     double2* base = (double2*)mtx + (long long)b * batch_stride;
@@ -1057,16 +988,10 @@ int sqg_apply_from_right(const sqg_circuit* c, const double* theta, void* mtx, i
   if (!workspace || ws_bytes < l.end) return fail(SQG_ERR_WORKSPACE, "workspace too small: need " + std::to_string(l.end));
   if (c->L == 0) return SQG_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  char* ws = (char*)workspace;
-  GateMat* gm = (GateMat*)(ws + l.gm_off);
-  double2* sc = (double2*)(ws + l.sc_off);
-  if ((st = launch_prep(c, theta, c->P, 1, gm, sc, s))) return st;
   TilePlan pl = plan_tiles(c->N, rows, false);
   TileArgs a;
   memset(&a, 0, sizeof(a));
-  a.gates = c->d_gates;
-  a.L = c->L; a.P = c->P; a.n = c->n; a.N = c->N;
-  a.gm = gm; a.sc = sc;
+  if ((st = launch_plan(c, theta, c->P, 1, rot_layout(c, 1, 0), (char*)workspace, a, s))) return st;
   a.mtx = (double2*)mtx;
   a.bstride = 0;
   a.rstride = stride;
@@ -1074,10 +999,8 @@ int sqg_apply_from_right(const sqg_circuit* c, const double* theta, void* mtx, i
   a.cols = rows;
   a.TC = pl.TC;
   a.tiles = pl.tiles;
-  a.reverse_order = 1;
-  a.orient = ORIENT_TRANS;
-  if ((st = set_smem(k_tile_forward<true, false>, pl.smem))) return st;
-  k_tile_forward<true, false><<<dim3(pl.tiles, 1), pl.threads, pl.smem, s>>>(a);
+  if ((st = set_smem(k_tile_forward<true, false, kRotTrans>, pl.smem))) return st;
+  k_tile_forward<true, false, kRotTrans><<<dim3(pl.tiles, 1), pl.threads, pl.smem, s>>>(a);
   return cuda_status(cudaGetLastError(), "k_tile_forward(right)");
 }
 
@@ -1143,30 +1066,34 @@ int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* stat
   if (c->L == 0) return SQG_OK;
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = (char*)workspace;
-  GateMat* gm = (GateMat*)(ws + l.gm_off);
-  double2* sc = (double2*)(ws + l.sc_off);
-  if ((st = launch_prep(c, theta, c->P, B, gm, sc, s))) return st;
   if (fused) {
     const size_t smem = sizeof(double2) << c->sK;
     if ((st = set_smem(k_state_block, smem))) return st;
+    TileArgs t;
+    if ((st = launch_plan(c, theta, c->P, B, rot_layout(c, B, 0), ws, t, s))) return st;
     StateArgs a;
     a.states = (double2*)states;
     a.stride = stride;
     a.n = c->n;
     a.K = c->sK;
     a.low = std::min(c->sK, kStateLow);
-    a.L = c->L;
-    a.lgates = c->d_lgates;
-    a.gm = gm;
+    a.nops = t.nops;
+    a.lops = c->d_lops;
+    a.recs = t.recs;
+    a.nphase = t.nphase;
     for (size_t k = 0; k < c->sblocks.size(); k++) {
-      a.g0 = c->sblocks[k].g0;
-      a.g1 = c->sblocks[k].g1;
+      a.k0 = c->sblocks[k].k0;
+      a.k1 = c->sblocks[k].k1;
+      a.phases = k == 0 && t.nphase > 0 ? t.phases : nullptr;
       a.hitab = c->d_hitab + 128 * k;
       a.inact = c->d_inact + 32 * k;
       k_state_block<<<dim3(1u << (c->n - c->sK), B), kStateThreads, smem, s>>>(a);
     }
     return cuda_status(cudaGetLastError(), "k_state_block");
   }
+  GateMat* gm = (GateMat*)(ws + l.gm_off);
+  double2* sc = (double2*)(ws + l.sc_off);
+  if ((st = launch_prep(c, theta, c->P, B, gm, sc, s))) return st;
   // unfused: one pass over the state per gate
   for (int b = 0; b < B; b++) {
     double2* base = (double2*)states + (long long)b * stride;

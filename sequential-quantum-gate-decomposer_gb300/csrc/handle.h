@@ -5,11 +5,12 @@
 #include <vector>
 
 #include "gates.cuh"
+#include "rot.cuh"
 
 // Fused state-vector passes (sqg_apply_state): consecutive gates whose qubits, together with
 // the lowest ones, fit one chunk of 2^K amplitudes form a block applied in shared memory.
 struct sqg_state_block {
-  int g0, g1;  // gates [g0, g1)
+  int k0, k1;  // operations [k0, k1) of the rotation plan
 };
 
 struct sqg_circuit {
@@ -17,21 +18,20 @@ struct sqg_circuit {
   int device = 0;
   sqg::Gate* d_gates = nullptr;
   std::vector<sqg::Gate> h_gates;
-  // state-vector plan: chunk qubits K, blocks, gate records with chunk-local qubit positions,
+  // state-vector plan: chunk qubits K, blocks, operations with chunk-local qubit positions,
   // per block the global offsets of the chunk's high local bits (2^(K - low) ints, padded to
   // 128) and the qubits that number the chunks (padded to 32)
   int sK = 0;
   std::vector<sqg_state_block> sblocks;
-  sqg::Gate* d_lgates = nullptr;
+  sqg::RotOp* d_lops = nullptr;
   int* d_hitab = nullptr;
   int* d_inact = nullptr;
-  // merged forward plan (Lm > 0 when it saves work): runs of single-qubit gates on one qubit
-  // with no two-qubit gate on that qubit between them become one general 2x2 gate; d_mgates
-  // holds the Lm records, members d_mmembers[d_mfirst[m] .. d_mfirst[m + 1]) their source gates
-  int Lm = 0;
-  sqg::Gate* d_mgates = nullptr;
-  int* d_mfirst = nullptr;
-  int* d_mmembers = nullptr;
+  // rotation plan (rot.cuh): the host's copy of the operations with the gate whose place each
+  // takes, and the device arrays, one allocation behind d_plan
+  std::vector<sqg::RotOp> h_ops;
+  std::vector<int> h_anchor;
+  void* d_plan = nullptr;
+  sqg::RotPlan plan = {};
 };
 
 namespace sqg {

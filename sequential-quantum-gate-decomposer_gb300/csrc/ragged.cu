@@ -13,6 +13,7 @@
 #include "../../include/sqg.h"
 #include "gates.cuh"
 #include "handle.h"
+#include "rotgrad.cuh"
 #include "tile.cuh"
 #include "tilekern.cuh"
 
@@ -23,9 +24,10 @@ namespace {
 constexpr int kRaggedThreads = 256;
 
 struct InstDesc {
-  const Gate* gates;
-  int L, P, n, N, cols, TC, tiles;
-  long long theta_off, target_off, gm_off, sc_off, tr_off, gr_off;
+  RotPlan plan;
+  int P, n, N, cols, TC, tiles;
+  // offsets of the instance in the packed arrays; gr_off counts overlaps
+  long long theta_off, target_off, rec_off, ph_off, tr_off, gr_off;
 };
 
 }  // namespace
@@ -35,56 +37,33 @@ struct sqg_ragged_batch {
   size_t smem = 0;
   InstDesc* d_desc = nullptr;
   int2* d_items = nullptr;     // (instance, tile), decreasing work
-  int2* d_gate_map = nullptr;  // (instance, gate) for every gate of the batch
-  int total_gates = 0, maxP = 1;
-  long long total_gm = 0, total_sc = 0, total_tr = 0, total_gr = 0;
+  int2* d_cta_map = nullptr;   // (instance, CTA of runs) of the plan and gradient kernels
+  int total_ctas = 0, max_overlaps = 0;
+  long long total_rec = 0, total_ph = 0, total_tr = 0, total_gr = 0;
   std::vector<long long> theta_off, target_off;
-  size_t off_gm = 0, off_sc = 0, off_tr = 0, off_gr = 0, ws_bytes = 0;
+  size_t off_rec = 0, off_ph = 0, off_tr = 0, off_gr = 0, ws_bytes = 0;
 };
 
 namespace {
 
 inline size_t a256(size_t v) { return (v + 255) / 256 * 256; }
 
-__global__ void k_ragged_prep(const InstDesc* __restrict__ desc, const int2* __restrict__ gate_map, int total_gates,
-                              const double* __restrict__ theta, GateMat* __restrict__ gm, double2* __restrict__ sc) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total_gates) return;
-  int2 m = gate_map[i];
+__global__ void __launch_bounds__(kRotThreads) k_ragged_plan(const InstDesc* __restrict__ desc,
+                                                             const int2* __restrict__ cta_map,
+                                                             const double* __restrict__ theta,
+                                                             RotRec* __restrict__ recs, double2* __restrict__ phases) {
+  const int2 m = cta_map[blockIdx.x];
   const InstDesc d = desc[m.x];
-  const Gate gt = d.gates[m.y];
-  const double* th = theta + d.theta_off + gt.pstart;
-  double2* scb = sc + d.sc_off + gt.pstart;
-  GateMat g;
-  g.u[0] = g.u[1] = g.u[2] = g.u[3] = make_double2(0.0, 0.0);
-  if (gt.type == G_U3) {
-    double st, ct, sp, cp, sl, cl;
-    sincos(th[0], &st, &ct);
-    sincos(th[1], &sp, &cp);
-    sincos(th[2], &sl, &cl);
-    scb[0] = make_double2(st, ct);
-    scb[1] = make_double2(sp, cp);
-    scb[2] = make_double2(sl, cl);
-    double spl = sp * cl + cp * sl, cpl = cp * cl - sp * sl;
-    g.u[0] = make_double2(ct, 0.0);
-    g.u[1] = make_double2(-st * cl, -st * sl);
-    g.u[2] = make_double2(st * cp, st * sp);
-    g.u[3] = make_double2(ct * cpl, ct * spl);
-  } else if (gate_param_num(gt.type) == 1) {
-    double s, c;
-    sincos(th[0], &s, &c);
-    scb[0] = make_double2(s, c);
-    g.u[0] = make_double2(c, s);
-  }
-  gm[d.gm_off + m.y] = g;
+  rot_plan_body(d.plan, m.y, theta + d.theta_off, recs + d.rec_off, phases + d.ph_off + m.y);
 }
 
-template <bool GRAD>
+// MODE 0: cost only; 1: gradient with real overlaps (FROBENIUS_NORM); 2: with complex ones.
+template <int MODE>
 __global__ void __launch_bounds__(kRaggedThreads) k_ragged_tiles(const InstDesc* __restrict__ desc,
                                                                  const int2* __restrict__ items, int n_items,
                                                                  int* __restrict__ counter, const double2* targets,
-                                                                 const GateMat* gm, const double2* sc, double2* ws_tr,
-                                                                 double2* ws_gr) {
+                                                                 const RotRec* recs, const double2* phases,
+                                                                 double2* ws_tr, double* ws_gr) {
   extern __shared__ double2 smem[];
   __shared__ int item_s;
   for (;;) {
@@ -96,10 +75,13 @@ __global__ void __launch_bounds__(kRaggedThreads) k_ragged_tiles(const InstDesc*
     const int2 it = items[item];
     const InstDesc d = desc[it.x];
     TileArgs a;
-    a.gates = d.gates;
-    a.L = d.L; a.P = d.P; a.n = d.n; a.N = d.N;
-    a.gm = gm + d.gm_off;
-    a.sc = sc + d.sc_off;
+    a.ops = d.plan.ops;
+    a.nops = d.plan.nops;
+    a.noverlaps = d.plan.noverlaps;
+    a.n = d.n; a.N = d.N;
+    a.recs = recs + d.rec_off;
+    a.phases = phases + d.ph_off;
+    a.nphase = d.plan.ncta;
     a.mtx = const_cast<double2*>(targets) + d.target_off;
     a.bstride = 0;
     a.rstride = d.cols;
@@ -108,63 +90,43 @@ __global__ void __launch_bounds__(kRaggedThreads) k_ragged_tiles(const InstDesc*
     a.TC = d.TC;
     a.tiles = d.tiles;
     a.trace_offset = 0;
-    a.reverse_order = 0;
-    a.orient = ORIENT_FWD;
     a.ws_tr = ws_tr + d.tr_off;
-    a.ws_gr = GRAD ? ws_gr + d.gr_off : nullptr;
+    a.ws_gr = MODE ? ws_gr + d.gr_off * MODE : nullptr;
     a.ckpt = nullptr;
     a.ckpt_interval = 0;
     a.nck = 0;
-    if (GRAD)
-      tile_adjoint_body(a, 0, it.y, smem);
+    if constexpr (MODE == 0)
+      tile_forward_body<false, true, kRotFwd>(a, 0, it.y, smem);
     else
-      tile_forward_body<false, true>(a, 0, it.y, smem);
+      tile_adjoint_body<MODE == 2>(a, 0, it.y, smem);
     __syncthreads();
   }
 }
 
-__global__ void k_ragged_finish(const InstDesc* __restrict__ desc, const double2* __restrict__ ws_tr,
-                                const double2* __restrict__ ws_gr, int variant, double* __restrict__ cost,
-                                double* __restrict__ grad) {
+// blockIdx.x: instance; W doubles per overlap.
+template <int W>
+__global__ void __launch_bounds__(32 * kSumGroups) k_ragged_sum(const InstDesc* __restrict__ desc, double2* ws_tr,
+                                                                double* ws_gr, int with_grad, int variant,
+                                                                double* __restrict__ cost) {
   const InstDesc d = desc[blockIdx.x];
-  double2 tr = make_double2(0.0, 0.0);
-  for (int t = 0; t < d.tiles; t++) {
-    double2 v = ws_tr[d.tr_off + t];
-    tr.x += v.x;
-    tr.y += v.y;
-  }
-  const double dc = d.cols;
-  if (blockIdx.y == 0 && threadIdx.x == 0) {
-    double f;
-    if (variant == SQG_FROBENIUS_NORM) {
-      f = 1.0 - tr.x / dc;
-    } else if (variant == SQG_HILBERT_SCHMIDT_TEST) {
-      double q = 1.0 / dc;
-      f = 1.0 - q * q * (tr.x * tr.x + tr.y * tr.y);
-    } else {
-      f = 1.0 - ((tr.x * tr.x + tr.y * tr.y) / dc + 1) / (dc + 1);
-    }
-    cost[blockIdx.x] = f;
-  }
-  if (!grad) return;
-  const int p = blockIdx.y * blockDim.x + threadIdx.x;
-  if (p >= d.P) return;
-  double2 dt = make_double2(0.0, 0.0);
-  for (int t = 0; t < d.tiles; t++) {
-    double2 v = ws_gr[d.gr_off + (long long)t * d.P + p];
-    dt.x += v.x;
-    dt.y += v.y;
-  }
-  double gv;
-  if (variant == SQG_FROBENIUS_NORM) {
-    gv = (1.0 - dt.x / dc) - 1.0;
-  } else if (variant == SQG_HILBERT_SCHMIDT_TEST) {
-    double q = 1.0 / dc;
-    gv = -2.0 * q * q * tr.x * dt.x - 2.0 * q * q * tr.y * dt.y;
-  } else {
-    gv = -2.0 / dc / (dc + 1) * tr.x * dt.x - 2.0 / dc / (dc + 1) * tr.y * dt.y;
-  }
-  grad[d.theta_off + p] = gv;
+  const int nov = with_grad ? d.plan.noverlaps : 0;
+  if (blockIdx.y > 0 && (int)blockIdx.y * 32 >= nov) return;
+  tile_sum_body<W>(blockIdx.y, ws_tr + d.tr_off, ws_gr + d.gr_off * W, d.tiles, nov, d.cols, variant,
+                   cost + blockIdx.x);
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(kRotThreads) k_ragged_grad(const InstDesc* __restrict__ desc,
+                                                             const int2* __restrict__ cta_map,
+                                                             const double* __restrict__ theta,
+                                                             const RotRec* __restrict__ recs,
+                                                             const double2* __restrict__ ws_tr,
+                                                             const double* __restrict__ ws_gr, int variant,
+                                                             double* __restrict__ grad) {
+  const int2 m = cta_map[blockIdx.x];
+  const InstDesc d = desc[m.x];
+  rot_grad_body<CPLX>(d.plan, m.y, theta + d.theta_off, recs + d.rec_off, ws_tr + d.tr_off,
+                      ws_gr + d.gr_off * (CPLX ? 2 : 1), d.cols, variant, grad + d.theta_off);
 }
 
 int cerr(cudaError_t e, const char* where) {
@@ -175,7 +137,7 @@ void free_batch(sqg_ragged_batch* r) {
   if (!r) return;
   cudaFree(r->d_desc);
   cudaFree(r->d_items);
-  cudaFree(r->d_gate_map);
+  cudaFree(r->d_cta_map);
   delete r;
 }
 
@@ -194,7 +156,7 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
   r->with_grad = with_grad ? 1 : 0;
   cudaGetDevice(&r->device);
   std::vector<InstDesc> desc(count);
-  std::vector<int2> gate_map;
+  std::vector<int2> cta_map;
   std::vector<std::pair<double, int2>> work;
   long long th = 0, tg = 0;
   size_t smem = 0;
@@ -213,8 +175,8 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
       return set_error(SQG_ERR_UNSUPPORTED, "gradient supports qbit_num <= 12");
     }
     InstDesc& d = desc[i];
-    d.gates = c->d_gates;
-    d.L = c->L; d.P = c->P; d.n = c->n; d.N = c->N; d.cols = cols[i];
+    d.plan = c->plan;
+    d.P = c->P; d.n = c->n; d.N = c->N; d.cols = cols[i];
     const size_t per = (size_t)c->N * sizeof(double2) * (with_grad ? 2 : 1);
     int tc;
     if (tile_cols && tile_cols[i] > 0) {
@@ -233,21 +195,21 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
     d.tiles = (cols[i] + tc - 1) / tc;
     d.theta_off = th;
     d.target_off = tg;
-    d.gm_off = r->total_gm;
-    d.sc_off = r->total_sc;
+    d.rec_off = r->total_rec;
+    d.ph_off = r->total_ph;
     d.tr_off = r->total_tr;
     d.gr_off = r->total_gr;
     r->theta_off.push_back(th);
     r->target_off.push_back(tg);
     th += c->P;
     tg += (long long)c->N * cols[i];
-    r->total_gm += std::max(c->L, 1);
-    r->total_sc += std::max(c->P, 1);
+    r->total_rec += c->plan.nops;
+    r->total_ph += c->plan.ncta;
     r->total_tr += d.tiles;
-    if (with_grad) r->total_gr += (long long)d.tiles * std::max(c->P, 1);
-    r->maxP = std::max(r->maxP, c->P);
+    if (with_grad) r->total_gr += (long long)d.tiles * c->plan.noverlaps;
+    r->max_overlaps = std::max(r->max_overlaps, c->plan.noverlaps);
     smem = std::max(smem, tile_smem_bytes(tc, c->N, with_grad));
-    for (int g = 0; g < c->L; g++) gate_map.push_back(make_int2(i, g));
+    for (int k = 0; k < c->plan.ncta; k++) cta_map.push_back(make_int2(i, k));
     const double w = (double)std::max(c->L, 1) * c->N * tc;
     for (int t = 0; t < d.tiles; t++) work.push_back({w, make_int2(i, t)});
   }
@@ -257,21 +219,21 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
   std::vector<int2> items(work.size());
   for (size_t k = 0; k < work.size(); k++) items[k] = work[k].second;
   r->n_items = (int)items.size();
-  r->total_gates = (int)gate_map.size();
+  r->total_ctas = (int)cta_map.size();
   r->smem = smem;
-  r->off_gm = 256;
-  r->off_sc = a256(r->off_gm + sizeof(GateMat) * r->total_gm);
-  r->off_tr = a256(r->off_sc + sizeof(double2) * r->total_sc);
+  r->off_rec = 256;
+  r->off_ph = a256(r->off_rec + sizeof(RotRec) * r->total_rec);
+  r->off_tr = a256(r->off_ph + sizeof(double2) * r->total_ph);
   r->off_gr = a256(r->off_tr + sizeof(double2) * r->total_tr);
   r->ws_bytes = a256(r->off_gr + sizeof(double2) * std::max<long long>(r->total_gr, 1));
   cudaError_t e = cudaMalloc(&r->d_desc, sizeof(InstDesc) * count);
   if (e == cudaSuccess) e = cudaMalloc(&r->d_items, sizeof(int2) * std::max<size_t>(items.size(), 1));
-  if (e == cudaSuccess) e = cudaMalloc(&r->d_gate_map, sizeof(int2) * std::max<size_t>(gate_map.size(), 1));
+  if (e == cudaSuccess) e = cudaMalloc(&r->d_cta_map, sizeof(int2) * std::max<size_t>(cta_map.size(), 1));
   if (e == cudaSuccess) e = cudaMemcpy(r->d_desc, desc.data(), sizeof(InstDesc) * count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !items.empty())
     e = cudaMemcpy(r->d_items, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !gate_map.empty())
-    e = cudaMemcpy(r->d_gate_map, gate_map.data(), sizeof(int2) * gate_map.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !cta_map.empty())
+    e = cudaMemcpy(r->d_cta_map, cta_map.data(), sizeof(int2) * cta_map.size(), cudaMemcpyHostToDevice);
   // kernel attributes are set here, at planning time and to the device's opt-in maximum
   // (the attribute is per kernel, shared by every batch), so that launches can be captured
   // in CUDA graphs
@@ -281,14 +243,12 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
     free_batch(r);
     return set_error(SQG_ERR_UNSUPPORTED, "work item does not fit in shared memory");
   }
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_ragged_tiles<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 64);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_ragged_tiles<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 64);
+  for (auto k : {k_ragged_tiles<0>, k_ragged_tiles<1>, k_ragged_tiles<2>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 64);
   int per_sm = 0, sms = 0;
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, with_grad ? k_ragged_tiles<true> : k_ragged_tiles<false>, kRaggedThreads, smem);
+        &per_sm, with_grad ? k_ragged_tiles<1> : k_ragged_tiles<0>, kRaggedThreads, smem);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
   if (e != cudaSuccess) {
     int st = cerr(e, "sqg_ragged_create");
@@ -331,27 +291,33 @@ int sqg_ragged_cost_grad(const sqg_ragged_batch* r, const double* theta, const v
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = (char*)workspace;
   int* counter = (int*)ws;
-  GateMat* gm = (GateMat*)(ws + r->off_gm);
-  double2* sc = (double2*)(ws + r->off_sc);
+  RotRec* recs = (RotRec*)(ws + r->off_rec);
+  double2* ph = (double2*)(ws + r->off_ph);
   double2* tr = (double2*)(ws + r->off_tr);
-  double2* gr = (double2*)(ws + r->off_gr);
+  double* gr = (double*)(ws + r->off_gr);
+  const double2* tg = (const double2*)targets;
   int st;
   if ((st = cerr(cudaMemsetAsync(counter, 0, sizeof(int), s), "cudaMemsetAsync"))) return st;
-  if (r->total_gates > 0) {
-    k_ragged_prep<<<(r->total_gates + 127) / 128, 128, 0, s>>>(r->d_desc, r->d_gate_map, r->total_gates, theta, gm, sc);
-    if ((st = cerr(cudaGetLastError(), "k_ragged_prep"))) return st;
+  if (r->total_ctas > 0) {
+    k_ragged_plan<<<r->total_ctas, kRotThreads, 0, s>>>(r->d_desc, r->d_cta_map, theta, recs, ph);
+    if ((st = cerr(cudaGetLastError(), "k_ragged_plan"))) return st;
   }
-  const bool g = grad != nullptr;
-  if (g)
-    k_ragged_tiles<true><<<r->grid, kRaggedThreads, r->smem, s>>>(r->d_desc, r->d_items, r->n_items, counter,
-                                                                  (const double2*)targets, gm, sc, tr, gr);
-  else
-    k_ragged_tiles<false><<<r->grid, kRaggedThreads, r->smem, s>>>(r->d_desc, r->d_items, r->n_items, counter,
-                                                                   (const double2*)targets, gm, sc, tr, gr);
+  const int mode = !grad ? 0 : variant == SQG_FROBENIUS_NORM ? 1 : 2;
+  auto tiles = mode == 0 ? k_ragged_tiles<0> : mode == 1 ? k_ragged_tiles<1> : k_ragged_tiles<2>;
+  tiles<<<r->grid, kRaggedThreads, r->smem, s>>>(r->d_desc, r->d_items, r->n_items, counter, tg, recs, ph, tr, gr);
   if ((st = cerr(cudaGetLastError(), "k_ragged_tiles"))) return st;
-  dim3 fgrid(r->count, g ? (r->maxP + 127) / 128 : 1);
-  k_ragged_finish<<<fgrid, 128, 0, s>>>(r->d_desc, tr, gr, variant, cost, g ? grad : nullptr);
-  return cerr(cudaGetLastError(), "k_ragged_finish");
+  const dim3 sgrid(r->count, grad ? std::max(1, (r->max_overlaps + 31) / 32) : 1);
+  if (mode < 2)
+    k_ragged_sum<1><<<sgrid, 32 * kSumGroups, 0, s>>>(r->d_desc, tr, gr, grad != nullptr, variant, cost);
+  else
+    k_ragged_sum<2><<<sgrid, 32 * kSumGroups, 0, s>>>(r->d_desc, tr, gr, 1, variant, cost);
+  if (grad && r->total_ctas > 0) {
+    if (mode == 1)
+      k_ragged_grad<false><<<r->total_ctas, kRotThreads, 0, s>>>(r->d_desc, r->d_cta_map, theta, recs, tr, gr, variant, grad);
+    else
+      k_ragged_grad<true><<<r->total_ctas, kRotThreads, 0, s>>>(r->d_desc, r->d_cta_map, theta, recs, tr, gr, variant, grad);
+  }
+  return cerr(cudaGetLastError(), "ragged sums and gradients");
 }
 
 }  // extern "C"

@@ -3,15 +3,17 @@
 // work item with all threads of the CTA; smem holds the tile(s) plus reduction scratch.
 #pragma once
 #include "gates.cuh"
+#include "rot.cuh"
 #include "tile.cuh"
 
 namespace sqg {
 
 struct TileArgs {
-  const Gate* gates;
-  int L, P, n, N;
-  const GateMat* gm;   // [B][L]
-  const double2* sc;   // [B][P]
+  const RotOp* ops;     // operations of the circuit's plan
+  int nops, noverlaps, n, N;
+  const RotRec* recs;   // [B][nops]
+  const double2* phases;  // [B][nphase]: factors of the phase common to all amplitudes
+  int nphase;
   // matrix source (target or in/out matrix); element (r, c) of instance b at
   // base + b*bstride + r*rstride + c*cstride
   double2* mtx;
@@ -20,14 +22,18 @@ struct TileArgs {
   int TC;            // vectors per tile
   int tiles;         // tiles per instance
   int trace_offset;  // row offset of the traced element (left application)
-  int reverse_order; // right application walks the gates from last to first
-  int orient;        // ORIENT_FWD or ORIENT_TRANS
   double2* ws_tr;    // [B][tiles] forward trace partials
-  double2* ws_gr;    // [B][tiles][P] derivative trace partials
+  double* ws_gr;     // [B][tiles][noverlaps] overlaps (complex: noverlaps double2)
   double2* ckpt;     // checkpoints [B][tiles][nck][TC][N] or null
-  int ckpt_interval;
+  int ckpt_interval;  // in operations
   int nck;
 };
+
+__device__ __forceinline__ double2 tile_phase(const TileArgs& a, int b) {
+  double2 p = make_double2(1.0, 0.0);
+  for (int k = 0; k < a.nphase; k++) p = cmul(p, a.phases[(long long)b * a.nphase + k]);
+  return p;
+}
 
 __device__ __forceinline__ void load_tile(double2* s, const TileArgs& a, int b, int v0, int tc) {
   const double2* base = a.mtx + (long long)b * a.bstride;
@@ -47,135 +53,303 @@ __device__ __forceinline__ void load_tile(double2* s, const TileArgs& a, int b, 
   }
 }
 
-__device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, int b, int v0, int tc) {
+// Writes the tile back times the instance's common phase.
+__device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, int b, int v0, int tc, double2 phase) {
   double2* base = a.mtx + (long long)b * a.bstride;
   const int total = a.N * tc;
   if (a.cstride == 1) {
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
       int r = e / tc, c = e - r * tc;
-      base[(long long)r * a.rstride + v0 + c] = s[c * a.N + r];
+      base[(long long)r * a.rstride + v0 + c] = cmul(phase, s[c * a.N + r]);
     }
   } else {
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
       int c = e / a.N, r = e - c * a.N;
-      base[(long long)(v0 + c) * a.rstride + r] = s[c * a.N + r];
+      base[(long long)(v0 + c) * a.rstride + r] = cmul(phase, s[c * a.N + r]);
     }
   }
 }
 
-// Gate records and 2x2 matrices are staged in shared memory kGateChunk at a time, so each
-// CTA reads them from global memory once instead of once per warp and gate.
-constexpr int kGateChunk = kStage;
-constexpr size_t kGateStageBytes = kGateChunk * (sizeof(Gate) + sizeof(GateMat));
+// Operations are staged in shared memory kRotChunk at a time, so each CTA reads them from
+// global memory once instead of once per warp and operation.
+constexpr size_t kStageBytes = kRotChunk * sizeof(StagedOp);
 
-// Forward (or right) application of the whole circuit to one tile; optionally writes
-// the tile back and/or the traced diagonal partial.
-template <bool WRITE_BACK, bool TRACE>
+// Application of the whole circuit to one tile (DIR kRotFwd: from the left; kRotTrans: to the
+// rows, from the right); optionally writes the tile back and/or the traced diagonal partial.
+template <bool WRITE_BACK, bool TRACE, int DIR>
 __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int tile, double2* smem) {
   double2* s = smem;
   double2* red = smem + (size_t)a.TC * a.N;
-  GateMat* gst = reinterpret_cast<GateMat*>(red + kTileMaxWarps);  // [kGateChunk]
-  Gate* gts = reinterpret_cast<Gate*>(gst + kGateChunk);            // [kGateChunk]
+  StagedOp* st = reinterpret_cast<StagedOp*>(red + kTileMaxWarps);  // [kRotChunk]
   const int v0 = tile * a.TC;
   const int tc = min(a.TC, a.cols - v0);
-  const int logN = a.n;
   load_tile(s, a, b, v0, tc);
-  const GateMat* gm = a.gm + (long long)b * a.L;
-  for (int k0 = 0; k0 < a.L; k0 += kGateChunk) {
-    const int kn = min(kGateChunk, a.L - k0);
-    __syncthreads();  // the previous chunk's records are no longer read
-    if (threadIdx.x < kn) {
-      const int k = k0 + threadIdx.x;
-      const int g = a.reverse_order ? a.L - 1 - k : k;
-      gts[threadIdx.x] = a.gates[g];
-      gst[threadIdx.x] = gm[g];
-    }
+  const RotRec* recs = a.recs + (long long)b * a.nops;
+  const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
+  for (int q = 0; q < nchunks; q++) {
+    const int k0 = (DIR == kRotFwd ? q : nchunks - 1 - q) * kRotChunk;
+    const int kn = min(kRotChunk, a.nops - k0);
+    __syncthreads();  // the previous chunk's operations are no longer read
+    stage_ops(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
-      const Gate gt = gts[j];
-      PairOp op = make_op(gt.type, gst[j], a.orient);
-      tile_apply(s, a.N, logN, tc, gt, op);
+      rot_tile<DIR>(s, a.N, a.n, tc, st[DIR == kRotFwd ? j : kn - 1 - j]);
       __syncthreads();
     }
   }
   __syncthreads();
+  const double2 phase = tile_phase(a, b);
   if (TRACE) {
     double2 t = tile_trace(s, a.N, tc, v0, a.trace_offset, reinterpret_cast<double*>(red));
-    if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = t;
+    if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
   }
-  if (WRITE_BACK) store_tile(s, a, b, v0, tc);
+  if (WRITE_BACK) store_tile(s, a, b, v0, tc, phase);
 }
 
-// Cost + adjoint gradient of one (instance, tile).
+// Adds the overlaps `mask` of one pair of psi (x, y) and lambda (lx, ly) to acc.  CPLX = false
+// (FROBENIUS_NORM needs only the real part of a derivative): acc = Im <X>, Im <Y>, Im of the
+// upper rows' <lambda|psi>; 4 + 4 + 2 instructions.  CPLX: acc = the complex overlaps
+// <lambda_0|psi_0>, <lambda_0|psi_1>, <lambda_1|psi_0>.
+template <bool CPLX, int mask>
+__device__ __forceinline__ void measure_pair(double2 x, double2 y, double2 lx, double2 ly,
+                                             double (&acc)[CPLX ? 6 : 3]) {
+  if (!CPLX) {
+    if (mask & 1) {  // Im(conj(lx) y + conj(ly) x)
+      acc[0] = fma(lx.x, y.y, fma(-lx.y, y.x, acc[0]));
+      acc[0] = fma(ly.x, x.y, fma(-ly.y, x.x, acc[0]));
+    }
+    if (mask & 2) {  // Im(i (conj(ly) x - conj(lx) y)) = Re(conj(ly) x - conj(lx) y)
+      acc[1] = fma(ly.x, x.x, fma(ly.y, x.y, acc[1]));
+      acc[1] = fma(-lx.x, y.x, fma(-lx.y, y.y, acc[1]));
+    }
+    if (mask & 4) acc[2] = fma(lx.x, x.y, fma(-lx.y, x.x, acc[2]));
+  } else {
+    if (mask & 4) {
+      acc[0] = fma(lx.x, x.x, fma(lx.y, x.y, acc[0]));
+      acc[1] = fma(lx.x, x.y, fma(-lx.y, x.x, acc[1]));
+    }
+    if (mask & 3) {
+      acc[2] = fma(lx.x, y.x, fma(lx.y, y.y, acc[2]));
+      acc[3] = fma(lx.x, y.y, fma(-lx.y, y.x, acc[3]));
+      acc[4] = fma(ly.x, x.x, fma(ly.y, x.y, acc[4]));
+      acc[5] = fma(ly.x, x.y, fma(-ly.y, x.x, acc[5]));
+    }
+  }
+}
+
+// One measured operation of the reverse sweep on a tile: the overlaps behind it, then its
+// adjoint on psi and lambda.
+template <bool CPLX, int KIND, int MASK, bool RS>
+__device__ __forceinline__ void adjoint_tile_kind(double2* psi, double2* lam, int N, int logN, int tc,
+                                                  const StagedOp& staged, double (&acc)[CPLX ? 6 : 3]) {
+  const DirOp op = directed<kRotAdj, KIND>(staged);
+  const int target = staged.qubits & 255, control = (staged.qubits >> 8) & 255;
+  constexpr bool ctrl = KIND == kOpCry;
+  const int lognp = ctrl ? logN - 2 : logN - 1;
+  const int npairs = 1 << lognp;
+  const int items = tc << lognp;
+  const int step = 1 << target;
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    const int col = it >> lognp;
+    const int p = it & (npairs - 1);
+    const int i = ctrl ? pair_index2(p, target, control) : pair_index1(p, target);
+    double2* ps = psi + col * N;
+    double2* ls = lam + col * N;
+    double2 x = ps[i], y = ps[i + step], lx = ls[i], ly = ls[i + step];
+    measure_pair<CPLX, MASK>(x, y, lx, ly, acc);
+    if (KIND == kOpPhase) {
+      rot_phase(y, op.zix, op.ziy, op.nzi);
+      rot_phase(ly, op.zix, op.ziy, op.nzi);
+    } else {
+      if (KIND == kOpCry) {
+        cry_pair(op, x, y);
+        cry_pair(op, lx, ly);
+      } else {
+        rot_pair<kRotAdj, KIND, RS>(op, x, y);
+        rot_pair<kRotAdj, KIND, RS>(op, lx, ly);
+      }
+      ps[i] = x;
+      ls[i] = lx;
+    }
+    ps[i + step] = y;
+    ls[i + step] = ly;
+  }
+}
+
+// The forms that build_rot_plan makes: each kind with the overlaps it is measured with.
+template <bool CPLX>
+__device__ __forceinline__ void adjoint_tile(double2* psi, double2* lam, int N, int logN, int tc, const StagedOp& st,
+                                             double (&acc)[CPLX ? 6 : 3]) {
+#define SQG_ROT_CASE(KIND, MASK) \
+  case (KIND) | (MASK) << 8: \
+    if (st.qubits & kStRescale) \
+      adjoint_tile_kind<CPLX, (KIND), (MASK), true>(psi, lam, N, logN, tc, st, acc); \
+    else \
+      adjoint_tile_kind<CPLX, (KIND), (MASK), false>(psi, lam, N, logN, tc, st, acc); \
+    break;
+  switch (st.kind | st.mask << 8) {
+    case kOpCry | 2 << 8: adjoint_tile_kind<CPLX, kOpCry, 2, false>(psi, lam, N, logN, tc, st, acc); break;
+    case kOpPhase | 4 << 8: adjoint_tile_kind<CPLX, kOpPhase, 4, false>(psi, lam, N, logN, tc, st, acc); break;
+    SQG_ROT_CASE(kOpRot, 2)
+    SQG_ROT_CASE(kOpRot | kOpX, 1)
+    SQG_ROT_CASE(kOpRot | kOpZi, 3)
+    SQG_ROT_CASE(kOpRot | kOpZi, 6)
+    SQG_ROT_CASE(kOpRot | kOpX | kOpZi, 5)
+    SQG_ROT_CASE(kOpRot | kOpZi | kOpZo, 7)
+  }
+#undef SQG_ROT_CASE
+}
+
+// Warp totals of the overlaps: lane l ends with value (l >> 3) & 3 (real) or (l >> 2) & 7.
+__device__ __forceinline__ double warp_reduce_scatter4(double r0, double r1, double r2) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 16;
+  double a = (hi ? r2 : r0) + __shfl_xor_sync(0xffffffffu, hi ? r0 : r2, 16);
+  double b = hi ? 0.0 : r1;
+  const double br = __shfl_xor_sync(0xffffffffu, r1, 16);  // the upper half's r1 goes to the lower half
+  if (!hi) b += br;
+  const bool odd = lane & 8;
+  const double send = odd ? a : b;
+  double v = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, send, 8);
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v;
+}
+
+// Cost trace and overlaps of one (instance, tile): forward sweep, then the adjoint sweep
+// psi <- G^dagger psi, lambda <- G^dagger lambda with lambda starting at e_{j + offset}.
+// Bound by FP64 instructions: a U3 run of a CNOT circuit costs 8 per pair forward and
+// 16 + 6 or 8 on the way back (a U3 by itself: 14, 28 and 16 with the gates as given).
+template <bool CPLX>
 __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int tile, double2* smem) {
+  constexpr int NV = CPLX ? 8 : 4;  // reduced values per operation (the last ones unused)
   const int N = a.N, logN = a.n;
   double2* psi = smem;
   double2* lam = smem + (size_t)a.TC * N;
-  double* redd = reinterpret_cast<double*>(lam + (size_t)a.TC * N);  // [kTileMaxWarps][8]
-  double* tot = redd + kTileMaxWarps * 8;                             // [8]
-  double* scratch = tot + 8;                                          // [kTileMaxWarps]
-  GateMat* gst = reinterpret_cast<GateMat*>(scratch + kTileMaxWarps);  // [kGateChunk]
-  Gate* gts = reinterpret_cast<Gate*>(gst + kGateChunk);              // [kGateChunk]
+  double* redd = reinterpret_cast<double*>(lam + (size_t)a.TC * N);  // [2][kTileMaxWarps][4 or 8]
+  StagedOp* st = reinterpret_cast<StagedOp*>(redd + kTileMaxWarps * 16);  // [kRotChunk]
   const int v0 = tile * a.TC;
   const int tc = min(a.TC, a.cols - v0);
   const size_t tile_elems = (size_t)a.TC * N;
   double2* ck = a.ckpt ? a.ckpt + ((long long)b * a.tiles + tile) * a.nck * tile_elems : nullptr;
+  const RotRec* recs = a.recs + (long long)b * a.nops;
+  const double2 phase = tile_phase(a, b);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 
   load_tile(psi, a, b, v0, tc);
-  // lambda_j = e_{j + offset}
+  // <lambda| carries the common phase: lambda_j = conj(phase) e_{j + offset}
   for (int e = threadIdx.x; e < tc * N; e += blockDim.x) {
     int c = e / N, r = e - c * N;
-    lam[e] = make_double2(r == v0 + c + a.trace_offset ? 1.0 : 0.0, 0.0);
+    lam[e] = r == v0 + c + a.trace_offset ? cconj(phase) : make_double2(0.0, 0.0);
+  }
+  // forward sweep, storing psi after every ckpt_interval-th operation
+  const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
+  for (int q = 0; q < nchunks; q++) {
+    const int k0 = q * kRotChunk, kn = min(kRotChunk, a.nops - k0);
+    __syncthreads();
+    stage_ops(st, a.ops, recs, k0, kn);
+    __syncthreads();
+    for (int j = 0; j < kn; j++) {
+      rot_tile<kRotFwd>(psi, N, logN, tc, st[j]);
+      __syncthreads();
+      if (ck && (k0 + j + 1) % a.ckpt_interval == 0 && (k0 + j + 1) / a.ckpt_interval <= a.nck) {
+        double2* dst = ck + (size_t)((k0 + j + 1) / a.ckpt_interval - 1) * tile_elems;
+        for (int e = threadIdx.x; e < tc * N; e += blockDim.x) dst[e] = psi[e];
+        __syncthreads();  // the next operation changes psi
+      }
+    }
   }
   __syncthreads();
-  const GateMat* gm = a.gm + (long long)b * a.L;
-  const double2* scb = a.sc + (long long)b * a.P;
-  // forward sweep, storing psi after every ckpt_interval-th gate
-  for (int g = 0; g < a.L; g++) {
-    const int j = g % kGateChunk;
-    if (j == 0) {
-      __syncthreads();
-      if ((int)threadIdx.x < min(kGateChunk, a.L - g)) {
-        gts[threadIdx.x] = a.gates[g + threadIdx.x];
-        gst[threadIdx.x] = gm[g + threadIdx.x];
+  double2 t = tile_trace(psi, N, tc, v0, a.trace_offset, redd);
+  if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
+
+  // reverse sweep.  The warps' totals of an operation are summed and written by the last warp
+  // while the next operation runs: redd alternates between two halves, one barrier per operation.
+  double* wgr = a.ws_gr + ((long long)b * a.tiles + tile) * a.noverlaps * (CPLX ? 2 : 1);
+  int pend_coff = 0, pend_mask = 0, pend_aw = 0, buf = 0;
+  double pend_fac = 0.0;
+  auto flush = [&]() {  // one thread per measured overlap
+    if (!pend_mask || warp != nw - 1 || lane >= 3) return;
+    const int axis = lane;  // 0 X, 1 Y, 2 Z
+    if (!((pend_mask >> axis) & 1)) return;
+    const double* rd = redd + (buf ^ 1) * kTileMaxWarps * 8;
+    const int pos = pend_coff + __popc(pend_mask & ((1 << axis) - 1));
+    if (!CPLX) {
+      double v = 0.0;
+      for (int w = 0; w < pend_aw; w++) v += rd[w * NV + axis];
+      wgr[pos] = v * pend_fac;
+    } else {
+      double o[6];
+      for (int k = 0; k < 6; k++) {
+        o[k] = 0.0;
+        for (int w = 0; w < pend_aw; w++) o[k] += rd[w * NV + k];
+        o[k] *= pend_fac;
       }
-      __syncthreads();
+      double2 v;
+      if (axis == 2) v = make_double2(o[0], o[1]);                       // <lambda_0|psi_0>
+      else if (axis == 0) v = make_double2(o[2] + o[4], o[3] + o[5]);     // <X>
+      else v = make_double2(-(o[5] - o[3]), o[4] - o[2]);                 // <Y> = i (m10 - m01)
+      reinterpret_cast<double2*>(wgr)[pos] = v;
     }
-    Gate gt = gts[j];
-    PairOp op = make_op(gt.type, gst[j], ORIENT_FWD);
-    tile_apply(psi, N, logN, tc, gt, op);
+  };
+  for (int q = nchunks - 1; q >= 0; q--) {
+    const int k0 = q * kRotChunk, kn = min(kRotChunk, a.nops - k0);
     __syncthreads();
-    if (ck && (g + 1) % a.ckpt_interval == 0 && (g + 1) / a.ckpt_interval <= a.nck) {
-      double2* dst = ck + (size_t)((g + 1) / a.ckpt_interval - 1) * tile_elems;
-      for (int e = threadIdx.x; e < tc * N; e += blockDim.x) dst[e] = psi[e];
+    stage_ops(st, a.ops, recs, k0, kn);
+    __syncthreads();
+    for (int j = kn - 1; j >= 0; j--) {
+      const int k = k0 + j;
+      // before step k, psi holds the state behind operation k; the stored copy replaces it at
+      // checkpoints, so that the error of undoing never spans more than ckpt_interval
+      // operations (the copy was made on the way forward: scaled by 1 / mfac against psi here)
+      if (ck && (k + 1) % a.ckpt_interval == 0 && (k + 1) / a.ckpt_interval <= a.nck && k + 1 < a.nops) {
+        const double2* src = ck + (size_t)((k + 1) / a.ckpt_interval - 1) * tile_elems;
+        const double f = 1.0 / st[j].mfac;
+        for (int e = threadIdx.x; e < tc * N; e += blockDim.x) psi[e] = cscale(src[e], f);
+        __syncthreads();
+      }
+      const int mask = st[j].mask;
+      if (mask == 0) {  // CNOT, CZ
+        rot_tile<kRotAdj>(psi, N, logN, tc, st[j]);
+        rot_tile<kRotAdj>(lam, N, logN, tc, st[j]);
+        __syncthreads();
+        continue;
+      }
+      double acc[CPLX ? 6 : 3];
+#pragma unroll
+      for (int r = 0; r < (CPLX ? 6 : 3); r++) acc[r] = 0.0;
+      adjoint_tile<CPLX>(psi, lam, N, logN, tc, st[j], acc);
+      const int items = tc << (st[j].kind == kOpCry ? logN - 2 : logN - 1);
+      const int aw = min(nw, (items + 31) >> 5);  // warps holding pairs
+      if (warp < aw) {
+        double* rd = redd + buf * kTileMaxWarps * 8;
+        if constexpr (CPLX) {
+          double r[8] = {acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], 0.0, 0.0};
+          const double v = warp_reduce_scatter8(r);
+          if ((lane & 3) == 0) rd[warp * NV + (lane >> 2)] = v;
+        } else {
+          const double v = warp_reduce_scatter4(acc[0], acc[1], acc[2]);
+          if ((lane & 7) == 0) rd[warp * NV + ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)] = v;
+        }
+      }
+      flush();  // the operation before this one
+      __syncthreads();
+      pend_coff = st[j].coff;
+      pend_mask = mask;
+      pend_aw = aw;
+      pend_fac = st[j].mfac;
+      buf ^= 1;
     }
   }
-  double2 t = tile_trace(psi, N, tc, v0, a.trace_offset, scratch);
-  if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = t;
-  double2* wgr = a.ws_gr + ((long long)b * a.tiles + tile) * a.P;
-  auto sink = [&](int, const Gate& gt, const double* R) {
-    if (threadIdx.x < gate_param_num(gt.type)) wgr[gt.pstart + threadIdx.x] = contract_derivative(gt, scb, threadIdx.x, R);
-  };
-  // before reverse step g, psi must hold the state after gate g; restore the stored copy
-  // at checkpoint boundaries so that uncomputation error never spans more than
-  // ckpt_interval gates
-  auto restore = [&](int g) {
-    if (ck && (g + 1) % a.ckpt_interval == 0 && (g + 1) / a.ckpt_interval <= a.nck && g + 1 < a.L) {
-      const double2* src = ck + (size_t)((g + 1) / a.ckpt_interval - 1) * tile_elems;
-      __syncthreads();
-      for (int e = threadIdx.x; e < tc * N; e += blockDim.x) psi[e] = src[e];
-      __syncthreads();
-    }
-  };
-  adjoint_sweep(psi, lam, N, logN, tc, a.gates, gm, scb, a.L, redd, tot, sink, restore, gts, gst);
+  flush();
 }
-
 
 // Shared memory bytes of one work item: tiles plus reduction scratch.
 __host__ __device__ inline size_t tile_smem_bytes(int TC, int N, bool grad) {
   size_t per = (size_t)N * sizeof(double2) * (grad ? 2 : 1);
-  size_t extra = grad ? (kTileMaxWarps * 8 + 8 + kTileMaxWarps) * sizeof(double) + kGateStageBytes
-                      : kTileMaxWarps * sizeof(double2) + kGateStageBytes;
+  size_t extra = grad ? kTileMaxWarps * 16 * sizeof(double) + kStageBytes
+                      : kTileMaxWarps * sizeof(double2) + kStageBytes;
   return per * TC + extra;
 }
 

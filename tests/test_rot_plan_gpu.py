@@ -1,0 +1,113 @@
+"""The rotation plan against the oracle: chains of rotations pushed through every kind of
+two-qubit gate, chains and operation counts at and around the plan's limits, angles at which its
+factorisations degenerate, and every direction and cost variant.
+
+Tolerance 1e-12 relative to max(1, |reference|), as for the engine's other parity tests: at most
+400 operations with a few roundings of 1.1e-16 each.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def close(a, b):
+    a, b = np.asarray(a), np.asarray(b)
+    assert np.max(np.abs(a - b)) <= 1e-12 * max(1.0, np.max(np.abs(b)))
+
+
+def circuit(sqg, n, kind, length):
+    """push_*: U3 runs on qubit 0 separated by gates that commute with one axis there."""
+    rng = np.random.default_rng(length)
+    c = sqg.Circuit(n)
+    for k in range(length):
+        if kind == "random":
+            t = ("U3", "RX", "RY", "RZ", "CNOT", "CZ", "CRY")[rng.integers(7)]
+            a, b = rng.choice(n, 2, replace=False)
+            getattr(c, "add_" + t)(int(a), int(b)) if t[0] == "C" else getattr(c, "add_" + t)(int(a))
+            continue
+        c.add_U3(0)
+        if k % 5 == 2:  # a run of several gates
+            c.add_RX(0)
+            c.add_RY(0)
+            c.add_RX(0)
+        if k % 3 == 1:
+            c.add_U3(1)
+        if kind == "push_z":
+            c.add_CNOT(1, 0) if k % 2 else c.add_CZ(0, 1)
+        elif kind == "push_x":
+            c.add_CNOT(0, 1)
+            if k % 4 == 0:
+                c.add_CNOT(0, n - 1)
+        elif kind == "push_y":
+            c.add_CRY(0, 1)
+        else:  # the axis changes from run to run
+            (c.add_CNOT, c.add_CRY, c.add_CZ)[k % 3](k % 2, 1 - k % 2)
+    return c
+
+
+def angles(P, which):
+    rng = np.random.default_rng(P)
+    if which == "any":
+        return rng.uniform(0, 2 * np.pi, P)
+    if which == "zero":
+        return np.zeros(P)
+    if which == "tiny":
+        return 1e-9 * rng.standard_normal(P)
+    return rng.integers(0, 8, P) * (np.pi / 4)  # exchanges, ties of the pivots, the gimbal case
+
+
+CASES = [(n, kind, length, which) for n, length in ((3, 15), (3, 16), (3, 17), (6, 33), (7, 70))
+         for kind in ("push_z", "push_x", "push_y", "mixed") for which in ("any", "eighths")]
+CASES += [(4, "random", 31, "any"), (4, "random", 32, "any"), (6, "random", 33, "zero"), (6, "random", 200, "tiny"),
+          (8, "random", 300, "eighths"), (2, "push_x", 140, "any"), (5, "mixed", 1, "any")]
+
+
+@pytest.mark.parametrize("n,kind,length,which", CASES)
+def test_plan_against_oracle(sqg, n, kind, length, which):
+    c = circuit(sqg, n, kind, length)
+    recs, P = c.gate_records(), c.get_Parameter_Num()
+    p = angles(P, which)
+    rng = np.random.default_rng(n)
+    N, cols = 1 << n, (1 << n) // 2 + 1  # too narrow for the environment-matrix evaluation
+    T = np.linalg.qr(rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N)))[0][:, :cols].copy()
+    M = O.get_matrix(n, recs, p)
+    A = T.copy()
+    c.apply_to(p, A)
+    close(A, M @ T)
+    R = np.ascontiguousarray(T.T)
+    c.apply_from_right(p, R)
+    close(R, T.T @ M)
+    psi = np.ascontiguousarray(T[:, 0])
+    c.apply_to(p, psi)
+    close(psi, M @ T[:, 0])
+    th = torch.from_numpy(p).cuda()
+    for variant, offset, step in ((0, 0, 0), (0, N - cols, 7), (3, 0, 0), (9, 0, 32)):
+        ev = sqg.CostEvaluator(c, T, trace_offset=offset, cost_variant=variant)
+        cost, grad = ev.cost_grad(th, checkpoint_interval=step)
+        rc, rg = O.cost_grad(n, recs, p, T, trace_offset=offset, variant=variant)
+        close(cost.item(), rc)
+        close(grad[0].cpu().numpy(), rg)
+        close(ev.cost_grad(th, with_grad=False)[0].item(), rc)
+
+
+def test_ragged_plans_share_a_launch(sqg):
+    from importlib import import_module
+    ragged = import_module("sequential-quantum-gate-decomposer_gb300.ragged")
+    cs = [circuit(sqg, n, kind, length) for n, kind, length in
+          ((3, "push_x", 40), (7, "random", 150), (5, "push_y", 3), (2, "push_z", 17), (6, "mixed", 50))]
+    rng = np.random.default_rng(3)
+    ts = [np.linalg.qr(rng.standard_normal((1 << c.qbit_num,) * 2) + 1j * rng.standard_normal((1 << c.qbit_num,) * 2))[0]
+          for c in cs]
+    th = [angles(c.get_Parameter_Num(), "any") for c in cs]
+    rb = ragged.RaggedBatch(cs, ts)
+    for variant in (0, 3, 9):
+        cost, grad = rb.cost_grad(rb.pack(th), variant=variant)
+        for i, (c, g) in enumerate(zip(cost.cpu().numpy(), rb.split(grad))):
+            rc, rg = O.cost_grad(cs[i].qbit_num, cs[i].gate_records(), th[i], ts[i], variant=variant)
+            close(c, rc)
+            close(g.cpu().numpy(), rg)
