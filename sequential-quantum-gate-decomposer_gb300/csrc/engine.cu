@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_plan(RotPlan pl, const doub
                                                           long long theta_stride, RotRec* __restrict__ recs,
                                                           double2* __restrict__ phases) {
   const long long b = blockIdx.y;
-  rot_plan_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nops, phases + b * pl.ncta + blockIdx.x);
+  rot_plan_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nrecs, phases + b * pl.ncta + blockIdx.x);
 }
 
 template <bool WRITE_BACK, bool TRACE, int DIR>
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_grad(RotPlan pl, const doub
                                                           const double* __restrict__ ws_gr, int tiles, int P, int cols,
                                                           int variant, double* __restrict__ grad) {
   const long long b = blockIdx.y;
-  rot_grad_body<CPLX>(pl, blockIdx.x, theta + b * P, recs + b * pl.nops, ws_tr + b * tiles,
+  rot_grad_body<CPLX>(pl, blockIdx.x, theta + b * P, recs + b * pl.nrecs, ws_tr + b * tiles,
                       ws_gr + b * tiles * pl.noverlaps * (CPLX ? 2 : 1), cols, variant, grad + b * P);
 }
 
@@ -346,7 +346,7 @@ struct RotLayout {
 RotLayout rot_layout(const sqg_circuit* c, int B, size_t start) {
   RotLayout l;
   l.rec_off = align_up(start, 256);
-  l.ph_off = align_up(l.rec_off + (size_t)B * c->plan.nops * sizeof(RotRec), 256);
+  l.ph_off = align_up(l.rec_off + (size_t)B * c->plan.nrecs * sizeof(RotRec), 256);
   l.end = align_up(l.ph_off + (size_t)B * c->plan.ncta * sizeof(double2), 256);
   return l;
 }
@@ -357,7 +357,9 @@ int launch_plan(const sqg_circuit* c, const double* theta, long long theta_strid
   RotRec* recs = (RotRec*)(ws + l.rec_off);
   double2* ph = (double2*)(ws + l.ph_off);
   a.ops = c->plan.ops;
+  a.ends = c->plan.ends;
   a.nops = c->plan.nops;
+  a.nrecs = c->plan.nrecs;
   a.noverlaps = c->plan.noverlaps;
   a.n = c->n;
   a.N = c->N;
@@ -430,8 +432,9 @@ constexpr int kStateThreads = 256;
 int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
   const int n = c->n, K = std::min(n, kStateK), low = std::min(K, kStateLow);
   c->sK = K;
-  std::vector<RotOp> lops(c->h_ops);
-  size_t done = 0;  // operations placed in blocks (they follow the order of their anchor gates)
+  std::vector<RotOp> lops;
+  std::vector<int> lends;
+  size_t done = 0;  // steps placed in blocks (they follow the order of their anchor gates)
   std::vector<int> hitab, inact;
   std::vector<int> inA(n, 0);
   auto close_block = [&](int g0, int g1) {
@@ -446,11 +449,10 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
     std::sort(A.begin(), A.end());
     std::vector<int> loc(n, -1);
     for (int j = 0; j < (int)A.size(); j++) loc[A[j]] = j;
-    const int k0 = (int)done;
-    for (; done < lops.size() && c->h_anchor[done] < g1; done++) {
-      const int t = lops[done].qubits & 255, ctl = lops[done].qubits >> 8;
-      lops[done].qubits = loc[t] | (lops[done].kind <= kOpCry ? loc[ctl] << 8 : 0);
-    }
+    const int s0 = (int)done, k0 = (int)lops.size();
+    while (done < c->h_steps.size() && c->h_steps[done].anchor < g1) done++;
+    lower_rot_steps(c->h_steps, s0, (int)done, K, loc, lops, lends);
+    lends.resize(16 * (c->sblocks.size() + 1), 0);
     (void)g0;
     const int hb = K - low;
     for (int h = 0; h < 128; h++) {
@@ -467,7 +469,7 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
         k++;
       }
     for (; k < 32; k++) inact.push_back(0);
-    c->sblocks.push_back({k0, (int)done});
+    c->sblocks.push_back({k0, (int)lops.size()});
     std::fill(inA.begin(), inA.end(), 0);
   };
   int g0 = 0, used = 0;
@@ -526,8 +528,11 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
   }
   if (c->L > 0) close_block(g0, c->L);
   if (c->L == 0) return SQG_OK;
+  lops.push_back(RotOp{});  // a block may have no operation left: never an empty array
   cudaError_t e = cudaMalloc(&c->d_lops, sizeof(RotOp) * lops.size());
   if (e == cudaSuccess) e = cudaMemcpy(c->d_lops, lops.data(), sizeof(RotOp) * lops.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMalloc(&c->d_lends, sizeof(int) * lends.size());
+  if (e == cudaSuccess) e = cudaMemcpy(c->d_lends, lends.data(), sizeof(int) * lends.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&c->d_hitab, sizeof(int) * hitab.size());
   if (e == cudaSuccess) e = cudaMemcpy(c->d_hitab, hitab.data(), sizeof(int) * hitab.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&c->d_inact, sizeof(int) * inact.size());
@@ -542,9 +547,10 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
 struct StateArgs {
   double2* states;
   long long stride;
-  int n, K, low, k0, k1, nops;
+  int n, K, low, k0, k1, nrecs;
   const RotOp* lops;
-  const RotRec* recs;     // [B][nops]
+  const int* ends;        // this block's places behind its last operation
+  const RotRec* recs;     // [B][nrecs]
   const double2* phases;  // [B][nphase], multiplied in by this pass; null: by another one
   int nphase;
   const int* hitab;
@@ -554,17 +560,19 @@ struct StateArgs {
 __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   extern __shared__ double2 sv[];
   __shared__ int hit[128];
+  __shared__ int ends[16 * kEndGroups];
   __shared__ StagedOp st[kRotChunk];
   const int b = blockIdx.y;
   const int KK = 1 << a.K, hb = a.K - a.low, lowmask = (1 << a.low) - 1;
   for (int h = threadIdx.x; h < (1 << hb); h += blockDim.x) hit[h] = a.hitab[h];
+  fill_end_table(ends, a.ends, a.K);
   long long cbase = 0;
   for (int j = 0; j < a.n - a.K; j++)
     if ((blockIdx.x >> j) & 1u) cbase |= 1LL << a.inact[j];
   double2* base = a.states + (long long)b * a.stride + cbase;
   __syncthreads();
   for (int l = threadIdx.x; l < KK; l += blockDim.x) sv[l] = base[(l & lowmask) + hit[l >> a.low]];
-  const RotRec* recs = a.recs + (long long)b * a.nops;
+  const RotRec* recs = a.recs + (long long)b * a.nrecs;
   for (int k0 = a.k0; k0 < a.k1; k0 += kRotChunk) {
     const int kn = min(kRotChunk, a.k1 - k0);
     __syncthreads();
@@ -578,9 +586,9 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   if (a.phases) {
     double2 p = make_double2(1.0, 0.0);
     for (int k = 0; k < a.nphase; k++) p = cmul(p, a.phases[(long long)b * a.nphase + k]);
-    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = cmul(p, sv[l]);
+    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = cmul(p, sv[end_place(ends, l)]);
   } else {
-    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = sv[l];
+    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = sv[end_place(ends, l)];
   }
 }
 
@@ -592,27 +600,44 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
 // Makes the rotation plan of the circuit and copies it to the device.
 static int make_rot_plan(sqg_circuit* c) {
   RotPlanHost h = build_rot_plan(c->n, c->h_gates);
-  c->h_ops = h.ops;
-  c->h_anchor = h.anchor;
+  c->h_steps = h.steps;
+  std::vector<RotOp> ops;
+  std::vector<int> ends;
+  if (c->n <= kMatrixQubits) {  // larger registers are applied in chunks only
+    std::vector<int> loc(c->n);
+    for (int q = 0; q < c->n; q++) loc[q] = q;
+    lower_rot_steps(h.steps, 0, (int)h.steps.size(), c->n, loc, ops, ends);
+  }
   RotPlan& p = c->plan;
   p.gates = c->d_gates;
-  p.nops = (int)h.ops.size();
+  p.nops = (int)ops.size();
+  p.nrecs = (int)h.steps.size();
   p.ncta = (int)h.cta.size() - 1;
   p.noverlaps = h.noverlaps;
-  const size_t ob = h.ops.size() * sizeof(RotOp), rb = h.runs.size() * sizeof(RotRun), mb = h.members.size() * sizeof(int),
-               cb = h.cta.size() * sizeof(int);
-  std::vector<char> blob(ob + rb + mb + cb);
-  if (ob) memcpy(blob.data(), h.ops.data(), ob);
-  if (rb) memcpy(blob.data() + ob, h.runs.data(), rb);
-  if (mb) memcpy(blob.data() + ob + rb, h.members.data(), mb);
-  memcpy(blob.data() + ob + rb + mb, h.cta.data(), cb);
+  std::vector<char> blob;
+  auto put = [&](const void* src, size_t bytes) {
+    const size_t at = blob.size();
+    blob.resize((at + bytes + 15) / 16 * 16);
+    if (bytes) memcpy(blob.data() + at, src, bytes);
+    return at;
+  };
+  const size_t o_ops = put(ops.data(), ops.size() * sizeof(RotOp));
+  const size_t o_runs = put(h.runs.data(), h.runs.size() * sizeof(RotRun));
+  const size_t o_mem = put(h.members.data(), h.members.size() * sizeof(int));
+  const size_t o_cta = put(h.cta.data(), h.cta.size() * sizeof(int));
+  const size_t o_par = put(h.params.data(), h.params.size() * sizeof(int));
+  const size_t o_cpar = put(h.cta_params.data(), h.cta_params.size() * sizeof(int));
+  const size_t o_ends = put(ends.data(), ends.size() * sizeof(int));
   cudaError_t e = cudaMalloc(&c->d_plan, blob.size());
   if (e == cudaSuccess) e = cudaMemcpy(c->d_plan, blob.data(), blob.size(), cudaMemcpyHostToDevice);
   char* d = (char*)c->d_plan;
-  p.ops = (const RotOp*)d;
-  p.runs = (const RotRun*)(d + ob);
-  p.members = (const int*)(d + ob + rb);
-  p.cta = (const int*)(d + ob + rb + mb);
+  p.ops = (const RotOp*)(d + o_ops);
+  p.runs = (const RotRun*)(d + o_runs);
+  p.members = (const int*)(d + o_mem);
+  p.cta = (const int*)(d + o_cta);
+  p.params = (const int*)(d + o_par);
+  p.cta_params = (const int*)(d + o_cpar);
+  p.ends = (const int*)(d + o_ends);
   return cuda_status(e, "rotation plan");
 }
 
@@ -703,9 +728,11 @@ int sqg_circuit_set_partitions(sqg_circuit* c, const int* part_ends, int nparts)
   cudaGetDevice(&dev);
   if (dev != c->device) return fail(SQG_ERR_INVALID_ARGUMENT, "circuit handle belongs to another device");
   cudaFree(c->d_lops);
+  cudaFree(c->d_lends);
   cudaFree(c->d_hitab);
   cudaFree(c->d_inact);
   c->d_lops = nullptr;
+  c->d_lends = nullptr;
   c->d_hitab = nullptr;
   c->d_inact = nullptr;
   c->sblocks.clear();
@@ -716,6 +743,7 @@ int sqg_circuit_destroy(sqg_circuit* c) {
   if (!c) return SQG_OK;
   if (c->d_gates) cudaFree(c->d_gates);
   if (c->d_lops) cudaFree(c->d_lops);
+  if (c->d_lends) cudaFree(c->d_lends);
   if (c->d_hitab) cudaFree(c->d_hitab);
   if (c->d_inact) cudaFree(c->d_inact);
   if (c->d_plan) cudaFree(c->d_plan);
@@ -1077,7 +1105,7 @@ int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* stat
     a.n = c->n;
     a.K = c->sK;
     a.low = std::min(c->sK, kStateLow);
-    a.nops = t.nops;
+    a.nrecs = t.nrecs;
     a.lops = c->d_lops;
     a.recs = t.recs;
     a.nphase = t.nphase;
@@ -1085,6 +1113,7 @@ int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* stat
       a.k0 = c->sblocks[k].k0;
       a.k1 = c->sblocks[k].k1;
       a.phases = k == 0 && t.nphase > 0 ? t.phases : nullptr;
+      a.ends = c->d_lends + 16 * k;
       a.hitab = c->d_hitab + 128 * k;
       a.inact = c->d_inact + 32 * k;
       k_state_block<<<dim3(1u << (c->n - c->sK), B), kStateThreads, smem, s>>>(a);

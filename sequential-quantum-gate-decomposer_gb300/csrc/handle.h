@@ -5,12 +5,12 @@
 #include <vector>
 
 #include "gates.cuh"
-#include "rot.cuh"
+#include "rotplan.h"
 
 // Fused state-vector passes (sqg_apply_state): consecutive gates whose qubits, together with
 // the lowest ones, fit one chunk of 2^K amplitudes form a block applied in shared memory.
 struct sqg_state_block {
-  int k0, k1;  // operations [k0, k1) of the rotation plan
+  int k0, k1;  // operations [k0, k1) of the state-vector plan
 };
 
 struct sqg_circuit {
@@ -18,20 +18,21 @@ struct sqg_circuit {
   int device = 0;
   sqg::Gate* d_gates = nullptr;
   std::vector<sqg::Gate> h_gates;
-  // state-vector plan: chunk qubits K, blocks, operations with chunk-local qubit positions,
-  // per block the global offsets of the chunk's high local bits (2^(K - low) ints, padded to
-  // 128) and the qubits that number the chunks (padded to 32)
+  // rotation plan (rot.cuh): the host's steps, from which the tile operations and those of the
+  // state-vector blocks are made, and the device arrays, one allocation behind d_plan
+  std::vector<sqg::RotStep> h_steps;
+  void* d_plan = nullptr;
+  sqg::RotPlan plan = {};
+  // state-vector plan: chunk qubits K, blocks, operations on chunk-local qubits, per block the
+  // places behind its last operation (K ints, padded to 16), the global offsets of the chunk's
+  // high local bits (2^(K - low) ints, padded to 128) and the qubits that number the chunks
+  // (padded to 32)
   int sK = 0;
   std::vector<sqg_state_block> sblocks;
   sqg::RotOp* d_lops = nullptr;
+  int* d_lends = nullptr;
   int* d_hitab = nullptr;
   int* d_inact = nullptr;
-  // rotation plan (rot.cuh): the host's copy of the operations with the gate whose place each
-  // takes, and the device arrays, one allocation behind d_plan
-  std::vector<sqg::RotOp> h_ops;
-  std::vector<int> h_anchor;
-  void* d_plan = nullptr;
-  sqg::RotPlan plan = {};
 };
 
 namespace sqg {

@@ -22,6 +22,7 @@ using namespace sqg;
 namespace {
 
 constexpr int kRaggedThreads = 256;
+constexpr int kRaggedStatic = 512;  // bound of the tile kernels' static shared memory
 
 struct InstDesc {
   RotPlan plan;
@@ -76,7 +77,9 @@ __global__ void __launch_bounds__(kRaggedThreads) k_ragged_tiles(const InstDesc*
     const InstDesc d = desc[it.x];
     TileArgs a;
     a.ops = d.plan.ops;
+    a.ends = d.plan.ends;
     a.nops = d.plan.nops;
+    a.nrecs = d.plan.nrecs;
     a.noverlaps = d.plan.noverlaps;
     a.n = d.n; a.N = d.N;
     a.recs = recs + d.rec_off;
@@ -203,7 +206,7 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
     r->target_off.push_back(tg);
     th += c->P;
     tg += (long long)c->N * cols[i];
-    r->total_rec += c->plan.nops;
+    r->total_rec += c->plan.nrecs;
     r->total_ph += c->plan.ncta;
     r->total_tr += d.tiles;
     if (with_grad) r->total_gr += (long long)d.tiles * c->plan.noverlaps;
@@ -239,12 +242,12 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
   // in CUDA graphs
   int optin = 0;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, r->device);
-  if (e == cudaSuccess && smem + 64 > (size_t)optin) {
+  if (e == cudaSuccess && smem + kRaggedStatic > (size_t)optin) {
     free_batch(r);
     return set_error(SQG_ERR_UNSUPPORTED, "work item does not fit in shared memory");
   }
   for (auto k : {k_ragged_tiles<0>, k_ragged_tiles<1>, k_ragged_tiles<2>})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 64);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - kRaggedStatic);
   int per_sm = 0, sms = 0;
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(

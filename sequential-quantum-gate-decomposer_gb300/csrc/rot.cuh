@@ -8,7 +8,7 @@
 //  * M = scalar * diag(1, zo) * R * diag(1, zi) with R a rotation.  R is applied without its
 //    cosine ([[1, -t], [t, 1]], |t| <= 1 after an exchange of the two rows where needed):
 //    4 multiply-adds per pair instead of 8.  The cosines of up to kRotChunk consecutive
-//    operations are multiplied back in one of them, so the scale never leaves [1, 2^16].
+//    operations are multiplied in with the first of them, so the scale stays in [2^-16, 1].
 //    A phase diag(1, z) touches one row of the pair: 4 instructions.
 //  * The rotation that M ends with is moved through the next two-qubit gate into the next run
 //    on the qubit where it commutes with that gate: Z through a control or a CZ, X through a
@@ -17,7 +17,8 @@
 //  * Phases common to all amplitudes are collected per instance and multiplied in once.
 //  * The gradient needs only <lambda| P |psi> for the Paulis P at the end of each run; the one
 //    along the axis that the run pushes equals that of the next run and is not measured, and
-//    the derivatives of the run's gates follow from these three numbers, once per run (rot_grad_body), not per amplitude.
+//    the derivatives of the run's gates follow from these three numbers, once per run
+//    (rot_grad_body) and not per amplitude.
 // Measured on GB300 against the gates as given (U3 14 instructions, merged runs 16): gradient at
 // 8 qubits, 360 blocks, 128 vectors 333 -> 182 ms; cost alone, 120 blocks, 200 vectors 41.5 ->
 // 25.3 ms; 2000 random gates on a 4096 x 4096 matrix 143 -> 99 ms; 829 gates on 24 qubits 128 ->
@@ -34,21 +35,31 @@ namespace sqg {
 enum : int { kOpCnot = 0, kOpCz = 1, kOpCry = 2, kOpPhase = 3, kOpRot = 4, kOpX = 8, kOpZi = 16, kOpZo = 32 };
 enum : int { kAxisNone = 0, kAxisX = 1, kAxisY = 2, kAxisZ = 3 };
 
-// One operation of the plan.  coff: first of its overlaps in the instance's overlap list;
-// mask: which are measured (1 X, 2 Y, 4 Z; kOpCry: 2, on the controlled half).
+// One operation of the plan as the sweeps apply it to 2^n amplitudes.  A CNOT moves no data: it
+// only changes which amplitude a place holds.  Place p holds the amplitude whose bit q is the
+// parity of p & row_q, and its partner under qubit q is p ^ pair_q; the plan follows these masks
+// through the CNOTs.  A CZ flips signs where two parities are odd; it rides on the next
+// operation that does not commute with it (cz0, cz1; none: 0) or is one of its own (kOpCz).
+// coff: first of the operation's overlaps in the instance's overlap list; mask: which are
+// measured (1 X, 2 Y, 4 Z; kOpCry: 2, on the controlled half).
 struct RotOp {
   int kind;
-  int qubits;  // target | control << 8
+  int rec;  // of its numbers
   int coff;
   int mask;
+  unsigned short pair, row, crow;  // the target's pair and row, a CRY control's row
+  unsigned short cz0, cz1;
+  unsigned short b0, b1;  // bits that number the pairs: set in pair; kOpCry: in crow, not b0
+  unsigned short pad;
 };
 
-// One run (or CRY gate): its operation, its gates members[first .. first + count), the axis it
+// One run (or CRY gate): its record, its gates members[first .. first + count), the axis it
 // pushes (kAxisNone: nothing) into the run right behind it in the chain order, whether the run
 // before it pushes into it, a copy of its operation's kind, coff and mask, and whether it is a
-// single U3.
+// single U3.  soff: place of its first parameter in its CTA's parameter list, the parameters of its
+// gates behind one another (-1: not listed).
 struct RotRun {
-  int op, first, count, push, pulled, kind, coff, mask, lone_u3;
+  int rec, first, count, push, pulled, kind, coff, mask, lone_u3, soff;
 };
 
 // Numbers of one operation.  t, c: tangent and cosine of the rotation (kOpCry: sine and
@@ -70,10 +81,14 @@ struct RotPlan {
   const RotRun* runs;
   const int* members;
   const int* cta;  // runs [cta[i], cta[i + 1]) are handled by one CTA of kRotThreads threads
-  int nops, ncta, noverlaps;
+  const int* params;  // parameters of CTA i's runs: params[cta_params[i] .. cta_params[i + 1])
+  const int* cta_params;
+  const int* ends;  // place of the amplitude 2^q behind the last operation (a sum of them: their XOR)
+  int nops, nrecs, ncta, noverlaps;
 };
 
 constexpr int kRotThreads = 128;  // runs per CTA of the per-instance kernels; no chain straddles two
+constexpr int kRotParams = 512;  // parameters listed per CTA
 constexpr int kRotChain = 16;     // runs linked by pushed rotations (their numbers are made one after another)
 constexpr int kRotChunk = 32;     // operations staged in shared memory together
 
@@ -88,6 +103,20 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double cnorm2(double2 a) { return fma(a.x, a.x, a.y * a.y); }
+// 1 / sqrt(x) and 1 / x for x in [2^-120, 2^120], to a rounding: from the single-precision value by
+// two Newton steps.  The chains of rot_plan_body wait for every one of their instructions, and
+// the general functions take several times as many.
+__device__ __forceinline__ double fast_rsqrt(double x) {
+  double y = (double)rsqrtf((float)x);
+  const double h = -0.5 * x;
+  y = fma(y, fma(h * y, y, 0.5), y);
+  return fma(y, fma(h * y, y, 0.5), y);
+}
+__device__ __forceinline__ double fast_rcp(double x) {
+  double y = (double)__frcp_rn((float)x);
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
 // One Newton step towards |z| = 1 for z that is a few roundings away from it.
 __device__ __forceinline__ double2 cunit(double2 z) { return cscale(z, fma(-0.5, cnorm2(z), 1.5)); }
 
@@ -100,18 +129,35 @@ __device__ __forceinline__ void matmul2(const double2 G[4], double2 M[4]) {
   M[3] = cadd(cmul(G[2], b), cmul(G[3], M[3]));
 }
 
-// Full 2x2 matrix of a single-qubit gate from its stored parameters.
-__device__ __forceinline__ void gate_matrix(int type, const double* th, double2 u[4]) {
+// (cos, sin) of every listed parameter of a CTA's runs, one per thread: a warp's FP64 instruction
+// costs the same for one lane as for 32.  sc: kRotParams entries of shared memory; the caller
+// synchronises.
+__device__ __forceinline__ void cta_sincos(const RotPlan& pl, int cta, const double* theta, double2* sc) {
+  const int first = pl.cta_params[cta], n = pl.cta_params[cta + 1] - first;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    double s, c;
+    sincos(theta[pl.params[first + k]], &s, &c);
+    sc[k] = make_double2(c, s);
+  }
+}
+// (cos, sin) of parameter k of a gate whose listed ones start at soff.
+__device__ __forceinline__ double2 param_sincos(const double2* sc, int soff, const double* th, int k) {
+  if (soff >= 0) return sc[soff + k];
   double s, c;
-  sincos(th[0], &s, &c);
+  sincos(th[k], &s, &c);
+  return make_double2(c, s);
+}
+
+// Full 2x2 matrix of a single-qubit gate.
+__device__ __forceinline__ void gate_matrix(int type, const double2* sc, int soff, const double* th, double2 u[4]) {
+  const double2 a = param_sincos(sc, soff, th, 0);
+  const double c = a.x, s = a.y;
   if (type == G_U3) {
-    double sp, cp, sl, cl;
-    sincos(th[1], &sp, &cp);
-    sincos(th[2], &sl, &cl);
+    const double2 ph = param_sincos(sc, soff, th, 1), la = param_sincos(sc, soff, th, 2);
     u[0] = make_double2(c, 0.0);
-    u[1] = make_double2(-s * cl, -s * sl);
-    u[2] = make_double2(s * cp, s * sp);
-    u[3] = make_double2(c * (cp * cl - sp * sl), c * (sp * cl + cp * sl));
+    u[1] = cscale(la, -s);
+    u[2] = cscale(ph, s);
+    u[3] = cscale(cmul(ph, la), c);
   } else if (type == G_RX) {
     u[0] = u[3] = make_double2(c, 0.0);
     u[1] = u[2] = make_double2(0.0, -s);
@@ -131,7 +177,7 @@ __device__ __forceinline__ void gate_matrix(int type, const double* th, double2 
 __device__ __forceinline__ void set_cosine(RotRec& r) {
   const double t2 = r.t * r.t, t2e = fma(r.t, r.t, -t2);
   const double s = 1.0 + t2, se = (1.0 - s) + t2 + t2e;
-  r.c = 1.0 / sqrt(s);
+  r.c = fast_rsqrt(s);
   const double c2 = r.c * r.c, c2e = fma(r.c, r.c, -c2);
   const double p = c2 * s, pe = fma(c2, s, -p) + fma(c2e, s, c2 * se);
   r.lo = 0.5 * r.c * ((1.0 - p) - pe);
@@ -144,48 +190,51 @@ __device__ __forceinline__ double2 split_zyz(const double2 M[4], RotRec& r) {
   const bool turn = nc > na;
   const double2 piv = turn ? M[2] : M[0], oth = turn ? M[0] : M[2];
   const double np = turn ? nc : na;
-  const double2 q = cscale(cmulc(oth, piv), 1.0 / np);  // f = 0: t zo, f = 1: -t / zo
-  const double t2 = cnorm2(q), t = sqrt(t2);
+  const double inp = fast_rcp(np);
+  const double2 q = cscale(cmulc(oth, piv), inp);  // f = 0: t zo, f = 1: -t / zo
+  const double t2 = cnorm2(q);
+  // t below 1e-17 is an entry lost in the rounding of the others: any phase does
+  const double rt = t2 > 1e-34 ? fast_rsqrt(t2) : 0.0, t = t2 * rt;
   double2 zo = make_double2(1.0, 0.0);
-  if (t2 > 1e-280) zo = cscale(turn ? make_double2(-q.x, q.y) : q, 1.0 / t);
+  if (t2 > 1e-34) zo = cscale(turn ? make_double2(-q.x, q.y) : q, rt);
   zo = cunit(zo);
   // turn = 0: zi = (d / a) / zo;  turn = 1: zi = -(b / c) zo
-  const double2 w = cscale(cmulc(turn ? M[1] : M[3], piv), 1.0 / np);
+  const double2 w = cscale(cmulc(turn ? M[1] : M[3], piv), inp);
   double2 zi = turn ? cmul(make_double2(-w.x, -w.y), zo) : cmulc(w, zo);
   zi = cunit(cunit(zi));
   r.turn = turn;
   r.t = t;
-  set_cosine(r);
   // the quarter turn (x, y) -> (-y, x) as an exchange: its sign goes into zi
   r.zi = turn ? make_double2(-zi.x, -zi.y) : zi;
   r.zo = zo;
-  const double2 u = cscale(piv, 1.0 / sqrt(np));
+  const double2 u = cscale(piv, fast_rsqrt(np));
   return turn ? cmulc(u, zo) : u;
 }
 
-// M (unitary) as W * Ry(atan t) * diag(1, zi) with W = phase * Rx: W is returned in w00, w01
-// (its diagonal and off-diagonal entry).  |t| <= 1 always.
-__device__ __forceinline__ void split_x(const double2 M[4], RotRec& r, double2& w00, double2& w01) {
-  // (M00^2 - M10^2) / det M = e^{-2 i gamma} cos 2 beta, with zi = e^{2 i gamma}
-  const double2 det = csub(cmul(M[0], M[3]), cmul(M[1], M[2]));
-  const double2 d = cmulc(csub(cmul(M[0], M[0]), cmul(M[2], M[2])), det);
-  const double nd2 = cnorm2(d), nd = sqrt(nd2);
-  const double s = cnorm2(M[0]) + cnorm2(M[2]);
-  double2 zi = make_double2(1.0, 0.0);
-  if (nd2 > 1e-280) zi = cunit(make_double2(d.x / nd, -d.y / nd));
-  const double sb = 2.0 * fma(M[0].x, M[2].x, M[0].y * M[2].y);
-  r.t = sb / (s + nd);
-  set_cosine(r);
-  const double c = r.c, sn = r.t * c;
-  // W = M diag(1, conj zi) Ry(-beta)
-  const double2 b = cmulc(M[1], zi);
-  w00 = csub(cscale(M[0], c), cscale(b, sn));
-  w01 = cadd(cscale(M[0], sn), cscale(b, c));
-  const double k = fma(-0.5, cnorm2(w00) + cnorm2(w01), 1.5);
-  w00 = cscale(w00, k);
-  w01 = cscale(w01, k);
+// A unitary with first column (p, q) and determinant det as W * Ry(atan t) * diag(1, zi) with W =
+// phase * Rx = [[w0, w1], [w1, w0]].  |t| <= 1 always.  The cosine is left to set_cosine.  On
+// return p, q, det are those of W.
+__device__ __forceinline__ void split_x(double2& p, double2& q, double2& det, RotRec& r) {
+  // (p^2 - q^2) / det = e^{-2 i gamma} cos 2 beta, with zi = e^{2 i gamma}
+  const double2 pq = cadd(p, q), mq = csub(p, q);
+  const double2 d = cmulc(cmul(pq, mq), det);
+  const double nd2 = cnorm2(d), rnd = nd2 > 1e-34 ? fast_rsqrt(nd2) : 0.0;
+  const double2 zi = nd2 > 1e-34 ? make_double2(d.x * rnd, -d.y * rnd) : make_double2(1.0, 0.0);
+  const double sb = fma(p.x, q.x, p.y * q.y);
+  const double t = 2.0 * sb * fast_rcp(fma(nd2, rnd, 1.0));
+  const double c = fast_rsqrt(fma(t, t, 1.0)), sn = t * c;
+  // W = A diag(1, conj zi) Ry(-beta); the second column of A is (-conj q, conj p) det
+  det = cmulc(det, zi);
+  const double2 b = cmulc(det, q);  // minus the upper entry of A diag(1, conj zi)
+  const double2 w0 = make_double2(fma(c, p.x, sn * b.x), fma(c, p.y, sn * b.y));
+  const double2 w1 = make_double2(fma(sn, p.x, -(c * b.x)), fma(sn, p.y, -(c * b.y)));
+  const double k = fma(-0.5, cnorm2(w0) + cnorm2(w1), 1.5);
+  p = cscale(w0, k);
+  q = cscale(w1, k);
+  det = cunit(det);
   r.turn = 0;
-  r.zi = zi;
+  r.t = t;
+  r.zi = cunit(zi);
 }
 
 // U3 = diag(1, phi) Ry(s, c) diag(1, lam), all three given as (cos, sin), times a phase: the
@@ -196,8 +245,8 @@ __device__ __forceinline__ double split_u3(double2 cs, double2 phi, double2 lam,
   // Ry(theta) = Ry(theta - pi/2) after the quarter turn
   const double c = turn ? cs.y : cs.x, s = turn ? -cs.x : cs.y;
   r.turn = turn;
-  r.t = s / c;
-  set_cosine(r);
+  const double rc = fast_rcp(c), t = s * rc;
+  r.t = fma(fma(-t, c, s), rc, t);
   r.zi = turn ? make_double2(-lam.x, -lam.y) : lam;
   r.zo = phi;
   return c < 0.0 ? -1.0 : 1.0;
@@ -210,40 +259,60 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
                                               double2* phase_out) {
   __shared__ double2 Ms[kRotThreads][4];
   __shared__ double2 ph[kRotThreads];
+  __shared__ int chain_of[kRotThreads], warp_heads[kRotThreads / 32];
   const int base = pl.cta[cta], n = pl.cta[cta + 1] - base, i = threadIdx.x;
   const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
+  __shared__ double2 sc[kRotParams];
+  cta_sincos(pl, cta, theta, sc);
+  __syncthreads();
   RotRun run;
   double2 phase = one;
   if (i < n) {
     run = pl.runs[base + i];
     double2 M[4];
     Gate g = pl.gates[pl.members[run.first]];
+    int soff = run.soff;
     if (run.lone_u3) {
-      double s, c;
-      for (int k = 0; k < 3; k++) {
-        sincos(theta[g.pstart + k], &s, &c);
-        M[k] = make_double2(c, s);
-      }
-      M[3] = zero;
+      for (int k = 0; k < 3; k++) M[k] = param_sincos(sc, soff, theta + g.pstart, k);
+      M[3] = cmul(M[1], M[2]);
     } else {
-      gate_matrix(g.type, theta + g.pstart, M);
+      gate_matrix(g.type, sc, soff, theta + g.pstart, M);
       for (int k = 1; k < run.count; k++) {
         double2 G[4];
+        if (soff >= 0) soff += gate_param_num(g.type);
         g = pl.gates[pl.members[run.first + k]];
-        gate_matrix(g.type, theta + g.pstart, G);
+        gate_matrix(g.type, sc, soff, theta + g.pstart, G);
         matmul2(G, M);
       }
     }
     for (int k = 0; k < 4; k++) Ms[i][k] = M[k];
   }
+  // Chains of two and more runs are few and take longest: they are dealt out over the warps, so
+  // that as few as possible wait for one another's branches.
+  const int warp = i >> 5, lane = i & 31;
+  const bool head = i < n && !run.pulled && run.push != kAxisNone;
+  const unsigned heads = __ballot_sync(0xffffffffu, head);
+  if (lane == 0) warp_heads[warp] = __popc(heads);
   __syncthreads();
-  if (i < n && !run.pulled) {
-    // the rotation pushed into the next run: diag(1, pz) times a phase (zpend), or a matrix
+  int rank = __popc(heads & ((1u << lane) - 1)), nheads = 0;
+  for (int w = 0; w < kRotThreads / 32; w++) {
+    if (w < warp) rank += warp_heads[w];
+    nheads += warp_heads[w];
+  }
+  if (head) chain_of[(rank % (kRotThreads / 32)) * 32 + rank / (kRotThreads / 32)] = i;
+  __syncthreads();
+  const bool walks = lane * (kRotThreads / 32) + warp < nheads;
+  for (int pass = 0; pass < 2; pass++) {
+    // first the runs by themselves, each by its own thread, then the chains
+    if (pass == 0 ? !(i < n && !run.pulled && run.push == kAxisNone) : !walks) continue;
+    // the rotation pushed into the next run: diag(1, pz) times pphase (zpend), or a unitary given
+    // by its first column (wp, wq); wdet: its determinant
     bool zpend = true;
-    double2 pz = one, pphase = one, pend[4];
-    int j = i;
+    double2 pz = one, pphase = one, wp = one, wq = zero, wdet = one;
+    int j = pass == 0 ? i : chain_of[i];
+    double2 own = one;
     for (int step = 0; step < kRotChain; step++, j++) {
-      if (step) run = pl.runs[base + j];
+      if (pass || step) run = pl.runs[base + j];
       RotRec r = {0.0, 1.0, one, one, 0.0, 0};
       double2 M[4];
       for (int k = 0; k < 4; k++) M[k] = Ms[j][k];
@@ -252,73 +321,77 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
         r.c = M[0].x;
       } else if (run.kind == kOpPhase) {  // diagonal
         r.zi = cunit(cmulc(M[3], M[0]));
-        phase = M[0];
+        own = M[0];
       } else if (!(run.kind & kOpZi)) {  // Ry or Rx by itself: M[0] = cos, M[2] = sin or -i sin
         const double2 cs = make_double2(M[0].x, (run.kind & kOpX) ? -M[2].y : M[2].x);
         const double sign = split_u3(cs, one, one, r);
         r.zi = one;
         // about X the quarter turn is -i times the exchange
-        phase = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
+        own = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
       } else if (run.lone_u3 && zpend && (run.push == kAxisNone || run.push == kAxisZ)) {
         const double2 lam = step ? cunit(cmul(M[2], pz)) : M[2];
         pphase = cscale(pphase, split_u3(M[0], M[1], lam, r));
         if (run.push == kAxisNone)
-          phase = pphase;
+          own = pphase;
         else
-          pz = M[1];
+          pz = M[1], wdet = cmul(cmul(pphase, pphase), pz);
       } else {
-        double2 A[4];
-        if (run.lone_u3) {
-          const double2 cs = M[0], pl2 = cmul(M[1], M[2]);
-          A[0] = make_double2(cs.x, 0.0);
-          A[1] = cscale(M[2], -cs.y);
-          A[2] = cscale(M[1], cs.y);
-          A[3] = cscale(pl2, cs.x);
+        // A = M * pushed, by its first column (p, q) and its determinant
+        double2 p, q, d;
+        if (run.lone_u3) {  // cos and sin, phi, lambda and phi lambda
+          const double2 y = zpend ? make_double2(0.0, 0.0) : cmul(M[2], wq);
+          const double2 u = zpend ? pphase : wp;
+          p = make_double2(fma(M[0].x, u.x, -(M[0].y * y.x)), fma(M[0].x, u.y, -(M[0].y * y.y)));
+          q = cmul(M[1], make_double2(fma(M[0].y, u.x, M[0].x * y.x), fma(M[0].y, u.y, M[0].x * y.y)));
+          d = cmul(M[3], wdet);
         } else {
-          for (int k = 0; k < 4; k++) A[k] = M[k];
+          p = zpend ? cmul(M[0], pphase) : cadd(cmul(M[0], wp), cmul(M[1], wq));
+          q = zpend ? cmul(M[2], pphase) : cadd(cmul(M[2], wp), cmul(M[3], wq));
+          d = cmul(csub(cmul(M[0], M[3]), cmul(M[1], M[2])), wdet);
         }
-        if (zpend) {
-          A[1] = cmul(A[1], pz);
-          A[3] = cmul(A[3], pz);
-          for (int k = 0; k < 4; k++) A[k] = cmul(A[k], pphase);
-        } else {
-          for (int k = 0; k < 4; k++) M[k] = A[k];
-          for (int k = 0; k < 4; k++) A[k] = pend[k];
-          matmul2(M, A);
-        }
-        if (run.push == kAxisNone) {
-          phase = split_zyz(A, r);
-        } else if (run.push == kAxisZ) {
-          pphase = cunit(split_zyz(A, r));
-          pz = r.zo;
-          zpend = true;
+        if (run.push == kAxisNone || run.push == kAxisZ) {
+          // the second column of a unitary: (-conj q, conj p) det
+          const double2 A[4] = {p, cmulc(make_double2(-d.x, -d.y), q), q, cmulc(d, p)};
+          const double2 ph = split_zyz(A, r);
+          if (run.push == kAxisNone) {
+            own = ph;
+          } else {
+            zpend = true;
+            pphase = cunit(ph);
+            pz = r.zo;
+            wdet = cmul(cmul(pphase, pphase), pz);
+          }
         } else {
           // Y: with S = diag(1, i), S A S^dagger = Rx(-alpha) Ry(beta) diag(1, zi)
-          if (run.push == kAxisY) {
-            A[1] = make_double2(A[1].y, -A[1].x);
-            A[2] = make_double2(-A[2].y, A[2].x);
-          }
-          double2 w0, w1;
-          split_x(A, r, w0, w1);
+          if (run.push == kAxisY) q = make_double2(-q.y, q.x);
+          split_x(p, q, d, r);
+          const double c2 = cnorm2(p) - cnorm2(q);
+          const double s2 = -2.0 * fma(p.x, q.y, -(p.y * q.x));  // sin of the full angle: -2 Im(conj(w0) w1)
           zpend = false;
-          pend[0] = pend[3] = w0;
-          pend[1] = pend[2] = w1;
-          const double c2 = cnorm2(w0) - cnorm2(w1);
-          double s2 = -2.0 * fma(w0.x, w1.y, -w0.y * w1.x);  // sin of the full angle: -2 Im(conj(w0) w1)
-          if (run.push == kAxisY) {
-            pend[1] = make_double2(-w1.y, w1.x);
-            pend[2] = make_double2(w1.y, -w1.x);
-            s2 = -s2;
-          }
-          r.zo = make_double2(c2, s2);
+          wp = p;
+          wq = run.push == kAxisY ? make_double2(q.y, -q.x) : q;
+          wdet = d;
+          r.zo = make_double2(c2, run.push == kAxisY ? -s2 : s2);
         }
       }
-      recs[run.op] = r;
+      recs[run.rec] = r;
       if (run.push == kAxisNone) break;
     }
+    phase = cmul(phase, own);
   }
   ph[i] = phase;
   __syncthreads();
+  // the cosines of all runs at once: the chains need not wait for them
+  if (i < n) {
+    const RotRun mine = pl.runs[base + i];
+    if (mine.kind & kOpRot) {
+      RotRec& r = recs[mine.rec];
+      RotRec v = r;
+      set_cosine(v);
+      r.c = v.c;
+      r.lo = v.lo;
+    }
+  }
   for (int o = kRotThreads / 2; o > 0; o >>= 1) {
     if (i < o) ph[i] = cmul(ph[i], ph[i + o]);
     __syncthreads();
@@ -327,31 +400,31 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
 }
 
 // ---- application ---------------------------------------------------------------------------
-// Operation staged for the sweeps.  Negated copies of its numbers (nt, nzi, nzo) are staged with
-// them: the sweeps would otherwise negate them once per thread, on the FP64 pipe.  scale: of the
-// operation that multiplies the chunk's cosines back in (kStRescale; t and nt include it), the
-// cosine of a kOpCry.  mfac: what the overlaps measured behind the operation, with both vectors
-// on the way back, are multiplied by.
+// Operation staged for the sweeps.  scale: of the operation that multiplies the chunk's cosines
+// in (kStRescale; t includes it), the cosine of a kOpCry.  mfac: what the overlaps measured
+// behind the operation, with both vectors on the way back, are multiplied by.
 struct StagedOp {
-  int kind, qubits, coff, mask;  // qubits: target | control << 8 | flags << 16
-  double t, nt, scale, mfac;
+  int kind, coff;  // kind | mask << 8 | flags
+  unsigned pair_row, crow_bits, cz;  // pair | row << 16, crow | b0 << 16 | b1 << 24, cz0 | cz1 << 16
+  int pad;
+  double t, scale, mfac;
   double2 zi, zo;
-  double nzi, nzo;
 };
 enum : int { kStTurn = 1 << 16, kStRescale = 1 << 17 };
 
 // Loads operations [k0, k0 + kn) (at most kRotChunk) into st with the first warp of the CTA.
-// The cosines that the chunk's rotations leave out are multiplied back in its last rotation.
+// The cosines that the chunk's rotations leave out are multiplied in by its first rotation: from
+// there the scale rises back to 1, and amplitudes never exceed what they were.
 // The caller synchronises before and after.
 __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   const bool on = lane < kn;
-  RotOp op = {kOpCnot, 0, 0, 0};
+  RotOp op = {kOpCnot, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   RotRec r = {0.0, 1.0, make_double2(1.0, 0.0), make_double2(1.0, 0.0), 0.0, 0};
   if (on) {
     op = ops[k0 + lane];
-    if (op.kind >= kOpCry) r = recs[k0 + lane];
+    if (op.kind >= kOpCry) r = recs[op.rec];
   }
   const bool rot = (op.kind & kOpRot) != 0;
   // product of the cosines up to and including this operation, as pre + plo
@@ -366,58 +439,102 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
   }
   const double all = __shfl_sync(0xffffffffu, pre + plo, 31);
   const unsigned rots = __ballot_sync(0xffffffffu, rot);
-  const int last = rots ? 31 - __clz(rots) : -1;
+  const int first = rots ? __ffs(rots) - 1 : 32;
   if (on) {
     StagedOp s;
-    s.kind = op.kind;
-    s.qubits = op.qubits | (r.turn ? kStTurn : 0) | (lane == last ? kStRescale : 0);
+    s.kind = op.kind | op.mask << 8 | (r.turn ? kStTurn : 0) | (lane == first ? kStRescale : 0);
     s.coff = op.coff;
-    s.mask = op.mask;
-    s.scale = lane == last ? all : op.kind == kOpCry ? r.c : 1.0;
-    s.t = lane == last ? r.t * all : r.t;
-    s.nt = dneg(s.t);
-    const double inv = 1.0 / pre;
-    s.mfac = lane < last ? inv * inv : 1.0;
+    s.pair_row = op.pair | (unsigned)op.row << 16;
+    s.crow_bits = op.crow | (unsigned)op.b0 << 16 | (unsigned)op.b1 << 24;
+    s.cz = op.cz0 | (unsigned)op.cz1 << 16;
+    s.pad = 0;
+    s.scale = lane == first ? all : op.kind == kOpCry ? r.c : 1.0;
+    s.t = lane == first ? r.t * all : r.t;
+    const double inv = all / (pre + plo);
+    s.mfac = lane >= first ? inv * inv : 1.0;
     s.zi = r.zi;
     s.zo = r.zo;
-    s.nzi = dneg(r.zi.y);
-    s.nzo = dneg(r.zo.y);
     st[lane] = s;
   }
 }
 
 enum { kRotFwd = 0, kRotAdj = 1, kRotTrans = 2 };  // G, G^dagger, G^T (right multiplication)
 
+// v with the sign bit `flip` changed (an integer operation).
+__device__ __forceinline__ double flip_sign(double v, unsigned flip) {
+  return __hiloint2double(__double2hiint(v) ^ (int)flip, __double2loint(v));
+}
+
 // The numbers of a staged operation in a direction: G^dagger takes -t and the conjugate phases,
-// G^T takes -t about Y (Rx^T = Rx).
+// G^T takes -t about Y (Rx^T = Rx).  The negated copies are made here with integer operations,
+// from a sign bit that the compiler cannot see: it would otherwise negate on the FP64 pipe, once
+// per thread and operation (18 % of a sweep).
 struct DirOp {
   double t, nt, scale;
   double zix, ziy, nzi, zox, zoy, nzo;
   unsigned flip;  // sign bit for a turned Ry without a zi that could hold its sign
   bool turn;
+  unsigned pair, row, crow, cz0, cz1;
+  int b0, b1;
 };
 
 template <int DIR, int KIND>
 __device__ __forceinline__ DirOp directed(const StagedOp& s) {
   DirOp o;
+  unsigned sign = 0x80000000u;
+  asm volatile("" : "+r"(sign));
   const bool neg = DIR == kRotAdj || (DIR == kRotTrans && !(KIND & kOpX));
-  o.t = neg ? s.nt : s.t;
-  o.nt = neg ? s.t : s.nt;
+  const double t = s.t, nt = flip_sign(t, sign);
+  o.t = neg ? nt : t;
+  o.nt = neg ? t : nt;
   o.scale = s.scale;
   o.zix = s.zi.x;
-  o.ziy = DIR == kRotAdj ? s.nzi : s.zi.y;
-  o.nzi = DIR == kRotAdj ? s.zi.y : s.nzi;
+  const double zi = s.zi.y, nzi = flip_sign(zi, sign);
+  o.ziy = DIR == kRotAdj ? nzi : zi;
+  o.nzi = DIR == kRotAdj ? zi : nzi;
   o.zox = s.zo.x;
-  o.zoy = DIR == kRotAdj ? s.nzo : s.zo.y;
-  o.nzo = DIR == kRotAdj ? s.zo.y : s.nzo;
-  o.turn = (s.qubits & kStTurn) != 0;
-  o.flip = o.turn ? 0x80000000u : 0u;
+  const double zo = s.zo.y, nzo = flip_sign(zo, sign);
+  o.zoy = DIR == kRotAdj ? nzo : zo;
+  o.nzo = DIR == kRotAdj ? zo : nzo;
+  o.turn = (s.kind & kStTurn) != 0;
+  o.flip = o.turn ? sign : 0u;
+  o.pair = s.pair_row & 0xffffu;
+  o.row = s.pair_row >> 16;
+  o.crow = s.crow_bits & 0xffffu;
+  o.b0 = (s.crow_bits >> 16) & 255;
+  o.b1 = s.crow_bits >> 24;
+  o.cz0 = s.cz & 0xffffu;
+  o.cz1 = s.cz >> 16;
   return o;
 }
 
-// v with the sign bit `flip` changed (an integer operation).
-__device__ __forceinline__ double flip_sign(double v, unsigned flip) {
-  return __hiloint2double(__double2hiint(v) ^ (int)flip, __double2loint(v));
+__device__ __forceinline__ unsigned parity(unsigned v) { return __popc(v) & 1u; }
+
+// Places of pair q of an operation: x with its target bit 0, y with 1 (kOpCry: control bit 1).
+template <int KIND>
+__device__ __forceinline__ void pair_places(const DirOp& op, int q, int& ix, int& iy) {
+  unsigned p;
+  if (KIND == kOpCry) {
+    const int lo = min(op.b0, op.b1), hi = max(op.b0, op.b1);
+    p = ((q >> lo) << (lo + 1)) | (q & ((1 << lo) - 1));
+    p = ((p >> hi) << (hi + 1)) | (p & ((1u << hi) - 1));
+    p |= (parity(p & op.crow) ^ 1u) << op.b1;
+  } else {
+    p = ((q >> op.b0) << (op.b0 + 1)) | (q & ((1 << op.b0) - 1));
+  }
+  const unsigned par = parity(p & op.row) ? op.pair : 0u;
+  ix = (int)(p ^ par);
+  iy = (int)(p ^ par ^ op.pair);
+}
+
+// Signs of the CZ that rides on an operation.
+__device__ __forceinline__ void pair_signs(const DirOp& op, int ix, int iy, double2& x, double2& y) {
+  if (op.cz0) {
+    const unsigned fx = (parity(ix & op.cz0) & parity(ix & op.cz1)) << 31;
+    const unsigned fy = (parity(iy & op.cz0) & parity(iy & op.cz1)) << 31;
+    x = make_double2(flip_sign(x.x, fx), flip_sign(x.y, fx));
+    y = make_double2(flip_sign(y.x, fy), flip_sign(y.y, fy));
+  }
 }
 
 // y <- z y, nzy = -z.y
@@ -502,38 +619,38 @@ __device__ __forceinline__ void cry_pair(const DirOp& op, double2& x, double2& y
 template <int DIR, int KIND, bool RS>
 __device__ __forceinline__ void rot_tile_kind(double2* s, int N, int logN, int tc, const StagedOp& staged) {
   const DirOp op = directed<DIR, KIND>(staged);
-  const int target = staged.qubits & 255, control = (staged.qubits >> 8) & 255;
-  constexpr bool ctrl = KIND <= kOpCry;
-  const int lognp = ctrl ? logN - 2 : logN - 1;
+  const int lognp = KIND == kOpCry ? logN - 2 : logN - 1;
   const int npairs = 1 << lognp;
   const int items = tc << lognp;
-  const int step = 1 << target;
   for (int it = threadIdx.x; it < items; it += blockDim.x) {
-    const int col = it >> lognp;
-    const int p = it & (npairs - 1);
-    const int i = ctrl ? pair_index2(p, target, control) : pair_index1(p, target);
-    double2* v = s + col * N;
-    if (KIND == kOpPhase || KIND == kOpCz) {  // the target = 0 row is not touched
-      double2 y = v[i + step];
-      if (KIND == kOpCz)
-        y = make_double2(dneg(y.x), dneg(y.y));
-      else
-        rot_phase(y, op.zix, op.ziy, op.nzi);
-      v[i + step] = y;
+    double2* v = s + (it >> lognp) * N;
+    int ix, iy;
+    pair_places<KIND>(op, it & (npairs - 1), ix, iy);
+    if (KIND == kOpPhase) {  // the target = 0 row is not touched
+      double2 y = v[iy];
+      rot_phase(y, op.zix, op.ziy, op.nzi);
+      v[iy] = y;
       continue;
     }
-    double2 x = v[i], y = v[i + step];
-    if (KIND == kOpCnot) {
-      const double2 o = x;
-      x = y;
-      y = o;
-    } else if (KIND == kOpCry) {
+    double2 x = v[ix], y = v[iy];
+    if (DIR == kRotFwd) pair_signs(op, ix, iy, x, y);
+    if (KIND == kOpCry)
       cry_pair(op, x, y);
-    } else {
+    else
       rot_pair<DIR, KIND, RS>(op, x, y);
-    }
-    v[i] = x;
-    v[i + step] = y;
+    if (DIR != kRotFwd) pair_signs(op, ix, iy, x, y);
+    v[ix] = x;
+    v[iy] = y;
+  }
+}
+
+// A CZ by itself.
+__device__ __forceinline__ void cz_tile(double2* s, int N, int tc, unsigned cz0, unsigned cz1) {
+  for (int e = threadIdx.x; e < tc * N; e += blockDim.x) {
+    const unsigned p = e & (N - 1);
+    if (!(parity(p & cz0) & parity(p & cz1))) continue;
+    const double2 v = s[e];
+    s[e] = make_double2(dneg(v.x), dneg(v.y));
   }
 }
 
@@ -541,14 +658,13 @@ template <int DIR>
 __device__ __forceinline__ void rot_tile(double2* s, int N, int logN, int tc, const StagedOp& st) {
 #define SQG_ROT_CASE(KIND) \
   case (KIND): \
-    if (st.qubits & kStRescale) \
+    if (st.kind & kStRescale) \
       rot_tile_kind<DIR, (KIND), true>(s, N, logN, tc, st); \
     else \
       rot_tile_kind<DIR, (KIND), false>(s, N, logN, tc, st); \
     break;
-  switch (st.kind) {
-    case kOpCnot: rot_tile_kind<DIR, kOpCnot, false>(s, N, logN, tc, st); break;
-    case kOpCz: rot_tile_kind<DIR, kOpCz, false>(s, N, logN, tc, st); break;
+  switch (st.kind & 255) {
+    case kOpCz: cz_tile(s, N, tc, st.cz & 0xffffu, st.cz >> 16); break;
     case kOpCry: rot_tile_kind<DIR, kOpCry, false>(s, N, logN, tc, st); break;
     case kOpPhase: rot_tile_kind<DIR, kOpPhase, false>(s, N, logN, tc, st); break;
     SQG_ROT_CASE(kOpRot)
@@ -558,6 +674,22 @@ __device__ __forceinline__ void rot_tile(double2* s, int N, int logN, int tc, co
     SQG_ROT_CASE(kOpRot | kOpZi | kOpZo)
   }
 #undef SQG_ROT_CASE
+}
+
+// Table of places behind the last operation, kEndGroups groups of 16 entries: the amplitude with
+// index r is at the XOR over its hexadecimal digits d of table[16 g + d].  ends: RotPlan::ends or a
+// state block's.  All threads of the CTA; the caller synchronises.
+constexpr int kEndGroups = 4;
+__device__ __forceinline__ void fill_end_table(int* table, const int* ends, int logN) {
+  for (int e = threadIdx.x; e < 16 * kEndGroups; e += blockDim.x) {
+    int p = 0;
+    for (int q = 0; q < 4; q++)
+      if (((e >> q) & 1) && (e >> 4) * 4 + q < logN) p ^= ends[(e >> 4) * 4 + q];
+    table[e] = p;
+  }
+}
+__device__ __forceinline__ int end_place(const int* table, int r) {
+  return table[r & 15] ^ table[16 + ((r >> 4) & 15)] ^ table[32 + ((r >> 8) & 15)] ^ table[48 + ((r >> 12) & 15)];
 }
 
 }  // namespace sqg

@@ -86,6 +86,11 @@ __device__ __forceinline__ void undo_coeffs(int axis, double c, double s, double
   r[q] = fma(s, a, c * b);
 }
 
+// (cos, sin) of the double angle.
+__device__ __forceinline__ double2 twice(double2 a) {
+  return make_double2((a.x - a.y) * (a.x + a.y), 2.0 * a.x * a.y);
+}
+
 // Gradient components of the gates of one CTA's runs (kRotThreads threads, thread i for run i).
 // tr: the trace; gr: the summed overlaps.  The overlap along the axis that a run pushed is the
 // one that the next run of its chain has in front of its gates.
@@ -93,15 +98,18 @@ template <bool CPLX>
 __device__ __forceinline__ void rot_grad_body(const RotPlan& pl, int cta, const double* theta, const RotRec* recs,
                                               const double2* tr, const double* gr, int cols, int variant,
                                               double* grad) {
+  __shared__ double2 sc[kRotParams];
   __shared__ double2 V[kRotThreads][3];
   __shared__ double R[kRotThreads][3];
   const int base = pl.cta[cta], n = pl.cta[cta + 1] - base, i = threadIdx.x;
   const double2 T = tr[0];
+  cta_sincos(pl, cta, theta, sc);
+  __syncthreads();
   RotRun run;
   double2 wrot = make_double2(1.0, 0.0);
   if (i < n) {
     run = pl.runs[base + i];
-    if (run.push != kAxisNone) wrot = recs[run.op].zo;
+    if (run.push != kAxisNone) wrot = recs[run.rec].zo;
     double2 v[3];
     int pos = run.coff;
     for (int axis = 0; axis < 3; axis++) {
@@ -115,21 +123,20 @@ __device__ __forceinline__ void rot_grad_body(const RotPlan& pl, int cta, const 
     if (run.pulled) {  // <axis pulled> in front of the run from <P> behind it
       double r[3] = {0.0, 0.0, 0.0};
       r[pl.runs[base + i - 1].push - 1] = 1.0;
+      int soff = run.soff;
       for (int k = 0; k < run.count; k++) {
         const Gate g = pl.gates[pl.members[run.first + k]];
         const double* th = theta + g.pstart;
-        double s, c;
+        const double2 a = twice(param_sincos(sc, soff, th, 0));
         if (g.type == G_U3) {
-          sincos(th[2], &s, &c);
-          undo_coeffs(kAxisZ, c, s, r);
-          sincos(2.0 * th[0], &s, &c);
-          undo_coeffs(kAxisY, c, s, r);
-          sincos(th[1], &s, &c);
-          undo_coeffs(kAxisZ, c, s, r);
+          const double2 ph = param_sincos(sc, soff, th, 1), la = param_sincos(sc, soff, th, 2);
+          undo_coeffs(kAxisZ, la.x, la.y, r);
+          undo_coeffs(kAxisY, a.x, a.y, r);
+          undo_coeffs(kAxisZ, ph.x, ph.y, r);
         } else {
-          sincos(2.0 * th[0], &s, &c);
-          undo_coeffs(g.type == G_RX ? kAxisX : g.type == G_RY ? kAxisY : kAxisZ, c, s, r);
+          undo_coeffs(g.type == G_RX ? kAxisX : g.type == G_RY ? kAxisY : kAxisZ, a.x, a.y, r);
         }
+        if (soff >= 0) soff += gate_param_num(g.type);
       }
       if (run.push != kAxisNone) undo_coeffs(run.push, wrot.x, -wrot.y, r);
       for (int axis = 0; axis < 3; axis++) R[i][axis] = r[axis];
@@ -156,28 +163,29 @@ __device__ __forceinline__ void rot_grad_body(const RotPlan& pl, int cta, const 
   auto put = [&](int p, double2 dt) { grad[p] = grad_from_trace(variant, T, dt, cols); };
   auto minus_i = [](double2 a) { return make_double2(a.y, -a.x); };                       // d/dangle of e^{-i angle P}
   auto half_i = [&](double2 z) { return make_double2(-0.5 * (T.y - z.y), 0.5 * (T.x - z.x)); };  // of diag(1, e^{i angle})
+  int soff = run.soff;
+  for (int k = 0; soff >= 0 && k < run.count; k++) soff += gate_param_num(pl.gates[pl.members[run.first + k]].type);
   for (int k = run.count - 1; k >= 0; k--) {
     const Gate g = pl.gates[pl.members[run.first + k]];
     const double* th = theta + g.pstart;
-    double s, c;
+    if (soff >= 0) soff -= gate_param_num(g.type);
     if (g.type == G_U3) {
+      const double2 ph = param_sincos(sc, soff, th, 1), a = twice(param_sincos(sc, soff, th, 0));
       put(g.pstart + 1, half_i(v[2]));
-      sincos(th[1], &s, &c);
-      undo_rotation(kAxisZ, c, s, v);
+      undo_rotation(kAxisZ, ph.x, ph.y, v);
       put(g.pstart, minus_i(v[1]));
-      sincos(2.0 * th[0], &s, &c);
-      undo_rotation(kAxisY, c, s, v);
+      undo_rotation(kAxisY, a.x, a.y, v);
       put(g.pstart + 2, half_i(v[2]));
       if (k > 0) {
-        sincos(th[2], &s, &c);
-        undo_rotation(kAxisZ, c, s, v);
+        const double2 la = param_sincos(sc, soff, th, 2);
+        undo_rotation(kAxisZ, la.x, la.y, v);
       }
     } else {
       const int axis = g.type == G_RX ? kAxisX : g.type == G_RZ ? kAxisZ : kAxisY;
       put(g.pstart, minus_i(v[axis - 1]));
       if (k > 0) {
-        sincos(2.0 * th[0], &s, &c);
-        undo_rotation(axis, c, s, v);
+        const double2 a = twice(param_sincos(sc, soff, th, 0));
+        undo_rotation(axis, a.x, a.y, v);
       }
     }
   }

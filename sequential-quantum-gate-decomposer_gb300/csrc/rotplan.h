@@ -8,11 +8,16 @@
 
 namespace sqg {
 
+// An operation before its qubits become masks; its index is that of its numbers.
+struct RotStep {
+  int kind, target, control, coff, mask;
+  int anchor;  // gate whose place it takes (the last gate of its run)
+};
+
 struct RotPlanHost {
-  std::vector<RotOp> ops;
-  std::vector<int> anchor;  // gate whose place an operation takes (the last gate of its run)
+  std::vector<RotStep> steps;
   std::vector<RotRun> runs;
-  std::vector<int> members, cta;
+  std::vector<int> members, cta, params, cta_params;
   int noverlaps = 0;
 };
 
@@ -101,16 +106,15 @@ inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates) {
   std::vector<Item> items;
   std::vector<int> item_of(runs.size(), -1);
   auto add_op = [&](int kind, int target, int control, int mask, int anchor) {
-    RotOp op = {kind, target | (std::max(control, 0) << 8), pl.noverlaps, mask};
+    const RotStep st = {kind, target, control, pl.noverlaps, mask, anchor};
     for (int m = mask; m; m &= m - 1) pl.noverlaps++;
-    pl.ops.push_back(op);
-    pl.anchor.push_back(anchor);
-    return op;
+    pl.steps.push_back(st);
+    return st;
   };
   std::vector<std::vector<int>> item_members;
-  auto add_item = [&](const RotOp& op, const std::vector<int>& members, int push, bool pulled) {
-    items.push_back({{(int)pl.ops.size() - 1, 0, (int)members.size(), push, pulled ? 1 : 0, op.kind, op.coff, op.mask,
-                      members.size() == 1 && gates[members[0]].type == G_U3 ? 1 : 0},
+  auto add_item = [&](const RotStep& op, const std::vector<int>& members, int push, bool pulled) {
+    items.push_back({{(int)pl.steps.size() - 1, 0, (int)members.size(), push, pulled ? 1 : 0, op.kind, op.coff, op.mask,
+                      members.size() == 1 && gates[members[0]].type == G_U3 ? 1 : 0, -1},
                      -1});
     item_members.push_back(members);
     return (int)items.size() - 1;
@@ -119,7 +123,7 @@ inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates) {
     const Gate& gt = gates[g];
     if (gate_controlled(gt.type)) {
       const bool cry = gt.type == G_CRY;
-      const RotOp op = add_op(cry ? kOpCry : gt.type == G_CNOT ? kOpCnot : kOpCz, gt.target, gt.control, cry ? 2 : 0, g);
+      const RotStep op = add_op(cry ? kOpCry : gt.type == G_CNOT ? kOpCnot : kOpCz, gt.target, gt.control, cry ? 2 : 0, g);
       if (cry) add_item(op, {g}, kAxisNone, false);
       continue;
     }
@@ -142,22 +146,112 @@ inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates) {
   }
   for (size_t i = 0; i < runs.size(); i++)
     if (runs[i].next >= 0) items[item_of[i]].next = item_of[runs[i].next];
-  // chain order: every chain contiguous and within one CTA
+  // chain order: every chain contiguous and within one CTA, whose parameters are listed together
+  auto gate_params = [&](int j) {
+    int np = 0;
+    for (int g : item_members[j]) np += gate_param_num(gates[g].type);
+    return np;
+  };
   pl.cta.push_back(0);
+  pl.cta_params.push_back(0);
+  auto close_cta = [&]() {
+    pl.cta.push_back((int)pl.runs.size());
+    pl.cta_params.push_back((int)pl.params.size());
+  };
   for (size_t i = 0; i < items.size(); i++) {
     if (items[i].r.pulled) continue;
-    int len = 0;
-    for (int j = (int)i; j >= 0; j = items[j].next) len++;
-    if ((int)pl.runs.size() + len - pl.cta.back() > kRotThreads) pl.cta.push_back((int)pl.runs.size());
+    int len = 0, np = 0;
+    for (int j = (int)i; j >= 0; j = items[j].next) {
+      len++;
+      np += gate_params(j);
+    }
+    const bool listed = np <= kRotParams;  // else the chain's threads take them one by one
+    if ((int)pl.runs.size() + len - pl.cta.back() > kRotThreads ||
+        (listed && (int)pl.params.size() + np - pl.cta_params.back() > kRotParams))
+      close_cta();
     for (int j = (int)i; j >= 0; j = items[j].next) {
       RotRun r = items[j].r;
       r.first = (int)pl.members.size();
-      pl.members.insert(pl.members.end(), item_members[j].begin(), item_members[j].end());
+      r.soff = listed ? (int)pl.params.size() - pl.cta_params.back() : -1;
+      for (int g : item_members[j]) {
+        pl.members.push_back(g);
+        for (int k = 0; listed && k < gate_param_num(gates[g].type); k++) pl.params.push_back(gates[g].pstart + k);
+      }
       pl.runs.push_back(r);
     }
   }
-  if ((int)pl.runs.size() > pl.cta.back()) pl.cta.push_back((int)pl.runs.size());
+  if ((int)pl.runs.size() > pl.cta.back()) close_cta();
   return pl;
+}
+
+// Steps [k0, k1) as operations on n qubits, qubit q of a step being loc[q]; appended to ops.
+// ends receives n places (RotPlan::ends).
+inline void lower_rot_steps(const std::vector<RotStep>& steps, int k0, int k1, int n, const std::vector<int>& loc,
+                            std::vector<RotOp>& ops, std::vector<int>& ends) {
+  // qubit q of the amplitude at place p is the parity of p & row[q]; the amplitude with bit q
+  // changed is at p ^ pair[q].  A CNOT adds its control's row to its target's.
+  std::vector<unsigned> row(n), pair(n);
+  for (int q = 0; q < n; q++) row[q] = pair[q] = 1u << q;
+  struct Cz {
+    unsigned a, b;
+  };
+  std::vector<Cz> waiting;
+  auto odd = [](unsigned v) { return __builtin_popcount(v) & 1; };
+  auto emit_cz = [&](const Cz& z) {
+    RotOp op = {};
+    op.kind = kOpCz;
+    op.cz0 = (unsigned short)z.a;
+    op.cz1 = (unsigned short)z.b;
+    ops.push_back(op);
+  };
+  for (int k = k0; k < k1; k++) {
+    const RotStep& s = steps[k];
+    const int t = loc[s.target], c = s.control >= 0 ? loc[s.control] : -1;
+    if (s.kind == kOpCnot) {
+      row[t] ^= row[c];
+      pair[c] ^= pair[t];
+      continue;
+    }
+    if (s.kind == kOpCz) {
+      waiting.push_back({row[t], row[c]});
+      continue;
+    }
+    RotOp op = {};
+    op.kind = s.kind;
+    op.rec = k;
+    op.coff = s.coff;
+    op.mask = s.mask;
+    op.pair = (unsigned short)pair[t];
+    op.row = (unsigned short)row[t];
+    // the highest bit of the pair mask numbers the pairs: the lower ones then run through
+    // consecutive places, without bank conflicts
+    op.b0 = (unsigned short)(31 - __builtin_clz(pair[t]));
+    if (s.kind == kOpCry) {
+      op.crow = (unsigned short)row[c];
+      op.b1 = (unsigned short)(31 - __builtin_clz(row[c] & ~(1u << op.b0)));
+    }
+    if (s.kind != kOpPhase) {  // diagonal operations commute with every CZ
+      bool first = true;
+      for (size_t i = 0; i < waiting.size();) {
+        const Cz z = waiting[i];
+        if (!odd(z.a & pair[t]) && !odd(z.b & pair[t])) {
+          i++;
+          continue;
+        }
+        waiting.erase(waiting.begin() + i);
+        if (first && s.kind != kOpCry) {  // a CRY visits half of the places only
+          op.cz0 = (unsigned short)z.a;
+          op.cz1 = (unsigned short)z.b;
+          first = false;
+        } else {
+          emit_cz(z);
+        }
+      }
+    }
+    ops.push_back(op);
+  }
+  for (const Cz& z : waiting) emit_cz(z);
+  for (int q = 0; q < n; q++) ends.push_back((int)pair[q]);
 }
 
 }  // namespace sqg

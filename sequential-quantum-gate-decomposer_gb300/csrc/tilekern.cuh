@@ -10,8 +10,9 @@ namespace sqg {
 
 struct TileArgs {
   const RotOp* ops;     // operations of the circuit's plan
-  int nops, noverlaps, n, N;
-  const RotRec* recs;   // [B][nops]
+  const int* ends;      // RotPlan::ends
+  int nops, nrecs, noverlaps, n, N;
+  const RotRec* recs;   // [B][nrecs]
   const double2* phases;  // [B][nphase]: factors of the phase common to all amplitudes
   int nphase;
   // matrix source (target or in/out matrix); element (r, c) of instance b at
@@ -35,7 +36,8 @@ __device__ __forceinline__ double2 tile_phase(const TileArgs& a, int b) {
   return p;
 }
 
-__device__ __forceinline__ void load_tile(double2* s, const TileArgs& a, int b, int v0, int tc) {
+// ends: table of the places behind the last operation (fill_end_table).
+__device__ __forceinline__ void load_tile(double2* s, const TileArgs& a, int b, int v0, int tc, const int* ends) {
   const double2* base = a.mtx + (long long)b * a.bstride;
   const int total = a.N * tc;
   if (a.cstride == 1) {
@@ -47,27 +49,42 @@ __device__ __forceinline__ void load_tile(double2* s, const TileArgs& a, int b, 
   } else {
     // right application: vector = row (contiguous)
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int c = e / a.N, r = e - c * a.N;
-      s[c * a.N + r] = base[(long long)(v0 + c) * a.rstride + r];
+      int c = e >> a.n, r = e & (a.N - 1);
+      s[c * a.N + end_place(ends, r)] = base[(long long)(v0 + c) * a.rstride + r];
     }
   }
 }
 
 // Writes the tile back times the instance's common phase.
-__device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, int b, int v0, int tc, double2 phase) {
+__device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, int b, int v0, int tc, double2 phase,
+                                           const int* ends) {
   double2* base = a.mtx + (long long)b * a.bstride;
   const int total = a.N * tc;
   if (a.cstride == 1) {
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
       int r = e / tc, c = e - r * tc;
-      base[(long long)r * a.rstride + v0 + c] = cmul(phase, s[c * a.N + r]);
+      base[(long long)r * a.rstride + v0 + c] = cmul(phase, s[c * a.N + end_place(ends, r)]);
     }
   } else {
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int c = e / a.N, r = e - c * a.N;
+      int c = e >> a.n, r = e & (a.N - 1);
       base[(long long)(v0 + c) * a.rstride + r] = cmul(phase, s[c * a.N + r]);
     }
   }
+}
+
+// Complex trace partial sum_c s[c][place of v0 + c + offset], returned to all threads.
+__device__ __forceinline__ double2 tile_trace_at(const double2* s, int N, int tc, int first, const int* ends,
+                                                 double* scratch) {
+  double2 t = make_double2(0.0, 0.0);
+  for (int c = threadIdx.x; c < tc; c += blockDim.x) {
+    const double2 v = s[c * N + end_place(ends, first + c)];
+    t.x += v.x;
+    t.y += v.y;
+  }
+  t.x = block_allsum(t.x, scratch);
+  t.y = block_allsum(t.y, scratch);
+  return t;
 }
 
 // Operations are staged in shared memory kRotChunk at a time, so each CTA reads them from
@@ -81,10 +98,13 @@ __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int 
   double2* s = smem;
   double2* red = smem + (size_t)a.TC * a.N;
   StagedOp* st = reinterpret_cast<StagedOp*>(red + kTileMaxWarps);  // [kRotChunk]
+  __shared__ int ends[16 * kEndGroups];
   const int v0 = tile * a.TC;
   const int tc = min(a.TC, a.cols - v0);
-  load_tile(s, a, b, v0, tc);
-  const RotRec* recs = a.recs + (long long)b * a.nops;
+  fill_end_table(ends, a.ends, a.n);
+  if (DIR == kRotTrans) __syncthreads();
+  load_tile(s, a, b, v0, tc, ends);
+  const RotRec* recs = a.recs + (long long)b * a.nrecs;
   const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
   for (int q = 0; q < nchunks; q++) {
     const int k0 = (DIR == kRotFwd ? q : nchunks - 1 - q) * kRotChunk;
@@ -100,10 +120,10 @@ __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int 
   __syncthreads();
   const double2 phase = tile_phase(a, b);
   if (TRACE) {
-    double2 t = tile_trace(s, a.N, tc, v0, a.trace_offset, reinterpret_cast<double*>(red));
+    double2 t = tile_trace_at(s, a.N, tc, v0 + a.trace_offset, ends, reinterpret_cast<double*>(red));
     if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
   }
-  if (WRITE_BACK) store_tile(s, a, b, v0, tc, phase);
+  if (WRITE_BACK) store_tile(s, a, b, v0, tc, phase, ends);
 }
 
 // Adds the overlaps `mask` of one pair of psi (x, y) and lambda (lx, ly) to acc.  CPLX = false
@@ -143,19 +163,16 @@ template <bool CPLX, int KIND, int MASK, bool RS>
 __device__ __forceinline__ void adjoint_tile_kind(double2* psi, double2* lam, int N, int logN, int tc,
                                                   const StagedOp& staged, double (&acc)[CPLX ? 6 : 3]) {
   const DirOp op = directed<kRotAdj, KIND>(staged);
-  const int target = staged.qubits & 255, control = (staged.qubits >> 8) & 255;
-  constexpr bool ctrl = KIND == kOpCry;
-  const int lognp = ctrl ? logN - 2 : logN - 1;
+  const int lognp = KIND == kOpCry ? logN - 2 : logN - 1;
   const int npairs = 1 << lognp;
   const int items = tc << lognp;
-  const int step = 1 << target;
   for (int it = threadIdx.x; it < items; it += blockDim.x) {
     const int col = it >> lognp;
-    const int p = it & (npairs - 1);
-    const int i = ctrl ? pair_index2(p, target, control) : pair_index1(p, target);
     double2* ps = psi + col * N;
     double2* ls = lam + col * N;
-    double2 x = ps[i], y = ps[i + step], lx = ls[i], ly = ls[i + step];
+    int ix, iy;
+    pair_places<KIND>(op, it & (npairs - 1), ix, iy);
+    double2 x = ps[ix], y = ps[iy], lx = ls[ix], ly = ls[iy];
     measure_pair<CPLX, MASK>(x, y, lx, ly, acc);
     if (KIND == kOpPhase) {
       rot_phase(y, op.zix, op.ziy, op.nzi);
@@ -168,11 +185,13 @@ __device__ __forceinline__ void adjoint_tile_kind(double2* psi, double2* lam, in
         rot_pair<kRotAdj, KIND, RS>(op, x, y);
         rot_pair<kRotAdj, KIND, RS>(op, lx, ly);
       }
-      ps[i] = x;
-      ls[i] = lx;
+      pair_signs(op, ix, iy, x, y);
+      pair_signs(op, ix, iy, lx, ly);
+      ps[ix] = x;
+      ls[ix] = lx;
     }
-    ps[i + step] = y;
-    ls[i + step] = ly;
+    ps[iy] = y;
+    ls[iy] = ly;
   }
 }
 
@@ -182,12 +201,12 @@ __device__ __forceinline__ void adjoint_tile(double2* psi, double2* lam, int N, 
                                              double (&acc)[CPLX ? 6 : 3]) {
 #define SQG_ROT_CASE(KIND, MASK) \
   case (KIND) | (MASK) << 8: \
-    if (st.qubits & kStRescale) \
+    if (st.kind & kStRescale) \
       adjoint_tile_kind<CPLX, (KIND), (MASK), true>(psi, lam, N, logN, tc, st, acc); \
     else \
       adjoint_tile_kind<CPLX, (KIND), (MASK), false>(psi, lam, N, logN, tc, st, acc); \
     break;
-  switch (st.kind | st.mask << 8) {
+  switch (st.kind & 0xffff) {
     case kOpCry | 2 << 8: adjoint_tile_kind<CPLX, kOpCry, 2, false>(psi, lam, N, logN, tc, st, acc); break;
     case kOpPhase | 4 << 8: adjoint_tile_kind<CPLX, kOpPhase, 4, false>(psi, lam, N, logN, tc, st, acc); break;
     SQG_ROT_CASE(kOpRot, 2)
@@ -233,16 +252,17 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   const int tc = min(a.TC, a.cols - v0);
   const size_t tile_elems = (size_t)a.TC * N;
   double2* ck = a.ckpt ? a.ckpt + ((long long)b * a.tiles + tile) * a.nck * tile_elems : nullptr;
-  const RotRec* recs = a.recs + (long long)b * a.nops;
+  const RotRec* recs = a.recs + (long long)b * a.nrecs;
   const double2 phase = tile_phase(a, b);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 
-  load_tile(psi, a, b, v0, tc);
+  __shared__ int ends[16 * kEndGroups];
+  fill_end_table(ends, a.ends, logN);
+  load_tile(psi, a, b, v0, tc, ends);
+  for (int e = threadIdx.x; e < tc * N; e += blockDim.x) lam[e] = make_double2(0.0, 0.0);
+  __syncthreads();
   // <lambda| carries the common phase: lambda_j = conj(phase) e_{j + offset}
-  for (int e = threadIdx.x; e < tc * N; e += blockDim.x) {
-    int c = e / N, r = e - c * N;
-    lam[e] = r == v0 + c + a.trace_offset ? cconj(phase) : make_double2(0.0, 0.0);
-  }
+  for (int c = threadIdx.x; c < tc; c += blockDim.x) lam[c * N + end_place(ends, v0 + c + a.trace_offset)] = cconj(phase);
   // forward sweep, storing psi after every ckpt_interval-th operation
   const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
   for (int q = 0; q < nchunks; q++) {
@@ -261,7 +281,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
     }
   }
   __syncthreads();
-  double2 t = tile_trace(psi, N, tc, v0, a.trace_offset, redd);
+  double2 t = tile_trace_at(psi, N, tc, v0 + a.trace_offset, ends, redd);
   if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
 
   // reverse sweep.  The warps' totals of an operation are summed and written by the last warp
@@ -309,8 +329,8 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
         for (int e = threadIdx.x; e < tc * N; e += blockDim.x) psi[e] = cscale(src[e], f);
         __syncthreads();
       }
-      const int mask = st[j].mask;
-      if (mask == 0) {  // CNOT, CZ
+      const int kind = st[j].kind & 255, mask = (st[j].kind >> 8) & 255;
+      if (mask == 0) {  // a CZ by itself
         rot_tile<kRotAdj>(psi, N, logN, tc, st[j]);
         rot_tile<kRotAdj>(lam, N, logN, tc, st[j]);
         __syncthreads();
@@ -320,7 +340,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
 #pragma unroll
       for (int r = 0; r < (CPLX ? 6 : 3); r++) acc[r] = 0.0;
       adjoint_tile<CPLX>(psi, lam, N, logN, tc, st[j], acc);
-      const int items = tc << (st[j].kind == kOpCry ? logN - 2 : logN - 1);
+      const int items = tc << (kind == kOpCry ? logN - 2 : logN - 1);
       const int aw = min(nw, (items + 31) >> 5);  // warps holding pairs
       if (warp < aw) {
         double* rd = redd + buf * kTileMaxWarps * 8;
