@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   for (int k0 = a.k0; k0 < a.k1; k0 += kRotChunk) {
     const int kn = min(kRotChunk, a.k1 - k0);
     __syncthreads();
-    stage_ops(st, a.lops, recs, k0, kn);
+    stage_ops<true, kRotGroup>(st, a.lops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
       rot_tile<kRotFwd>(sv, KK, a.K, 1, st[j]);
@@ -819,6 +819,7 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   a.ckpt = l.nck > 0 ? (double2*)(ws + l.ck_off) : nullptr;
   a.ckpt_interval = checkpoint_interval;
   a.nck = l.nck;
+  a.fixed = 1;
   const dim3 grid(l.plan.tiles, B);
   if (!with_grad) {
     if ((st = set_smem(k_tile_forward<false, true, kRotFwd>, l.plan.smem))) return st;

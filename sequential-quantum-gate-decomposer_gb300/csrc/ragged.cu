@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kRaggedThreads) k_ragged_tiles(const InstDesc*
     a.ckpt = nullptr;
     a.ckpt_interval = 0;
     a.nck = 0;
+    a.fixed = 1;
     if constexpr (MODE == 0)
       tile_forward_body<false, true, kRotFwd>(a, 0, it.y, smem);
     else

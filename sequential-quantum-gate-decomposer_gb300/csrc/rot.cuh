@@ -7,8 +7,8 @@
 //    them, is one 2x2 unitary M.
 //  * M = scalar * diag(1, zo) * R * diag(1, zi) with R a rotation.  R is applied without its
 //    cosine ([[1, -t], [t, 1]], |t| <= 1 after an exchange of the two rows where needed):
-//    4 multiply-adds per pair instead of 8.  The cosines of up to kRotChunk consecutive
-//    operations are multiplied in with the first of them, so the scale stays in [2^-16, 1].
+//    4 multiply-adds per pair instead of 8.  The cosines of a group of consecutive operations are
+//    multiplied in with the first of them, so the scale never exceeds 1.
 //    A phase diag(1, z) touches one row of the pair: 4 instructions.
 //  * The rotation that M ends with is moved through the next two-qubit gate into the next run
 //    on the qubit where it commutes with that gate: Z through a control or a CZ, X through a
@@ -90,7 +90,11 @@ struct RotPlan {
 constexpr int kRotThreads = 128;  // runs per CTA of the per-instance kernels; no chain straddles two
 constexpr int kRotParams = 512;  // parameters listed per CTA
 constexpr int kRotChain = 16;     // runs linked by pushed rotations (their numbers are made one after another)
-constexpr int kRotChunk = 32;     // operations staged in shared memory together
+constexpr int kRotChunk = 32;     // operations staged in shared memory together (a warp)
+// Operations whose cosines are multiplied in together.  In FP64 the scale costs no precision, so
+// the whole chunk; in fixed point the overlaps lose the square of it (2^-8 at worst), at 4
+// more products per group: 16 a group costs 3 % of a gradient against 32, 8 costs 6 %.
+constexpr int kRotGroup = kRotChunk, kFxGroup = 16;
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
@@ -384,14 +388,18 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
   // the cosines of all runs at once: the chains need not wait for them
   if (i < n) {
     const RotRun mine = pl.runs[base + i];
+    RotRec& r = recs[mine.rec];
+    RotRec v = r;
     if (mine.kind & kOpRot) {
-      RotRec& r = recs[mine.rec];
-      RotRec v = r;
       set_cosine(v);
       r.c = v.c;
       r.lo = v.lo;
     }
+    // a NaN anywhere (an infinite angle, say) is one of the phase too: sweeps in fixed point look
+    // for it there
+    ph[i].x = fma(0.0, v.t + v.c + v.zi.x + v.zi.y + v.zo.x + v.zo.y, ph[i].x);
   }
+  __syncthreads();
   for (int o = kRotThreads / 2; o > 0; o >>= 1) {
     if (i < o) ph[i] = cmul(ph[i], ph[i + o]);
     __syncthreads();
@@ -400,9 +408,9 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
 }
 
 // ---- application ---------------------------------------------------------------------------
-// Operation staged for the sweeps.  scale: of the operation that multiplies the chunk's cosines
-// in (kStRescale; t includes it), the cosine of a kOpCry.  mfac: what the overlaps measured
-// behind the operation, with both vectors on the way back, are multiplied by.
+// Operation staged for the sweeps.  scale: the product of its group's cosines, multiplied in by the
+// operation with kStRescale (its t includes it).  zi.x of a kOpCry: its cosine.  mfac: what the
+// overlaps measured behind the operation, with both vectors on the way back, are multiplied by.
 struct StagedOp {
   int kind, coff;  // kind | mask << 8 | flags
   unsigned pair_row, crow_bits, cz;  // pair | row << 16, crow | b0 << 16 | b1 << 24, cz0 | cz1 << 16
@@ -410,12 +418,14 @@ struct StagedOp {
   double t, scale, mfac;
   double2 zi, zo;
 };
-enum : int { kStTurn = 1 << 16, kStRescale = 1 << 17 };
+// kStInside: from the group's first rotation to before its last.
+enum : int { kStTurn = 1 << 16, kStRescale = 1 << 17, kStInside = 1 << 18 };
 
 // Loads operations [k0, k0 + kn) (at most kRotChunk) into st with the first warp of the CTA.
-// The cosines that the chunk's rotations leave out are multiplied in by its first rotation: from
-// there the scale rises back to 1, and amplitudes never exceed what they were.
-// The caller synchronises before and after.
+// The cosines that a group's rotations leave out are multiplied in by the first rotation in the
+// direction of travel (FWD: the group's first, else its last): from there the scale rises back to
+// 1, and amplitudes never exceed what they were.  The caller synchronises before and after.
+template <bool FWD, int GROUP>
 __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
@@ -427,32 +437,35 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
     if (op.kind >= kOpCry) r = recs[op.rec];
   }
   const bool rot = (op.kind & kOpRot) != 0;
-  // product of the cosines up to and including this operation, as pre + plo
+  // product of the cosines of the group up to and including this operation, as pre + plo
+  const int in_group = lane & (GROUP - 1), base = lane - in_group;
   double pre = rot ? r.c : 1.0, plo = rot ? r.lo : 0.0;
-  for (int o = 1; o < 32; o <<= 1) {
+  for (int o = 1; o < GROUP; o <<= 1) {
     const double v = __shfl_up_sync(0xffffffffu, pre, o), vlo = __shfl_up_sync(0xffffffffu, plo, o);
-    if (lane >= o) {
+    if (in_group >= o) {
       const double p = pre * v;
       plo = fma(pre, v, -p) + fma(pre, vlo, plo * v);
       pre = p;
     }
   }
-  const double all = __shfl_sync(0xffffffffu, pre + plo, 31);
-  const unsigned rots = __ballot_sync(0xffffffffu, rot);
-  const int first = rots ? __ffs(rots) - 1 : 32;
+  const double all = __shfl_sync(0xffffffffu, pre + plo, base + GROUP - 1);
+  const unsigned rots = (__ballot_sync(0xffffffffu, rot) >> base) & (0xffffffffu >> (32 - GROUP));
+  const int first = rots ? base + __ffs(rots) - 1 : 32, last = rots ? base + 31 - __clz(rots) : 32;
+  const bool rescale = lane == (FWD ? first : last);
   if (on) {
     StagedOp s;
-    s.kind = op.kind | op.mask << 8 | (r.turn ? kStTurn : 0) | (lane == first ? kStRescale : 0);
+    s.kind = op.kind | op.mask << 8 | (r.turn ? kStTurn : 0) | (rescale ? kStRescale : 0) |
+             (lane >= first && lane < last ? kStInside : 0);
     s.coff = op.coff;
     s.pair_row = op.pair | (unsigned)op.row << 16;
     s.crow_bits = op.crow | (unsigned)op.b0 << 16 | (unsigned)op.b1 << 24;
     s.cz = op.cz0 | (unsigned)op.cz1 << 16;
     s.pad = 0;
-    s.scale = lane == first ? all : op.kind == kOpCry ? r.c : 1.0;
-    s.t = lane == first ? r.t * all : r.t;
-    const double inv = all / (pre + plo);
-    s.mfac = lane >= first ? inv * inv : 1.0;
-    s.zi = r.zi;
+    s.scale = all;
+    s.t = rescale ? r.t * all : r.t;
+    const double inv = 1.0 / (pre + plo);
+    s.mfac = lane < last ? inv * inv : 1.0;
+    s.zi = op.kind == kOpCry ? make_double2(r.c, 0.0) : r.zi;
     s.zo = r.zo;
     st[lane] = s;
   }
@@ -474,8 +487,6 @@ struct DirOp {
   double zix, ziy, nzi, zox, zoy, nzo;
   unsigned flip;  // sign bit for a turned Ry without a zi that could hold its sign
   bool turn;
-  unsigned pair, row, crow, cz0, cz1;
-  int b0, b1;
 };
 
 template <int DIR, int KIND>
@@ -498,6 +509,16 @@ __device__ __forceinline__ DirOp directed(const StagedOp& s) {
   o.nzo = DIR == kRotAdj ? zo : nzo;
   o.turn = (s.kind & kStTurn) != 0;
   o.flip = o.turn ? sign : 0u;
+  return o;
+}
+
+// Where a staged operation finds its pairs, as in RotOp.
+struct OpPlaces {
+  unsigned pair, row, crow, cz0, cz1;
+  int b0, b1;
+};
+__device__ __forceinline__ OpPlaces op_places(const StagedOp& s) {
+  OpPlaces o;
   o.pair = s.pair_row & 0xffffu;
   o.row = s.pair_row >> 16;
   o.crow = s.crow_bits & 0xffffu;
@@ -512,7 +533,7 @@ __device__ __forceinline__ unsigned parity(unsigned v) { return __popc(v) & 1u; 
 
 // Places of pair q of an operation: x with its target bit 0, y with 1 (kOpCry: control bit 1).
 template <int KIND>
-__device__ __forceinline__ void pair_places(const DirOp& op, int q, int& ix, int& iy) {
+__device__ __forceinline__ void pair_places(const OpPlaces& op, int q, int& ix, int& iy) {
   unsigned p;
   if (KIND == kOpCry) {
     const int lo = min(op.b0, op.b1), hi = max(op.b0, op.b1);
@@ -528,7 +549,7 @@ __device__ __forceinline__ void pair_places(const DirOp& op, int q, int& ix, int
 }
 
 // Signs of the CZ that rides on an operation.
-__device__ __forceinline__ void pair_signs(const DirOp& op, int ix, int iy, double2& x, double2& y) {
+__device__ __forceinline__ void pair_signs(const OpPlaces& op, int ix, int iy, double2& x, double2& y) {
   if (op.cz0) {
     const unsigned fx = (parity(ix & op.cz0) & parity(ix & op.cz1)) << 31;
     const unsigned fy = (parity(iy & op.cz0) & parity(iy & op.cz1)) << 31;
@@ -603,15 +624,9 @@ __device__ __forceinline__ void rot_pair(const DirOp& op, double2& x, double2& y
   }
 }
 
-// Controlled Ry on a pair with its control bit set: [[c, ns], [s, c]].
+// Controlled Ry on a pair with its control bit set: [[c, nt], [t, c]], t its sine.
 __device__ __forceinline__ void cry_pair(const DirOp& op, double2& x, double2& y) {
-  double2 nx, ny;
-  nx.x = fma(op.scale, x.x, op.nt * y.x);
-  nx.y = fma(op.scale, x.y, op.nt * y.y);
-  ny.x = fma(op.t, x.x, op.scale * y.x);
-  ny.y = fma(op.t, x.y, op.scale * y.y);
-  x = nx;
-  y = ny;
+  rot_turnless<false, true>(x, y, op.t, op.nt, op.zix);
 }
 
 // Applies one staged operation to every vector of a tile: tc vectors of length N = 2^logN, one
@@ -619,13 +634,14 @@ __device__ __forceinline__ void cry_pair(const DirOp& op, double2& x, double2& y
 template <int DIR, int KIND, bool RS>
 __device__ __forceinline__ void rot_tile_kind(double2* s, int N, int logN, int tc, const StagedOp& staged) {
   const DirOp op = directed<DIR, KIND>(staged);
+  const OpPlaces pl = op_places(staged);
   const int lognp = KIND == kOpCry ? logN - 2 : logN - 1;
   const int npairs = 1 << lognp;
   const int items = tc << lognp;
   for (int it = threadIdx.x; it < items; it += blockDim.x) {
     double2* v = s + (it >> lognp) * N;
     int ix, iy;
-    pair_places<KIND>(op, it & (npairs - 1), ix, iy);
+    pair_places<KIND>(pl, it & (npairs - 1), ix, iy);
     if (KIND == kOpPhase) {  // the target = 0 row is not touched
       double2 y = v[iy];
       rot_phase(y, op.zix, op.ziy, op.nzi);
@@ -633,12 +649,12 @@ __device__ __forceinline__ void rot_tile_kind(double2* s, int N, int logN, int t
       continue;
     }
     double2 x = v[ix], y = v[iy];
-    if (DIR == kRotFwd) pair_signs(op, ix, iy, x, y);
+    if (DIR == kRotFwd) pair_signs(pl, ix, iy, x, y);
     if (KIND == kOpCry)
       cry_pair(op, x, y);
     else
       rot_pair<DIR, KIND, RS>(op, x, y);
-    if (DIR != kRotFwd) pair_signs(op, ix, iy, x, y);
+    if (DIR != kRotFwd) pair_signs(pl, ix, iy, x, y);
     v[ix] = x;
     v[iy] = y;
   }

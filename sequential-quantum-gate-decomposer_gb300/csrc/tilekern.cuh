@@ -2,6 +2,7 @@
 // persistent ragged-batch launch (ragged.cu).  Each body processes one (instance, tile)
 // work item with all threads of the CTA; smem holds the tile(s) plus reduction scratch.
 #pragma once
+#include "fx.cuh"
 #include "gates.cuh"
 #include "rot.cuh"
 #include "tile.cuh"
@@ -28,6 +29,7 @@ struct TileArgs {
   double2* ckpt;     // checkpoints [B][tiles][nck][TC][N] or null
   int ckpt_interval;  // in operations
   int nck;
+  int fixed;         // cost and gradient: sweep finite tiles in fixed point
 };
 
 __device__ __forceinline__ double2 tile_phase(const TileArgs& a, int b) {
@@ -73,54 +75,126 @@ __device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, 
   }
 }
 
-// Complex trace partial sum_c s[c][place of v0 + c + offset], returned to all threads.
+// Operations are staged in shared memory kRotChunk at a time, so each CTA reads them from
+// global memory once instead of once per warp and operation.
+constexpr size_t kStageBytes = kRotChunk * sizeof(StagedOp);
+
+// Turns a tile of tc vectors of N doubles into fixed point in place (Fx2): |amplitude| <= 2^62 under
+// the power of two that the largest of the vectors' norms allows.  Returns false, and leaves the
+// tile, if it holds an infinity or NaN.  unit: what a result / 2^62 is multiplied by, as two
+// factors.  All threads; scratch: kTileMaxWarps doubles.
+struct FxUnit {
+  double a, b;
+};
+__device__ __forceinline__ bool fx_from_tile(double2* s, int N, int tc, double* scratch, FxUnit& unit) {
+  const int total = tc * N, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  int top = 0;  // largest upper word without its sign
+  __syncthreads();
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    const double2 v = s[e];
+    top = max(top, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
+  }
+  for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  int* tops = reinterpret_cast<int*>(scratch);
+  if (lane == 0) tops[warp] = top;
+  __syncthreads();
+  for (int w = 0; w < nw; w++) top = max(top, tops[w]);
+  __syncthreads();
+  if (top >= 0x7ff00000) return false;
+  // every component is below 2^(e0 + 1); zeros and denormals count as 2^-1023
+  const int e0 = top < 0x00100000 ? -1023 : (top >> 20) - 1023;
+  auto pow2 = [](int k) { return __hiloint2double((1023 + k) << 20, 0); };
+  // 2^-e0 in two factors: e0 spans the whole exponent range
+  const int h0 = -e0 / 2, h1 = -e0 - h0;
+  const double f0 = pow2(h0), f1 = pow2(h1);
+  double norm2 = 0.0;  // the largest of this warp's vectors
+  for (int c = warp; c < tc; c += nw) {
+    double q = 0.0;
+    for (int r = lane; r < N; r += 32) {
+      const double2 v = s[c * N + r];
+      const double x = v.x * f0 * f1, y = v.y * f0 * f1;
+      q = fma(x, x, fma(y, y, q));
+    }
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    norm2 = fmax(norm2, q);
+  }
+  if (lane == 0) scratch[warp] = norm2;
+  __syncthreads();
+  for (int w = 0; w < nw; w++) norm2 = fmax(norm2, scratch[w]);
+  // norm < 2^e1
+  const int e1 = norm2 >= 1.0 ? ((__double2hiint(norm2) >> 20) - 1023) / 2 + 1 : 1;
+  const double f2 = pow2(kFxBits - e1);
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    const double2 v = s[e];
+    Fx2 w;
+    w.x = __double2ll_rn(v.x * f0 * f1 * f2);
+    w.y = __double2ll_rn(v.y * f0 * f1 * f2);
+    reinterpret_cast<Fx2*>(s)[e] = w;
+  }
+  __syncthreads();
+  unit.a = pow2(-h0);
+  unit.b = pow2(e1 - h1);
+  return true;
+}
+
+// Complex trace partial sum_c s[c][place of first + c], returned to all threads.
 __device__ __forceinline__ double2 tile_trace_at(const double2* s, int N, int tc, int first, const int* ends,
-                                                 double* scratch) {
+                                                 double* scratch, bool fixed, const FxUnit& unit) {
   double2 t = make_double2(0.0, 0.0);
   for (int c = threadIdx.x; c < tc; c += blockDim.x) {
-    const double2 v = s[c * N + end_place(ends, first + c)];
+    double2 v = s[c * N + end_place(ends, first + c)];
+    if (fixed)
+      v = make_double2((double)__double_as_longlong(v.x) * 0x1p-62, (double)__double_as_longlong(v.y) * 0x1p-62);
     t.x += v.x;
     t.y += v.y;
   }
   t.x = block_allsum(t.x, scratch);
   t.y = block_allsum(t.y, scratch);
+  if (fixed) t = make_double2(t.x * unit.a * unit.b, t.y * unit.a * unit.b);
   return t;
 }
 
-// Operations are staged in shared memory kRotChunk at a time, so each CTA reads them from
-// global memory once instead of once per warp and operation.
-constexpr size_t kStageBytes = kRotChunk * sizeof(StagedOp);
-
 // Application of the whole circuit to one tile (DIR kRotFwd: from the left; kRotTrans: to the
 // rows, from the right); optionally writes the tile back and/or the traced diagonal partial.
+// Without write-back (cost only) the sweep runs in fixed point.
 template <bool WRITE_BACK, bool TRACE, int DIR>
 __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int tile, double2* smem) {
   double2* s = smem;
-  double2* red = smem + (size_t)a.TC * a.N;
-  StagedOp* st = reinterpret_cast<StagedOp*>(red + kTileMaxWarps);  // [kRotChunk]
+  double* red = reinterpret_cast<double*>(smem + (size_t)a.TC * a.N);
+  StagedOp* st = reinterpret_cast<StagedOp*>(red + 2 * kTileMaxWarps);  // [kRotChunk]
   __shared__ int ends[16 * kEndGroups];
   const int v0 = tile * a.TC;
   const int tc = min(a.TC, a.cols - v0);
+  const double2 phase = tile_phase(a, b);
   fill_end_table(ends, a.ends, a.n);
   if (DIR == kRotTrans) __syncthreads();
   load_tile(s, a, b, v0, tc, ends);
+  bool fixed = false;
+  FxUnit unit;
+  if (!WRITE_BACK && a.fixed && isfinite(phase.x) && isfinite(phase.y))
+    fixed = fx_from_tile(s, a.N, tc, red, unit);
   const RotRec* recs = a.recs + (long long)b * a.nrecs;
   const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
   for (int q = 0; q < nchunks; q++) {
     const int k0 = (DIR == kRotFwd ? q : nchunks - 1 - q) * kRotChunk;
     const int kn = min(kRotChunk, a.nops - k0);
     __syncthreads();  // the previous chunk's operations are no longer read
-    stage_ops(st, a.ops, recs, k0, kn);
+    if (!WRITE_BACK && fixed)
+      fx_stage_ops<true>(st, a.ops, recs, k0, kn);
+    else
+      stage_ops<DIR == kRotFwd, kRotGroup>(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
-      rot_tile<DIR>(s, a.N, a.n, tc, st[DIR == kRotFwd ? j : kn - 1 - j]);
+      if (!WRITE_BACK && fixed)
+        fx_tile(reinterpret_cast<Fx2*>(s), a.N, a.n, tc, st[j]);
+      else
+        rot_tile<DIR>(s, a.N, a.n, tc, st[DIR == kRotFwd ? j : kn - 1 - j]);
       __syncthreads();
     }
   }
   __syncthreads();
-  const double2 phase = tile_phase(a, b);
   if (TRACE) {
-    double2 t = tile_trace_at(s, a.N, tc, v0 + a.trace_offset, ends, reinterpret_cast<double*>(red));
+    const double2 t = tile_trace_at(s, a.N, tc, v0 + a.trace_offset, ends, red, fixed, unit);
     if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
   }
   if (WRITE_BACK) store_tile(s, a, b, v0, tc, phase, ends);
@@ -163,6 +237,7 @@ template <bool CPLX, int KIND, int MASK, bool RS>
 __device__ __forceinline__ void adjoint_tile_kind(double2* psi, double2* lam, int N, int logN, int tc,
                                                   const StagedOp& staged, double (&acc)[CPLX ? 6 : 3]) {
   const DirOp op = directed<kRotAdj, KIND>(staged);
+  const OpPlaces pl = op_places(staged);
   const int lognp = KIND == kOpCry ? logN - 2 : logN - 1;
   const int npairs = 1 << lognp;
   const int items = tc << lognp;
@@ -171,7 +246,7 @@ __device__ __forceinline__ void adjoint_tile_kind(double2* psi, double2* lam, in
     double2* ps = psi + col * N;
     double2* ls = lam + col * N;
     int ix, iy;
-    pair_places<KIND>(op, it & (npairs - 1), ix, iy);
+    pair_places<KIND>(pl, it & (npairs - 1), ix, iy);
     double2 x = ps[ix], y = ps[iy], lx = ls[ix], ly = ls[iy];
     measure_pair<CPLX, MASK>(x, y, lx, ly, acc);
     if (KIND == kOpPhase) {
@@ -185,8 +260,8 @@ __device__ __forceinline__ void adjoint_tile_kind(double2* psi, double2* lam, in
         rot_pair<kRotAdj, KIND, RS>(op, x, y);
         rot_pair<kRotAdj, KIND, RS>(op, lx, ly);
       }
-      pair_signs(op, ix, iy, x, y);
-      pair_signs(op, ix, iy, lx, ly);
+      pair_signs(pl, ix, iy, x, y);
+      pair_signs(pl, ix, iy, lx, ly);
       ps[ix] = x;
       ls[ix] = lx;
     }
@@ -238,11 +313,13 @@ __device__ __forceinline__ double warp_reduce_scatter4(double r0, double r1, dou
 
 // Cost trace and overlaps of one (instance, tile): forward sweep, then the adjoint sweep
 // psi <- G^dagger psi, lambda <- G^dagger lambda with lambda starting at e_{j + offset}.
-// Bound by FP64 instructions: a U3 run of a CNOT circuit costs 8 per pair forward and
-// 16 + 6 or 8 on the way back (a U3 by itself: 14, 28 and 16 with the gates as given).
+// A U3 run of a CNOT circuit takes 8 products per pair forward and 16 + 6 or 8 on the way back (a
+// U3 by itself: 14, 28 and 16 with the gates as given); in fixed point (fx.cuh) unless the tile
+// holds infinities or NaN or checkpoints are kept.
 template <bool CPLX>
 __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int tile, double2* smem) {
   constexpr int NV = CPLX ? 8 : 4;  // reduced values per operation (the last ones unused)
+  constexpr int NA = CPLX ? 6 : 3;
   const int N = a.N, logN = a.n;
   double2* psi = smem;
   double2* lam = smem + (size_t)a.TC * N;
@@ -260,18 +337,35 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   fill_end_table(ends, a.ends, logN);
   load_tile(psi, a, b, v0, tc, ends);
   for (int e = threadIdx.x; e < tc * N; e += blockDim.x) lam[e] = make_double2(0.0, 0.0);
+  bool fixed = false;
+  FxUnit unit;
+  if (!ck && a.fixed && (tc <= kFxItems || tc * (N / 2) <= kFxItems * (int)blockDim.x) &&
+      isfinite(phase.x) && isfinite(phase.y))
+    fixed = fx_from_tile(psi, N, tc, redd, unit);
   __syncthreads();
   // <lambda| carries the common phase: lambda_j = conj(phase) e_{j + offset}
-  for (int c = threadIdx.x; c < tc; c += blockDim.x) lam[c * N + end_place(ends, v0 + c + a.trace_offset)] = cconj(phase);
+  for (int c = threadIdx.x; c < tc; c += blockDim.x) {
+    double2 v = cconj(phase);
+    if (fixed)
+      v = make_double2(__longlong_as_double(__double2ll_rn(v.x * 0x1p62)),
+                       __longlong_as_double(__double2ll_rn(v.y * 0x1p62)));
+    lam[c * N + end_place(ends, v0 + c + a.trace_offset)] = v;
+  }
   // forward sweep, storing psi after every ckpt_interval-th operation
   const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
   for (int q = 0; q < nchunks; q++) {
     const int k0 = q * kRotChunk, kn = min(kRotChunk, a.nops - k0);
     __syncthreads();
-    stage_ops(st, a.ops, recs, k0, kn);
+    if (fixed)
+      fx_stage_ops<true>(st, a.ops, recs, k0, kn);
+    else
+      stage_ops<true, kRotGroup>(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
-      rot_tile<kRotFwd>(psi, N, logN, tc, st[j]);
+      if (fixed)
+        fx_tile(reinterpret_cast<Fx2*>(psi), N, logN, tc, st[j]);
+      else
+        rot_tile<kRotFwd>(psi, N, logN, tc, st[j]);
       __syncthreads();
       if (ck && (k0 + j + 1) % a.ckpt_interval == 0 && (k0 + j + 1) / a.ckpt_interval <= a.nck) {
         double2* dst = ck + (size_t)((k0 + j + 1) / a.ckpt_interval - 1) * tile_elems;
@@ -281,76 +375,104 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
     }
   }
   __syncthreads();
-  double2 t = tile_trace_at(psi, N, tc, v0 + a.trace_offset, ends, redd);
+  double2 t = tile_trace_at(psi, N, tc, v0 + a.trace_offset, ends, redd, fixed, unit);
   if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
+  __syncthreads();
 
   // reverse sweep.  The warps' totals of an operation are summed and written by the last warp
   // while the next operation runs: redd alternates between two halves, one barrier per operation.
   double* wgr = a.ws_gr + ((long long)b * a.tiles + tile) * a.noverlaps * (CPLX ? 2 : 1);
   int pend_coff = 0, pend_mask = 0, pend_aw = 0, buf = 0;
   double pend_fac = 0.0;
+  const int shift = fx_sum_shift(tc);
+  const double fx_unit = 0x1p-60 * (double)(1 << shift);
   auto flush = [&]() {  // one thread per measured overlap
     if (!pend_mask || warp != nw - 1 || lane >= 3) return;
     const int axis = lane;  // 0 X, 1 Y, 2 Z
     if (!((pend_mask >> axis) & 1)) return;
     const double* rd = redd + (buf ^ 1) * kTileMaxWarps * 8;
     const int pos = pend_coff + __popc(pend_mask & ((1 << axis) - 1));
-    if (!CPLX) {
-      double v = 0.0;
-      for (int w = 0; w < pend_aw; w++) v += rd[w * NV + axis];
-      wgr[pos] = v * pend_fac;
-    } else {
-      double o[6];
-      for (int k = 0; k < 6; k++) {
-        o[k] = 0.0;
-        for (int w = 0; w < pend_aw; w++) o[k] += rd[w * NV + k];
-        o[k] *= pend_fac;
+    auto total = [&](int k) {
+      if (fixed) {
+        long long v = 0;
+        for (int w = 0; w < pend_aw; w++) v += __double_as_longlong(rd[w * NV + k]);
+        return (double)v * fx_unit * unit.a * unit.b * pend_fac;
       }
+      double v = 0.0;
+      for (int w = 0; w < pend_aw; w++) v += rd[w * NV + k];
+      return v * pend_fac;
+    };
+    if (!CPLX) {
+      wgr[pos] = total(axis);
+    } else {
       double2 v;
-      if (axis == 2) v = make_double2(o[0], o[1]);                       // <lambda_0|psi_0>
-      else if (axis == 0) v = make_double2(o[2] + o[4], o[3] + o[5]);     // <X>
-      else v = make_double2(-(o[5] - o[3]), o[4] - o[2]);                 // <Y> = i (m10 - m01)
+      if (axis == 2) v = make_double2(total(0), total(1));                           // <lambda_0|psi_0>
+      else if (axis == 0) v = make_double2(total(2) + total(4), total(3) + total(5));  // <X>
+      else v = make_double2(total(3) - total(5), total(4) - total(2));                 // <Y> = i (m10 - m01)
       reinterpret_cast<double2*>(wgr)[pos] = v;
     }
   };
   for (int q = nchunks - 1; q >= 0; q--) {
     const int k0 = q * kRotChunk, kn = min(kRotChunk, a.nops - k0);
     __syncthreads();
-    stage_ops(st, a.ops, recs, k0, kn);
+    if (fixed)
+      fx_stage_ops<false>(st, a.ops, recs, k0, kn);
+    else
+      stage_ops<false, kRotGroup>(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = kn - 1; j >= 0; j--) {
       const int k = k0 + j;
       // before step k, psi holds the state behind operation k; the stored copy replaces it at
       // checkpoints, so that the error of undoing never spans more than ckpt_interval
-      // operations (the copy was made on the way forward: scaled by 1 / mfac against psi here)
+      // operations.  Between a group's first and last rotation the copy's scale is all / pre (pre:
+      // its cosines up to here, all: of the group) and the one on the way back pre.
       if (ck && (k + 1) % a.ckpt_interval == 0 && (k + 1) / a.ckpt_interval <= a.nck && k + 1 < a.nops) {
         const double2* src = ck + (size_t)((k + 1) / a.ckpt_interval - 1) * tile_elems;
-        const double f = 1.0 / st[j].mfac;
+        const double f = st[j].kind & kStInside ? 1.0 / (st[j].mfac * st[j].scale) : 1.0;
         for (int e = threadIdx.x; e < tc * N; e += blockDim.x) psi[e] = cscale(src[e], f);
         __syncthreads();
       }
       const int kind = st[j].kind & 255, mask = (st[j].kind >> 8) & 255;
       if (mask == 0) {  // a CZ by itself
-        rot_tile<kRotAdj>(psi, N, logN, tc, st[j]);
-        rot_tile<kRotAdj>(lam, N, logN, tc, st[j]);
+        if (fixed) {
+          fx_tile(reinterpret_cast<Fx2*>(psi), N, logN, tc, st[j]);
+          fx_tile(reinterpret_cast<Fx2*>(lam), N, logN, tc, st[j]);
+        } else {
+          rot_tile<kRotAdj>(psi, N, logN, tc, st[j]);
+          rot_tile<kRotAdj>(lam, N, logN, tc, st[j]);
+        }
         __syncthreads();
         continue;
       }
-      double acc[CPLX ? 6 : 3];
-#pragma unroll
-      for (int r = 0; r < (CPLX ? 6 : 3); r++) acc[r] = 0.0;
-      adjoint_tile<CPLX>(psi, lam, N, logN, tc, st[j], acc);
       const int items = tc << (kind == kOpCry ? logN - 2 : logN - 1);
       const int aw = min(nw, (items + 31) >> 5);  // warps holding pairs
-      if (warp < aw) {
-        double* rd = redd + buf * kTileMaxWarps * 8;
-        if constexpr (CPLX) {
-          double r[8] = {acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], 0.0, 0.0};
-          const double v = warp_reduce_scatter8(r);
-          if ((lane & 3) == 0) rd[warp * NV + (lane >> 2)] = v;
-        } else {
-          const double v = warp_reduce_scatter4(acc[0], acc[1], acc[2]);
-          if ((lane & 7) == 0) rd[warp * NV + ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)] = v;
+      double* rd = redd + buf * kTileMaxWarps * 8 + warp * NV;
+      if (fixed) {
+        long long acc[NA];
+#pragma unroll
+        for (int r = 0; r < NA; r++) acc[r] = 0;
+        fx_adjoint<CPLX>(reinterpret_cast<Fx2*>(psi), reinterpret_cast<Fx2*>(lam), N, logN, tc, st[j], acc);
+        if (warp < aw) {
+          long long r[8] = {};
+#pragma unroll
+          for (int i = 0; i < NA; i++) r[i] = fx_scaled(acc[i], shift);
+          const long long v = fx_reduce_scatter8(r);
+          if ((lane & 3) == 0 && (lane >> 2) < NV) rd[lane >> 2] = __longlong_as_double(v);
+        }
+      } else {
+        double acc[NA];
+#pragma unroll
+        for (int r = 0; r < NA; r++) acc[r] = 0.0;
+        adjoint_tile<CPLX>(psi, lam, N, logN, tc, st[j], acc);
+        if (warp < aw) {
+          if constexpr (CPLX) {
+            double r[8] = {acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], 0.0, 0.0};
+            const double v = warp_reduce_scatter8(r);
+            if ((lane & 3) == 0) rd[lane >> 2] = v;
+          } else {
+            const double v = warp_reduce_scatter4(acc[0], acc[1], acc[2]);
+            if ((lane & 7) == 0) rd[((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)] = v;
+          }
         }
       }
       flush();  // the operation before this one
