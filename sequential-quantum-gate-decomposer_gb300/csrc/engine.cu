@@ -109,13 +109,15 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_plan(RotPlan pl, const doub
 }
 
 template <bool WRITE_BACK, bool TRACE, int DIR>
-__global__ void __launch_bounds__(kMaxThreads) k_tile_forward(TileArgs a) {
+__global__ void __launch_bounds__(kMaxThreads, 3) k_tile_forward(TileArgs a) {
   extern __shared__ double2 smem[];
   tile_forward_body<WRITE_BACK, TRACE, DIR>(a, blockIdx.y, blockIdx.x, smem);
 }
 
-template <bool CPLX>
-__global__ void __launch_bounds__(kMaxThreads) k_tile_adjoint(TileArgs a) {
+// MINB: CTAs per SM that the registers are cut to.  Three where the launch fills the device with
+// tiles (the sweeps wait on the integer pipes' latencies), one where it does not (no spills).
+template <bool CPLX, int MINB>
+__global__ void __launch_bounds__(kMaxThreads, MINB) k_tile_adjoint(TileArgs a) {
   extern __shared__ double2 smem[];
   tile_adjoint_body<CPLX>(a, blockIdx.y, blockIdx.x, smem);
 }
@@ -831,16 +833,18 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   const int nov = c->plan.noverlaps;
   const dim3 sgrid((nov + 31) / 32, B), ggrid(c->plan.ncta, B);
   // the other variants multiply the derivative of the trace by the trace: complex overlaps
-  if (variant == SQG_FROBENIUS_NORM) {
-    if ((st = set_smem(k_tile_adjoint<false>, l.plan.smem))) return st;
-    k_tile_adjoint<false><<<grid, l.plan.threads, l.plan.smem, s>>>(a);
-    k_tile_sum<1><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
-    k_rot_grad<false><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
-  } else {
-    if ((st = set_smem(k_tile_adjoint<true>, l.plan.smem))) return st;
-    k_tile_adjoint<true><<<grid, l.plan.threads, l.plan.smem, s>>>(a);
+  const bool cplx = variant != SQG_FROBENIUS_NORM;
+  const bool full = (long long)l.plan.tiles * B >= 3LL * device_sms();
+  auto adjoint = cplx ? (full ? k_tile_adjoint<true, 3> : k_tile_adjoint<true, 1>)
+                      : (full ? k_tile_adjoint<false, 3> : k_tile_adjoint<false, 1>);
+  if ((st = set_smem(adjoint, l.plan.smem))) return st;
+  adjoint<<<grid, l.plan.threads, l.plan.smem, s>>>(a);
+  if (cplx) {
     k_tile_sum<2><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
     k_rot_grad<true><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
+  } else {
+    k_tile_sum<1><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
+    k_rot_grad<false><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
   }
   return cuda_status(cudaGetLastError(), "cost and gradient kernels");
 }

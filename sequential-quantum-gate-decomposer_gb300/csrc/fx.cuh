@@ -34,45 +34,43 @@ __device__ __forceinline__ unsigned long long fx_encode(double c) {
   return m << 1 | ((unsigned)__double2hiint(c) >> 31);
 }
 
-// The same, split for fx_mul.  add: -2^63 2^64|c| / 2^64 for the offset of the amplitude, one for the
-// two halves that the truncated products lose, less one where the result is complemented.
+// The same, split for fx_mul.  xl, xh: what the halves of the amplitude w are exclusive-or'd with: to
+// w + 2^63, or to its complement (2^63 - w - 1) for a negative coefficient.  k: what is added to
+// fx_mul: less the offset's share 2^63 2^64|c| / 2^64, and the mean of what fx_mul drops (1.25, and
+// |c| for the complement's one).
 struct FxCoef {
-  unsigned h, l;
-  unsigned long long add;
-  unsigned neg;  // all ones for a negative coefficient
+  unsigned h, l, xl, xh;
+  unsigned long long k;
 };
 __device__ __forceinline__ FxCoef fx_coef(unsigned long long enc, bool flip) {
   FxCoef c;
-  const unsigned neg = ((unsigned)enc & 1u) ^ (flip ? 1u : 0u);
+  const unsigned neg = 0u - (((unsigned)enc & 1u) ^ (flip ? 1u : 0u));
   c.h = (unsigned)(enc >> 32);
   c.l = (unsigned)enc & ~1u;
-  c.add = 1ULL - (enc >> 1) - neg;
-  c.neg = 0u - neg;
+  c.xl = neg;
+  c.xh = 0x80000000u ^ neg;
+  c.k = (neg && c.h >= 0x40000000u ? 2ULL : 1ULL) - (enc >> 1);
   return c;
 }
 
-// c * w for |w| <= 2^62, within a unit and without bias: (w + 2^63) * 2^64 |c| / 2^64 from three of the
-// four half products, less the offset's share.
+// c * w - c.k for |w| <= 2^62, within a unit: three of the four half products of (w + 2^63) * 2^64 |c| /
+// 2^64.  In PTX: with the sum written in C++ the compiler (CUDA 13.0) lost a carry.
 __device__ __forceinline__ unsigned long long fx_mul(long long w, const FxCoef& c) {
-  const unsigned wh = (unsigned)((unsigned long long)w >> 32) ^ 0x80000000u, wl = (unsigned)w;
-  unsigned lo, hi;
-  // in PTX: with the sum written in C++ the compiler (CUDA 13.0) lost a carry between `add` and the
-  // complement where |c| = 1
+  const unsigned wh = (unsigned)((unsigned long long)w >> 32) ^ c.xh, wl = (unsigned)w ^ c.xl;
+  unsigned long long p;
   asm("{\n\t"
-      ".reg .u64 p;\n\t"
-      ".reg .u32 a, b;\n\t"
-      "mad.wide.u32 p, %2, %4, %6;\n\t"
-      "mul.hi.u32 a, %2, %5;\n\t"
-      "mul.hi.u32 b, %3, %4;\n\t"
-      "mov.b64 {%0, %1}, p;\n\t"
-      "add.cc.u32 %0, %0, a;\n\t"
-      "addc.u32 %1, %1, 0;\n\t"
-      "add.cc.u32 %0, %0, b;\n\t"
-      "addc.u32 %1, %1, 0;\n\t"
+      ".reg .u64 q;\n\t"
+      ".reg .u32 a, b, n;\n\t"
+      "mul.hi.u32 a, %1, %4;\n\t"
+      "mul.hi.u32 b, %2, %3;\n\t"
+      "add.cc.u32 a, a, b;\n\t"
+      "addc.u32 n, 0, 0;\n\t"
+      "mov.b64 q, {a, n};\n\t"
+      "mad.wide.u32 %0, %1, %3, q;\n\t"
       "}"
-      : "=&r"(lo), "=&r"(hi)
-      : "r"(wh), "r"(wl), "r"(c.h), "r"(c.l), "l"(c.add));
-  return ((unsigned long long)(hi ^ c.neg) << 32) | (lo ^ c.neg);
+      : "=l"(p)
+      : "r"(wh), "r"(wl), "r"(c.h), "r"(c.l));
+  return p;
 }
 
 // Numbers of a staged operation (its doubles replaced by fx_encode) in a direction.
@@ -115,8 +113,8 @@ __device__ __forceinline__ long long fx_neg_if(long long v, unsigned neg) {
 
 // y <- z y
 __device__ __forceinline__ void fx_phase(Fx2& y, const FxCoef& zx, const FxCoef& zy, const FxCoef& nzy) {
-  const long long re = (long long)(fx_mul(y.x, zx) + fx_mul(y.y, nzy));
-  y.y = (long long)(fx_mul(y.y, zx) + fx_mul(y.x, zy));
+  const long long re = (long long)(fx_mul(y.x, zx) + fx_mul(y.y, nzy) + (zx.k + nzy.k));
+  y.y = (long long)(fx_mul(y.y, zx) + fx_mul(y.x, zy) + (zx.k + zy.k));
   y.x = re;
 }
 
@@ -126,16 +124,17 @@ __device__ __forceinline__ void fx_turnless(Fx2& x, Fx2& y, const FxCoef& t, con
   Fx2 nx, ny;
   const unsigned long long xx = AX ? fx_mul(y.y, t) : fx_mul(y.x, nt), xy = AX ? fx_mul(y.x, nt) : fx_mul(y.y, nt);
   const unsigned long long yx = AX ? fx_mul(x.y, t) : fx_mul(x.x, t), yy = AX ? fx_mul(x.x, nt) : fx_mul(x.y, t);
+  const unsigned long long kxx = AX ? t.k : nt.k, kxy = nt.k, kyx = t.k, kyy = AX ? nt.k : t.k;
   if (!RS) {
-    nx.x = x.x + (long long)xx;
-    nx.y = x.y + (long long)xy;
-    ny.x = y.x + (long long)yx;
-    ny.y = y.y + (long long)yy;
+    nx.x = x.x + (long long)(xx + kxx);
+    nx.y = x.y + (long long)(xy + kxy);
+    ny.x = y.x + (long long)(yx + kyx);
+    ny.y = y.y + (long long)(yy + kyy);
   } else {
-    nx.x = (long long)(fx_mul(x.x, scale) + xx);
-    nx.y = (long long)(fx_mul(x.y, scale) + xy);
-    ny.x = (long long)(fx_mul(y.x, scale) + yx);
-    ny.y = (long long)(fx_mul(y.y, scale) + yy);
+    nx.x = (long long)(fx_mul(x.x, scale) + xx + (scale.k + kxx));
+    nx.y = (long long)(fx_mul(x.y, scale) + xy + (scale.k + kxy));
+    ny.x = (long long)(fx_mul(y.x, scale) + yx + (scale.k + kyx));
+    ny.y = (long long)(fx_mul(y.y, scale) + yy + (scale.k + kyy));
   }
   x = nx;
   y = ny;
@@ -258,7 +257,9 @@ __device__ __forceinline__ FxHalf fx_half(long long v) {
   const int l = (int)v;
   return {(int)(v >> 32) - (l >> 31), l};
 }
-// Sum of products of amplitudes / 2^64, its low part kept until fx_fold.
+// Sum of at most four products of amplitudes of two pairs / 2^64, its low part kept to 64 bits until
+// fx_less: rounding each product would leave a bias that depends on which components are zero, and
+// sum it over the amplitudes.
 struct FxSum {
   long long hi, mid;
 };
@@ -267,7 +268,10 @@ __device__ __forceinline__ void fx_add(FxSum& s, FxHalf a, FxHalf b) {
   s.mid += (long long)a.h * b.l;
   s.mid += (long long)a.l * b.h;
 }
-__device__ __forceinline__ long long fx_fold(const FxSum& s) { return s.hi + ((s.mid + 0x80000000LL) >> 32); }
+__device__ __forceinline__ long long fx_less(const FxSum& s, const FxSum& u) {
+  return (s.hi - u.hi) + ((s.mid - u.mid + 0x80000000LL) >> 32);
+}
+
 // A thread's sum (|sum| <= 2^60 per vector, at most kFxItems vectors) / 2^shift, so that those of a
 // whole tile can be added; halves to the even side: a bias of half a unit's last place would add
 // up over the threads.
@@ -283,27 +287,26 @@ __device__ __forceinline__ void fx_measure(const Fx2& x, const Fx2& y, const Fx2
                                            long long (&acc)[CPLX ? 6 : 3]) {
   const FxHalf xx = fx_half(x.x), xy = fx_half(x.y), yx = fx_half(y.x), yy = fx_half(y.y);
   const FxHalf lxx = fx_half(lx.x), lxy = fx_half(lx.y), lyx = fx_half(ly.x), lyy = fx_half(ly.y);
-  auto sum2 = [](FxSum& s, FxHalf a, FxHalf b, FxHalf c, FxHalf d) {  // a b + c d
+  // (a b + c d) - (e f + g h)
+  auto folded = [](FxHalf a, FxHalf b, FxHalf c, FxHalf d, FxHalf e, FxHalf f, FxHalf g, FxHalf h) {
+    FxSum s = {0, 0}, u = {0, 0};
     fx_add(s, a, b);
     fx_add(s, c, d);
+    fx_add(u, e, f);
+    fx_add(u, g, h);
+    return fx_less(s, u);
   };
-  // (a b + c d) - (e f + g h)
-  auto folded = [&](FxHalf a, FxHalf b, FxHalf c, FxHalf d, FxHalf e, FxHalf f, FxHalf g, FxHalf h) {
-    FxSum s = {0, 0}, u = {0, 0};
-    sum2(s, a, b, c, d);
-    sum2(u, e, f, g, h);
-    return fx_fold({s.hi - u.hi, s.mid - u.mid});
-  };
-  auto plus = [&](FxHalf a, FxHalf b, FxHalf c, FxHalf d) {
+  auto plus = [](FxHalf a, FxHalf b, FxHalf c, FxHalf d) {
     FxSum s = {0, 0};
-    sum2(s, a, b, c, d);
-    return fx_fold(s);
+    fx_add(s, a, b);
+    fx_add(s, c, d);
+    return fx_less(s, {0, 0});
   };
-  auto minus = [&](FxHalf a, FxHalf b, FxHalf c, FxHalf d) {  // a b - c d
+  auto minus = [](FxHalf a, FxHalf b, FxHalf c, FxHalf d) {  // a b - c d
     FxSum s = {0, 0}, u = {0, 0};
     fx_add(s, a, b);
     fx_add(u, c, d);
-    return fx_fold({s.hi - u.hi, s.mid - u.mid});
+    return fx_less(s, u);
   };
   if (!CPLX) {
     if (MASK & 1) acc[0] += folded(lxx, yy, lyx, xy, lxy, yx, lyy, xx);

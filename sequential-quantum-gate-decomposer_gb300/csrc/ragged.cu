@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kRotThreads) k_ragged_plan(const InstDesc* __r
 
 // MODE 0: cost only; 1: gradient with real overlaps (FROBENIUS_NORM); 2: with complex ones.
 template <int MODE>
-__global__ void __launch_bounds__(kRaggedThreads) k_ragged_tiles(const InstDesc* __restrict__ desc,
+__global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged_tiles(const InstDesc* __restrict__ desc,
                                                                  const int2* __restrict__ items, int n_items,
                                                                  int* __restrict__ counter, const double2* targets,
                                                                  const RotRec* recs, const double2* phases,
