@@ -26,12 +26,14 @@ struct Fx2 {
 };
 static_assert(sizeof(Fx2) == sizeof(double2), "tiles are converted in place");
 
-// Coefficient c of |c| <= 1: upper 63 bits of 2^64 |c|, its sign in the lowest.
+// Coefficient c of |c| <= 1: upper 63 bits of 2^64 |c|, its sign in the lowest.  By shifts of its
+// significand (no FP64 instruction); 1 itself becomes 1 - 2^-63.
 __device__ __forceinline__ unsigned long long fx_encode(double c) {
-  const double a = fabs(c);
-  // 2^63 |c| is whole from 2^-10 on; 1 itself becomes 1 - 2^-63
-  unsigned long long m = a >= 1.0 ? 0x7fffffffffffffffULL : (unsigned long long)__double2ll_rn(a * 0x1p63);
-  return m << 1 | ((unsigned)__double2hiint(c) >> 31);
+  const unsigned long long v = (unsigned long long)__double_as_longlong(c);
+  const int s = (int)((v >> 52) & 0x7ff) - 1012;  // 2^63 |c| = significand * 2^s
+  const unsigned long long sig = (v & 0xfffffffffffffULL) | 0x10000000000000ULL;
+  const unsigned long long m = s > 10 ? 0x7fffffffffffffffULL : s >= 0 ? sig << s : s > -64 ? sig >> -s : 0ULL;
+  return m << 1 | v >> 63;
 }
 
 // The same, split for fx_mul.  xl, xh: what the halves of the amplitude w are exclusive-or'd with: to

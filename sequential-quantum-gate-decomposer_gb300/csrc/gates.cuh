@@ -50,43 +50,57 @@ __device__ __forceinline__ int pair_index2(int p, int t, int c) {
   return i | (1 << c);
 }
 
+// v with the sign bit `flip` changed (an integer operation).
+__device__ __forceinline__ double flip_sign(double v, unsigned flip) {
+  return __hiloint2double(__double2hiint(v) ^ (int)flip, __double2loint(v));
+}
+// The sign bit, as a value that the compiler cannot see: it turns a negation of a loop invariant
+// that it recognises into an FP64 instruction per thread (a fifth of a gate on one pair).
+__device__ __forceinline__ unsigned opaque_sign() {
+  unsigned sign = 0x80000000u;
+  asm("" : "+r"(sign));
+  return sign;
+}
+
 // ---- per-pair update rules (x = row with target bit 0, y = partner row) ----------
+// The imaginary parts and sines come with their negatives (nb = -u01.y and so on, ns = -s).
 // U3 with real u00: 14 FP64 instructions.
-__device__ __forceinline__ void rule_u3(double2& x, double2& y, double u00, double2 u01, double2 u10, double2 u11) {
+__device__ __forceinline__ void rule_u3(double2& x, double2& y, double u00, double2 u01, double2 u10, double2 u11,
+                                        double nb, double nc, double nd) {
   double2 nx, ny;
-  nx.x = fma(u00, x.x, fma(u01.x, y.x, -u01.y * y.y));
+  nx.x = fma(u00, x.x, fma(u01.x, y.x, nb * y.y));
   nx.y = fma(u00, x.y, fma(u01.x, y.y, u01.y * y.x));
-  ny.x = fma(u10.x, x.x, fma(-u10.y, x.y, fma(u11.x, y.x, -u11.y * y.y)));
+  ny.x = fma(u10.x, x.x, fma(nc, x.y, fma(u11.x, y.x, nd * y.y)));
   ny.y = fma(u10.x, x.y, fma(u10.y, x.x, fma(u11.x, y.y, u11.y * y.x)));
   x = nx;
   y = ny;
 }
 // RY / CRY [[c, -s], [s, c]]: 8 FP64 instructions.
-__device__ __forceinline__ void rule_ry(double2& x, double2& y, double c, double s) {
+__device__ __forceinline__ void rule_ry(double2& x, double2& y, double c, double s, double ns) {
   double2 nx, ny;
-  nx.x = fma(c, x.x, -s * y.x);
-  nx.y = fma(c, x.y, -s * y.y);
+  nx.x = fma(c, x.x, ns * y.x);
+  nx.y = fma(c, x.y, ns * y.y);
   ny.x = fma(s, x.x, c * y.x);
   ny.y = fma(s, x.y, c * y.y);
   x = nx;
   y = ny;
 }
 // RX [[c, -i s], [-i s, c]].
-__device__ __forceinline__ void rule_rx(double2& x, double2& y, double c, double s) {
+__device__ __forceinline__ void rule_rx(double2& x, double2& y, double c, double s, double ns) {
   double2 nx, ny;
   nx.x = fma(c, x.x, s * y.y);
-  nx.y = fma(c, x.y, -s * y.x);
+  nx.y = fma(c, x.y, ns * y.x);
   ny.x = fma(c, y.x, s * x.y);
-  ny.y = fma(c, y.y, -s * x.x);
+  ny.y = fma(c, y.y, ns * x.x);
   x = nx;
   y = ny;
 }
 // RZ diag(c - i s, c + i s).
-__device__ __forceinline__ void rule_rz(double2& x, double2& y, double c, double s) {
+__device__ __forceinline__ void rule_rz(double2& x, double2& y, double c, double s, double ns) {
   double2 nx, ny;
   nx.x = fma(c, x.x, s * x.y);
-  nx.y = fma(c, x.y, -s * x.x);
-  ny.x = fma(c, y.x, -s * y.y);
+  nx.y = fma(c, x.y, ns * x.x);
+  ny.x = fma(c, y.x, ns * y.y);
   ny.y = fma(c, y.y, s * y.x);
   x = nx;
   y = ny;
@@ -98,52 +112,42 @@ __device__ __forceinline__ void rule_rz(double2& x, double2& y, double c, double
 struct PairOp {
   int kind;  // G_U3, G_RY (also CRY), G_RX, G_RZ, G_CNOT, G_CZ
   double a;  // u00 (U3) or cos
-  double s;  // sin (signed for adjoint)
+  double s, ns;  // sin (signed for adjoint), its negative
   double2 b, c, d;  // u01, u10, u11 (U3)
+  double nb, nc, nd;  // negatives of their imaginary parts
 };
 
 enum Orientation { ORIENT_FWD = 0, ORIENT_ADJ = 1, ORIENT_TRANS = 2, ORIENT_CONJ = 3 };
 
-// Sign flips go through dneg (an integer operation): a negated double that is stored,
-// rather than folded into the consuming FMA, would cost an FP64 instruction per gate.
 __device__ __forceinline__ PairOp make_op(int type, const GateMat& m, int orient) {
   PairOp op;
+  const unsigned sign = opaque_sign();
+  const bool conj = orient == ORIENT_ADJ || orient == ORIENT_CONJ, swap = orient == ORIENT_ADJ || orient == ORIENT_TRANS;
   op.kind = (type == G_CRY) ? G_RY : type;
   op.a = m.u[0].x;
-  op.s = m.u[0].y;
-  op.b = m.u[1];
-  op.c = m.u[2];
-  op.d = m.u[3];
-  if (type == G_U3) {
-    op.a = m.u[0].x;
-    if (orient == ORIENT_ADJ) {  // [[u00, conj u10], [conj u01, conj u11]]
-      op.b = make_double2(m.u[2].x, dneg(m.u[2].y));
-      op.c = make_double2(m.u[1].x, dneg(m.u[1].y));
-      op.d = make_double2(m.u[3].x, dneg(m.u[3].y));
-    } else if (orient == ORIENT_TRANS) {  // [[u00, u10], [u01, u11]]
-      op.b = m.u[2];
-      op.c = m.u[1];
-    } else if (orient == ORIENT_CONJ) {  // [[u00, conj u01], [conj u10, conj u11]]
-      op.b = make_double2(m.u[1].x, dneg(m.u[1].y));
-      op.c = make_double2(m.u[2].x, dneg(m.u[2].y));
-      op.d = make_double2(m.u[3].x, dneg(m.u[3].y));
-    }
-  } else if (type == G_RY || type == G_CRY) {
-    // RY^dagger = RY^T = RY(-theta); RY is real, so conj RY = RY
-    if (orient == ORIENT_ADJ || orient == ORIENT_TRANS) op.s = dneg(op.s);
-  } else if (type == G_RX || type == G_RZ) {
-    // RX, RZ are symmetric: RX^T = RX, RZ^T = RZ; adjoint and conjugate flip the sine.
-    if (orient == ORIENT_ADJ || orient == ORIENT_CONJ) op.s = dneg(op.s);
-  }
+  // RY^dagger = RY^T = RY(-theta), RY is real; RX and RZ are symmetric: adjoint and conjugate
+  // flip the sine
+  const bool neg = (type == G_RY || type == G_CRY) ? swap : conj;
+  op.s = flip_sign(m.u[0].y, neg ? sign : 0u);
+  op.ns = flip_sign(m.u[0].y, neg ? 0u : sign);
+  // U3: [[u00, u01], [u10, u11]], transposed and conjugated as asked
+  const unsigned fy = conj ? sign : 0u, fn = conj ? 0u : sign;
+  const double2 b = swap ? m.u[2] : m.u[1], c = swap ? m.u[1] : m.u[2], d = m.u[3];
+  op.b = make_double2(b.x, flip_sign(b.y, fy));
+  op.c = make_double2(c.x, flip_sign(c.y, fy));
+  op.d = make_double2(d.x, flip_sign(d.y, fy));
+  op.nb = flip_sign(b.y, fn);
+  op.nc = flip_sign(c.y, fn);
+  op.nd = flip_sign(d.y, fn);
   return op;
 }
 
 __device__ __forceinline__ void apply_op(const PairOp& op, double2& x, double2& y) {
   switch (op.kind) {
-    case G_U3: rule_u3(x, y, op.a, op.b, op.c, op.d); break;
-    case G_RY: rule_ry(x, y, op.a, op.s); break;
-    case G_RX: rule_rx(x, y, op.a, op.s); break;
-    case G_RZ: rule_rz(x, y, op.a, op.s); break;
+    case G_U3: rule_u3(x, y, op.a, op.b, op.c, op.d, op.nb, op.nc, op.nd); break;
+    case G_RY: rule_ry(x, y, op.a, op.s, op.ns); break;
+    case G_RX: rule_rx(x, y, op.a, op.s, op.ns); break;
+    case G_RZ: rule_rz(x, y, op.a, op.s, op.ns); break;
     case G_CNOT: { double2 t = x; x = y; y = t; } break;
     case G_CZ: y.x = dneg(y.x); y.y = dneg(y.y); break;
   }

@@ -473,15 +473,9 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
 
 enum { kRotFwd = 0, kRotAdj = 1, kRotTrans = 2 };  // G, G^dagger, G^T (right multiplication)
 
-// v with the sign bit `flip` changed (an integer operation).
-__device__ __forceinline__ double flip_sign(double v, unsigned flip) {
-  return __hiloint2double(__double2hiint(v) ^ (int)flip, __double2loint(v));
-}
-
 // The numbers of a staged operation in a direction: G^dagger takes -t and the conjugate phases,
-// G^T takes -t about Y (Rx^T = Rx).  The negated copies are made here with integer operations,
-// from a sign bit that the compiler cannot see: it would otherwise negate on the FP64 pipe, once
-// per thread and operation (18 % of a sweep).
+// G^T takes -t about Y (Rx^T = Rx).  The negated copies are made here with integer operations
+// (opaque_sign): the compiler's own took 18 % of a sweep's FP64 instructions.
 struct DirOp {
   double t, nt, scale;
   double zix, ziy, nzi, zox, zoy, nzo;
@@ -492,8 +486,7 @@ struct DirOp {
 template <int DIR, int KIND>
 __device__ __forceinline__ DirOp directed(const StagedOp& s) {
   DirOp o;
-  unsigned sign = 0x80000000u;
-  asm volatile("" : "+r"(sign));
+  const unsigned sign = opaque_sign();
   const bool neg = DIR == kRotAdj || (DIR == kRotTrans && !(KIND & kOpX));
   const double t = s.t, nt = flip_sign(t, sign);
   o.t = neg ? nt : t;
