@@ -103,9 +103,9 @@ __global__ void k_prep(const Gate* __restrict__ gates, int L, int P, const doubl
 // Numbers of the plan's operations, one CTA per (CTA of runs, instance).
 __global__ void __launch_bounds__(kRotThreads) k_rot_plan(RotPlan pl, const double* __restrict__ theta,
                                                           long long theta_stride, RotRec* __restrict__ recs,
-                                                          double2* __restrict__ phases) {
+                                                          double2* __restrict__ phases, int deal) {
   const long long b = blockIdx.y;
-  rot_plan_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nrecs, phases + b * pl.ncta + blockIdx.x);
+  rot_plan_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nrecs, phases + b * pl.ncta + blockIdx.x, deal);
 }
 
 template <bool WRITE_BACK, bool TRACE, int DIR>
@@ -345,35 +345,37 @@ PrepLayout prep_layout(const sqg_circuit* c, int B, size_t start) {
 struct RotLayout {
   size_t rec_off, ph_off, end;
 };
-RotLayout rot_layout(const sqg_circuit* c, int B, size_t start) {
+RotLayout rot_layout(const RotPlan& p, int B, size_t start) {
   RotLayout l;
   l.rec_off = align_up(start, 256);
-  l.ph_off = align_up(l.rec_off + (size_t)B * c->plan.nrecs * sizeof(RotRec), 256);
-  l.end = align_up(l.ph_off + (size_t)B * c->plan.ncta * sizeof(double2), 256);
+  l.ph_off = align_up(l.rec_off + (size_t)B * p.nrecs * sizeof(RotRec), 256);
+  l.end = align_up(l.ph_off + (size_t)B * p.ncta * sizeof(double2), 256);
   return l;
 }
 
 // Makes the plan's numbers for B parameter vectors in the workspace and points `a` at them.
-int launch_plan(const sqg_circuit* c, const double* theta, long long theta_stride, int B, const RotLayout& l, char* ws,
+int launch_plan(const sqg_circuit* c, const RotPlan& p, const double* theta, long long theta_stride, int B, const RotLayout& l, char* ws,
                 TileArgs& a, cudaStream_t st) {
   RotRec* recs = (RotRec*)(ws + l.rec_off);
   double2* ph = (double2*)(ws + l.ph_off);
-  a.ops = c->plan.ops;
-  a.ends = c->plan.ends;
-  a.nops = c->plan.nops;
-  a.nrecs = c->plan.nrecs;
-  a.noverlaps = c->plan.noverlaps;
+  a.ops = p.ops;
+  a.ends = p.ends;
+  a.nops = p.nops;
+  a.nrecs = p.nrecs;
+  a.noverlaps = p.noverlaps;
   a.n = c->n;
   a.N = c->N;
   a.recs = recs;
   a.phases = ph;
-  a.nphase = c->plan.ncta;
-  if (c->plan.ncta == 0) return SQG_OK;
-  k_rot_plan<<<dim3(c->plan.ncta, B), kRotThreads, 0, st>>>(c->plan, theta, theta_stride, recs, ph);
+  a.nphase = p.ncta;
+  if (p.ncta == 0) return SQG_OK;
+  k_rot_plan<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, theta, theta_stride, recs, ph,
+                                                           (long long)p.ncta * B > 2LL * device_sms() ? 2 : 4);
   return cuda_status(cudaGetLastError(), "k_rot_plan");
 }
 
 struct EvalLayout {
+  const RotPlan* rp;
   RotLayout rot;
   size_t tr_off, gr_off, ck_off, end;
   TilePlan plan;
@@ -383,14 +385,15 @@ struct EvalLayout {
 // only their imaginary parts, uses half of that.
 EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckpt_interval) {
   EvalLayout l;
-  l.rot = rot_layout(c, B, 0);
   l.plan = plan_tiles(c->N, cols, grad, B);
+  l.rp = (long long)B * l.plan.tiles < 3LL * device_sms() ? &c->short_plan : &c->plan;
+  l.rot = rot_layout(*l.rp, B, 0);
   l.tr_off = l.rot.end;
   l.gr_off = align_up(l.tr_off + (size_t)B * l.plan.tiles * sizeof(double2), 256);
-  size_t gr_bytes = grad ? (size_t)B * l.plan.tiles * std::max(c->plan.noverlaps, 1) * sizeof(double2) : 0;
+  size_t gr_bytes = grad ? (size_t)B * l.plan.tiles * std::max(l.rp->noverlaps, 1) * sizeof(double2) : 0;
   l.ck_off = align_up(l.gr_off + gr_bytes, 256);
   l.nck = 0;
-  if (grad && ckpt_interval > 0) l.nck = c->plan.nops / ckpt_interval;
+  if (grad && ckpt_interval > 0) l.nck = l.rp->nops / ckpt_interval;
   size_t ck_bytes = (size_t)B * l.plan.tiles * l.nck * (size_t)l.plan.TC * c->N * sizeof(double2);
   l.end = align_up(l.ck_off + ck_bytes, 256);
   return l;
@@ -423,6 +426,14 @@ constexpr int kStateQubits = 30;   // largest register of sqg_apply_state (2^30 
 constexpr int kStateK = 12;        // qubits per chunk: 4096 amplitudes, 64 KB of shared memory
 constexpr int kStateLow = 5;       // the lowest qubits belong to every chunk (512-byte coalesced runs)
 constexpr int kStateThreads = 256;
+
+// Appends bytes to a blob on a 16-byte boundary; returns their offset.
+size_t blob_put(std::vector<char>& blob, const void* src, size_t bytes) {
+  const size_t at = blob.size();
+  blob.resize((at + bytes + 15) / 16 * 16);
+  if (bytes) memcpy(blob.data() + at, src, bytes);
+  return at;
+}
 
 // Groups the gates into blocks: a block grows while the qubits it touches, together with the
 // lowest kStateLow ones, number at most K; each block is one pass over the state.  With
@@ -530,15 +541,18 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
   }
   if (c->L > 0) close_block(g0, c->L);
   if (c->L == 0) return SQG_OK;
-  lops.push_back(RotOp{});  // a block may have no operation left: never an empty array
-  cudaError_t e = cudaMalloc(&c->d_lops, sizeof(RotOp) * lops.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_lops, lops.data(), sizeof(RotOp) * lops.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_lends, sizeof(int) * lends.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_lends, lends.data(), sizeof(int) * lends.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_hitab, sizeof(int) * hitab.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_hitab, hitab.data(), sizeof(int) * hitab.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_inact, sizeof(int) * inact.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_inact, inact.data(), sizeof(int) * inact.size(), cudaMemcpyHostToDevice);
+  std::vector<char> blob;
+  const size_t o_ops = blob_put(blob, lops.data(), lops.size() * sizeof(RotOp));
+  const size_t o_ends = blob_put(blob, lends.data(), lends.size() * sizeof(int));
+  const size_t o_hi = blob_put(blob, hitab.data(), hitab.size() * sizeof(int));
+  const size_t o_in = blob_put(blob, inact.data(), inact.size() * sizeof(int));
+  cudaError_t e = cudaMalloc(&c->d_state, blob.size());
+  if (e == cudaSuccess) e = cudaMemcpy(c->d_state, blob.data(), blob.size(), cudaMemcpyHostToDevice);
+  const char* d = (const char*)c->d_state;
+  c->d_lops = (RotOp*)(d + o_ops);
+  c->d_lends = (int*)(d + o_ends);
+  c->d_hitab = (int*)(d + o_hi);
+  c->d_inact = (int*)(d + o_in);
   return cuda_status(e, "state plan");
 }
 
@@ -599,48 +613,52 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
 // =====================================================================================
 // C ABI
 // =====================================================================================
-// Makes the rotation plan of the circuit and copies it to the device.
-static int make_rot_plan(sqg_circuit* c) {
-  RotPlanHost h = build_rot_plan(c->n, c->h_gates);
-  c->h_steps = h.steps;
-  std::vector<RotOp> ops;
-  std::vector<int> ends;
-  if (c->n <= kMatrixQubits) {  // larger registers are applied in chunks only
-    std::vector<int> loc(c->n);
-    for (int q = 0; q < c->n; q++) loc[q] = q;
-    lower_rot_steps(h.steps, 0, (int)h.steps.size(), c->n, loc, ops, ends);
-  }
-  RotPlan& p = c->plan;
-  p.gates = c->d_gates;
-  p.nops = (int)ops.size();
-  p.nrecs = (int)h.steps.size();
-  p.ncta = (int)h.cta.size() - 1;
-  p.noverlaps = h.noverlaps;
+// Makes the rotation plans of the circuit and copies them to the device with its gates, in one
+// allocation.
+static int make_rot_plans(sqg_circuit* c) {
   std::vector<char> blob;
-  auto put = [&](const void* src, size_t bytes) {
-    const size_t at = blob.size();
-    blob.resize((at + bytes + 15) / 16 * 16);
-    if (bytes) memcpy(blob.data() + at, src, bytes);
-    return at;
-  };
-  const size_t o_ops = put(ops.data(), ops.size() * sizeof(RotOp));
-  const size_t o_runs = put(h.runs.data(), h.runs.size() * sizeof(RotRun));
-  const size_t o_mem = put(h.members.data(), h.members.size() * sizeof(int));
-  const size_t o_cta = put(h.cta.data(), h.cta.size() * sizeof(int));
-  const size_t o_par = put(h.params.data(), h.params.size() * sizeof(int));
-  const size_t o_cpar = put(h.cta_params.data(), h.cta_params.size() * sizeof(int));
-  const size_t o_ends = put(ends.data(), ends.size() * sizeof(int));
+  const size_t o_gates = blob_put(blob, c->h_gates.data(), c->h_gates.size() * sizeof(Gate));
+  RotPlan* plans[2] = {&c->plan, &c->short_plan};
+  size_t off[2][7];
+  for (int k = 0; k < 2; k++) {
+    const RotPlanHost h = build_rot_plan(c->n, c->h_gates, k ? kRotShortChain : kRotChain);
+    std::vector<RotOp> ops;
+    std::vector<int> ends;
+    if (c->n <= kMatrixQubits) {  // larger registers are applied in chunks only
+      std::vector<int> loc(c->n);
+      for (int q = 0; q < c->n; q++) loc[q] = q;
+      lower_rot_steps(h.steps, 0, (int)h.steps.size(), c->n, loc, ops, ends);
+    }
+    RotPlan& p = *plans[k];
+    p.nops = (int)ops.size();
+    p.nrecs = (int)h.steps.size();
+    p.ncta = (int)h.cta.size() - 1;
+    p.noverlaps = h.noverlaps;
+    off[k][0] = blob_put(blob, ops.data(), ops.size() * sizeof(RotOp));
+    off[k][1] = blob_put(blob, h.runs.data(), h.runs.size() * sizeof(RotRun));
+    off[k][2] = blob_put(blob, h.members.data(), h.members.size() * sizeof(int));
+    off[k][3] = blob_put(blob, h.cta.data(), h.cta.size() * sizeof(int));
+    off[k][4] = blob_put(blob, h.params.data(), h.params.size() * sizeof(int));
+    off[k][5] = blob_put(blob, h.cta_params.data(), h.cta_params.size() * sizeof(int));
+    off[k][6] = blob_put(blob, ends.data(), ends.size() * sizeof(int));
+    if (k == 0) c->h_steps = h.steps;
+  }
   cudaError_t e = cudaMalloc(&c->d_plan, blob.size());
   if (e == cudaSuccess) e = cudaMemcpy(c->d_plan, blob.data(), blob.size(), cudaMemcpyHostToDevice);
-  char* d = (char*)c->d_plan;
-  p.ops = (const RotOp*)(d + o_ops);
-  p.runs = (const RotRun*)(d + o_runs);
-  p.members = (const int*)(d + o_mem);
-  p.cta = (const int*)(d + o_cta);
-  p.params = (const int*)(d + o_par);
-  p.cta_params = (const int*)(d + o_cpar);
-  p.ends = (const int*)(d + o_ends);
-  return cuda_status(e, "rotation plan");
+  const char* d = (const char*)c->d_plan;
+  c->d_gates = (Gate*)(d + o_gates);
+  for (int k = 0; k < 2; k++) {
+    RotPlan& p = *plans[k];
+    p.gates = c->d_gates;
+    p.ops = (const RotOp*)(d + off[k][0]);
+    p.runs = (const RotRun*)(d + off[k][1]);
+    p.members = (const int*)(d + off[k][2]);
+    p.cta = (const int*)(d + off[k][3]);
+    p.params = (const int*)(d + off[k][4]);
+    p.cta_params = (const int*)(d + off[k][5]);
+    p.ends = (const int*)(d + off[k][6]);
+  }
+  return cuda_status(e, "circuit handle");
 }
 
 extern "C" {
@@ -699,16 +717,7 @@ int sqg_circuit_create(int qbit_num, const sqg_gate* gates, int gate_num, sqg_ci
   }
   c->P = p;
   cudaGetDevice(&c->device);
-  if (gate_num > 0) {
-    cudaError_t e = cudaMalloc(&c->d_gates, sizeof(Gate) * gate_num);
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_gates, c->h_gates.data(), sizeof(Gate) * gate_num, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      int st = cuda_status(e, "sqg_circuit_create");
-      sqg_circuit_destroy(c);
-      return st;
-    }
-  }
-  int st = make_rot_plan(c);
+  int st = make_rot_plans(c);
   if (!st) st = build_state_plan(c);
   if (st) {
     sqg_circuit_destroy(c);
@@ -729,26 +738,16 @@ int sqg_circuit_set_partitions(sqg_circuit* c, const int* part_ends, int nparts)
   int dev = -1;
   cudaGetDevice(&dev);
   if (dev != c->device) return fail(SQG_ERR_INVALID_ARGUMENT, "circuit handle belongs to another device");
-  cudaFree(c->d_lops);
-  cudaFree(c->d_lends);
-  cudaFree(c->d_hitab);
-  cudaFree(c->d_inact);
-  c->d_lops = nullptr;
-  c->d_lends = nullptr;
-  c->d_hitab = nullptr;
-  c->d_inact = nullptr;
+  cudaFree(c->d_state);
+  c->d_state = nullptr;
   c->sblocks.clear();
   return build_state_plan(c, cuts);
 }
 
 int sqg_circuit_destroy(sqg_circuit* c) {
   if (!c) return SQG_OK;
-  if (c->d_gates) cudaFree(c->d_gates);
-  if (c->d_lops) cudaFree(c->d_lops);
-  if (c->d_lends) cudaFree(c->d_lends);
-  if (c->d_hitab) cudaFree(c->d_hitab);
-  if (c->d_inact) cudaFree(c->d_inact);
   if (c->d_plan) cudaFree(c->d_plan);
+  if (c->d_state) cudaFree(c->d_state);
   delete c;
   return SQG_OK;
 }
@@ -787,16 +786,39 @@ static int cost_grad_args(const sqg_circuit* c, const double* theta, int B, cons
   return SQG_OK;
 }
 
+// Whether the tile kernels are faster than the environment-matrix evaluation where both can run.
+// Measured on GB300, environment matrix against tiles: three qubits 71 against 115 us (one vector,
+// 14 blocks), 434 against 1222 us (4096 vectors); four qubits, 40 blocks 322 against 228 us (one
+// vector), 1210 against 1045 us (1024), 10 blocks 130 against 110 us (one), 20 blocks 551 against 667
+// us (1024); five qubits, 3 blocks 164 against 74 us (one) and 254 against 236 us (512), 20 blocks 406
+// against 154 us and 1090 against 665 us.
+static bool tiles_first(const sqg_circuit* c, int B) {
+  if (c->n >= 5) return true;
+  return c->n == 4 && c->L >= (B > 2 * device_sms() ? 96 : 32);
+}
+
 int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
                   long long target_batch_stride, int trace_offset, int variant, double* cost, double* grad,
                   int checkpoint_interval, void* workspace, size_t ws_bytes, void* stream) {
+  return sqg::cost_grad(c, theta, B, target, cols, target_batch_stride, trace_offset, variant, cost, grad,
+                        checkpoint_interval, workspace, ws_bytes, stream, false);
+}
+
+}  // extern "C"
+
+int sqg::cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
+                   long long target_batch_stride, int trace_offset, int variant, double* cost, double* grad,
+                   int checkpoint_interval, void* workspace, size_t ws_bytes, void* stream, bool env_first) {
   int st = cost_grad_args(c, theta, B, target, cols, trace_offset, variant, cost, grad, checkpoint_interval);
   if (st) return st;
   const int off = variant == SQG_FROBENIUS_NORM ? trace_offset : 0;
   const bool with_grad = grad != nullptr && c->P > 0;
   if (with_grad && checkpoint_interval == 0) {
-    // up to five qubits: one CTA per vector with the environment-matrix evaluation
-    st = sqg::env_cost_grad(c, theta, B, target, cols, target_batch_stride, off, variant, cost, grad, stream);
+    // up to five qubits: one CTA per vector with the environment-matrix evaluation, which also
+    // takes the calls without a workspace
+    const bool tiles = !env_first && tiles_first(c, B) && workspace && ws_bytes >= eval_layout(c, B, cols, true, 0).end;
+    st = tiles ? SQG_ERR_UNSUPPORTED
+               : sqg::env_cost_grad(c, theta, B, target, cols, target_batch_stride, off, variant, cost, grad, stream);
     if (st != SQG_ERR_UNSUPPORTED) return st;
     st = SQG_OK;
   }
@@ -807,7 +829,7 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   double2* wtr = (double2*)(ws + l.tr_off);
   double* wgr = (double*)(ws + l.gr_off);
   TileArgs a;
-  if ((st = launch_plan(c, theta, c->P, B, l.rot, ws, a, s))) return st;
+  if ((st = launch_plan(c, *l.rp, theta, c->P, B, l.rot, ws, a, s))) return st;
   a.mtx = (double2*)target;
   a.bstride = target_batch_stride;
   a.rstride = cols;
@@ -830,8 +852,8 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
     k_tile_sum<1><<<dim3(1, B), 32 * kSumGroups, 0, s>>>(wtr, nullptr, l.plan.tiles, 0, cols, variant, cost);
     return cuda_status(cudaGetLastError(), "k_tile_sum");
   }
-  const int nov = c->plan.noverlaps;
-  const dim3 sgrid((nov + 31) / 32, B), ggrid(c->plan.ncta, B);
+  const int nov = l.rp->noverlaps;
+  const dim3 sgrid((nov + 31) / 32, B), ggrid(l.rp->ncta, B);
   // the other variants multiply the derivative of the trace by the trace: complex overlaps
   const bool cplx = variant != SQG_FROBENIUS_NORM;
   const bool full = (long long)l.plan.tiles * B >= 3LL * device_sms();
@@ -841,15 +863,13 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   adjoint<<<grid, l.plan.threads, l.plan.smem, s>>>(a);
   if (cplx) {
     k_tile_sum<2><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
-    k_rot_grad<true><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
+    k_rot_grad<true><<<ggrid, kRotThreads, 0, s>>>(*l.rp, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
   } else {
     k_tile_sum<1><<<sgrid, 32 * kSumGroups, 0, s>>>(wtr, wgr, l.plan.tiles, nov, cols, variant, cost);
-    k_rot_grad<false><<<ggrid, kRotThreads, 0, s>>>(c->plan, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
+    k_rot_grad<false><<<ggrid, kRotThreads, 0, s>>>(*l.rp, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
   }
   return cuda_status(cudaGetLastError(), "cost and gradient kernels");
 }
-
-}  // extern "C"
 
 // ---- allocation-free cost/gradient ---------------------------------------------------
 // The scratch of sqg_cost_grad_noalloc: a file-scope device array of fixed size.  In host
@@ -973,7 +993,7 @@ int sqg_apply(const sqg_circuit* c, const double* theta, int B, void* mtx, int c
     TilePlan pl = plan_tiles(c->N, cols, false);
     TileArgs a;
     memset(&a, 0, sizeof(a));
-    if ((st = launch_plan(c, theta, c->P, B, rot_layout(c, B, 0), ws, a, s))) return st;
+    if ((st = launch_plan(c, c->plan, theta, c->P, B, rot_layout(c->plan, B, 0), ws, a, s))) return st;
     a.mtx = (double2*)mtx;
     a.bstride = batch_stride;
     a.rstride = stride;
@@ -1024,7 +1044,7 @@ int sqg_apply_from_right(const sqg_circuit* c, const double* theta, void* mtx, i
   TilePlan pl = plan_tiles(c->N, rows, false);
   TileArgs a;
   memset(&a, 0, sizeof(a));
-  if ((st = launch_plan(c, theta, c->P, 1, rot_layout(c, 1, 0), (char*)workspace, a, s))) return st;
+  if ((st = launch_plan(c, c->plan, theta, c->P, 1, rot_layout(c->plan, 1, 0), (char*)workspace, a, s))) return st;
   a.mtx = (double2*)mtx;
   a.bstride = 0;
   a.rstride = stride;
@@ -1103,7 +1123,7 @@ int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* stat
     const size_t smem = sizeof(double2) << c->sK;
     if ((st = set_smem(k_state_block, smem))) return st;
     TileArgs t;
-    if ((st = launch_plan(c, theta, c->P, B, rot_layout(c, B, 0), ws, t, s))) return st;
+    if ((st = launch_plan(c, c->plan, theta, c->P, B, rot_layout(c->plan, B, 0), ws, t, s))) return st;
     StateArgs a;
     a.states = (double2*)states;
     a.stride = stride;

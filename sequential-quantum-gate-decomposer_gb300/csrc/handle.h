@@ -18,17 +18,19 @@ struct sqg_circuit {
   int device = 0;
   sqg::Gate* d_gates = nullptr;
   std::vector<sqg::Gate> h_gates;
-  // rotation plan (rot.cuh): the host's steps, from which the tile operations and those of the
-  // state-vector blocks are made, and the device arrays, one allocation behind d_plan
+  // rotation plan (rot.cuh): the host's steps, from which the operations of the state-vector
+  // blocks are made, and the device arrays, one allocation with the gates behind d_plan.
+  // short_plan: the same with short chains, for launches that wait for the chains.
   std::vector<sqg::RotStep> h_steps;
   void* d_plan = nullptr;
-  sqg::RotPlan plan = {};
+  sqg::RotPlan plan = {}, short_plan = {};
   // state-vector plan: chunk qubits K, blocks, operations on chunk-local qubits, per block the
   // places behind its last operation (K ints, padded to 16), the global offsets of the chunk's
   // high local bits (2^(K - low) ints, padded to 128) and the qubits that number the chunks
   // (padded to 32)
   int sK = 0;
   std::vector<sqg_state_block> sblocks;
+  void* d_state = nullptr;  // the arrays' allocation
   sqg::RotOp* d_lops = nullptr;
   int* d_lends = nullptr;
   int* d_hitab = nullptr;
@@ -42,4 +44,9 @@ int set_error(int status, const std::string& msg);
 // for shapes it does not take.
 int env_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols, long long tstride,
                   int off, int variant, double* cost, double* grad, void* stream);
+// sqg_cost_grad; env_first: with the arithmetic of the decomposition kernels wherever they have it
+// (up to five qubits), which the device loops repeat bit for bit.
+int cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
+              long long target_batch_stride, int trace_offset, int variant, double* cost, double* grad,
+              int checkpoint_interval, void* workspace, size_t ws_bytes, void* stream, bool env_first);
 }  // namespace sqg

@@ -415,8 +415,8 @@ int run_loop_graph(const sqg_circuit* c, const void* target, int cols, int trace
   if (e != cudaSuccess) {
     st = cuda_fail(e, "building the decomposition graph");
   } else {
-    st = sqg_cost_grad(c, x_eval, 1, target, cols, 0, trace_offset, cost_variant, cost_eval, g_eval, 0, eval_ws,
-                       eval_bytes, cap);
+    st = sqg::cost_grad(c, x_eval, 1, target, cols, 0, trace_offset, cost_variant, cost_eval, g_eval, 0, eval_ws,
+                        eval_bytes, cap, true);
     if (st == SQG_OK) {
       step(cap, handle);
       e = cudaGetLastError();

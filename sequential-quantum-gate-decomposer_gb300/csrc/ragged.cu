@@ -39,7 +39,7 @@ struct sqg_ragged_batch {
   InstDesc* d_desc = nullptr;
   int2* d_items = nullptr;     // (instance, tile), decreasing work
   int2* d_cta_map = nullptr;   // (instance, CTA of runs) of the plan and gradient kernels
-  int total_ctas = 0, max_overlaps = 0;
+  int total_ctas = 0, max_overlaps = 0, sms = 1;
   long long total_rec = 0, total_ph = 0, total_tr = 0, total_gr = 0;
   std::vector<long long> theta_off, target_off;
   size_t off_rec = 0, off_ph = 0, off_tr = 0, off_gr = 0, ws_bytes = 0;
@@ -52,10 +52,11 @@ inline size_t a256(size_t v) { return (v + 255) / 256 * 256; }
 __global__ void __launch_bounds__(kRotThreads) k_ragged_plan(const InstDesc* __restrict__ desc,
                                                              const int2* __restrict__ cta_map,
                                                              const double* __restrict__ theta,
-                                                             RotRec* __restrict__ recs, double2* __restrict__ phases) {
+                                                             RotRec* __restrict__ recs, double2* __restrict__ phases,
+                                                             int deal) {
   const int2 m = cta_map[blockIdx.x];
   const InstDesc d = desc[m.x];
-  rot_plan_body(d.plan, m.y, theta + d.theta_off, recs + d.rec_off, phases + d.ph_off + m.y);
+  rot_plan_body(d.plan, m.y, theta + d.theta_off, recs + d.rec_off, phases + d.ph_off + m.y, deal);
 }
 
 // MODE 0: cost only; 1: gradient with real overlaps (FROBENIUS_NORM); 2: with complex ones.
@@ -259,6 +260,7 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
     free_batch(r);
     return st;
   }
+  r->sms = sms;
   r->grid = std::max(1, std::min(r->n_items, std::max(per_sm, 1) * sms));
   *out = r;
   return SQG_OK;
@@ -303,7 +305,8 @@ int sqg_ragged_cost_grad(const sqg_ragged_batch* r, const double* theta, const v
   int st;
   if ((st = cerr(cudaMemsetAsync(counter, 0, sizeof(int), s), "cudaMemsetAsync"))) return st;
   if (r->total_ctas > 0) {
-    k_ragged_plan<<<r->total_ctas, kRotThreads, 0, s>>>(r->d_desc, r->d_cta_map, theta, recs, ph);
+    k_ragged_plan<<<r->total_ctas, kRotThreads, 0, s>>>(r->d_desc, r->d_cta_map, theta, recs, ph,
+                                                        r->total_ctas > 2 * r->sms ? 2 : 4);
     if ((st = cerr(cudaGetLastError(), "k_ragged_plan"))) return st;
   }
   const int mode = !grad ? 0 : variant == SQG_FROBENIUS_NORM ? 1 : 2;

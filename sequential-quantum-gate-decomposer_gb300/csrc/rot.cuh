@@ -89,7 +89,10 @@ struct RotPlan {
 
 constexpr int kRotThreads = 128;  // runs per CTA of the per-instance kernels; no chain straddles two
 constexpr int kRotParams = 512;  // parameters listed per CTA
-constexpr int kRotChain = 16;     // runs linked by pushed rotations (their numbers are made one after another)
+// Runs linked by pushed rotations.  Their numbers are made one after another, 4 us a run, and the
+// run that ends a chain costs 4 products more per pair and vector: 3 % at 16, 12 % at 4.  A launch
+// that does not fill the device waits for the chains: 46 U3 of one vector 52 us at 16, 29 us at 4.
+constexpr int kRotChain = 16, kRotShortChain = 4;
 constexpr int kRotChunk = 32;     // operations staged in shared memory together (a warp)
 // Operations whose cosines are multiplied in together.  In FP64 the scale costs no precision, so
 // the whole chunk; in fixed point the overlaps lose the square of it (2^-8 at worst), at 4
@@ -260,7 +263,7 @@ __device__ __forceinline__ double split_u3(double2 cs, double2 phi, double2 lam,
 // makes the matrix of run i (the factors of a lone U3); the first thread of each chain of pushed
 // rotations then walks it.  phase_out receives the product of the runs' phases.
 __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const double* theta, RotRec* recs,
-                                              double2* phase_out) {
+                                              double2* phase_out, int deal) {
   __shared__ double2 Ms[kRotThreads][4];
   __shared__ double2 ph[kRotThreads];
   __shared__ int chain_of[kRotThreads], warp_heads[kRotThreads / 32];
@@ -291,8 +294,10 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
     }
     for (int k = 0; k < 4; k++) Ms[i][k] = M[k];
   }
-  // Chains of two and more runs are few and take longest: they are dealt out over the warps, so
-  // that as few as possible wait for one another's branches.
+  // Chains of two and more runs are few and take longest: they are dealt out over `deal` warps.  All
+  // four where the launch waits for one CTA (as few as possible wait for one another's branches),
+  // two, which hold the most there can be, where the FP64 pipe is shared by many CTAs and takes
+  // as long for a warp of two chains as for one of 32.
   const int warp = i >> 5, lane = i & 31;
   const bool head = i < n && !run.pulled && run.push != kAxisNone;
   const unsigned heads = __ballot_sync(0xffffffffu, head);
@@ -303,9 +308,9 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
     if (w < warp) rank += warp_heads[w];
     nheads += warp_heads[w];
   }
-  if (head) chain_of[(rank % (kRotThreads / 32)) * 32 + rank / (kRotThreads / 32)] = i;
+  if (head) chain_of[(rank % deal) * 32 + rank / deal] = i;
   __syncthreads();
-  const bool walks = lane * (kRotThreads / 32) + warp < nheads;
+  const bool walks = warp < deal && lane * deal + warp < nheads;
   for (int pass = 0; pass < 2; pass++) {
     // first the runs by themselves, each by its own thread, then the chains
     if (pass == 0 ? !(i < n && !run.pulled && run.push == kAxisNone) : !walks) continue;

@@ -29,7 +29,8 @@ inline int rot_commuting_axis(int type, bool on_control) {
 
 inline int rot_letter(int type) { return type == G_RX ? kAxisX : type == G_RY ? kAxisY : kAxisZ; }
 
-inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates) {
+// max_chain: runs linked by pushed rotations, at most kRotChain.
+inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates, int max_chain) {
   // A run whose gates are single-axis rotations about at most two axes in turn (`letters`, equal
   // neighbours merged) stays as one operation per axis: 4 instructions each, no more than any
   // other form, and only their own overlaps.  Every other run is a general 2x2 unitary.
@@ -75,9 +76,9 @@ inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates) {
     if (letters > 2) r.general = true;
   }
   // A general run pushes into the next run of its qubit if that run is general too and every
-  // two-qubit gate between them commutes with the same axis.  Chains end after kRotChain runs:
-  // their numbers are made one after another, and the run that ends a chain costs 4
-  // instructions more per pair (3 % at 16).
+  // two-qubit gate between them commutes with the same axis.  Chains end after max_chain runs:
+  // their numbers are made one after another, and the run that ends a chain costs 4 products more
+  // per pair and vector.
   for (int q = 0; q < n; q++) {
     const std::vector<Event>& ev = events[q];
     for (size_t i = 0; i < ev.size(); i++) {
@@ -91,7 +92,7 @@ inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates) {
       if (j >= ev.size() || ev[j].run < 0) continue;
       Run& r = runs[ev[i].run];
       Run& s = runs[ev[j].run];
-      if (!s.general || r.depth + 1 >= kRotChain) continue;
+      if (!s.general || r.depth + 1 >= max_chain) continue;
       r.push = axis;
       r.next = ev[j].run;
       s.prev = ev[i].run;
