@@ -108,6 +108,21 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_plan(RotPlan pl, const doub
   rot_plan_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nrecs, phases + b * pl.ncta + blockIdx.x, deal);
 }
 
+// The same for many vectors in three launches.
+__global__ void __launch_bounds__(kRotThreads) k_rot_matrices(RotPlan pl, const double* __restrict__ theta,
+                                                              long long theta_stride, RotRec* recs) {
+  const long long b = blockIdx.y;
+  batch_matrices_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nrecs);
+}
+__global__ void __launch_bounds__(kRotThreads) k_rot_chains(RotPlan pl, int B, RotRec* recs) {
+  const long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (b < B) batch_chain_body(pl, blockIdx.y, recs + b * pl.nrecs);
+}
+__global__ void __launch_bounds__(kRotThreads) k_rot_finish(RotPlan pl, RotRec* recs, double2* __restrict__ phases) {
+  const long long b = blockIdx.y;
+  batch_finish_body(pl, blockIdx.x, recs + b * pl.nrecs, phases + b * pl.ncta + blockIdx.x);
+}
+
 template <bool WRITE_BACK, bool TRACE, int DIR>
 __global__ void __launch_bounds__(kMaxThreads, 3) k_tile_forward(TileArgs a) {
   extern __shared__ double2 smem[];
@@ -353,6 +368,10 @@ RotLayout rot_layout(const RotPlan& p, int B, size_t start) {
   return l;
 }
 
+// Vectors from which the plan's numbers are made in three launches.  Below, warps of k_rot_chains
+// would idle.
+constexpr int kRotBatch = 32;
+
 // Makes the plan's numbers for B parameter vectors in the workspace and points `a` at them.
 int launch_plan(const sqg_circuit* c, const RotPlan& p, const double* theta, long long theta_stride, int B, const RotLayout& l, char* ws,
                 TileArgs& a, cudaStream_t st) {
@@ -369,8 +388,14 @@ int launch_plan(const sqg_circuit* c, const RotPlan& p, const double* theta, lon
   a.phases = ph;
   a.nphase = p.ncta;
   if (p.ncta == 0) return SQG_OK;
-  k_rot_plan<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, theta, theta_stride, recs, ph,
-                                                           (long long)p.ncta * B > 2LL * device_sms() ? 2 : 4);
+  if (B >= kRotBatch) {
+    k_rot_matrices<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, theta, theta_stride, recs);
+    k_rot_chains<<<dim3((B + 31) / 32, p.nheads), 32, 0, st>>>(p, B, recs);
+    k_rot_finish<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, recs, ph);
+  } else {
+    k_rot_plan<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, theta, theta_stride, recs, ph,
+                                                         p.ncta * B > 2 * device_sms() ? 2 : 4);
+  }
   return cuda_status(cudaGetLastError(), "k_rot_plan");
 }
 
@@ -619,7 +644,7 @@ static int make_rot_plans(sqg_circuit* c) {
   std::vector<char> blob;
   const size_t o_gates = blob_put(blob, c->h_gates.data(), c->h_gates.size() * sizeof(Gate));
   RotPlan* plans[2] = {&c->plan, &c->short_plan};
-  size_t off[2][7];
+  size_t off[2][8];
   for (int k = 0; k < 2; k++) {
     const RotPlanHost h = build_rot_plan(c->n, c->h_gates, k ? kRotShortChain : kRotChain);
     std::vector<RotOp> ops;
@@ -641,6 +666,8 @@ static int make_rot_plans(sqg_circuit* c) {
     off[k][4] = blob_put(blob, h.params.data(), h.params.size() * sizeof(int));
     off[k][5] = blob_put(blob, h.cta_params.data(), h.cta_params.size() * sizeof(int));
     off[k][6] = blob_put(blob, ends.data(), ends.size() * sizeof(int));
+    off[k][7] = blob_put(blob, h.heads.data(), h.heads.size() * sizeof(int));
+    p.nheads = (int)h.heads.size();
     if (k == 0) c->h_steps = h.steps;
   }
   cudaError_t e = cudaMalloc(&c->d_plan, blob.size());
@@ -657,6 +684,7 @@ static int make_rot_plans(sqg_circuit* c) {
     p.params = (const int*)(d + off[k][4]);
     p.cta_params = (const int*)(d + off[k][5]);
     p.ends = (const int*)(d + off[k][6]);
+    p.heads = (const int*)(d + off[k][7]);
   }
   return cuda_status(e, "circuit handle");
 }
@@ -787,14 +815,14 @@ static int cost_grad_args(const sqg_circuit* c, const double* theta, int B, cons
 }
 
 // Whether the tile kernels are faster than the environment-matrix evaluation where both can run.
-// Measured on GB300, environment matrix against tiles: three qubits 71 against 115 us (one vector,
-// 14 blocks), 434 against 1222 us (4096 vectors); four qubits, 40 blocks 322 against 228 us (one
-// vector), 1210 against 1045 us (1024), 10 blocks 130 against 110 us (one), 20 blocks 551 against 667
-// us (1024); five qubits, 3 blocks 164 against 74 us (one) and 254 against 236 us (512), 20 blocks 406
-// against 154 us and 1090 against 665 us.
+// Measured on GB300, environment matrix against tiles: three qubits, 14 blocks 71 against 116 us (one
+// vector), 434 against 551 us (4096); four qubits, 5 blocks 77 against 80 us (one) and 171 against 224
+// us (1024), 10 blocks 130 against 110 us (one), 20 blocks 551 against 488 us (1024), 40 blocks 322
+// against 226 us and 1210 against 790 us; five qubits, 3 blocks 164 against 74 us (one) and 254
+// against 225 us (512), 20 blocks 406 against 154 us and 1090 against 607 us.
 static bool tiles_first(const sqg_circuit* c, int B) {
   if (c->n >= 5) return true;
-  return c->n == 4 && c->L >= (B > 2 * device_sms() ? 96 : 32);
+  return c->n == 4 && c->L >= (B > 2 * device_sms() ? 48 : 32);
 }
 
 int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,

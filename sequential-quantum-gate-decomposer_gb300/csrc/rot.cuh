@@ -70,7 +70,7 @@ struct RotRec {
   double t, c;
   double2 zi, zo;
   double lo;
-  long long turn;
+  double turn;  // 0 or 1 (all members are doubles: batch_matrices_body keeps matrices here)
 };
 static_assert(sizeof(RotRec) == sizeof(GateMat), "the workspace counts both as 64 bytes");
 
@@ -83,8 +83,9 @@ struct RotPlan {
   const int* cta;  // runs [cta[i], cta[i + 1]) are handled by one CTA of kRotThreads threads
   const int* params;  // parameters of CTA i's runs: params[cta_params[i] .. cta_params[i + 1])
   const int* cta_params;
+  const int* heads;  // first runs of the chains, those of two and more runs first
   const int* ends;  // place of the amplitude 2^q behind the last operation (a sum of them: their XOR)
-  int nops, nrecs, ncta, noverlaps;
+  int nops, nrecs, ncta, noverlaps, nheads;
 };
 
 constexpr int kRotThreads = 128;  // runs per CTA of the per-instance kernels; no chain straddles two
@@ -259,40 +260,145 @@ __device__ __forceinline__ double split_u3(double2 cs, double2 phi, double2 lam,
   return c < 0.0 ? -1.0 : 1.0;
 }
 
-// The numbers of all operations of the runs of one CTA, for one parameter vector: thread i
-// makes the matrix of run i (the factors of a lone U3); the first thread of each chain of pushed
-// rotations then walks it.  phase_out receives the product of the runs' phases.
+// Matrix of a run (a lone U3: (cos, sin) of its three angles and phi lambda) from its CTA's
+// parameters.
+__device__ __forceinline__ void run_matrix(const RotPlan& pl, const RotRun& run, const double2* sc,
+                                           const double* theta, double2 M[4]) {
+  Gate g = pl.gates[pl.members[run.first]];
+  int soff = run.soff;
+  if (run.lone_u3) {
+    for (int k = 0; k < 3; k++) M[k] = param_sincos(sc, soff, theta + g.pstart, k);
+    M[3] = cmul(M[1], M[2]);
+    return;
+  }
+  gate_matrix(g.type, sc, soff, theta + g.pstart, M);
+  for (int k = 1; k < run.count; k++) {
+    double2 G[4];
+    if (soff >= 0) soff += gate_param_num(g.type);
+    g = pl.gates[pl.members[run.first + k]];
+    gate_matrix(g.type, sc, soff, theta + g.pstart, G);
+    matmul2(G, M);
+  }
+}
+
+// Walks the chain that starts with run `first` (a run by itself: a chain of one), mat(j, M)
+// giving the matrix of run j: writes their records, but for the cosines of rotations.  Returns
+// the phase that the chain leaves.
+template <class Mat>
+__device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotRec* recs, Mat mat) {
+  const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
+  // the rotation pushed into the next run: diag(1, pz) times pphase (zpend), or a unitary given
+  // by its first column (wp, wq); wdet: its determinant
+  bool zpend = true;
+  double2 pz = one, pphase = one, wp = one, wq = zero, wdet = one, own = one;
+  for (int step = 0; step < kRotChain; step++) {
+    const RotRun run = pl.runs[first + step];
+    RotRec r = {0.0, 1.0, one, one, 0.0, 0.0};
+    double2 M[4];
+    mat(first + step, run, M);
+    if (run.kind == kOpCry) {
+      r.t = M[2].x;
+      r.c = M[0].x;
+    } else if (run.kind == kOpPhase) {  // diagonal
+      r.zi = cunit(cmulc(M[3], M[0]));
+      own = M[0];
+    } else if (!(run.kind & kOpZi)) {  // Ry or Rx by itself: M[0] = cos, M[2] = sin or -i sin
+      const double2 cs = make_double2(M[0].x, (run.kind & kOpX) ? -M[2].y : M[2].x);
+      const double sign = split_u3(cs, one, one, r);
+      r.zi = one;
+      // about X the quarter turn is -i times the exchange
+      own = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
+    } else if (run.lone_u3 && zpend && (run.push == kAxisNone || run.push == kAxisZ)) {
+      const double2 lam = step ? cunit(cmul(M[2], pz)) : M[2];
+      pphase = cscale(pphase, split_u3(M[0], M[1], lam, r));
+      if (run.push == kAxisNone)
+        own = pphase;
+      else
+        pz = M[1], wdet = cmul(cmul(pphase, pphase), pz);
+    } else {
+      // A = M * pushed, by its first column (p, q) and its determinant
+      double2 p, q, d;
+      if (run.lone_u3) {  // cos and sin, phi, lambda and phi lambda
+        const double2 y = zpend ? make_double2(0.0, 0.0) : cmul(M[2], wq);
+        const double2 u = zpend ? pphase : wp;
+        p = make_double2(fma(M[0].x, u.x, -(M[0].y * y.x)), fma(M[0].x, u.y, -(M[0].y * y.y)));
+        q = cmul(M[1], make_double2(fma(M[0].y, u.x, M[0].x * y.x), fma(M[0].y, u.y, M[0].x * y.y)));
+        d = cmul(M[3], wdet);
+      } else {
+        p = zpend ? cmul(M[0], pphase) : cadd(cmul(M[0], wp), cmul(M[1], wq));
+        q = zpend ? cmul(M[2], pphase) : cadd(cmul(M[2], wp), cmul(M[3], wq));
+        d = cmul(csub(cmul(M[0], M[3]), cmul(M[1], M[2])), wdet);
+      }
+      if (run.push == kAxisNone || run.push == kAxisZ) {
+        // the second column of a unitary: (-conj q, conj p) det
+        const double2 A[4] = {p, cmulc(make_double2(-d.x, -d.y), q), q, cmulc(d, p)};
+        const double2 ph = split_zyz(A, r);
+        if (run.push == kAxisNone) {
+          own = ph;
+        } else {
+          zpend = true;
+          pphase = cunit(ph);
+          pz = r.zo;
+          wdet = cmul(cmul(pphase, pphase), pz);
+        }
+      } else {
+        // Y: with S = diag(1, i), S A S^dagger = Rx(-alpha) Ry(beta) diag(1, zi)
+        if (run.push == kAxisY) q = make_double2(-q.y, q.x);
+        split_x(p, q, d, r);
+        const double c2 = cnorm2(p) - cnorm2(q);
+        const double s2 = -2.0 * fma(p.x, q.y, -(p.y * q.x));  // sin of the full angle: -2 Im(conj(w0) w1)
+        zpend = false;
+        wp = p;
+        wq = run.push == kAxisY ? make_double2(q.y, -q.x) : q;
+        wdet = d;
+        r.zo = make_double2(c2, run.push == kAxisY ? -s2 : s2);
+      }
+    }
+    recs[run.rec] = r;
+    if (run.push == kAxisNone) break;
+  }
+  return own;
+}
+
+// The cosines of a run's record, and its share of the phase: a NaN anywhere (an infinite angle, say)
+// becomes one of the phase too, where sweeps in fixed point look for it.
+__device__ __forceinline__ double2 finish_record(const RotRun& run, RotRec& r, double2 phase) {
+  RotRec v = r;
+  if (run.kind & kOpRot) set_cosine(v);
+  r.c = v.c;
+  r.lo = v.lo;
+  phase.x = fma(0.0, v.t + v.c + v.zi.x + v.zi.y + v.zo.x + v.zo.y, phase.x);
+  return phase;
+}
+
+// Product of the threads' phases (kRotThreads of them), written by thread 0.
+__device__ __forceinline__ void phase_product(double2 phase, double2* out) {
+  __shared__ double2 ph[kRotThreads];
+  const int i = threadIdx.x;
+  ph[i] = phase;
+  __syncthreads();
+  for (int o = kRotThreads / 2; o > 0; o >>= 1) {
+    if (i < o) ph[i] = cmul(ph[i], ph[i + o]);
+    __syncthreads();
+  }
+  if (i == 0) *out = ph[0];
+}
+
+// The numbers of all operations of the runs of one CTA, for one parameter vector, in one go:
+// thread i makes the matrix of run i, the first thread of each chain walks it.  phase_out receives
+// the product of the runs' phases.
 __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const double* theta, RotRec* recs,
                                               double2* phase_out, int deal) {
   __shared__ double2 Ms[kRotThreads][4];
-  __shared__ double2 ph[kRotThreads];
   __shared__ int chain_of[kRotThreads], warp_heads[kRotThreads / 32];
-  const int base = pl.cta[cta], n = pl.cta[cta + 1] - base, i = threadIdx.x;
-  const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
   __shared__ double2 sc[kRotParams];
+  const int base = pl.cta[cta], n = pl.cta[cta + 1] - base, i = threadIdx.x;
   cta_sincos(pl, cta, theta, sc);
   __syncthreads();
   RotRun run;
-  double2 phase = one;
   if (i < n) {
     run = pl.runs[base + i];
-    double2 M[4];
-    Gate g = pl.gates[pl.members[run.first]];
-    int soff = run.soff;
-    if (run.lone_u3) {
-      for (int k = 0; k < 3; k++) M[k] = param_sincos(sc, soff, theta + g.pstart, k);
-      M[3] = cmul(M[1], M[2]);
-    } else {
-      gate_matrix(g.type, sc, soff, theta + g.pstart, M);
-      for (int k = 1; k < run.count; k++) {
-        double2 G[4];
-        if (soff >= 0) soff += gate_param_num(g.type);
-        g = pl.gates[pl.members[run.first + k]];
-        gate_matrix(g.type, sc, soff, theta + g.pstart, G);
-        matmul2(G, M);
-      }
-    }
-    for (int k = 0; k < 4; k++) Ms[i][k] = M[k];
+    run_matrix(pl, run, sc, theta, Ms[i]);
   }
   // Chains of two and more runs are few and take longest: they are dealt out over `deal` warps.  All
   // four where the launch waits for one CTA (as few as possible wait for one another's branches),
@@ -311,105 +417,66 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
   if (head) chain_of[(rank % deal) * 32 + rank / deal] = i;
   __syncthreads();
   const bool walks = warp < deal && lane * deal + warp < nheads;
+  double2 phase = make_double2(1.0, 0.0);
+  auto mat = [&](int j, const RotRun&, double2 M[4]) {
+    for (int k = 0; k < 4; k++) M[k] = Ms[j - base][k];
+  };
   for (int pass = 0; pass < 2; pass++) {
     // first the runs by themselves, each by its own thread, then the chains
     if (pass == 0 ? !(i < n && !run.pulled && run.push == kAxisNone) : !walks) continue;
-    // the rotation pushed into the next run: diag(1, pz) times pphase (zpend), or a unitary given
-    // by its first column (wp, wq); wdet: its determinant
-    bool zpend = true;
-    double2 pz = one, pphase = one, wp = one, wq = zero, wdet = one;
-    int j = pass == 0 ? i : chain_of[i];
-    double2 own = one;
-    for (int step = 0; step < kRotChain; step++, j++) {
-      if (pass || step) run = pl.runs[base + j];
-      RotRec r = {0.0, 1.0, one, one, 0.0, 0};
-      double2 M[4];
-      for (int k = 0; k < 4; k++) M[k] = Ms[j][k];
-      if (run.kind == kOpCry) {
-        r.t = M[2].x;
-        r.c = M[0].x;
-      } else if (run.kind == kOpPhase) {  // diagonal
-        r.zi = cunit(cmulc(M[3], M[0]));
-        own = M[0];
-      } else if (!(run.kind & kOpZi)) {  // Ry or Rx by itself: M[0] = cos, M[2] = sin or -i sin
-        const double2 cs = make_double2(M[0].x, (run.kind & kOpX) ? -M[2].y : M[2].x);
-        const double sign = split_u3(cs, one, one, r);
-        r.zi = one;
-        // about X the quarter turn is -i times the exchange
-        own = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
-      } else if (run.lone_u3 && zpend && (run.push == kAxisNone || run.push == kAxisZ)) {
-        const double2 lam = step ? cunit(cmul(M[2], pz)) : M[2];
-        pphase = cscale(pphase, split_u3(M[0], M[1], lam, r));
-        if (run.push == kAxisNone)
-          own = pphase;
-        else
-          pz = M[1], wdet = cmul(cmul(pphase, pphase), pz);
-      } else {
-        // A = M * pushed, by its first column (p, q) and its determinant
-        double2 p, q, d;
-        if (run.lone_u3) {  // cos and sin, phi, lambda and phi lambda
-          const double2 y = zpend ? make_double2(0.0, 0.0) : cmul(M[2], wq);
-          const double2 u = zpend ? pphase : wp;
-          p = make_double2(fma(M[0].x, u.x, -(M[0].y * y.x)), fma(M[0].x, u.y, -(M[0].y * y.y)));
-          q = cmul(M[1], make_double2(fma(M[0].y, u.x, M[0].x * y.x), fma(M[0].y, u.y, M[0].x * y.y)));
-          d = cmul(M[3], wdet);
-        } else {
-          p = zpend ? cmul(M[0], pphase) : cadd(cmul(M[0], wp), cmul(M[1], wq));
-          q = zpend ? cmul(M[2], pphase) : cadd(cmul(M[2], wp), cmul(M[3], wq));
-          d = cmul(csub(cmul(M[0], M[3]), cmul(M[1], M[2])), wdet);
-        }
-        if (run.push == kAxisNone || run.push == kAxisZ) {
-          // the second column of a unitary: (-conj q, conj p) det
-          const double2 A[4] = {p, cmulc(make_double2(-d.x, -d.y), q), q, cmulc(d, p)};
-          const double2 ph = split_zyz(A, r);
-          if (run.push == kAxisNone) {
-            own = ph;
-          } else {
-            zpend = true;
-            pphase = cunit(ph);
-            pz = r.zo;
-            wdet = cmul(cmul(pphase, pphase), pz);
-          }
-        } else {
-          // Y: with S = diag(1, i), S A S^dagger = Rx(-alpha) Ry(beta) diag(1, zi)
-          if (run.push == kAxisY) q = make_double2(-q.y, q.x);
-          split_x(p, q, d, r);
-          const double c2 = cnorm2(p) - cnorm2(q);
-          const double s2 = -2.0 * fma(p.x, q.y, -(p.y * q.x));  // sin of the full angle: -2 Im(conj(w0) w1)
-          zpend = false;
-          wp = p;
-          wq = run.push == kAxisY ? make_double2(q.y, -q.x) : q;
-          wdet = d;
-          r.zo = make_double2(c2, run.push == kAxisY ? -s2 : s2);
-        }
-      }
-      recs[run.rec] = r;
-      if (run.push == kAxisNone) break;
-    }
-    phase = cmul(phase, own);
+    phase = cmul(phase, walk_chain(pl, base + (pass == 0 ? i : chain_of[i]), recs, mat));
   }
-  ph[i] = phase;
   __syncthreads();
   // the cosines of all runs at once: the chains need not wait for them
-  if (i < n) {
-    const RotRun mine = pl.runs[base + i];
-    RotRec& r = recs[mine.rec];
-    RotRec v = r;
-    if (mine.kind & kOpRot) {
-      set_cosine(v);
-      r.c = v.c;
-      r.lo = v.lo;
-    }
-    // a NaN anywhere (an infinite angle, say) is one of the phase too: sweeps in fixed point look
-    // for it there
-    ph[i].x = fma(0.0, v.t + v.c + v.zi.x + v.zi.y + v.zo.x + v.zo.y, ph[i].x);
-  }
+  if (i < n) phase = finish_record(run, recs[run.rec], phase);
+  phase_product(phase, phase_out);
+}
+
+// The same in three launches for many parameter vectors, the matrices kept in the records: a
+// thread walks one chain of one vector, and the 32 of a warp the same chain of 32 vectors, so no
+// lane idles or takes another's branch.
+__device__ __forceinline__ void batch_matrices_body(const RotPlan& pl, int cta, const double* theta, RotRec* recs) {
+  __shared__ double2 sc[kRotParams];
+  const int base = pl.cta[cta], n = pl.cta[cta + 1] - base;
+  cta_sincos(pl, cta, theta, sc);
   __syncthreads();
-  for (int o = kRotThreads / 2; o > 0; o >>= 1) {
-    if (i < o) ph[i] = cmul(ph[i], ph[i + o]);
-    __syncthreads();
+  if ((int)threadIdx.x >= n) return;
+  const RotRun run = pl.runs[base + threadIdx.x];
+  double2 M[4];
+  run_matrix(pl, run, sc, theta, M);
+  double2* out = reinterpret_cast<double2*>(recs + run.rec);
+  for (int k = 0; k < 4; k++) out[k] = M[k];
+}
+// The phase of a chain is left in the place of its last run's cosine.
+__device__ __forceinline__ void batch_chain_body(const RotPlan& pl, int head, RotRec* recs) {
+  int last = 0;
+  auto mat = [&](int, const RotRun& run, double2 M[4]) {
+    const double2* in = reinterpret_cast<const double2*>(recs + run.rec);
+    for (int k = 0; k < 4; k++) M[k] = in[k];
+    last = run.rec;
+  };
+  const int first = pl.heads[head];
+  const double2 phase = walk_chain(pl, first, recs, mat);
+  if (pl.runs[first].kind == kOpCry) return;  // its cosine is in use, its phase 1
+  recs[last].c = phase.x;
+  recs[last].lo = phase.y;
+}
+__device__ __forceinline__ void batch_finish_body(const RotPlan& pl, int cta, RotRec* recs, double2* phase_out) {
+  const int base = pl.cta[cta], n = pl.cta[cta + 1] - base;
+  double2 phase = make_double2(1.0, 0.0);
+  if ((int)threadIdx.x < n) {
+    const RotRun run = pl.runs[base + threadIdx.x];
+    RotRec r = recs[run.rec];
+    if (run.kind != kOpCry) {
+      if (run.push == kAxisNone) phase = make_double2(r.c, r.lo);
+      r.c = 1.0;
+      r.lo = 0.0;
+    }
+    phase = finish_record(run, r, phase);
+    recs[run.rec].c = r.c;
+    recs[run.rec].lo = r.lo;
   }
-  if (i == 0) *phase_out = ph[0];
+  phase_product(phase, phase_out);
 }
 
 // ---- application ---------------------------------------------------------------------------
@@ -436,7 +503,7 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
   const int lane = threadIdx.x;
   const bool on = lane < kn;
   RotOp op = {kOpCnot, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  RotRec r = {0.0, 1.0, make_double2(1.0, 0.0), make_double2(1.0, 0.0), 0.0, 0};
+  RotRec r = {0.0, 1.0, make_double2(1.0, 0.0), make_double2(1.0, 0.0), 0.0, 0.0};
   if (on) {
     op = ops[k0 + lane];
     if (op.kind >= kOpCry) r = recs[op.rec];

@@ -17,7 +17,7 @@ struct RotStep {
 struct RotPlanHost {
   std::vector<RotStep> steps;
   std::vector<RotRun> runs;
-  std::vector<int> members, cta, params, cta_params;
+  std::vector<int> members, cta, params, cta_params, heads;
   int noverlaps = 0;
 };
 
@@ -182,6 +182,9 @@ inline RotPlanHost build_rot_plan(int n, const std::vector<Gate>& gates, int max
     }
   }
   if ((int)pl.runs.size() > pl.cta.back()) close_cta();
+  for (int longer = 1; longer >= 0; longer--)
+    for (int i = 0; i < (int)pl.runs.size(); i++)
+      if (!pl.runs[i].pulled && (pl.runs[i].push != kAxisNone) == (longer == 1)) pl.heads.push_back(i);
   return pl;
 }
 

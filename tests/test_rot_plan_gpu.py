@@ -111,3 +111,18 @@ def test_ragged_plans_share_a_launch(sqg):
             rc, rg = O.cost_grad(cs[i].qbit_num, cs[i].gate_records(), th[i], ts[i], variant=variant)
             close(c, rc)
             close(g.cpu().numpy(), rg)
+
+
+@pytest.mark.parametrize("batch", [1, 31, 32, 33, 70])
+def test_batches_make_the_same_numbers(sqg, batch):
+    """Plans of many vectors are made in three launches, those of a few in one."""
+    c = circuit(sqg, 5, "mixed", 60)
+    recs, P = c.gate_records(), c.get_Parameter_Num()
+    rng = np.random.default_rng(batch)
+    p = np.concatenate([angles(P, "eighths")[None], rng.uniform(0, 2 * np.pi, (batch - 1, P))])
+    T = np.linalg.qr(rng.standard_normal((32, 32)) + 1j * rng.standard_normal((32, 32)))[0][:, :17].copy()
+    cost, grad = sqg.CostEvaluator(c, T).cost_grad(torch.from_numpy(p).cuda())
+    for b in {0, batch // 2, batch - 1}:
+        rc, rg = O.cost_grad(5, recs, p[b], T)
+        close(cost[b].item(), rc)
+        close(grad[b].cpu().numpy(), rg)
