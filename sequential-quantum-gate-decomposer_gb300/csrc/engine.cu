@@ -467,16 +467,21 @@ size_t blob_put(std::vector<char>& blob, const void* src, size_t bytes) {
 // is then split gate by gate).  Fills the chunk with further qubits (lowest first), maps every
 // gate of the block to chunk-local qubit positions and tabulates the global offsets of the
 // chunk's high local bits and the qubits that number the chunks.
-int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
-  const int n = c->n, K = std::min(n, kStateK), low = std::min(K, kStateLow);
-  c->sK = K;
+struct StatePlanHost {
   std::vector<RotOp> lops;
-  std::vector<int> lends;
+  std::vector<int> lends, hitab, inact;
+  std::vector<sqg_state_block> blocks;
+};
+StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<int>& cuts) {
+  const int n = c->n, low = std::min(K, kStateLow);
+  StatePlanHost out;
+  std::vector<RotOp>& lops = out.lops;
+  std::vector<int>&lends = out.lends, &hitab = out.hitab, &inact = out.inact;
   size_t done = 0;  // steps placed in blocks (they follow the order of their anchor gates)
-  std::vector<int> hitab, inact;
-  std::vector<int> inA(n, 0);
+  std::vector<int> inA(n, 0), A, loc(n);
+  lops.reserve(c->h_steps.size() + 16);
   auto close_block = [&](int g0, int g1) {
-    std::vector<int> A;
+    A.clear();
     for (int q = 0; q < n; q++)
       if (q < low || inA[q]) A.push_back(q);
     for (int q = 0; q < n && (int)A.size() < K; q++)
@@ -485,21 +490,18 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
         inA[q] = 1;
       }
     std::sort(A.begin(), A.end());
-    std::vector<int> loc(n, -1);
+    std::fill(loc.begin(), loc.end(), -1);
     for (int j = 0; j < (int)A.size(); j++) loc[A[j]] = j;
     const int s0 = (int)done, k0 = (int)lops.size();
     while (done < c->h_steps.size() && c->h_steps[done].anchor < g1) done++;
     lower_rot_steps(c->h_steps, s0, (int)done, K, loc, lops, lends);
-    lends.resize(16 * (c->sblocks.size() + 1), 0);
+    lends.resize(16 * (out.blocks.size() + 1), 0);
     (void)g0;
     const int hb = K - low;
-    for (int h = 0; h < 128; h++) {
-      int off = 0;
-      if (h < (1 << hb))
-        for (int j = 0; j < hb; j++)
-          if ((h >> j) & 1) off |= 1 << A[low + j];
-      hitab.push_back(off);
-    }
+    const size_t h0 = hitab.size();
+    hitab.resize(h0 + 128, 0);
+    for (int h = 1; h < (1 << hb); h++)
+      hitab[h0 + h] = hitab[h0 + (h & (h - 1))] | 1 << A[low + __builtin_ctz(h)];
     int k = 0;
     for (int q = 0; q < n; q++)
       if (loc[q] < 0) {
@@ -507,7 +509,7 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
         k++;
       }
     for (; k < 32; k++) inact.push_back(0);
-    c->sblocks.push_back({k0, (int)lops.size()});
+    out.blocks.push_back({k0, (int)lops.size()});
     std::fill(inA.begin(), inA.end(), 0);
   };
   int g0 = 0, used = 0;
@@ -565,20 +567,63 @@ int build_state_plan(sqg_circuit* c, const std::vector<int>& cuts = {}) {
     }
   }
   if (c->L > 0) close_block(g0, c->L);
-  if (c->L == 0) return SQG_OK;
+  return out;
+}
+
+// Makes the state-vector plans of the circuit: chunks of 2^12 amplitudes, and, for registers whose
+// chunks are too few for the device, smaller ones down to 2^9.
+int make_state_plans(sqg_circuit* c, const std::vector<int>& cuts = {}) {
+  c->splans.clear();
   std::vector<char> blob;
-  const size_t o_ops = blob_put(blob, lops.data(), lops.size() * sizeof(RotOp));
-  const size_t o_ends = blob_put(blob, lends.data(), lends.size() * sizeof(int));
-  const size_t o_hi = blob_put(blob, hitab.data(), hitab.size() * sizeof(int));
-  const size_t o_in = blob_put(blob, inact.data(), inact.size() * sizeof(int));
+  std::vector<size_t> off;
+  const int largest = std::min(c->n, kStateK);
+  for (int K = largest; K >= (c->n <= 20 ? std::min(largest, 9) : largest); K--) {
+    const StatePlanHost h = build_state_plan(c, K, cuts);
+    sqg_state_plan p;
+    p.K = K;
+    p.nops = (int)h.lops.size();
+    p.blocks = h.blocks;
+    c->splans.push_back(p);
+    off.push_back(blob_put(blob, h.lops.data(), h.lops.size() * sizeof(RotOp)));
+    off.push_back(blob_put(blob, h.lends.data(), h.lends.size() * sizeof(int)));
+    off.push_back(blob_put(blob, h.hitab.data(), h.hitab.size() * sizeof(int)));
+    off.push_back(blob_put(blob, h.inact.data(), h.inact.size() * sizeof(int)));
+  }
+  if (blob.empty()) return SQG_OK;
   cudaError_t e = cudaMalloc(&c->d_state, blob.size());
   if (e == cudaSuccess) e = cudaMemcpy(c->d_state, blob.data(), blob.size(), cudaMemcpyHostToDevice);
   const char* d = (const char*)c->d_state;
-  c->d_lops = (RotOp*)(d + o_ops);
-  c->d_lends = (int*)(d + o_ends);
-  c->d_hitab = (int*)(d + o_hi);
-  c->d_inact = (int*)(d + o_in);
+  for (size_t k = 0; k < c->splans.size(); k++) {
+    sqg_state_plan& p = c->splans[k];
+    p.d_lops = (const RotOp*)(d + off[4 * k]);
+    p.d_lends = (const int*)(d + off[4 * k + 1]);
+    p.d_hitab = (const int*)(d + off[4 * k + 2]);
+    p.d_inact = (const int*)(d + off[4 * k + 3]);
+  }
   return cuda_status(e, "state plan");
+}
+
+// The plan for `batch` states: the least of the modelled times.  An operation takes 1 ns per
+// amplitude of an SM's chunks (the FP64 pipe), at least 0.7 us (its latency and the barrier), a block
+// two operations' worth for loading and storing and 2.5 us for its launch.  Measured on GB300, 300 to
+// 400 gates, chunks of 2^12 against the choice: 12 qubits 1146 -> 454 us, 15 qubits, 7 states 1247 ->
+// 858 us, 17 qubits 1808 -> 760 us, 20 qubits 3162 -> 2111 us (the first and the last two before the
+// rotation plan).
+const sqg_state_plan& choose_state_plan(const sqg_circuit* c, int batch) {
+  const int sms = device_sms();
+  const sqg_state_plan* best = &c->splans[0];
+  double best_t = 0.0;
+  for (const sqg_state_plan& p : c->splans) {
+    const double ctas = (double)batch * (double)(1LL << (c->n - p.K));
+    const double per_sm = ctas <= 4.0 * sms ? (double)(((long long)ctas + sms - 1) / sms) : ctas / sms;
+    const double op = std::max(0.7, per_sm * (1 << p.K) * 1e-3);
+    const double t = p.nops * op + p.blocks.size() * (2.0 * op + 2.5);
+    if (&p == best || t < best_t) {
+      best = &p;
+      best_t = t;
+    }
+  }
+  return *best;
 }
 
 // One block of gates applied to every chunk of 2^K amplitudes of a state vector.  The
@@ -613,6 +658,7 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   double2* base = a.states + (long long)b * a.stride + cbase;
   __syncthreads();
   for (int l = threadIdx.x; l < KK; l += blockDim.x) sv[l] = base[(l & lowmask) + hit[l >> a.low]];
+  __syncthreads();  // a block of CNOTs alone has no operation, only places to exchange
   const RotRec* recs = a.recs + (long long)b * a.nrecs;
   for (int k0 = a.k0; k0 < a.k1; k0 += kRotChunk) {
     const int kn = min(kRotChunk, a.k1 - k0);
@@ -645,7 +691,8 @@ static int make_rot_plans(sqg_circuit* c) {
   const size_t o_gates = blob_put(blob, c->h_gates.data(), c->h_gates.size() * sizeof(Gate));
   RotPlan* plans[2] = {&c->plan, &c->short_plan};
   size_t off[2][8];
-  for (int k = 0; k < 2; k++) {
+  const int nplans = c->n <= kMatrixQubits ? 2 : 1;  // state vectors use the first alone
+  for (int k = 0; k < nplans; k++) {
     const RotPlanHost h = build_rot_plan(c->n, c->h_gates, k ? kRotShortChain : kRotChain);
     std::vector<RotOp> ops;
     std::vector<int> ends;
@@ -674,7 +721,7 @@ static int make_rot_plans(sqg_circuit* c) {
   if (e == cudaSuccess) e = cudaMemcpy(c->d_plan, blob.data(), blob.size(), cudaMemcpyHostToDevice);
   const char* d = (const char*)c->d_plan;
   c->d_gates = (Gate*)(d + o_gates);
-  for (int k = 0; k < 2; k++) {
+  for (int k = 0; k < nplans; k++) {
     RotPlan& p = *plans[k];
     p.gates = c->d_gates;
     p.ops = (const RotOp*)(d + off[k][0]);
@@ -746,7 +793,7 @@ int sqg_circuit_create(int qbit_num, const sqg_gate* gates, int gate_num, sqg_ci
   c->P = p;
   cudaGetDevice(&c->device);
   int st = make_rot_plans(c);
-  if (!st) st = build_state_plan(c);
+  if (!st) st = make_state_plans(c);
   if (st) {
     sqg_circuit_destroy(c);
     return st;
@@ -768,8 +815,7 @@ int sqg_circuit_set_partitions(sqg_circuit* c, const int* part_ends, int nparts)
   if (dev != c->device) return fail(SQG_ERR_INVALID_ARGUMENT, "circuit handle belongs to another device");
   cudaFree(c->d_state);
   c->d_state = nullptr;
-  c->sblocks.clear();
-  return build_state_plan(c, cuts);
+  return make_state_plans(c, cuts);
 }
 
 int sqg_circuit_destroy(sqg_circuit* c) {
@@ -1133,7 +1179,7 @@ size_t sqg_state_workspace_bytes(const sqg_circuit* c, int batch) {
   return prep_layout(c, batch, 0).end;
 }
 
-int sqg_state_block_count(const sqg_circuit* c) { return c ? (int)c->sblocks.size() : -1; }
+int sqg_state_block_count(const sqg_circuit* c) { return c ? (int)c->splans[0].blocks.size() : -1; }
 
 int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* states, long long stride, int fused,
                     void* workspace, size_t ws_bytes, void* stream) {
@@ -1148,28 +1194,29 @@ int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* stat
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = (char*)workspace;
   if (fused) {
-    const size_t smem = sizeof(double2) << c->sK;
-    if ((st = set_smem(k_state_block, smem))) return st;
+    const sqg_state_plan& sp = choose_state_plan(c, B);
+    const size_t smem = sizeof(double2) << sp.K;
+    if ((st = set_smem(k_state_block, sizeof(double2) << c->splans[0].K))) return st;
     TileArgs t;
     if ((st = launch_plan(c, c->plan, theta, c->P, B, rot_layout(c->plan, B, 0), ws, t, s))) return st;
     StateArgs a;
     a.states = (double2*)states;
     a.stride = stride;
     a.n = c->n;
-    a.K = c->sK;
-    a.low = std::min(c->sK, kStateLow);
+    a.K = sp.K;
+    a.low = std::min(sp.K, kStateLow);
     a.nrecs = t.nrecs;
-    a.lops = c->d_lops;
+    a.lops = sp.d_lops;
     a.recs = t.recs;
     a.nphase = t.nphase;
-    for (size_t k = 0; k < c->sblocks.size(); k++) {
-      a.k0 = c->sblocks[k].k0;
-      a.k1 = c->sblocks[k].k1;
+    for (size_t k = 0; k < sp.blocks.size(); k++) {
+      a.k0 = sp.blocks[k].k0;
+      a.k1 = sp.blocks[k].k1;
       a.phases = k == 0 && t.nphase > 0 ? t.phases : nullptr;
-      a.ends = c->d_lends + 16 * k;
-      a.hitab = c->d_hitab + 128 * k;
-      a.inact = c->d_inact + 32 * k;
-      k_state_block<<<dim3(1u << (c->n - c->sK), B), kStateThreads, smem, s>>>(a);
+      a.ends = sp.d_lends + 16 * k;
+      a.hitab = sp.d_hitab + 128 * k;
+      a.inact = sp.d_inact + 32 * k;
+      k_state_block<<<dim3(1u << (c->n - sp.K), B), kStateThreads, smem, s>>>(a);
     }
     return cuda_status(cudaGetLastError(), "k_state_block");
   }

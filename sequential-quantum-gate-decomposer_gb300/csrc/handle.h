@@ -13,6 +13,16 @@ struct sqg_state_block {
   int k0, k1;  // operations [k0, k1) of the state-vector plan
 };
 
+// A plan of such passes: chunk qubits K, blocks, operations on chunk-local qubits, per block the
+// places behind its last operation (K ints, padded to 16), the global offsets of the chunk's high
+// local bits (2^(K - low) ints, padded to 128) and the qubits that number the chunks (padded to 32).
+struct sqg_state_plan {
+  int K = 0, nops = 0;
+  std::vector<sqg_state_block> blocks;
+  const sqg::RotOp* d_lops = nullptr;
+  const int *d_lends = nullptr, *d_hitab = nullptr, *d_inact = nullptr;
+};
+
 struct sqg_circuit {
   int n = 0, N = 0, L = 0, P = 0;
   int device = 0;
@@ -24,17 +34,9 @@ struct sqg_circuit {
   std::vector<sqg::RotStep> h_steps;
   void* d_plan = nullptr;
   sqg::RotPlan plan = {}, short_plan = {};
-  // state-vector plan: chunk qubits K, blocks, operations on chunk-local qubits, per block the
-  // places behind its last operation (K ints, padded to 16), the global offsets of the chunk's
-  // high local bits (2^(K - low) ints, padded to 128) and the qubits that number the chunks
-  // (padded to 32)
-  int sK = 0;
-  std::vector<sqg_state_block> sblocks;
-  void* d_state = nullptr;  // the arrays' allocation
-  sqg::RotOp* d_lops = nullptr;
-  int* d_lends = nullptr;
-  int* d_hitab = nullptr;
-  int* d_inact = nullptr;
+  // state-vector plans, the first with the largest chunks; their device arrays are one allocation
+  std::vector<sqg_state_plan> splans;
+  void* d_state = nullptr;
 };
 
 namespace sqg {

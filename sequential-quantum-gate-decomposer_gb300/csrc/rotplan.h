@@ -194,7 +194,7 @@ inline void lower_rot_steps(const std::vector<RotStep>& steps, int k0, int k1, i
                             std::vector<RotOp>& ops, std::vector<int>& ends) {
   // qubit q of the amplitude at place p is the parity of p & row[q]; the amplitude with bit q
   // changed is at p ^ pair[q].  A CNOT adds its control's row to its target's.
-  std::vector<unsigned> row(n), pair(n);
+  unsigned row[32], pair[32];
   for (int q = 0; q < n; q++) row[q] = pair[q] = 1u << q;
   struct Cz {
     unsigned a, b;

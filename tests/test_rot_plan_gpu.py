@@ -126,3 +126,23 @@ def test_batches_make_the_same_numbers(sqg, batch):
         rc, rg = O.cost_grad(5, recs, p[b], T)
         close(cost[b].item(), rc)
         close(grad[b].cpu().numpy(), rg)
+
+
+@pytest.mark.parametrize("n,batch", [(9, 1), (10, 3), (13, 1), (14, 2), (16, 1), (17, 1)])
+def test_states_in_small_chunks(sqg, n, batch):
+    """Registers whose chunks would leave the device idle are applied in smaller ones, with blocks of
+    CNOTs alone among them."""
+    rng = np.random.default_rng(n)
+    c = circuit(sqg, n, "random", 120)
+    for k in range(40):
+        c.add_CNOT(*(int(q) for q in rng.choice(n, 2, replace=False)))
+    for q in range(0, n, 3):
+        c.add_U3(q)
+    recs, P = c.gate_records(), c.get_Parameter_Num()
+    p = rng.uniform(0, 2 * np.pi, (batch, P))
+    v = rng.standard_normal((batch, 1 << n)) + 1j * rng.standard_normal((batch, 1 << n))
+    v /= np.linalg.norm(v, axis=1, keepdims=True)
+    d = torch.from_numpy(v.copy()).cuda()
+    c.apply_state_device(torch.from_numpy(p).cuda(), d)
+    for b in range(batch):
+        close(d[b].cpu().numpy(), O.apply_to(n, recs, p[b], v[b].reshape(-1, 1).copy()).reshape(-1))
