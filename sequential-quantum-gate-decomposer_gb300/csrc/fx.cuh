@@ -10,9 +10,9 @@
 // Cost and gradient are sums over all amplitudes, so an absolute resolution is what they need;
 // matrices and state vectors that go back to the caller stay in FP64.  Tiles with infinities or
 // NaN, and sweeps with checkpoints, stay in FP64 too.
-// GB300, FP64 sweeps -> these: gradient at 8 qubits, 360 blocks, 128 vectors 179 -> 79 ms; at 10
-// qubits, 300 blocks, 6 vectors 116 -> 51 ms; cost alone at 8 qubits, 120 blocks, 200 vectors 24.7
-// -> 10.6 ms.  Error of the gradient against 64-bit reference values: 3.2e-14 (3.1e-14) at 8 and
+// GB300, FP64 sweeps -> these: gradient at 8 qubits, 360 blocks, 128 vectors 179 -> 75 ms; at 10
+// qubits, 300 blocks, 6 vectors 116 -> 49 ms; cost alone at 8 qubits, 120 blocks, 200 vectors 24.7
+// -> 10.4 ms.  Error of the gradient against 64-bit reference values: 3.2e-14 (3.1e-14) at 8 and
 // 8.9e-14 (8.9e-14) at 10 qubits.
 #pragma once
 #include "rot.cuh"
@@ -179,13 +179,16 @@ __device__ __forceinline__ void fx_signs(const OpPlaces& pl, int ix, int iy, Fx2
   }
 }
 
-// stage_ops with the numbers encoded.
+// stage_ops with the numbers encoded; mfac times `unit`, what 2^60 of a sum of overlaps
+// is worth: done here once per chunk, not in the serial end of each operation.
 template <bool FWD>
-__device__ __forceinline__ void fx_stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn) {
+__device__ __forceinline__ void fx_stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn,
+                                             double unit) {
   stage_ops<FWD, kFxGroup>(st, ops, recs, k0, kn);
   if ((int)threadIdx.x >= kn) return;  // each thread the operation that it staged
   StagedOp& s = st[threadIdx.x];
   auto enc = [](double c) { return __longlong_as_double((long long)fx_encode(c)); };
+  if (!FWD) s.mfac *= unit;
   s.t = enc(s.t);
   s.scale = enc(s.scale);
   s.zi = make_double2(enc(s.zi.x), enc(s.zi.y));

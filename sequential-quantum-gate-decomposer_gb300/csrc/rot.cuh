@@ -535,8 +535,11 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
     s.pad = 0;
     s.scale = all;
     s.t = rescale ? r.t * all : r.t;
-    const double inv = 1.0 / (pre + plo);
-    s.mfac = lane < last ? inv * inv : 1.0;
+    s.mfac = 1.0;
+    if (!FWD && lane < last) {
+      const double inv = fast_rcp(pre + plo);
+      s.mfac = inv * inv;
+    }
     s.zi = op.kind == kOpCry ? make_double2(r.c, 0.0) : r.zi;
     s.zo = r.zo;
     st[lane] = s;

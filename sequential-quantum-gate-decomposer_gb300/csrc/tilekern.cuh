@@ -180,7 +180,7 @@ __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int 
     const int kn = min(kRotChunk, a.nops - k0);
     __syncthreads();  // the previous chunk's operations are no longer read
     if (!WRITE_BACK && fixed)
-      fx_stage_ops<true>(st, a.ops, recs, k0, kn);
+      fx_stage_ops<true>(st, a.ops, recs, k0, kn, 1.0);
     else
       stage_ops<DIR == kRotFwd, kRotGroup>(st, a.ops, recs, k0, kn);
     __syncthreads();
@@ -357,7 +357,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
     const int k0 = q * kRotChunk, kn = min(kRotChunk, a.nops - k0);
     __syncthreads();
     if (fixed)
-      fx_stage_ops<true>(st, a.ops, recs, k0, kn);
+      fx_stage_ops<true>(st, a.ops, recs, k0, kn, 1.0);
     else
       stage_ops<true, kRotGroup>(st, a.ops, recs, k0, kn);
     __syncthreads();
@@ -385,7 +385,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   int pend_coff = 0, pend_mask = 0, pend_aw = 0, buf = 0;
   double pend_fac = 0.0;
   const int shift = fx_sum_shift(tc);
-  const double fx_unit = 0x1p-60 * (double)(1 << shift);
+  const double fx_unit = fixed ? (double)(1 << shift) * (unit.a * unit.b) : 1.0;
   auto flush = [&]() {  // one thread per measured overlap
     if (!pend_mask || warp != nw - 1 || lane >= 3) return;
     const int axis = lane;  // 0 X, 1 Y, 2 Z
@@ -396,7 +396,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
       if (fixed) {
         long long v = 0;
         for (int w = 0; w < pend_aw; w++) v += __double_as_longlong(rd[w * NV + k]);
-        return (double)v * fx_unit * unit.a * unit.b * pend_fac;
+        return (double)v * 0x1p-60 * pend_fac;
       }
       double v = 0.0;
       for (int w = 0; w < pend_aw; w++) v += rd[w * NV + k];
@@ -416,7 +416,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
     const int k0 = q * kRotChunk, kn = min(kRotChunk, a.nops - k0);
     __syncthreads();
     if (fixed)
-      fx_stage_ops<false>(st, a.ops, recs, k0, kn);
+      fx_stage_ops<false>(st, a.ops, recs, k0, kn, fx_unit);
     else
       stage_ops<false, kRotGroup>(st, a.ops, recs, k0, kn);
     __syncthreads();
