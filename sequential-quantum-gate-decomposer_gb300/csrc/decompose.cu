@@ -80,7 +80,7 @@ struct Sh {
 // Gate matrices of parameter vector xv: one sincos per parameter (threads over
 // parameters, so every warp instruction of the FP64 series works on full warps), then the
 // 2x2 kernels from the stored (sin, cos) (threads over gates).  Same formulas as
-// build_gate_mats.
+// k_prep in engine.cu.
 __device__ void dec_build(const DecArgs& a, const Sh& sh, const double* xv) {
   for (int p = threadIdx.x; p < a.P; p += blockDim.x) {
     double s, c;
@@ -460,8 +460,7 @@ __device__ __noinline__ double dec_eval(const DecArgs& a, const Sh& sh, const do
   adjoint_sweep(sh.psi, sh.lam, N, a.n, cols, sh.gates, sh.gm, sh.sc, a.L, sh.redd, sh.tot,
                 [&](int g, const Gate&, const double* R) {
                   if (threadIdx.x < 8) Rb[g * 8 + threadIdx.x] = R[threadIdx.x];
-                },
-                [](int) {});
+                });
   __syncthreads();
   return dec_finish(a, sh, tr, gv);
 }

@@ -139,34 +139,16 @@ __device__ __forceinline__ double2 tile_trace(const double2* s, int N, int tc, i
 // Im R10, Re R11, Im R11) and sink(g, gate, tot) is called by every thread.
 // Only the warps that own amplitude pairs of the gate take part in the reduction: the
 // FP64 pipe is charged per warp instruction whatever the number of active lanes.
-// redd: kTileMaxWarps * 8 doubles, tot: 8 doubles.  restore(g) is called at the start of
-// each reverse step and may overwrite psi (checkpoints); it must contain its own barriers.
-// stage_gates / stage_mats (kStage entries each, or null): shared-memory staging of the
-// gate records and matrices when gates / gm are in global memory.
-constexpr int kStage = 32;
-
-template <class Sink, class Restore>
+// redd: kTileMaxWarps * 8 doubles, tot: 8 doubles.
+template <class Sink>
 __device__ __forceinline__ void adjoint_sweep(double2* psi, double2* lam, int N, int logN, int tc, const Gate* gates,
                                               const GateMat* gm, const double2* sc, int L, double* redd, double* tot,
-                                              Sink sink, Restore restore, Gate* stage_gates = nullptr,
-                                              GateMat* stage_mats = nullptr) {
+                                              Sink sink) {
   const int nw = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool staged = stage_gates != nullptr;
   for (int g = L - 1; g >= 0; g--) {
-    const int j = (L - 1 - g) % kStage;  // position of gate g in its staged chunk
-    if (staged && j == 0) {
-      __syncthreads();
-      const int kn = min(kStage, g + 1);
-      if ((int)threadIdx.x < kn) {
-        stage_gates[threadIdx.x] = gates[g - threadIdx.x];
-        stage_mats[threadIdx.x] = gm[g - threadIdx.x];
-      }
-      __syncthreads();
-    }
-    restore(g);
-    Gate gt = staged ? stage_gates[j] : gates[g];
-    PairOp op = make_op(gt.type, staged ? stage_mats[j] : gm[g], ORIENT_ADJ);
+    Gate gt = gates[g];
+    PairOp op = make_op(gt.type, gm[g], ORIENT_ADJ);
     const int np = gate_param_num(gt.type);
     if (np == 0) {
       tile_apply(psi, N, logN, tc, gt, op);
@@ -240,36 +222,6 @@ __device__ __forceinline__ double2 contract_derivative(const Gate& gt, const dou
     ti = fma(D[q].x, ri, fma(D[q].y, rr, ti));
   }
   return make_double2(tr, ti);
-}
-
-// Builds the gate matrices and per-parameter (sin, cos) of one parameter vector
-// (threads over gates).  Same formulas as k_prep in engine.cu.
-__device__ __forceinline__ void build_gate_mats(const Gate* gates, int L, const double* th, GateMat* gm, double2* sc) {
-  for (int g = threadIdx.x; g < L; g += blockDim.x) {
-    Gate gt = gates[g];
-    GateMat m;
-    m.u[0] = m.u[1] = m.u[2] = m.u[3] = make_double2(0.0, 0.0);
-    if (gt.type == G_U3) {
-      double st, ct, sp, cp, sl, cl;
-      sincos(th[gt.pstart], &st, &ct);
-      sincos(th[gt.pstart + 1], &sp, &cp);
-      sincos(th[gt.pstart + 2], &sl, &cl);
-      sc[gt.pstart] = make_double2(st, ct);
-      sc[gt.pstart + 1] = make_double2(sp, cp);
-      sc[gt.pstart + 2] = make_double2(sl, cl);
-      double spl = sp * cl + cp * sl, cpl = cp * cl - sp * sl;
-      m.u[0] = make_double2(ct, 0.0);
-      m.u[1] = make_double2(-st * cl, -st * sl);
-      m.u[2] = make_double2(st * cp, st * sp);
-      m.u[3] = make_double2(ct * cpl, ct * spl);
-    } else if (gate_param_num(gt.type) == 1) {
-      double s, c;
-      sincos(th[gt.pstart], &s, &c);
-      sc[gt.pstart] = make_double2(s, c);
-      m.u[0] = make_double2(c, s);
-    }
-    gm[g] = m;
-  }
 }
 
 }  // namespace sqg

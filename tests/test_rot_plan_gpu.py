@@ -146,3 +146,31 @@ def test_states_in_small_chunks(sqg, n, batch):
     c.apply_state_device(torch.from_numpy(p).cuda(), d)
     for b in range(batch):
         close(d[b].cpu().numpy(), O.apply_to(n, recs, p[b], v[b].reshape(-1, 1).copy()).reshape(-1))
+
+
+@pytest.mark.parametrize("n,gates,batch", [(3, 40, 2), (4, 31, 1), (4, 32, 1), (4, 47, 400), (4, 48, 400), (5, 1, 1),
+                                           (5, 60, 3)])
+def test_small_registers_with_and_without_a_workspace(sqg, n, gates, batch):
+    """Up to five qubits the environment-matrix evaluation takes the calls that bring no workspace,
+    and those where it is the faster one; both agree with the oracle."""
+    from importlib import import_module
+    native = import_module("sequential-quantum-gate-decomposer_gb300._native")
+    c = circuit(sqg, n, "random", gates)
+    recs, P = c.gate_records(), c.get_Parameter_Num()
+    rng = np.random.default_rng(gates)
+    p = rng.uniform(0, 2 * np.pi, (batch, P))
+    N = 1 << n
+    T = np.linalg.qr(rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N)))[0]
+    th, tgt = torch.from_numpy(p).cuda(), torch.from_numpy(T.copy()).cuda()
+    ev = sqg.CostEvaluator(c, T)
+    room = torch.empty(ev.workspace_bytes(batch, True), dtype=torch.uint8, device="cuda")
+    for ws, size in ((None, 0), (room.data_ptr(), room.numel() // 2), (room.data_ptr(), room.numel())):
+        cost = torch.full((batch,), np.nan, dtype=torch.float64, device="cuda")
+        grad = torch.full((batch, P), np.nan, dtype=torch.float64, device="cuda")
+        native.check(native.lib().sqg_cost_grad(
+            ev.native.handle, th.data_ptr(), batch, tgt.data_ptr(), N, 0, 0, 0, cost.data_ptr(), grad.data_ptr(), 0, ws,
+            size, torch.cuda.current_stream().cuda_stream), "sqg_cost_grad")
+        for b in {0, batch - 1}:
+            rc, rg = O.cost_grad(n, recs, p[b], T)
+            close(cost[b].item(), rc)
+            close(grad[b].cpu().numpy(), rg)
