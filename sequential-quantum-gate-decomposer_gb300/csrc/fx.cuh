@@ -12,8 +12,8 @@
 // NaN, and sweeps with checkpoints, stay in FP64 too.
 // GB300, FP64 sweeps -> these: gradient at 8 qubits, 360 blocks, 128 vectors 179 -> 75 ms; at 10
 // qubits, 300 blocks, 6 vectors 116 -> 49 ms; cost alone at 8 qubits, 120 blocks, 200 vectors 24.7
-// -> 10.4 ms.  Error of the gradient against 64-bit reference values: 3.2e-14 (3.1e-14) at 8 and
-// 8.9e-14 (8.9e-14) at 10 qubits.
+// -> 10.4 ms.  Error of the gradient against 64-bit reference values: 2.3e-14 at 8 and 8.8e-14 at
+// 10 qubits, as with the gates as given in FP64.
 #pragma once
 #include "rot.cuh"
 

@@ -125,8 +125,10 @@ __device__ __forceinline__ double fast_rcp(double x) {
   y = fma(y, fma(-x, y, 1.0), y);
   return fma(y, fma(-x, y, 1.0), y);
 }
-// One Newton step towards |z| = 1 for z that is a few roundings away from it.
-__device__ __forceinline__ double2 cunit(double2 z) { return cscale(z, fma(-0.5, cnorm2(z), 1.5)); }
+// One Newton step towards |z| = 1 for z that is a few roundings away from it, as z + e z: a factor
+// 1 + e would be rounded, more coarsely above 1 than below, and hundreds of runs would shrink.
+__device__ __forceinline__ double2 cgrow(double2 z, double e) { return make_double2(fma(z.x, e, z.x), fma(z.y, e, z.y)); }
+__device__ __forceinline__ double2 cunit(double2 z) { return cgrow(z, -0.5 * fma(z.x, z.x, fma(z.y, z.y, -1.0))); }
 
 // M <- G M
 __device__ __forceinline__ void matmul2(const double2 G[4], double2 M[4]) {
@@ -236,9 +238,9 @@ __device__ __forceinline__ void split_x(double2& p, double2& q, double2& det, Ro
   const double2 b = cmulc(det, q);  // minus the upper entry of A diag(1, conj zi)
   const double2 w0 = make_double2(fma(c, p.x, sn * b.x), fma(c, p.y, sn * b.y));
   const double2 w1 = make_double2(fma(sn, p.x, -(c * b.x)), fma(sn, p.y, -(c * b.y)));
-  const double k = fma(-0.5, cnorm2(w0) + cnorm2(w1), 1.5);
-  p = cscale(w0, k);
-  q = cscale(w1, k);
+  const double e = -0.5 * (fma(w0.x, w0.x, fma(w0.y, w0.y, -1.0)) + cnorm2(w1));
+  p = cgrow(w0, e);
+  q = cgrow(w1, e);
   det = cunit(det);
   r.turn = 0;
   r.t = t;

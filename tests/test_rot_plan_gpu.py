@@ -174,3 +174,14 @@ def test_small_registers_with_and_without_a_workspace(sqg, n, gates, batch):
             rc, rg = O.cost_grad(n, recs, p[b], T)
             close(cost[b].item(), rc)
             close(grad[b].cpu().numpy(), rg)
+
+
+@pytest.mark.parametrize("kind", ["push_x", "push_y", "push_z"])
+def test_long_chains_keep_the_norm(sqg, kind):
+    """The roundings of the plan's numbers have no preferred sign: over L runs the norm walks at random
+    by about 1.5e-16 sqrt(L); five times that is allowed."""
+    L = 10000
+    c = circuit(sqg, 3, kind, L)
+    A = np.eye(8, dtype=np.complex128)
+    c.apply_to(angles(c.get_Parameter_Num(), "any"), A)
+    assert abs(np.mean(np.linalg.norm(A, axis=0)) - 1.0) < 5 * 1.5e-16 * np.sqrt(2 * L)
