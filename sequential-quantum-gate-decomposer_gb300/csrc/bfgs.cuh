@@ -11,10 +11,11 @@
 
 namespace sqg {
 
-// Z entries per load batch in the row and column passes.  4 since the evaluation of the batched
-// decomposition kernel is no longer inlined: with it out of line, chunks of 4 gave 10060
-// decompositions/s against 9536 with chunks of 8 (the same evaluation counts).
-constexpr int kChunk = 4;
+// Z entries per load batch in the row and column passes (CHUNK; the order of the arithmetic does not
+// depend on it).  4 in the batched decomposition kernel, whose many CTAs hide each other's latency:
+// 10060 decompositions/s against 9536 with chunks of 8.  16 in the graph-driven loop, whose one CTA
+// waits for every batch: an evaluation of the loop at 6 qubits, P = 138, 205 -> 193 us.
+constexpr int kChunk = 4, kLoopChunk = 16;
 constexpr double kNumPrecision = 1.42e-14;  // grad_descend.cpp:37
 constexpr double kTwoPi = 6.283185307179586476925286766559;
 
@@ -125,7 +126,7 @@ static __device__ __forceinline__ int block_allmax_int(int v, double* scratch) {
 //   y'_col = alpha_col * sum_{i>=col} y_i z_i - beta_col * y_{col-1},
 //   alpha_col = z_{col-1} / (r_{col-1} r_col),  beta_col = r_col / r_{col-1}.
 // Keeping alpha_col as the column's new scale leaves two FP64 operations per entry.
-template <class ZA>
+template <int CHUNK, class ZA>
 static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, const ZA& za) {
   double* Z = sh.Z;
   double red[4] = {0.0, 0.0, 0.0, 0.0};
@@ -140,7 +141,7 @@ static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, c
   }
   for (int c = threadIdx.x; c < P; c += blockDim.x) {
     double s = 0.0;
-#pragma unroll 8
+#pragma unroll 2 * CHUNK
     for (int r = 0; r < P; r++) s = fma(za.ld(Z + (long long)r * P + c), sh.g[r], s);
     sh.v[c] = s * sh.cs[c];
   }
@@ -189,20 +190,20 @@ static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, c
       zero_alpha = true;
   }
   zero_alpha = __syncthreads_or(zero_alpha);
-  // Rows in chunks of kChunk columns: all loads of a chunk are issued before its stores,
+  // Rows in chunks of CHUNK columns: all loads of a chunk are issued before its stores,
   // so a row costs one memory round trip per chunk instead of one per column (a lone
   // CTA, as at the end of a batch, sees the full L2 latency).
   for (int r = threadIdx.x; r < P; r += blockDim.x) {
     double* row = Z + (long long)r * P;
     if (m < 1) break;
     double sd = 0.0, ycur = za.ld(row + m);
-    for (int col = m; col >= 1; col -= kChunk) {
-      double yp[kChunk], out[kChunk];
+    for (int col = m; col >= 1; col -= CHUNK) {
+      double yp[CHUNK], out[CHUNK];
 #pragma unroll
-      for (int j = 0; j < kChunk; j++) yp[j] = col - 1 - j >= 0 ? za.ld(row + col - 1 - j) : 0.0;
+      for (int j = 0; j < CHUNK; j++) yp[j] = col - 1 - j >= 0 ? za.ld(row + col - 1 - j) : 0.0;
       if (!zero_alpha) {
 #pragma unroll
-        for (int j = 0; j < kChunk; j++) {
+        for (int j = 0; j < CHUNK; j++) {
           const int cc = max(col - j, 1);
           sd = fma(ycur, sh.zs[cc], sd);
           out[j] = fma(sh.gtz[cc], yp[j], sd);  // times alpha_cc (the column's scale)
@@ -210,7 +211,7 @@ static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, c
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < kChunk; j++) {
+        for (int j = 0; j < CHUNK; j++) {
           const int cc = max(col - j, 1);
           sd = fma(ycur, sh.zs[cc], sd);
           out[j] = fma(sh.nz[cc], sd, -sh.sdv[cc] * yp[j]);
@@ -218,7 +219,7 @@ static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, c
         }
       }
 #pragma unroll
-      for (int j = 0; j < kChunk; j++)
+      for (int j = 0; j < CHUNK; j++)
         if (col - j >= 1) za.st(row + col - j, out[j]);
     }
   }
@@ -249,19 +250,19 @@ static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, c
     }
     const double cs = sh.cs[c], gtz = sh.vp[c] * idtg, gc = gtz / cs;
     double s = 0.0;
-    for (int r0 = 0; r0 < P; r0 += kChunk) {
-      double zv[kChunk];
+    for (int r0 = 0; r0 < P; r0 += CHUNK) {
+      double zv[CHUNK];
 #pragma unroll
-      for (int j = 0; j < kChunk; j++) zv[j] = r0 + j < P ? za.ld(Z + (long long)(r0 + j) * P + c) : 0.0;
+      for (int j = 0; j < CHUNK; j++) zv[j] = r0 + j < P ? za.ld(Z + (long long)(r0 + j) * P + c) : 0.0;
 #pragma unroll
-      for (int j = 0; j < kChunk; j++) {
+      for (int j = 0; j < CHUNK; j++) {
         if (r0 + j < P) {
           zv[j] = zv[j] - gc * sh.delta[r0 + j];
           s = fma(zv[j], zv[j], s);
         }
       }
 #pragma unroll
-      for (int j = 0; j < kChunk; j++)
+      for (int j = 0; j < CHUNK; j++)
         if (r0 + j < P) za.st(Z + (long long)(r0 + j) * P + c, zv[j]);
     }
     const double nzc = s * cs * cs;
@@ -278,14 +279,14 @@ static __device__ double bfgs_update(int P, const BfgsVecs& sh, double norm_Z, c
 // Search direction d = -Z Z^T g with Z = Zs diag(cs) (get_search_direction,
 // BFGS_Powell.cpp:407-446); Z^T g (ztg) and cs * Z^T g (zs) come from the last update or, for
 // Z = I, are g itself.  Returns d.g, the maximal step and g.g.
-template <class ZA>
+template <int CHUNK, class ZA>
 static __device__ void bfgs_direction(int P, const BfgsVecs& sh, double& dg, double& max_step, double& gn,
                                       const ZA& za) {
   const double* Z = sh.Z;
   for (int r = threadIdx.x; r < P; r += blockDim.x) {
     const double* row = Z + (long long)r * P;
     double s = 0.0;
-#pragma unroll 8
+#pragma unroll 2 * CHUNK
     for (int c = 0; c < P; c++) s = fma(-za.ld(row + c), sh.zs[c], s);
     sh.d[r] = s;
   }

@@ -492,7 +492,7 @@ __device__ double dec_bfgs(const DecArgs& a, const Sh& sh, int b, int& calls, in
   double fprev = fabs(f + f + 1.0);
   for (;;) {
     double dg, max_step, gn;
-    bfgs_direction(P, bv, dg, max_step, gn, za);
+    bfgs_direction<kChunk>(P, bv, dg, max_step, gn, za);
     if (gn <= 1e-19 * 1e-19 || dg >= 0.0 || f >= fprev) break;
     fprev = f;
     if (run >= a.max_calls) break;
@@ -551,7 +551,7 @@ __device__ double dec_bfgs(const DecArgs& a, const Sh& sh, int b, int& calls, in
       __syncthreads();
     }
     if (step == 0.0) break;
-    norm_Z = bfgs_update(P, bv, norm_Z, za);
+    norm_Z = bfgs_update<kChunk>(P, bv, norm_Z, za);
   }
   return f;
 }
