@@ -325,6 +325,24 @@ TilePlan plan_tiles(int N, int cols, bool grad, int B = 0) {
   return pl;
 }
 
+// Threads of a fixed-point evaluation: up to four pairs each, so that an operation's numbers are
+// decoded for more than one, and more tiles are resident, while every SM keeps a warp per
+// scheduler.  Measured on GB300 with one, two and four pairs per thread (40 blocks; gradient): four
+// qubits, 1024 vectors 788, 669, 682 us, 200 vectors 269, 301, 301 us; five qubits, 200 vectors 690,
+// 629, 522 us, 2500 vectors 3.69, 3.69, 3.45 ms; seven qubits, 30 blocks, 32 vectors 789, 789, 703 us,
+// one vector 191, 236, 236 us.  One warp per tile was never better than two.
+int eval_threads(const TilePlan& pl, int N, int B) {
+  const int items = pl.TC * (N / 2);
+  int t = pl.threads;
+  for (int pairs = 2; pairs <= 4; pairs *= 2) {
+    const int fewer = std::max(64, (items / pairs + 31) / 32 * 32);
+    if (fewer >= t) continue;
+    if ((long long)B * pl.tiles * (fewer / 32) < 4LL * device_sms()) break;
+    t = fewer;
+  }
+  return t;
+}
+
 // Raises a kernel's dynamic shared memory limit to the device's opt-in maximum (never
 // lowers it: the attribute is shared by every caller of the kernel).
 template <typename K>
@@ -411,6 +429,7 @@ struct EvalLayout {
 EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckpt_interval) {
   EvalLayout l;
   l.plan = plan_tiles(c->N, cols, grad, B);
+  if (ckpt_interval == 0) l.plan.threads = eval_threads(l.plan, c->N, B);
   l.rp = (long long)B * l.plan.tiles < 3LL * device_sms() ? &c->short_plan : &c->plan;
   l.rot = rot_layout(*l.rp, B, 0);
   l.tr_off = l.rot.end;
@@ -864,7 +883,7 @@ static int cost_grad_args(const sqg_circuit* c, const double* theta, int B, cons
 // Measured on GB300, environment matrix against tiles: three qubits, 14 blocks 71 against 116 us (one
 // vector), 434 against 551 us (4096); four qubits, 5 blocks 77 against 80 us (one) and 171 against 224
 // us (1024), 10 blocks 130 against 110 us (one), 20 blocks 551 against 488 us (1024), 40 blocks 322
-// against 226 us and 1210 against 790 us; five qubits, 3 blocks 164 against 74 us (one) and 254
+// against 226 us and 1210 against 669 us; five qubits, 3 blocks 164 against 74 us (one) and 254
 // against 225 us (512), 20 blocks 406 against 154 us and 1090 against 607 us.
 static bool tiles_first(const sqg_circuit* c, int B) {
   if (c->n >= 5) return true;

@@ -185,3 +185,24 @@ def test_long_chains_keep_the_norm(sqg, kind):
     A = np.eye(8, dtype=np.complex128)
     c.apply_to(angles(c.get_Parameter_Num(), "any"), A)
     assert abs(np.mean(np.linalg.norm(A, axis=0)) - 1.0) < 5 * 1.5e-16 * np.sqrt(2 * L)
+
+
+@pytest.mark.parametrize("n,batch,cols", [(4, 700, 16), (5, 200, 32), (5, 700, 31), (6, 90, 50), (7, 40, 128)])
+def test_batches_with_several_pairs_per_thread(sqg, n, batch, cols):
+    """Launches with warps to spare take two or four pairs per thread."""
+    c = circuit(sqg, n, "random", 60)
+    recs, P = c.gate_records(), c.get_Parameter_Num()
+    rng = np.random.default_rng(batch)
+    p = rng.uniform(0, 2 * np.pi, (batch, P))
+    N = 1 << n
+    T = np.linalg.qr(rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N)))[0][:, :cols].copy()
+    th = torch.from_numpy(p).cuda()
+    for variant in (0, 3):
+        ev = sqg.CostEvaluator(c, T, cost_variant=variant)
+        cost, grad = ev.cost_grad(th)
+        only = ev.cost_grad(th, with_grad=False)[0]
+        for b in (0, batch - 1):
+            rc, rg = O.cost_grad(n, recs, p[b], T, variant=variant)
+            close(cost[b].item(), rc)
+            close(only[b].item(), rc)
+            close(grad[b].cpu().numpy(), rg)
