@@ -148,6 +148,27 @@ void free_batch(sqg_ragged_batch* r) {
 
 }  // namespace
 
+// Work of an item: pairs of amplitudes times gates.
+static double item_work(const sqg_circuit* c, int tile_cols) {
+  return (double)std::max(c->L, 1) * c->N * tile_cols;
+}
+
+// Default tile width: as many columns as 100 KB take, then halved, down to a pair for every thread of
+// four warps, while one item is more than 1.3 times a resident CTA's share of the batch: the launch
+// would wait for a few items.  Measured on GB300, full width against narrowed: 20 instances of 3 to 8
+// qubits 2.05 against 1.55 ms, 10 of 3 to 7 1.13 against 0.51 ms, 60 of 3 to 6 0.86 against 0.43 ms,
+// 40 of 3 to 5 379 against 249 us.  Batches with enough items lose by it (60 instances of 3 to 8
+// qubits 2.69 against 2.87 ms, 400 12.4 against 13.2 ms) and stay as they are.
+static int default_tile_cols(const sqg_circuit* c, int cols, bool with_grad, double share) {
+  const size_t per = (size_t)c->N * sizeof(double2) * (with_grad ? 2 : 1);
+  const int most = (int)std::max<size_t>(1, (size_t)100 * 1024 / per);
+  int tc = 1;
+  while (tc * 2 <= most) tc *= 2;
+  tc = std::min(tc, cols);
+  while (tc > 1 && (tc / 2) * (c->N / 2) >= 128 && item_work(c, tc) > 1.3 * share) tc /= 2;
+  return tc;
+}
+
 extern "C" {
 
 int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int count, int with_grad,
@@ -165,6 +186,11 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
   std::vector<std::pair<double, int2>> work;
   long long th = 0, tg = 0;
   size_t smem = 0;
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
+  double share = 0.0;  // of a resident CTA (three per SM) of the batch's work
+  for (int i = 0; i < count; i++)
+    if (circuits[i] && cols[i] > 0) share += item_work(circuits[i], cols[i]) / (3.0 * std::max(sms, 1));
   for (int i = 0; i < count; i++) {
     const sqg_circuit* c = circuits[i];
     if (!c || c->device != r->device || cols[i] <= 0 || cols[i] > (c ? c->N : 0)) {
@@ -182,16 +208,8 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
     InstDesc& d = desc[i];
     d.plan = c->plan;
     d.P = c->P; d.n = c->n; d.N = c->N; d.cols = cols[i];
-    const size_t per = (size_t)c->N * sizeof(double2) * (with_grad ? 2 : 1);
-    int tc;
-    if (tile_cols && tile_cols[i] > 0) {
-      tc = std::min(tile_cols[i], cols[i]);
-    } else {
-      tc = (int)std::max<size_t>(1, (size_t)100 * 1024 / per);
-      int p2 = 1;
-      while (p2 * 2 <= tc) p2 *= 2;
-      tc = std::min(p2, cols[i]);
-    }
+    const int tc = tile_cols && tile_cols[i] > 0 ? std::min(tile_cols[i], cols[i])
+                                                 : default_tile_cols(c, cols[i], with_grad, share);
     if (tile_smem_bytes(tc, c->N, with_grad) > 220 * 1024) {
       free_batch(r);
       return set_error(SQG_ERR_UNSUPPORTED, "instance " + std::to_string(i) + ": tile does not fit in shared memory");
@@ -215,7 +233,7 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
     r->max_overlaps = std::max(r->max_overlaps, c->plan.noverlaps);
     smem = std::max(smem, tile_smem_bytes(tc, c->N, with_grad));
     for (int k = 0; k < c->plan.ncta; k++) cta_map.push_back(make_int2(i, k));
-    const double w = (double)std::max(c->L, 1) * c->N * tc;
+    const double w = item_work(c, tc);
     for (int t = 0; t < d.tiles; t++) work.push_back({w, make_int2(i, t)});
   }
   r->theta_off.push_back(th);
@@ -250,11 +268,10 @@ int sqg_ragged_create(const sqg_circuit* const* circuits, const int* cols, int c
   }
   for (auto k : {k_ragged_tiles<0>, k_ragged_tiles<1>, k_ragged_tiles<2>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - kRaggedStatic);
-  int per_sm = 0, sms = 0;
+  int per_sm = 0;
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, with_grad ? k_ragged_tiles<1> : k_ragged_tiles<0>, kRaggedThreads, smem);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
   if (e != cudaSuccess) {
     int st = cerr(e, "sqg_ragged_create");
     free_batch(r);

@@ -206,3 +206,23 @@ def test_batches_with_several_pairs_per_thread(sqg, n, batch, cols):
             close(cost[b].item(), rc)
             close(only[b].item(), rc)
             close(grad[b].cpu().numpy(), rg)
+
+
+@pytest.mark.parametrize("count", [1, 7, 400])
+def test_ragged_tile_widths(sqg, count):
+    """Batches of few items get narrower tiles; every width gives the same numbers."""
+    from importlib import import_module
+    ragged = import_module("sequential-quantum-gate-decomposer_gb300.ragged")
+    rng = np.random.default_rng(count)
+    cs = [circuit(sqg, 3 + (2 * i + 3) % 5, "random", 30) for i in range(count)]
+    ts = [np.linalg.qr(rng.standard_normal((1 << c.qbit_num,) * 2) + 1j * rng.standard_normal((1 << c.qbit_num,) * 2))[0]
+          for c in cs]
+    th = [rng.uniform(0, 2 * np.pi, c.get_Parameter_Num()) for c in cs]
+    for width in (None, 3, 8):
+        rb = ragged.RaggedBatch(cs, ts, tile_cols=None if width is None else [width] * count)
+        cost, grad = rb.cost_grad(rb.pack(th))
+        grads = rb.split(grad)
+        for i in {0, count // 2, count - 1}:
+            rc, rg = O.cost_grad(cs[i].qbit_num, cs[i].gate_records(), th[i], ts[i])
+            close(cost[i].item(), rc)
+            close(grads[i].cpu().numpy(), rg)
