@@ -880,14 +880,21 @@ static int cost_grad_args(const sqg_circuit* c, const double* theta, int B, cons
 }
 
 // Whether the tile kernels are faster than the environment-matrix evaluation where both can run.
-// Measured on GB300, environment matrix against tiles: three qubits, 14 blocks 71 against 116 us (one
-// vector), 434 against 551 us (4096); four qubits, 5 blocks 77 against 80 us (one) and 171 against 224
-// us (1024), 10 blocks 130 against 110 us (one), 20 blocks 551 against 488 us (1024), 40 blocks 322
-// against 226 us and 1210 against 669 us; five qubits, 3 blocks 164 against 74 us (one) and 254
-// against 225 us (512), 20 blocks 406 against 154 us and 1090 against 607 us.
+// The latter takes one CTA per vector, two per SM, and its time grows faster with the gates; the tiles
+// pay for the plan's numbers first.  Measured on GB300, environment matrix against tiles, us:
+// three qubits, 14 blocks 72 / 116 (one vector), 318 / 411 (3000); 30 blocks 313 / 332 (1024), 772 /
+// 666 (3000); 60 blocks 259 / 281 (one), 775 / 494 (700).
+// Four qubits, 6 blocks 89 / 84 (one), 91 / 121 (300), 194 / 208 (1024); 8 blocks 109 / 103, 113 / 137,
+// 241 / 235; 12 blocks 152 / 147 (64), 159 / 164 (300); 14 blocks 173 / 123, 181 / 179, 381 / 315; 40
+// blocks 1210 / 667 (1024).
+// Five qubits, one block 102 / 64 (one), 105 / 128 (300), 203 / 195 (700); two 138 / 142 (300); three 164 /
+// 74, 170 / 152, 329 / 241.
 static bool tiles_first(const sqg_circuit* c, int B) {
-  if (c->n >= 5) return true;
-  return c->n == 4 && c->L >= (B > 2 * device_sms() ? 48 : 32);
+  const bool waves = B > 2 * device_sms();  // more vectors than resident CTAs
+  if (c->n >= 6) return true;
+  if (c->n == 5) return c->L >= 11 || 2 * B <= device_sms();
+  if (c->n == 4) return c->L >= (B <= 4 ? 24 : waves ? 28 : 40);
+  return c->n == 3 && waves && c->L >= 112;
 }
 
 int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,

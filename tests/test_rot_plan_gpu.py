@@ -148,8 +148,9 @@ def test_states_in_small_chunks(sqg, n, batch):
         close(d[b].cpu().numpy(), O.apply_to(n, recs, p[b], v[b].reshape(-1, 1).copy()).reshape(-1))
 
 
-@pytest.mark.parametrize("n,gates,batch", [(3, 40, 2), (4, 31, 1), (4, 32, 1), (4, 47, 400), (4, 48, 400), (5, 1, 1),
-                                           (5, 60, 3)])
+@pytest.mark.parametrize("n,gates,batch", [(3, 40, 2), (4, 31, 1), (4, 32, 1), (4, 27, 400), (4, 28, 400), (5, 1, 1),
+                                           (5, 60, 3), (3, 111, 400), (3, 112, 400), (4, 39, 64), (4, 40, 64),
+                                           (4, 23, 4), (4, 24, 4), (5, 10, 100), (5, 11, 100)])
 def test_small_registers_with_and_without_a_workspace(sqg, n, gates, batch):
     """Up to five qubits the environment-matrix evaluation takes the calls that bring no workspace,
     and those where it is the faster one; both agree with the oracle."""
