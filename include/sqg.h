@@ -95,7 +95,8 @@ size_t sqg_cost_grad_workspace_bytes(const sqg_circuit* circuit, int batch, int 
  * optimization_problem_batched (:940-1033) and optimization_problem_combined_non_static
  * (:1145-1485) of the CPU reference, for the cost variants listed above.  The gradient
  * is the adjoint (reverse-sweep) gradient; checkpoint_interval > 0 stores the forward
- * state every that many gates in the workspace and restores it during the reverse sweep
+ * state every that many operations (at most one per gate: runs of single-qubit gates count
+ * as one, CNOTs as none) in the workspace and restores it during the reverse sweep
  * instead of relying on uncomputation alone (0 = pure uncomputation). */
 int sqg_cost_grad(const sqg_circuit* circuit, const double* theta_dev, int batch, const void* target_dev, int cols,
                   long long target_batch_stride, int trace_offset, int cost_variant, double* cost_dev,
