@@ -304,8 +304,14 @@ int device_sms() {
 // Column tiles of a launch over B instances of `cols` columns.  A tile holds as many columns
 // as the shared-memory budget takes (a power of two); when the whole launch would then not
 // give every SM two CTAs (small batches: a single decomposition's evaluation), tiles are
-// narrowed down to one column each, so the FP64 work of one instance spreads over the GPU.
-TilePlan plan_tiles(int N, int cols, bool grad, int B = 0) {
+// narrowed down to one column each, so the work of one instance spreads over the GPU.  even: one
+// step more for a launch of two to three CTAs per SM, which are two on some SMs and three on others,
+// while that leaves 128 pairs per tile.  Measured on GB300, gradient, without and with: 5 qubits, 40
+// blocks, 310 vectors 864, 741 us; 6 qubits, 160 vectors 1506, 1063 us; 7 qubits, 30 blocks, 40 vectors
+// 1194, 832 us, 10 vectors 412, 384 us; 8 qubits, 10 vectors 1212, 841 us, 3 vectors 420, 410 us.  With 64
+// pairs 7 qubits, 5 vectors 277, 294 us; 4 qubits, 400 vectors 366, 397 us.  The cost alone gains as
+// often as it loses.
+TilePlan plan_tiles(int N, int cols, bool grad, int B = 0, bool even = false) {
   const size_t per = (size_t)N * sizeof(double2) * (grad ? 2 : 1);
   size_t budget = grad ? kSmemBudgetGrad : kSmemBudgetFwd;
   int tc = (int)std::max<size_t>(1, budget / per);
@@ -314,8 +320,10 @@ TilePlan plan_tiles(int N, int cols, bool grad, int B = 0) {
   while (p2 * 2 <= tc) p2 *= 2;
   tc = std::min(p2, cols);
   if (B > 0) {
-    const long long want = 2LL * device_sms();
-    while (tc > 1 && (long long)B * ((cols + tc - 1) / tc) < want) tc >>= 1;
+    const long long sms = device_sms();
+    auto ctas = [&] { return (long long)B * ((cols + tc - 1) / tc); };
+    while (tc > 1 && ctas() < 2 * sms) tc >>= 1;
+    if (even && ctas() < 3 * sms && (tc / 2) * (N / 2) >= 128) tc >>= 1;
   }
   TilePlan pl;
   pl.TC = tc;
@@ -426,9 +434,9 @@ struct EvalLayout {
 };
 // The overlaps take two doubles each, whatever the cost variant: FROBENIUS_NORM, which needs
 // only their imaginary parts, uses half of that.
-EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckpt_interval) {
+EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckpt_interval, bool even = true) {
   EvalLayout l;
-  l.plan = plan_tiles(c->N, cols, grad, B);
+  l.plan = plan_tiles(c->N, cols, grad, B, even && grad && ckpt_interval == 0);
   if (ckpt_interval == 0) l.plan.threads = eval_threads(l.plan, c->N, B);
   l.rp = (long long)B * l.plan.tiles < 3LL * device_sms() ? &c->short_plan : &c->plan;
   l.rot = rot_layout(*l.rp, B, 0);
@@ -441,6 +449,13 @@ EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckp
   size_t ck_bytes = (size_t)B * l.plan.tiles * l.nck * (size_t)l.plan.TC * c->N * sizeof(double2);
   l.end = align_up(l.ck_off + ck_bytes, 256);
   return l;
+}
+
+// The layout for a workspace of ws_bytes: without the last step of plan_tiles, which takes more
+// bytes, where it does not fit.
+EvalLayout eval_layout_within(const sqg_circuit* c, int B, int cols, bool grad, int ckpt_interval, size_t ws_bytes) {
+  const EvalLayout l = eval_layout(c, B, cols, grad, ckpt_interval);
+  return l.end <= ws_bytes ? l : eval_layout(c, B, cols, grad, ckpt_interval, false);
 }
 
 int launch_prep(const sqg_circuit* c, const double* theta, long long theta_stride, int B, GateMat* gm, double2* sc,
@@ -916,13 +931,13 @@ int sqg::cost_grad(const sqg_circuit* c, const double* theta, int B, const void*
   if (with_grad && checkpoint_interval == 0) {
     // up to five qubits: one CTA per vector with the environment-matrix evaluation, which also
     // takes the calls without a workspace
-    const bool tiles = !env_first && tiles_first(c, B) && workspace && ws_bytes >= eval_layout(c, B, cols, true, 0).end;
+    const bool tiles = !env_first && tiles_first(c, B) && workspace && ws_bytes >= eval_layout(c, B, cols, true, 0, false).end;
     st = tiles ? SQG_ERR_UNSUPPORTED
                : sqg::env_cost_grad(c, theta, B, target, cols, target_batch_stride, off, variant, cost, grad, stream);
     if (st != SQG_ERR_UNSUPPORTED) return st;
     st = SQG_OK;
   }
-  EvalLayout l = eval_layout(c, B, cols, with_grad, with_grad ? checkpoint_interval : 0);
+  EvalLayout l = eval_layout_within(c, B, cols, with_grad, with_grad ? checkpoint_interval : 0, ws_bytes);
   if (!workspace || ws_bytes < l.end) return fail(SQG_ERR_WORKSPACE, "workspace too small: need " + std::to_string(l.end));
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = (char*)workspace;
@@ -1060,7 +1075,8 @@ int sqg_cost_grad_noalloc(const sqg_circuit* c, const double* theta, int B, cons
     st = sqg::env_cost_grad(c, theta, B, target, cols, target_batch_stride, off, variant, cost, grad, stream);
     if (st != SQG_ERR_UNSUPPORTED) return st;
   }
-  const size_t need = eval_layout(c, B, cols, with_grad, with_grad ? checkpoint_interval : 0).end;
+  const size_t need =
+      eval_layout_within(c, B, cols, with_grad, with_grad ? checkpoint_interval : 0, SQG_NOALLOC_SCRATCH_BYTES).end;
   if (need > SQG_NOALLOC_SCRATCH_BYTES)
     return fail(SQG_ERR_WORKSPACE, "sqg_cost_grad_noalloc: this call needs " + std::to_string(need) +
                                        " bytes of scratch but the built-in array holds " +

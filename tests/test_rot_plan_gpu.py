@@ -227,3 +227,34 @@ def test_ragged_tile_widths(sqg, count):
             rc, rg = O.cost_grad(cs[i].qbit_num, cs[i].gate_records(), th[i], ts[i])
             close(cost[i].item(), rc)
             close(grads[i].cpu().numpy(), rg)
+
+
+@pytest.mark.parametrize("n,batch", [(5, 160), (6, 160), (7, 40), (8, 11), (8, 3)])
+def test_narrow_tiles_and_a_workspace_for_wide_ones(sqg, n, batch):
+    """Launches of two to three CTAs per SM take narrower tiles where the workspace has room for
+    them; one that was large enough for the wide tiles still is."""
+    from importlib import import_module
+    native = import_module("sequential-quantum-gate-decomposer_gb300._native")
+    c = circuit(sqg, n, "random", 25)
+    recs, P = c.gate_records(), c.get_Parameter_Num()
+    rng = np.random.default_rng(n)
+    p = rng.uniform(0, 2 * np.pi, (batch, P))
+    N = 1 << n
+    T = np.linalg.qr(rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N)))[0]
+    th, tgt = torch.from_numpy(p).cuda(), torch.from_numpy(T.copy()).cuda()
+    ev = sqg.CostEvaluator(c, T)
+    size = ev.workspace_bytes(batch, True)
+    wide = ev.workspace_bytes(batch, True, 1000)  # checkpointed, none of them stored: wide tiles
+    assert wide <= size
+    for have in (size, wide):
+        guard = torch.full((have + 4096,), 7, dtype=torch.uint8, device="cuda")
+        cost = torch.full((batch,), np.nan, dtype=torch.float64, device="cuda")
+        grad = torch.full((batch, P), np.nan, dtype=torch.float64, device="cuda")
+        native.check(native.lib().sqg_cost_grad(
+            ev.native.handle, th.data_ptr(), batch, tgt.data_ptr(), N, 0, 0, 0, cost.data_ptr(), grad.data_ptr(), 0,
+            guard.data_ptr(), have, torch.cuda.current_stream().cuda_stream), "sqg_cost_grad")
+        assert bool((guard[have:] == 7).all())
+        for b in (0, batch - 1):
+            rc, rg = O.cost_grad(n, recs, p[b], T)
+            close(cost[b].item(), rc)
+            close(grad[b].cpu().numpy(), rg)
