@@ -14,7 +14,7 @@ namespace sqg {
 // Z entries per load batch in the row and column passes (CHUNK; the order of the arithmetic does not
 // depend on it).  4 in the batched decomposition kernel, whose many CTAs hide each other's latency:
 // 10060 decompositions/s against 9536 with chunks of 8.  16 in the graph-driven loop, whose one CTA
-// waits for every batch: an evaluation of the loop at 6 qubits, P = 138, 205 -> 193 us.
+// waits for every batch: an evaluation of the loop at 6 qubits, P = 138, 321 -> 291 us.
 constexpr int kChunk = 4, kLoopChunk = 16;
 constexpr double kNumPrecision = 1.42e-14;  // grad_descend.cpp:37
 constexpr double kTwoPi = 6.283185307179586476925286766559;

@@ -29,6 +29,7 @@
 
 #include "../../include/sqg.h"
 #include "gates.cuh"
+#include "gatetile.cuh"
 #include "handle.h"
 #include "rotgrad.cuh"
 #include "rotplan.h"
@@ -155,6 +156,23 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_grad(RotPlan pl, const doub
   const long long b = blockIdx.y;
   rot_grad_body<CPLX>(pl, blockIdx.x, theta + b * P, recs + b * pl.nrecs, ws_tr + b * tiles,
                       ws_gr + b * tiles * pl.noverlaps * (CPLX ? 2 : 1), cols, variant, grad + b * P);
+}
+
+// The optimizer loops' evaluation (gatetile.cuh) and the sum of its tiles in their order.
+__global__ void __launch_bounds__(kMaxThreads) k_gate_adjoint(GateTileArgs a) {
+  extern __shared__ double2 smem[];
+  gate_adjoint_body(a, blockIdx.x, smem);
+}
+__global__ void k_gate_finish(const double2* __restrict__ ws_tr, const double2* __restrict__ ws_gr, int tiles, int P,
+                              int cols, int variant, double* __restrict__ cost, double* __restrict__ grad) {
+  double2 tr = make_double2(0.0, 0.0);
+  for (int t = 0; t < tiles; t++) tr = cadd(tr, ws_tr[t]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cost = cost_from_trace(variant, tr, cols);
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P) return;
+  double2 dt = make_double2(0.0, 0.0);
+  for (int t = 0; t < tiles; t++) dt = cadd(dt, ws_gr[(long long)t * P + p]);
+  grad[p] = grad_from_trace(variant, tr, dt, cols);
 }
 
 // -------------------------------------------------------------------------------------
@@ -915,15 +933,6 @@ static bool tiles_first(const sqg_circuit* c, int B) {
 int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
                   long long target_batch_stride, int trace_offset, int variant, double* cost, double* grad,
                   int checkpoint_interval, void* workspace, size_t ws_bytes, void* stream) {
-  return sqg::cost_grad(c, theta, B, target, cols, target_batch_stride, trace_offset, variant, cost, grad,
-                        checkpoint_interval, workspace, ws_bytes, stream, false);
-}
-
-}  // extern "C"
-
-int sqg::cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
-                   long long target_batch_stride, int trace_offset, int variant, double* cost, double* grad,
-                   int checkpoint_interval, void* workspace, size_t ws_bytes, void* stream, bool env_first) {
   int st = cost_grad_args(c, theta, B, target, cols, trace_offset, variant, cost, grad, checkpoint_interval);
   if (st) return st;
   const int off = variant == SQG_FROBENIUS_NORM ? trace_offset : 0;
@@ -931,7 +940,7 @@ int sqg::cost_grad(const sqg_circuit* c, const double* theta, int B, const void*
   if (with_grad && checkpoint_interval == 0) {
     // up to five qubits: one CTA per vector with the environment-matrix evaluation, which also
     // takes the calls without a workspace
-    const bool tiles = !env_first && tiles_first(c, B) && workspace && ws_bytes >= eval_layout(c, B, cols, true, 0, false).end;
+    const bool tiles = tiles_first(c, B) && workspace && ws_bytes >= eval_layout(c, B, cols, true, 0, false).end;
     st = tiles ? SQG_ERR_UNSUPPORTED
                : sqg::env_cost_grad(c, theta, B, target, cols, target_batch_stride, off, variant, cost, grad, stream);
     if (st != SQG_ERR_UNSUPPORTED) return st;
@@ -984,6 +993,57 @@ int sqg::cost_grad(const sqg_circuit* c, const double* theta, int B, const void*
     k_rot_grad<false><<<ggrid, kRotThreads, 0, s>>>(*l.rp, theta, a.recs, wtr, wgr, l.plan.tiles, c->P, cols, variant, grad);
   }
   return cuda_status(cudaGetLastError(), "cost and gradient kernels");
+}
+
+}  // extern "C"
+
+// ---- the optimizer loops' evaluation ---------------------------------------------------
+namespace {
+struct LoopEvalLayout {
+  TilePlan plan;
+  PrepLayout prep;
+  size_t tr_off, gr_off, end;
+};
+LoopEvalLayout loop_eval_layout(const sqg_circuit* c, int cols) {
+  LoopEvalLayout l;
+  l.plan = plan_tiles(c->N, cols, true, 1);
+  l.plan.smem = gate_tile_smem_bytes(l.plan.TC, c->N);
+  l.prep = prep_layout(c, 1, 0);
+  l.tr_off = l.prep.end;
+  l.gr_off = align_up(l.tr_off + (size_t)l.plan.tiles * sizeof(double2), 256);
+  l.end = align_up(l.gr_off + (size_t)l.plan.tiles * std::max(c->P, 1) * sizeof(double2), 256);
+  return l;
+}
+}  // namespace
+
+size_t sqg::loop_cost_grad_bytes(const sqg_circuit* c, int cols) { return loop_eval_layout(c, cols).end; }
+
+int sqg::loop_cost_grad(const sqg_circuit* c, const double* theta, const void* target, int cols, int off, int variant,
+                        double* cost, double* grad, void* workspace, size_t ws_bytes, void* stream) {
+  int st = sqg::env_cost_grad(c, theta, 1, target, cols, 0, off, variant, cost, grad, stream);
+  if (st != SQG_ERR_UNSUPPORTED) return st;
+  const LoopEvalLayout l = loop_eval_layout(c, cols);
+  if (!workspace || ws_bytes < l.end) return fail(SQG_ERR_WORKSPACE, "workspace too small: need " + std::to_string(l.end));
+  cudaStream_t s = (cudaStream_t)stream;
+  char* ws = (char*)workspace;
+  GateMat* gm = (GateMat*)(ws + l.prep.gm_off);
+  double2* sc = (double2*)(ws + l.prep.sc_off);
+  if ((st = launch_prep(c, theta, c->P, 1, gm, sc, s))) return st;
+  GateTileArgs a;
+  a.gates = c->d_gates;
+  a.gm = gm;
+  a.sc = sc;
+  a.target = (const double2*)target;
+  a.L = c->L; a.P = c->P; a.n = c->n; a.N = c->N; a.cols = cols;
+  a.TC = l.plan.TC;
+  a.tiles = l.plan.tiles;
+  a.trace_offset = off;
+  a.ws_tr = (double2*)(ws + l.tr_off);
+  a.ws_gr = (double2*)(ws + l.gr_off);
+  if ((st = set_smem(k_gate_adjoint, l.plan.smem))) return st;
+  k_gate_adjoint<<<l.plan.tiles, l.plan.threads, l.plan.smem, s>>>(a);
+  k_gate_finish<<<(c->P + 127) / 128, 128, 0, s>>>(a.ws_tr, a.ws_gr, l.plan.tiles, c->P, cols, variant, cost, grad);
+  return cuda_status(cudaGetLastError(), "optimizer loop evaluation");
 }
 
 // ---- allocation-free cost/gradient ---------------------------------------------------

@@ -46,9 +46,10 @@ int set_error(int status, const std::string& msg);
 // for shapes it does not take.
 int env_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols, long long tstride,
                   int off, int variant, double* cost, double* grad, void* stream);
-// sqg_cost_grad; env_first: with the arithmetic of the decomposition kernels wherever they have it
-// (up to five qubits), which the device loops repeat bit for bit.
-int cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
-              long long target_batch_stride, int trace_offset, int variant, double* cost, double* grad,
-              int checkpoint_interval, void* workspace, size_t ws_bytes, void* stream, bool env_first);
+// Cost and gradient of one vector inside the device optimizer loops: env_cost_grad where it takes the
+// call, else gate by gate in FP64 (gatetile.cuh).  Arguments as checked by the loops; off: the trace
+// offset that the variant uses.
+size_t loop_cost_grad_bytes(const sqg_circuit* c, int cols);
+int loop_cost_grad(const sqg_circuit* c, const double* theta, const void* target, int cols, int off, int variant,
+                   double* cost, double* grad, void* workspace, size_t ws_bytes, void* stream);
 }  // namespace sqg

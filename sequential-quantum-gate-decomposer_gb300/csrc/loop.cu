@@ -68,7 +68,7 @@ LoopLayout loop_layout(const sqg_circuit* c, int cols) {
   for (size_t& v : l.vec) v = take(sizeof(double) * (size_t)c->P);
   l.f0 = take(sizeof(double) * 100);
   l.dec = take(sizeof(int) * 20);
-  l.eval = take(sqg_cost_grad_workspace_bytes(c, 1, cols, 1));
+  l.eval = take(sqg::loop_cost_grad_bytes(c, cols));
   l.end = off;
   return l;
 }
@@ -188,7 +188,7 @@ BfgsLayout bfgs_layout(const sqg_circuit* c, int cols) {
   l.cost = take(sizeof(double));
   for (size_t& v : l.vec) v = take(sizeof(double) * (size_t)c->P);
   l.Z = take(sizeof(double) * (size_t)c->P * c->P);
-  l.eval = take(sqg_cost_grad_workspace_bytes(c, 1, cols, 1));
+  l.eval = take(sqg::loop_cost_grad_bytes(c, cols));
   l.end = off;
   return l;
 }
@@ -415,8 +415,8 @@ int run_loop_graph(const sqg_circuit* c, const void* target, int cols, int trace
   if (e != cudaSuccess) {
     st = cuda_fail(e, "building the decomposition graph");
   } else {
-    st = sqg::cost_grad(c, x_eval, 1, target, cols, 0, trace_offset, cost_variant, cost_eval, g_eval, 0, eval_ws,
-                        eval_bytes, cap, true);
+    const int off = cost_variant == SQG_FROBENIUS_NORM ? trace_offset : 0;
+    st = sqg::loop_cost_grad(c, x_eval, target, cols, off, cost_variant, cost_eval, g_eval, eval_ws, eval_bytes, cap);
     if (st == SQG_OK) {
       step(cap, handle);
       e = cudaGetLastError();
