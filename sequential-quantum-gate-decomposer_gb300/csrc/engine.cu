@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   for (int k0 = a.k0; k0 < a.k1; k0 += kRotChunk) {
     const int kn = min(kRotChunk, a.k1 - k0);
     __syncthreads();
-    stage_ops<true, kRotGroup>(st, a.lops, recs, k0, kn);
+    stage_ops<true, false>(st, a.lops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
       rot_tile<kRotFwd>(sv, KK, a.K, 1, st[j]);

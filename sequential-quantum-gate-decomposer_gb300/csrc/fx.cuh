@@ -5,14 +5,14 @@
 // are bounded by its norm, so they fit 64-bit fixed point under one power of two, and a product
 // with a coefficient of 62 bits costs three such multiplies and six adds and exclusive-ors
 // instead of one FP64 instruction: about 6 clocks against 16, with a tenth of the latency.  The
-// resolution is 2^-61 of the tile's norm, below the rounding of FP64 amplitudes (2^-53 of each,
-// 2^-57 at 8 qubits), and every product rounds to nearest.
+// resolution is 2^-62 of the largest vector's norm, 2^-60 where a group of rotations has made the vectors
+// shorter (kFxGroupBits); FP64 amplitudes round to 2^-53 of each, 2^-57 of the norm at 8 qubits.
 // Cost and gradient are sums over all amplitudes, so an absolute resolution is what they need;
 // matrices and state vectors that go back to the caller stay in FP64.  Tiles with infinities or
 // NaN, and sweeps with checkpoints, stay in FP64 too.
-// GB300, FP64 sweeps -> these: gradient at 8 qubits, 360 blocks, 128 vectors 179 -> 75 ms; at 10
-// qubits, 300 blocks, 6 vectors 116 -> 49 ms; cost alone at 8 qubits, 120 blocks, 200 vectors 24.7
-// -> 10.4 ms.  Error of the gradient against 64-bit reference values: 2.3e-14 at 8 and 8.8e-14 at
+// GB300, FP64 sweeps -> these: gradient at 8 qubits, 360 blocks, 128 vectors 179 -> 76 ms; at 10
+// qubits, 300 blocks, 6 vectors 116 -> 50 ms; cost alone at 8 qubits, 120 blocks, 200 vectors 24.7
+// -> 10.5 ms.  Error of the gradient against 64-bit reference values: 2.3e-14 at 8 and 8.8e-14 at
 // 10 qubits, as with the gates as given in FP64.
 #pragma once
 #include "rot.cuh"
@@ -184,7 +184,7 @@ __device__ __forceinline__ void fx_signs(const OpPlaces& pl, int ix, int iy, Fx2
 template <bool FWD>
 __device__ __forceinline__ void fx_stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn,
                                              double unit) {
-  stage_ops<FWD, kFxGroup>(st, ops, recs, k0, kn);
+  stage_ops<FWD, true>(st, ops, recs, k0, kn);
   if ((int)threadIdx.x >= kn) return;  // each thread the operation that it staged
   StagedOp& s = st[threadIdx.x];
   auto enc = [](double c) { return __longlong_as_double((long long)fx_encode(c)); };
@@ -218,6 +218,27 @@ __device__ __forceinline__ void fx_tile_kind(Fx2* s, int N, int logN, int tc, co
     fx_pair<kRotFwd, KIND, RS>(op, x, y);
     v[ix] = x;
     v[iy] = y;
+  }
+}
+
+// Multiplies a group's scale into a tile behind the rotation that it belongs to, each thread on the pairs
+// that it has rotated (no barrier between); until then amplitudes may reach 2^62.5.  The way back takes
+// this pass of its own: with the scale in the rotation, as on the way up, every kind has a second form of
+// 20 KB of code, which small tiles wait for.  GB300, gradients, in the rotation against here: four qubits, 1024
+// vectors 744, 685 us; eight qubits, 128 vectors 75.4, 75.9 ms; 60 instances of 3 to 8 qubits 2.76, 2.78 ms.
+__device__ __forceinline__ void fx_rescale(Fx2* s, int N, int logN, int tc, const StagedOp& staged) {
+  const OpPlaces pl = op_places(staged);
+  const FxCoef c = fx_coef(fx_bits(staged.scale), false);
+  auto scaled = [&](Fx2 v) {
+    return Fx2{(long long)(fx_mul(v.x, c) + c.k), (long long)(fx_mul(v.y, c) + c.k)};
+  };
+  const int npairs = 1 << (logN - 1);
+  for (int it = threadIdx.x; it < tc << (logN - 1); it += blockDim.x) {
+    Fx2* v = s + (it >> (logN - 1)) * N;
+    int ix, iy;
+    pair_places<kOpRot>(pl, it & (npairs - 1), ix, iy);
+    v[ix] = scaled(v[ix]);
+    v[iy] = scaled(v[iy]);
   }
 }
 
@@ -331,10 +352,10 @@ __device__ __forceinline__ void fx_measure(const Fx2& x, const Fx2& y, const Fx2
   }
 }
 
-template <bool CPLX, int KIND, int MASK, bool RS>
+template <bool CPLX, int KIND, int MASK>
 __device__ __forceinline__ void fx_adjoint_kind(Fx2* psi, Fx2* lam, int N, int logN, int tc, const StagedOp& staged,
                                                 long long (&acc)[CPLX ? 6 : 3]) {
-  const FxOp op = fx_directed<kRotAdj, KIND, RS>(staged);
+  const FxOp op = fx_directed<kRotAdj, KIND, false>(staged);
   const OpPlaces pl = op_places(staged);
   const int lognp = KIND == kOpCry ? logN - 2 : logN - 1;
   const int npairs = 1 << lognp;
@@ -351,9 +372,9 @@ __device__ __forceinline__ void fx_adjoint_kind(Fx2* psi, Fx2* lam, int N, int l
       fx_phase(y, op.zix, op.ziy, op.nzi);
       fx_phase(ly, op.zix, op.ziy, op.nzi);
     } else {
-      fx_pair<kRotAdj, KIND, RS>(op, x, y);
+      fx_pair<kRotAdj, KIND, false>(op, x, y);
       fx_signs(pl, ix, iy, x, y);
-      fx_pair<kRotAdj, KIND, RS>(op, lx, ly);
+      fx_pair<kRotAdj, KIND, false>(op, lx, ly);
       fx_signs(pl, ix, iy, lx, ly);
       ps[ix] = x;
       ls[ix] = lx;
@@ -367,15 +388,10 @@ template <bool CPLX>
 __device__ __forceinline__ void fx_adjoint(Fx2* psi, Fx2* lam, int N, int logN, int tc, const StagedOp& st,
                                            long long (&acc)[CPLX ? 6 : 3]) {
 #define SQG_ROT_CASE(KIND, MASK) \
-  case (KIND) | (MASK) << 8: \
-    if (st.kind & kStRescale) \
-      fx_adjoint_kind<CPLX, (KIND), (MASK), true>(psi, lam, N, logN, tc, st, acc); \
-    else \
-      fx_adjoint_kind<CPLX, (KIND), (MASK), false>(psi, lam, N, logN, tc, st, acc); \
-    break;
+  case (KIND) | (MASK) << 8: fx_adjoint_kind<CPLX, (KIND), (MASK)>(psi, lam, N, logN, tc, st, acc); break;
   switch (st.kind & 0xffff) {
-    case kOpCry | 2 << 8: fx_adjoint_kind<CPLX, kOpCry, 2, false>(psi, lam, N, logN, tc, st, acc); break;
-    case kOpPhase | 4 << 8: fx_adjoint_kind<CPLX, kOpPhase, 4, false>(psi, lam, N, logN, tc, st, acc); break;
+    case kOpCry | 2 << 8: fx_adjoint_kind<CPLX, kOpCry, 2>(psi, lam, N, logN, tc, st, acc); break;
+    case kOpPhase | 4 << 8: fx_adjoint_kind<CPLX, kOpPhase, 4>(psi, lam, N, logN, tc, st, acc); break;
     SQG_ROT_CASE(kOpRot, 2)
     SQG_ROT_CASE(kOpRot | kOpX, 1)
     SQG_ROT_CASE(kOpRot | kOpZi, 3)
@@ -384,6 +400,10 @@ __device__ __forceinline__ void fx_adjoint(Fx2* psi, Fx2* lam, int N, int logN, 
     SQG_ROT_CASE(kOpRot | kOpZi | kOpZo, 7)
   }
 #undef SQG_ROT_CASE
+  if (st.kind & kStRescale) {
+    fx_rescale(psi, N, logN, tc, st);
+    fx_rescale(lam, N, logN, tc, st);
+  }
 }
 
 // Warp totals of up to eight sums: lane l ends with value (l >> 2) & 7.

@@ -95,10 +95,15 @@ constexpr int kRotParams = 512;  // parameters listed per CTA
 // that does not fill the device waits for the chains: 46 U3 of one vector 52 us at 16, 29 us at 4.
 constexpr int kRotChain = 16, kRotShortChain = 4;
 constexpr int kRotChunk = 32;     // operations staged in shared memory together (a warp)
-// Operations whose cosines are multiplied in together.  In FP64 the scale costs no precision, so
-// the whole chunk; in fixed point the overlaps lose the square of it (2^-8 at worst), at 4
-// more products per group: 16 a group costs 3 % of a gradient against 32, 8 costs 6 %.
-constexpr int kRotGroup = kRotChunk, kFxGroup = 16;
+// The cosines of a group of consecutive operations are multiplied in together.  In FP64 the scale costs no
+// precision: the whole chunk is a group.  In fixed point it costs amplitudes its size and overlaps its
+// square, so a group ends before the cosines of all but its last rotation pass 2^-1.5: after three
+// operations at angles of pi/4, ten at uniform ones.  Error of gradients against long double over 6 to 12
+// qubits, 1 to 256 columns, angles uniform and at or near multiples of pi/4, as a multiple of that of the gates
+// as given in FP64: 0.7 to 1.1 in the mean, 3 at worst; groups of 16 operations whatever their cosines
+// 1.0 to 6.4, 2800 at worst.  Bounds of 2^-1, 2^-2: gradients at four qubits, 1024 vectors 5 % slower, 3 % faster;
+// single columns of 4096 rows at uniform angles 1.4, 3.7 times the error of FP64 at worst (2^-1.5: 1.7).
+constexpr int kFxGroupBits = (3 << 20) / 2;  // 1.5, in units of 2^-20
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
@@ -483,7 +488,7 @@ __device__ __forceinline__ void batch_finish_body(const RotPlan& pl, int cta, Ro
 
 // ---- application ---------------------------------------------------------------------------
 // Operation staged for the sweeps.  scale: the product of its group's cosines, multiplied in by the
-// operation with kStRescale (its t includes it).  zi.x of a kOpCry: its cosine.  mfac: what the
+// operation with kStRescale (whose t includes it; fixed point on the way back: fx_rescale).  zi.x of a kOpCry: its cosine.  mfac: what the
 // overlaps measured behind the operation, with both vectors on the way back, are multiplied by.
 struct StagedOp {
   int kind, coff;  // kind | mask << 8 | flags
@@ -498,8 +503,9 @@ enum : int { kStTurn = 1 << 16, kStRescale = 1 << 17, kStInside = 1 << 18 };
 // Loads operations [k0, k0 + kn) (at most kRotChunk) into st with the first warp of the CTA.
 // The cosines that a group's rotations leave out are multiplied in by the first rotation in the
 // direction of travel (FWD: the group's first, else its last): from there the scale rises back to
-// 1, and amplitudes never exceed what they were.  The caller synchronises before and after.
-template <bool FWD, int GROUP>
+// 1, and amplitudes never exceed what they were.  FX: groups as kFxGroupBits ends them; both directions
+// make the same ones.  The caller synchronises before and after.
+template <bool FWD, bool FX>
 __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
@@ -511,20 +517,36 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
     if (op.kind >= kOpCry) r = recs[op.rec];
   }
   const bool rot = (op.kind & kOpRot) != 0;
+  int base = 0, end = 31;  // this lane's group
+  if (FX) {
+    // bits in front of this operation, in units of 2^-20: a group starts where they pass a multiple of
+    // kFxGroupBits, so those of all but its last rotation stay below
+    const int bits = rot ? (int)(-0x1p20f * __log2f((float)r.c)) : 0;
+    int upto = bits;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int before = (upto - bits) / kFxGroupBits, last = __shfl_up_sync(0xffffffffu, before, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != last);
+    base = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    const unsigned later = heads & ~(0xffffffffu >> (31 - lane));
+    if (later) end = __ffs(later) - 2;
+  }
   // product of the cosines of the group up to and including this operation, as pre + plo
-  const int in_group = lane & (GROUP - 1), base = lane - in_group;
   double pre = rot ? r.c : 1.0, plo = rot ? r.lo : 0.0;
-  for (int o = 1; o < GROUP; o <<= 1) {
+  for (int o = 1; o < 32; o <<= 1) {
+    if (FX && !__any_sync(0xffffffffu, lane - base >= o)) break;
     const double v = __shfl_up_sync(0xffffffffu, pre, o), vlo = __shfl_up_sync(0xffffffffu, plo, o);
-    if (in_group >= o) {
+    if (lane - base >= o) {
       const double p = pre * v;
       plo = fma(pre, v, -p) + fma(pre, vlo, plo * v);
       pre = p;
     }
   }
-  const double all = __shfl_sync(0xffffffffu, pre + plo, base + GROUP - 1);
-  const unsigned rots = (__ballot_sync(0xffffffffu, rot) >> base) & (0xffffffffu >> (32 - GROUP));
-  const int first = rots ? base + __ffs(rots) - 1 : 32, last = rots ? base + 31 - __clz(rots) : 32;
+  const double all = __shfl_sync(0xffffffffu, pre + plo, end);
+  const unsigned rots = __ballot_sync(0xffffffffu, rot) & (0xffffffffu >> (31 - end)) & (0xffffffffu << base);
+  const int first = rots ? __ffs(rots) - 1 : 32, last = rots ? 31 - __clz(rots) : 32;
   const bool rescale = lane == (FWD ? first : last);
   if (on) {
     StagedOp s;
@@ -536,7 +558,7 @@ __device__ __forceinline__ void stage_ops(StagedOp* st, const RotOp* ops, const 
     s.cz = op.cz0 | (unsigned)op.cz1 << 16;
     s.pad = 0;
     s.scale = all;
-    s.t = rescale ? r.t * all : r.t;
+    s.t = rescale && (FWD || !FX) ? r.t * all : r.t;
     s.mfac = 1.0;
     if (!FWD && lane < last) {
       const double inv = fast_rcp(pre + plo);

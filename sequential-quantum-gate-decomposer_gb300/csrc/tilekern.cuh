@@ -182,7 +182,7 @@ __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int 
     if (!WRITE_BACK && fixed)
       fx_stage_ops<true>(st, a.ops, recs, k0, kn, 1.0);
     else
-      stage_ops<DIR == kRotFwd, kRotGroup>(st, a.ops, recs, k0, kn);
+      stage_ops<DIR == kRotFwd, false>(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
       if (!WRITE_BACK && fixed)
@@ -359,7 +359,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
     if (fixed)
       fx_stage_ops<true>(st, a.ops, recs, k0, kn, 1.0);
     else
-      stage_ops<true, kRotGroup>(st, a.ops, recs, k0, kn);
+      stage_ops<true, false>(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = 0; j < kn; j++) {
       if (fixed)
@@ -418,7 +418,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
     if (fixed)
       fx_stage_ops<false>(st, a.ops, recs, k0, kn, fx_unit);
     else
-      stage_ops<false, kRotGroup>(st, a.ops, recs, k0, kn);
+      stage_ops<false, false>(st, a.ops, recs, k0, kn);
     __syncthreads();
     for (int j = kn - 1; j >= 0; j--) {
       const int k = k0 + j;
