@@ -46,3 +46,20 @@ def test_small_cosines(sqg, n, cols, blocks, angle, kind):
     assert np.max(np.abs(rg)) < 0.15
     assert abs(cost.item() - rc) <= 2e-15
     assert np.max(np.abs(grad[0].cpu().numpy() - rg)) <= 2e-15
+
+
+@pytest.mark.parametrize("kind", ["ry", "u3"])
+def test_deep_circuit_on_the_identity(sqg, kind):
+    """A thousand runs on amplitudes that start as zeros and ones: what a product adds to a zero must not
+    gather."""
+    n = 8
+    rng = np.random.default_rng(8)
+    c = circuit(sqg, n, 500, rng, kind)
+    P = c.get_Parameter_Num()
+    p = rng.choice([1, 3, 5, 7], P) * (np.pi / 4) + 1e-3 * rng.standard_normal(P)
+    T = np.eye(1 << n).astype(np.complex128)
+    ev = sqg.CostEvaluator(c, T)
+    cost, grad = ev.cost_grad(torch.from_numpy(p).cuda())
+    cost64, grad64 = ev.cost_grad(torch.from_numpy(p).cuda(), checkpoint_interval=50)  # swept in FP64
+    assert abs(cost.item() - cost64.item()) <= 2e-15
+    assert torch.max(torch.abs(grad - grad64)).item() <= 2e-15
