@@ -183,8 +183,8 @@ __device__ __forceinline__ void fx_signs(const OpPlaces& pl, int ix, int iy, Fx2
   }
 }
 
-// stage_ops with the numbers encoded; mfac times `unit`, what 2^60 of a sum of overlaps
-// is worth: done here once per chunk, not in the serial end of each operation.
+// stage_ops with the numbers encoded; mfac times `unit`, the power of two that a sum of overlaps
+// is multiplied by: done here once per chunk, not in the serial end of each operation.
 template <bool FWD>
 __device__ __forceinline__ void fx_stage_ops(StagedOp* st, const RotOp* ops, const RotRec* recs, int k0, int kn,
                                              double unit) {

@@ -338,7 +338,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   load_tile(psi, a, b, v0, tc, ends);
   for (int e = threadIdx.x; e < tc * N; e += blockDim.x) lam[e] = make_double2(0.0, 0.0);
   bool fixed = false;
-  FxUnit unit;
+  FxUnit unit = {1.0, 1.0};
   if (!ck && a.fixed && (tc <= kFxItems || tc * (N / 2) <= kFxItems * (int)blockDim.x) &&
       isfinite(phase.x) && isfinite(phase.y))
     fixed = fx_from_tile(psi, N, tc, redd, unit);
@@ -385,7 +385,9 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   int pend_coff = 0, pend_mask = 0, pend_aw = 0, buf = 0;
   double pend_fac = 0.0;
   const int shift = fx_sum_shift(tc);
-  const double fx_unit = fixed ? (double)(1 << shift) * (unit.a * unit.b) : 1.0;
+  // the 2^-60 of a sum goes into the unit where that could exceed the range of a double without it
+  const double sum_unit = unit.b >= 1.0 ? 1.0 : 0x1p-60;
+  const double fx_unit = fixed ? (double)(1 << shift) * (unit.b >= 1.0 ? 0x1p-60 : 1.0) * unit.a * unit.b : 1.0;
   auto flush = [&]() {  // one thread per measured overlap
     if (!pend_mask || warp != nw - 1 || lane >= 3) return;
     const int axis = lane;  // 0 X, 1 Y, 2 Z
@@ -396,7 +398,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
       if (fixed) {
         long long v = 0;
         for (int w = 0; w < pend_aw; w++) v += __double_as_longlong(rd[w * NV + k]);
-        return (double)v * 0x1p-60 * pend_fac;
+        return (double)v * sum_unit * pend_fac;
       }
       double v = 0.0;
       for (int w = 0; w < pend_aw; w++) v += rd[w * NV + k];
