@@ -115,9 +115,11 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_matrices(RotPlan pl, const 
   const long long b = blockIdx.y;
   batch_matrices_body(pl, blockIdx.x, theta + b * theta_stride, recs + b * pl.nrecs);
 }
-__global__ void __launch_bounds__(kRotThreads) k_rot_chains(RotPlan pl, int B, RotRec* recs) {
-  const long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (b < B) batch_chain_body(pl, blockIdx.y, recs + b * pl.nrecs);
+// A warp per (chain, 32 vectors), counted in one dimension: circuits have more chains than a grid is
+// high.  The chains of two and more runs come first for all vectors.
+__global__ void __launch_bounds__(32) k_rot_chains(RotPlan pl, int B, int groups, RotRec* recs) {
+  const long long b = (blockIdx.x % groups) * 32LL + threadIdx.x;
+  if (b < B) batch_chain_body(pl, blockIdx.x / groups, recs + b * pl.nrecs);
 }
 __global__ void __launch_bounds__(kRotThreads) k_rot_finish(RotPlan pl, RotRec* recs, double2* __restrict__ phases) {
   const long long b = blockIdx.y;
@@ -434,7 +436,8 @@ int launch_plan(const sqg_circuit* c, const RotPlan& p, const double* theta, lon
   if (p.ncta == 0) return SQG_OK;
   if (B >= kRotBatch) {
     k_rot_matrices<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, theta, theta_stride, recs);
-    k_rot_chains<<<dim3((B + 31) / 32, p.nheads), 32, 0, st>>>(p, B, recs);
+    const int groups = (B + 31) / 32;
+    k_rot_chains<<<(unsigned)groups * p.nheads, 32, 0, st>>>(p, B, groups, recs);
     k_rot_finish<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, recs, ph);
   } else {
     k_rot_plan<<<dim3(p.ncta, B), kRotThreads, 0, st>>>(p, theta, theta_stride, recs, ph,
