@@ -108,16 +108,17 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged_tiles(const InstDe
   }
 }
 
-// blockIdx.x: instance; W doubles per overlap.
+// blockIdx.x: instance, blockIdx.y and so on: 32 of its overlaps, W doubles each.
 template <int W>
 __global__ void __launch_bounds__(32 * kSumGroups) k_ragged_sum(const InstDesc* __restrict__ desc, double2* ws_tr,
                                                                 double* ws_gr, int with_grad, int variant,
                                                                 double* __restrict__ cost) {
   const InstDesc d = desc[blockIdx.x];
   const int nov = with_grad ? d.plan.noverlaps : 0;
-  if (blockIdx.y > 0 && (int)blockIdx.y * 32 >= nov) return;
-  tile_sum_body<W>(blockIdx.y, ws_tr + d.tr_off, ws_gr + d.gr_off * W, d.tiles, nov, d.cols, variant,
-                   cost + blockIdx.x);
+  for (int part = blockIdx.y; part == 0 || part < (nov + 31) / 32; part += gridDim.y) {
+    tile_sum_body<W>(part, ws_tr + d.tr_off, ws_gr + d.gr_off * W, d.tiles, nov, d.cols, variant, cost + blockIdx.x);
+    __syncthreads();  // its sums are no longer read
+  }
 }
 
 template <bool CPLX>
@@ -330,7 +331,7 @@ int sqg_ragged_cost_grad(const sqg_ragged_batch* r, const double* theta, const v
   auto tiles = mode == 0 ? k_ragged_tiles<0> : mode == 1 ? k_ragged_tiles<1> : k_ragged_tiles<2>;
   tiles<<<r->grid, kRaggedThreads, r->smem, s>>>(r->d_desc, r->d_items, r->n_items, counter, tg, recs, ph, tr, gr);
   if ((st = cerr(cudaGetLastError(), "k_ragged_tiles"))) return st;
-  const dim3 sgrid(r->count, grad ? std::max(1, (r->max_overlaps + 31) / 32) : 1);
+  const dim3 sgrid(r->count, grad ? std::min(std::max(1, (r->max_overlaps + 31) / 32), 65535) : 1);
   if (mode < 2)
     k_ragged_sum<1><<<sgrid, 32 * kSumGroups, 0, s>>>(r->d_desc, tr, gr, grad != nullptr, variant, cost);
   else
