@@ -727,8 +727,9 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
   }
   if (a.phases) {
     double2 p = make_double2(1.0, 0.0);
-    for (int k = 0; k < a.nphase; k++) p = cmul(p, a.phases[(long long)b * a.nphase + k]);
-    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = cmul(p, sv[end_place(ends, l)]);
+    bool finite;  // no matter here
+    for (int k = 0; k < a.nphase; k++) p = cmul(p, phase_factor(a.phases[(long long)b * a.nphase + k], finite));
+    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = phase_mul(p, sv[end_place(ends, l)]);
   } else {
     for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = sv[end_place(ends, l)];
   }

@@ -367,28 +367,46 @@ __device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotR
   return own;
 }
 
-// The cosines of a run's record, and its share of the phase: a NaN anywhere (an infinite angle, say)
-// becomes one of the phase too, where sweeps in fixed point look for it.
-__device__ __forceinline__ double2 finish_record(const RotRun& run, RotRec& r, double2 phase) {
+// The cosines of a run's record.  Returns whether its numbers are all finite (an infinite angle, say, makes
+// NaN of some).
+__device__ __forceinline__ bool finish_record(const RotRun& run, RotRec& r) {
   RotRec v = r;
   if (run.kind & kOpRot) set_cosine(v);
   r.c = v.c;
   r.lo = v.lo;
-  phase.x = fma(0.0, v.t + v.c + v.zi.x + v.zi.y + v.zo.x + v.zo.y, phase.x);
-  return phase;
+  return isfinite(v.t + v.c + v.zi.x + v.zi.y + v.zo.x + v.zo.y);
 }
 
-// Product of the threads' phases (kRotThreads of them), written by thread 0.
-__device__ __forceinline__ void phase_product(double2 phase, double2* out) {
+// Product of the threads' phases (kRotThreads of them), written by thread 0; twice that if a record of the
+// CTA's runs is not finite, which sweeps in fixed point need to know and amplitudes that do not meet
+// that record must not notice (phase_factor).
+__device__ __forceinline__ void phase_product(double2 phase, bool finite, double2* out) {
   __shared__ double2 ph[kRotThreads];
   const int i = threadIdx.x;
   ph[i] = phase;
-  __syncthreads();
+  finite = __syncthreads_and(finite);
   for (int o = kRotThreads / 2; o > 0; o >>= 1) {
     if (i < o) ph[i] = cmul(ph[i], ph[i + o]);
     __syncthreads();
   }
-  if (i == 0) *out = ph[0];
+  if (i == 0) *out = finite ? ph[0] : cadd(ph[0], ph[0]);
+}
+
+// A phase as phase_product left it, and whether the records behind it are finite.  The larger component of
+// a phase is at most 1 and a few roundings, that of a doubled one at least 1.41.
+__device__ __forceinline__ double2 phase_factor(double2 p, bool& finite) {
+  const int top = max(__double2hiint(p.x) & 0x7fffffff, __double2hiint(p.y) & 0x7fffffff);
+  if (top < 0x3ff40000) return p;  // 1.25
+  finite = false;
+  return cscale(p, 0.5);
+}
+
+// The common phase times an amplitude.  Phases of 1, -1, i and -i (none at all; rotations about X and Y, CRY)
+// move components as they are: an infinite one must not make NaN of the other.
+__device__ __forceinline__ double2 phase_mul(double2 p, double2 v) {
+  if (p.y == 0.0) return p.x == 1.0 ? v : cscale(v, p.x);
+  if (p.x == 0.0) return make_double2(-p.y * v.y, p.y * v.x);
+  return cmul(p, v);
 }
 
 // The numbers of all operations of the runs of one CTA, for one parameter vector, in one go:
@@ -435,8 +453,8 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
   }
   __syncthreads();
   // the cosines of all runs at once: the chains need not wait for them
-  if (i < n) phase = finish_record(run, recs[run.rec], phase);
-  phase_product(phase, phase_out);
+  const bool finite = i >= n || finish_record(run, recs[run.rec]);
+  phase_product(phase, finite, phase_out);
 }
 
 // The same in three launches for many parameter vectors, the matrices kept in the records: a
@@ -471,6 +489,7 @@ __device__ __forceinline__ void batch_chain_body(const RotPlan& pl, int head, Ro
 __device__ __forceinline__ void batch_finish_body(const RotPlan& pl, int cta, RotRec* recs, double2* phase_out) {
   const int base = pl.cta[cta], n = pl.cta[cta + 1] - base;
   double2 phase = make_double2(1.0, 0.0);
+  bool finite = true;
   if ((int)threadIdx.x < n) {
     const RotRun run = pl.runs[base + threadIdx.x];
     RotRec r = recs[run.rec];
@@ -479,11 +498,11 @@ __device__ __forceinline__ void batch_finish_body(const RotPlan& pl, int cta, Ro
       r.c = 1.0;
       r.lo = 0.0;
     }
-    phase = finish_record(run, r, phase);
+    finite = finish_record(run, r);
     recs[run.rec].c = r.c;
     recs[run.rec].lo = r.lo;
   }
-  phase_product(phase, phase_out);
+  phase_product(phase, finite, phase_out);
 }
 
 // ---- application ---------------------------------------------------------------------------

@@ -32,9 +32,11 @@ struct TileArgs {
   int fixed;         // cost and gradient: sweep finite tiles in fixed point
 };
 
-__device__ __forceinline__ double2 tile_phase(const TileArgs& a, int b) {
+// The instance's common phase; finite: whether the numbers of its operations are.
+__device__ __forceinline__ double2 tile_phase(const TileArgs& a, int b, bool& finite) {
   double2 p = make_double2(1.0, 0.0);
-  for (int k = 0; k < a.nphase; k++) p = cmul(p, a.phases[(long long)b * a.nphase + k]);
+  finite = true;
+  for (int k = 0; k < a.nphase; k++) p = cmul(p, phase_factor(a.phases[(long long)b * a.nphase + k], finite));
   return p;
 }
 
@@ -65,12 +67,12 @@ __device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, 
   if (a.cstride == 1) {
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
       int r = e / tc, c = e - r * tc;
-      base[(long long)r * a.rstride + v0 + c] = cmul(phase, s[c * a.N + end_place(ends, r)]);
+      base[(long long)r * a.rstride + v0 + c] = phase_mul(phase, s[c * a.N + end_place(ends, r)]);
     }
   } else {
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
       int c = e >> a.n, r = e & (a.N - 1);
-      base[(long long)(v0 + c) * a.rstride + r] = cmul(phase, s[c * a.N + r]);
+      base[(long long)(v0 + c) * a.rstride + r] = phase_mul(phase, s[c * a.N + r]);
     }
   }
 }
@@ -165,13 +167,14 @@ __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int 
   __shared__ int ends[16 * kEndGroups];
   const int v0 = tile * a.TC;
   const int tc = min(a.TC, a.cols - v0);
-  const double2 phase = tile_phase(a, b);
+  bool finite;
+  const double2 phase = tile_phase(a, b, finite);
   fill_end_table(ends, a.ends, a.n);
   if (DIR == kRotTrans) __syncthreads();
   load_tile(s, a, b, v0, tc, ends);
   bool fixed = false;
   FxUnit unit;
-  if (!WRITE_BACK && a.fixed && isfinite(phase.x) && isfinite(phase.y))
+  if (!WRITE_BACK && a.fixed && finite)
     fixed = fx_from_tile(s, a.N, tc, red, unit);
   const RotRec* recs = a.recs + (long long)b * a.nrecs;
   const int nchunks = (a.nops + kRotChunk - 1) / kRotChunk;
@@ -195,7 +198,7 @@ __device__ __forceinline__ void tile_forward_body(const TileArgs& a, int b, int 
   __syncthreads();
   if (TRACE) {
     const double2 t = tile_trace_at(s, a.N, tc, v0 + a.trace_offset, ends, red, fixed, unit);
-    if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
+    if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = phase_mul(phase, t);
   }
   if (WRITE_BACK) store_tile(s, a, b, v0, tc, phase, ends);
 }
@@ -330,7 +333,8 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   const size_t tile_elems = (size_t)a.TC * N;
   double2* ck = a.ckpt ? a.ckpt + ((long long)b * a.tiles + tile) * a.nck * tile_elems : nullptr;
   const RotRec* recs = a.recs + (long long)b * a.nrecs;
-  const double2 phase = tile_phase(a, b);
+  bool finite;
+  const double2 phase = tile_phase(a, b, finite);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 
   __shared__ int ends[16 * kEndGroups];
@@ -339,8 +343,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   for (int e = threadIdx.x; e < tc * N; e += blockDim.x) lam[e] = make_double2(0.0, 0.0);
   bool fixed = false;
   FxUnit unit = {1.0, 1.0};
-  if (!ck && a.fixed && (tc <= kFxItems || tc * (N / 2) <= kFxItems * (int)blockDim.x) &&
-      isfinite(phase.x) && isfinite(phase.y))
+  if (!ck && a.fixed && finite && (tc <= kFxItems || tc * (N / 2) <= kFxItems * (int)blockDim.x))
     fixed = fx_from_tile(psi, N, tc, redd, unit);
   __syncthreads();
   // <lambda| carries the common phase: lambda_j = conj(phase) e_{j + offset}
@@ -376,7 +379,7 @@ __device__ __forceinline__ void tile_adjoint_body(const TileArgs& a, int b, int 
   }
   __syncthreads();
   double2 t = tile_trace_at(psi, N, tc, v0 + a.trace_offset, ends, redd, fixed, unit);
-  if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = cmul(phase, t);
+  if (threadIdx.x == 0) a.ws_tr[(long long)b * a.tiles + tile] = phase_mul(phase, t);
   __syncthreads();
 
   // reverse sweep.  The warps' totals of an operation are summed and written by the last warp
