@@ -171,8 +171,10 @@ int sqg_apply(const sqg_circuit* circuit, const double* theta_dev, int batch, vo
  * examples/simulation/QC_sim_benchmark.py).  fused != 0 groups consecutive gates whose qubits,
  * together with the five lowest, number at most 12 into blocks (the role of the reference's
  * partitioning into fused blocks, squander/partitioning) and applies each block to chunks of
- * 4096 amplitudes in shared memory: one read and write of the state per block
- * (sqg_state_block_count); fused == 0 makes one pass per gate.  Circuit handles of more than
+ * 4096 amplitudes in shared memory: one read and write of the state per block.  Registers of up to 20
+ * qubits whose chunks are too few for the device take smaller ones, of 2^9 amplitudes and more, with as
+ * many fewer qubits per block.  sqg_state_block_count: the passes over one state (batch 1); more states
+ * may take fewer passes, in larger chunks.  fused == 0 makes one pass per gate.  Circuit handles of more than
  * 13 qubits are accepted only by this entry point.  Workspace: sqg_state_workspace_bytes. */
 size_t sqg_state_workspace_bytes(const sqg_circuit* circuit, int batch);
 int sqg_state_block_count(const sqg_circuit* circuit);
@@ -180,7 +182,8 @@ int sqg_state_block_count(const sqg_circuit* circuit);
 /* Hands a partitioning of the gate list to the fused state-vector plan: part_ends[i] is the
  * gate index after partition i (non-decreasing, the last equal to gate_num).  Fused passes
  * then start only at partition boundaries, consecutive partitions merged while their qubits
- * with the five lowest number at most 12 (a partition larger than that is split gate by gate);
+ * with the five lowest fit a chunk, of 12 qubits or fewer (a partition of more than 12 with the five
+ * lowest is split gate by gate; smaller chunks split no other);
  * nparts == 0 restores the gate-by-gate plan.  The partitions come from the partitioner
  * (squander/partitioning/partition.py:PartitionCircuit, kahn.py), which reorders the gates so
  * that each partition spans few qubits.  Rebuilds the plan synchronously; no work that uses

@@ -526,6 +526,7 @@ struct StatePlanHost {
   std::vector<RotOp> lops;
   std::vector<int> lends, hitab, inact;
   std::vector<sqg_state_block> blocks;
+  int split = 0;  // partitions larger than a chunk
 };
 StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<int>& cuts) {
   const int n = c->n, low = std::min(K, kStateLow);
@@ -607,6 +608,7 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
         mark[q] = 0;
       }
       if (low + own > K) {  // the partition alone exceeds the chunk
+        out.split++;
         for (int g = s0; g < e; g++) take_gate(g);
       } else {
         if (low + used + add > K) {
@@ -626,14 +628,18 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
 }
 
 // Makes the state-vector plans of the circuit: chunks of 2^12 amplitudes, and, for registers whose
-// chunks are too few for the device, smaller ones down to 2^9.
+// chunks are too few for the device, smaller ones down to 2^9, where they split no partition that the
+// largest hold.
 int make_state_plans(sqg_circuit* c, const std::vector<int>& cuts = {}) {
   c->splans.clear();
   std::vector<char> blob;
   std::vector<size_t> off;
   const int largest = std::min(c->n, kStateK);
+  int split = 0;
   for (int K = largest; K >= (c->n <= 20 ? std::min(largest, 9) : largest); K--) {
     const StatePlanHost h = build_state_plan(c, K, cuts);
+    if (K == largest) split = h.split;
+    if (h.split > split) break;  // so would those of still smaller chunks
     sqg_state_plan p;
     p.K = K;
     p.nops = (int)h.lops.size();
@@ -1285,7 +1291,7 @@ size_t sqg_state_workspace_bytes(const sqg_circuit* c, int batch) {
   return prep_layout(c, batch, 0).end;
 }
 
-int sqg_state_block_count(const sqg_circuit* c) { return c ? (int)c->splans[0].blocks.size() : -1; }
+int sqg_state_block_count(const sqg_circuit* c) { return c ? (int)choose_state_plan(c, 1).blocks.size() : -1; }
 
 int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* states, long long stride, int fused,
                     void* workspace, size_t ws_bytes, void* stream) {
