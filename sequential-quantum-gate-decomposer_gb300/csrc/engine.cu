@@ -535,27 +535,28 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
   std::vector<int>&lends = out.lends, &hitab = out.hitab, &inact = out.inact;
   size_t done = 0;  // steps placed in blocks (they follow the order of their anchor gates)
   std::vector<int> inA(n, 0), A, loc(n);
+  std::vector<RotCz> scratch;
   lops.reserve(c->h_steps.size() + 16);
-  auto close_block = [&](int g0, int g1) {
-    A.clear();
-    for (int q = 0; q < n; q++)
-      if (q < low || inA[q]) A.push_back(q);
-    for (int q = 0; q < n && (int)A.size() < K; q++)
-      if (!(q < low || inA[q])) {
-        A.push_back(q);
+  const int hb = K - low;
+  int used = 0;  // qubits of the block's gates above the lowest
+  auto close_block = [&](int g1) {  // its gates end before g1
+    int free = K - low - used;
+    for (int q = low; q < n && free > 0; q++)
+      if (!inA[q]) {
         inA[q] = 1;
+        free--;
       }
-    std::sort(A.begin(), A.end());
-    std::fill(loc.begin(), loc.end(), -1);
-    for (int j = 0; j < (int)A.size(); j++) loc[A[j]] = j;
+    A.clear();
+    for (int q = 0; q < n; q++) {
+      loc[q] = q < low || inA[q] ? (int)A.size() : -1;
+      if (loc[q] >= 0) A.push_back(q);
+    }
     const int s0 = (int)done, k0 = (int)lops.size();
     while (done < c->h_steps.size() && c->h_steps[done].anchor < g1) done++;
-    lower_rot_steps(c->h_steps, s0, (int)done, K, loc, lops, lends);
+    lower_rot_steps(c->h_steps, s0, (int)done, K, loc, lops, lends, scratch);
     lends.resize(16 * (out.blocks.size() + 1), 0);
-    (void)g0;
-    const int hb = K - low;
     const size_t h0 = hitab.size();
-    hitab.resize(h0 + 128, 0);
+    hitab.resize(h0 + (size_t(1) << hb), 0);
     for (int h = 1; h < (1 << hb); h++)
       hitab[h0 + h] = hitab[h0 + (h & (h - 1))] | 1 << A[low + __builtin_ctz(h)];
     int k = 0;
@@ -567,8 +568,8 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
     for (; k < 32; k++) inact.push_back(0);
     out.blocks.push_back({k0, (int)lops.size()});
     std::fill(inA.begin(), inA.end(), 0);
+    used = 0;
   };
-  int g0 = 0, used = 0;
   auto take_gate = [&](int g) {  // gate by gate: break wherever the chunk would overflow
     const Gate& gt = c->h_gates[g];
     int add = 0;
@@ -576,9 +577,7 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
     for (int q : qs)
       if (q >= low && !inA[q]) add++;
     if (low + used + add > K) {
-      close_block(g0, g);
-      g0 = g;
-      used = 0;
+      close_block(g);
     }
     for (int q : qs)
       if (q >= low && !inA[q]) {
@@ -612,9 +611,7 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
         for (int g = s0; g < e; g++) take_gate(g);
       } else {
         if (low + used + add > K) {
-          close_block(g0, s0);
-          g0 = s0;
-          used = 0;
+          close_block(s0);
           add = own;
         }
         for (int q : fresh) inA[q] = 1;
@@ -623,45 +620,55 @@ StatePlanHost build_state_plan(const sqg_circuit* c, int K, const std::vector<in
       s0 = e;
     }
   }
-  if (c->L > 0) close_block(g0, c->L);
+  if (c->L > 0) close_block(c->L);
   return out;
 }
 
 // Makes the state-vector plans of the circuit: chunks of 2^12 amplitudes, and, for registers whose
 // chunks are too few for the device, smaller ones down to 2^9, where they split no partition that the
-// largest hold.
-int make_state_plans(sqg_circuit* c, const std::vector<int>& cuts = {}) {
-  c->splans.clear();
-  std::vector<char> blob;
-  std::vector<size_t> off;
+// largest hold.  They are appended to the blob, their device pointers counted from null until state_plans_at.
+std::vector<sqg_state_plan> make_state_plans(const sqg_circuit* c, const std::vector<int>& cuts,
+                                             std::vector<char>& blob) {
+  std::vector<sqg_state_plan> plans;
   const int largest = std::min(c->n, kStateK);
   int split = 0;
   for (int K = largest; K >= (c->n <= 20 ? std::min(largest, 9) : largest); K--) {
-    const StatePlanHost h = build_state_plan(c, K, cuts);
+    StatePlanHost h = build_state_plan(c, K, cuts);
     if (K == largest) split = h.split;
     if (h.split > split) break;  // so would those of still smaller chunks
     sqg_state_plan p;
     p.K = K;
     p.nops = (int)h.lops.size();
-    p.blocks = h.blocks;
-    c->splans.push_back(p);
-    off.push_back(blob_put(blob, h.lops.data(), h.lops.size() * sizeof(RotOp)));
-    off.push_back(blob_put(blob, h.lends.data(), h.lends.size() * sizeof(int)));
-    off.push_back(blob_put(blob, h.hitab.data(), h.hitab.size() * sizeof(int)));
-    off.push_back(blob_put(blob, h.inact.data(), h.inact.size() * sizeof(int)));
+    p.blocks = std::move(h.blocks);
+    p.lops = blob_put(blob, h.lops.data(), h.lops.size() * sizeof(RotOp));
+    p.lends = blob_put(blob, h.lends.data(), h.lends.size() * sizeof(int));
+    p.hitab = blob_put(blob, h.hitab.data(), h.hitab.size() * sizeof(int));
+    p.inact = blob_put(blob, h.inact.data(), h.inact.size() * sizeof(int));
+    plans.push_back(std::move(p));
   }
-  if (blob.empty()) return SQG_OK;
-  cudaError_t e = cudaMalloc(&c->d_state, blob.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_state, blob.data(), blob.size(), cudaMemcpyHostToDevice);
-  const char* d = (const char*)c->d_state;
-  for (size_t k = 0; k < c->splans.size(); k++) {
-    sqg_state_plan& p = c->splans[k];
-    p.d_lops = (const RotOp*)(d + off[4 * k]);
-    p.d_lends = (const int*)(d + off[4 * k + 1]);
-    p.d_hitab = (const int*)(d + off[4 * k + 2]);
-    p.d_inact = (const int*)(d + off[4 * k + 3]);
+  return plans;
+}
+void state_plans_at(std::vector<sqg_state_plan>& plans, const void* base) {
+  const char* d = (const char*)base;
+  for (sqg_state_plan& p : plans) {
+    p.d_lops = (const RotOp*)(d + p.lops);
+    p.d_lends = (const int*)(d + p.lends);
+    p.d_hitab = (const int*)(d + p.hitab);
+    p.d_inact = (const int*)(d + p.inact);
   }
-  return cuda_status(e, "state plan");
+}
+
+// The blob on the device; *out is set on success only.
+int blob_to_device(const std::vector<char>& blob, void** out, const char* where) {
+  void* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, std::max<size_t>(blob.size(), 1));
+  if (e == cudaSuccess) e = cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    if (d) cudaFree(d);
+    return cuda_status(e, where);
+  }
+  *out = d;
+  return SQG_OK;
 }
 
 // The plan for `batch` states: the least of the modelled times.  An operation takes 1 ns per
@@ -746,22 +753,27 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
 // =====================================================================================
 // C ABI
 // =====================================================================================
-// Makes the rotation plans of the circuit and copies them to the device with its gates, in one
-// allocation.
-static int make_rot_plans(sqg_circuit* c) {
+// Makes the rotation and state-vector plans of the circuit and copies them to the device with its gates,
+// in one allocation.  Host time is what a handle costs: GB300's host, 42 gates on three qubits 107 us (131 us
+// with two allocations, lists of lists for the runs and 128 offsets for every block), 2000 gates on twelve
+// 588 us (924 us).
+static int make_plans(sqg_circuit* c) {
   std::vector<char> blob;
   const size_t o_gates = blob_put(blob, c->h_gates.data(), c->h_gates.size() * sizeof(Gate));
   RotPlan* plans[2] = {&c->plan, &c->short_plan};
   size_t off[2][8];
   const int nplans = c->n <= kMatrixQubits ? 2 : 1;  // state vectors use the first alone
+  const RotRuns runs = find_rot_runs(c->n, c->h_gates);
   for (int k = 0; k < nplans; k++) {
-    const RotPlanHost h = build_rot_plan(c->n, c->h_gates, k ? kRotShortChain : kRotChain);
+    RotPlanHost h = build_rot_plan(runs, c->h_gates, k ? kRotShortChain : kRotChain);
     std::vector<RotOp> ops;
     std::vector<int> ends;
     if (c->n <= kMatrixQubits) {  // larger registers are applied in chunks only
       std::vector<int> loc(c->n);
+      std::vector<RotCz> scratch;
+      ops.reserve(h.steps.size() + 16);
       for (int q = 0; q < c->n; q++) loc[q] = q;
-      lower_rot_steps(h.steps, 0, (int)h.steps.size(), c->n, loc, ops, ends);
+      lower_rot_steps(h.steps, 0, (int)h.steps.size(), c->n, loc, ops, ends, scratch);
     }
     RotPlan& p = *plans[k];
     p.nops = (int)ops.size();
@@ -777,11 +789,13 @@ static int make_rot_plans(sqg_circuit* c) {
     off[k][6] = blob_put(blob, ends.data(), ends.size() * sizeof(int));
     off[k][7] = blob_put(blob, h.heads.data(), h.heads.size() * sizeof(int));
     p.nheads = (int)h.heads.size();
-    if (k == 0) c->h_steps = h.steps;
+    if (k == 0) c->h_steps = std::move(h.steps);
   }
-  cudaError_t e = cudaMalloc(&c->d_plan, blob.size());
-  if (e == cudaSuccess) e = cudaMemcpy(c->d_plan, blob.data(), blob.size(), cudaMemcpyHostToDevice);
+  c->splans = make_state_plans(c, {}, blob);
+  const int st = blob_to_device(blob, &c->d_plan, "circuit handle");
+  if (st) return st;
   const char* d = (const char*)c->d_plan;
+  state_plans_at(c->splans, d);
   c->d_gates = (Gate*)(d + o_gates);
   for (int k = 0; k < nplans; k++) {
     RotPlan& p = *plans[k];
@@ -795,7 +809,7 @@ static int make_rot_plans(sqg_circuit* c) {
     p.ends = (const int*)(d + off[k][6]);
     p.heads = (const int*)(d + off[k][7]);
   }
-  return cuda_status(e, "circuit handle");
+  return SQG_OK;
 }
 
 extern "C" {
@@ -854,8 +868,7 @@ int sqg_circuit_create(int qbit_num, const sqg_gate* gates, int gate_num, sqg_ci
   }
   c->P = p;
   cudaGetDevice(&c->device);
-  int st = make_rot_plans(c);
-  if (!st) st = make_state_plans(c);
+  int st = make_plans(c);
   if (st) {
     sqg_circuit_destroy(c);
     return st;
@@ -875,9 +888,16 @@ int sqg_circuit_set_partitions(sqg_circuit* c, const int* part_ends, int nparts)
   int dev = -1;
   cudaGetDevice(&dev);
   if (dev != c->device) return fail(SQG_ERR_INVALID_ARGUMENT, "circuit handle belongs to another device");
+  std::vector<char> blob;
+  std::vector<sqg_state_plan> plans = make_state_plans(c, cuts, blob);
+  void* d = nullptr;
+  const int st = blob_to_device(blob, &d, "state plan");
+  if (st) return st;  // the plan that was there stays
+  state_plans_at(plans, d);
+  c->splans = std::move(plans);
   cudaFree(c->d_state);
-  c->d_state = nullptr;
-  return make_state_plans(c, cuts);
+  c->d_state = d;
+  return SQG_OK;
 }
 
 int sqg_circuit_destroy(sqg_circuit* c) {
@@ -1326,7 +1346,7 @@ int sqg_apply_state(const sqg_circuit* c, const double* theta, int B, void* stat
       a.k1 = sp.blocks[k].k1;
       a.phases = k == 0 && t.nphase > 0 ? t.phases : nullptr;
       a.ends = sp.d_lends + 16 * k;
-      a.hitab = sp.d_hitab + 128 * k;
+      a.hitab = sp.d_hitab + (k << (a.K - a.low));
       a.inact = sp.d_inact + 32 * k;
       k_state_block<<<dim3(1u << (c->n - sp.K), B), kStateThreads, smem, s>>>(a);
     }

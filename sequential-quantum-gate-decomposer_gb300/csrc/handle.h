@@ -15,10 +15,12 @@ struct sqg_state_block {
 
 // A plan of such passes: chunk qubits K, blocks, operations on chunk-local qubits, per block the
 // places behind its last operation (K ints, padded to 16), the global offsets of the chunk's high
-// local bits (2^(K - low) ints, padded to 128) and the qubits that number the chunks (padded to 32).
+// local bits (2^(K - low) ints) and the qubits that number the chunks (padded to 32).  lops to inact: where
+// these arrays are in their device allocation.
 struct sqg_state_plan {
   int K = 0, nops = 0;
   std::vector<sqg_state_block> blocks;
+  size_t lops = 0, lends = 0, hitab = 0, inact = 0;
   const sqg::RotOp* d_lops = nullptr;
   const int *d_lends = nullptr, *d_hitab = nullptr, *d_inact = nullptr;
 };
@@ -29,12 +31,14 @@ struct sqg_circuit {
   sqg::Gate* d_gates = nullptr;
   std::vector<sqg::Gate> h_gates;
   // rotation plan (rot.cuh): the host's steps, from which the operations of the state-vector
-  // blocks are made, and the device arrays, one allocation with the gates behind d_plan.
+  // blocks are made, and the device arrays, one allocation with the gates and state-vector plans behind
+  // d_plan.
   // short_plan: the same with short chains, for launches that wait for the chains.
   std::vector<sqg::RotStep> h_steps;
   void* d_plan = nullptr;
   sqg::RotPlan plan = {}, short_plan = {};
-  // state-vector plans, the first with the largest chunks; their device arrays are one allocation
+  // state-vector plans, the first with the largest chunks; d_state: the arrays of those that follow
+  // handed-over partitions
   std::vector<sqg_state_plan> splans;
   void* d_state = nullptr;
 };
