@@ -116,9 +116,9 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double cnorm2(double2 a) { return fma(a.x, a.x, a.y * a.y); }
-// 1 / sqrt(x) and 1 / x for x in [2^-120, 2^120], to a rounding: from the single-precision value by
-// two Newton steps.  The chains of rot_plan_body wait for every one of their instructions, and
-// the general functions take several times as many.
+// 1 / sqrt(x) and 1 / x for x in [2^-120, 2^120], to 1.5 and 1 times 2^-53 (relative): from the
+// single-precision value by two Newton steps.  The chains of rot_plan_body wait for every one of their
+// instructions, and the general functions take several times as many.
 __device__ __forceinline__ double fast_rsqrt(double x) {
   double y = (double)rsqrtf((float)x);
   const double h = -0.5 * x;
