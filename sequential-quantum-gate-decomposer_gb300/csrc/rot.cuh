@@ -112,7 +112,6 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // a * conj(b)
   return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
 }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double cnorm2(double2 a) { return fma(a.x, a.x, a.y * a.y); }
@@ -135,13 +134,42 @@ __device__ __forceinline__ double fast_rcp(double x) {
 __device__ __forceinline__ double2 cgrow(double2 z, double e) { return make_double2(fma(z.x, e, z.x), fma(z.y, e, z.y)); }
 __device__ __forceinline__ double2 cunit(double2 z) { return cgrow(z, -0.5 * fma(z.x, z.x, fma(z.y, z.y, -1.0))); }
 
+// ---- numbers of the chains: 64-bit fixed point --------------------------------------------------
+// The entries of unitaries, in units of 2^-62.  What a chain hands from run to run passes some
+// twenty products, whose roundings in FP64 would be as large as those of all amplitudes: with the chains
+// in FP64 the error of circuits of U3 and CNOT was 1.1 to 1.6 times that of the gates as given.  Here a product
+// is good to 2^-60 and answers in a tenth of the time.
+struct Q2 {
+  long long x, y;
+};
+constexpr long long kQOne = 1LL << 62;
+__device__ __forceinline__ long long q_of(double v) { return __double2ll_rn(v * 0x1p62); }
+__device__ __forceinline__ Q2 q_of(double2 v) { return {q_of(v.x), q_of(v.y)}; }
+__device__ __forceinline__ double q_to(long long v) { return (double)v * 0x1p-62; }
+__device__ __forceinline__ double2 q_to(Q2 v) { return make_double2(q_to(v.x), q_to(v.y)); }
+// Four units of the sum are those of the upper words; half of what their floors drop is put back.
+__device__ __forceinline__ long long q_mul(long long a, long long b) { return __mul64hi(a, b) * 4 + 2; }
+__device__ __forceinline__ long long q_sum(long long a, long long b, long long c, long long d) {  // a b + c d
+  return (__mul64hi(a, b) + __mul64hi(c, d)) * 4 + 4;
+}
+__device__ __forceinline__ long long q_diff(long long a, long long b, long long c, long long d) {  // a b - c d
+  return (__mul64hi(a, b) - __mul64hi(c, d)) * 4;
+}
+__device__ __forceinline__ Q2 q_mul(Q2 a, Q2 b) { return {q_diff(a.x, b.x, a.y, b.y), q_sum(a.x, b.y, a.y, b.x)}; }
+__device__ __forceinline__ Q2 q_mulc(Q2 a, Q2 b) {  // a * conj(b)
+  return {q_sum(a.x, b.x, a.y, b.y), q_diff(a.y, b.x, a.x, b.y)};
+}
+__device__ __forceinline__ Q2 q_scale(Q2 a, long long s) { return {q_mul(a.x, s), q_mul(a.y, s)}; }
+__device__ __forceinline__ Q2 q_add(Q2 a, Q2 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ Q2 q_sub(Q2 a, Q2 b) { return {a.x - b.x, a.y - b.y}; }
+
 // M <- G M
-__device__ __forceinline__ void matmul2(const double2 G[4], double2 M[4]) {
-  const double2 a = M[0], b = M[1];
-  M[0] = cadd(cmul(G[0], a), cmul(G[1], M[2]));
-  M[1] = cadd(cmul(G[0], b), cmul(G[1], M[3]));
-  M[2] = cadd(cmul(G[2], a), cmul(G[3], M[2]));
-  M[3] = cadd(cmul(G[2], b), cmul(G[3], M[3]));
+__device__ __forceinline__ void q_matmul(const Q2 G[4], Q2 M[4]) {
+  const Q2 a = M[0], b = M[1];
+  M[0] = q_add(q_mul(G[0], a), q_mul(G[1], M[2]));
+  M[1] = q_add(q_mul(G[0], b), q_mul(G[1], M[3]));
+  M[2] = q_add(q_mul(G[2], a), q_mul(G[3], M[2]));
+  M[3] = q_add(q_mul(G[2], b), q_mul(G[3], M[3]));
 }
 
 // (cos, sin) of every listed parameter of a CTA's runs, one per thread: a warp's FP64 instruction
@@ -163,17 +191,10 @@ __device__ __forceinline__ double2 param_sincos(const double2* sc, int soff, con
   return make_double2(c, s);
 }
 
-// Full 2x2 matrix of a single-qubit gate.
-__device__ __forceinline__ void gate_matrix(int type, const double2* sc, int soff, const double* th, double2 u[4]) {
-  const double2 a = param_sincos(sc, soff, th, 0);
+// Full 2x2 matrix of a gate of one parameter, given as (cos, sin).
+__device__ __forceinline__ void gate_matrix(int type, double2 a, double2 u[4]) {
   const double c = a.x, s = a.y;
-  if (type == G_U3) {
-    const double2 ph = param_sincos(sc, soff, th, 1), la = param_sincos(sc, soff, th, 2);
-    u[0] = make_double2(c, 0.0);
-    u[1] = cscale(la, -s);
-    u[2] = cscale(ph, s);
-    u[3] = cscale(cmul(ph, la), c);
-  } else if (type == G_RX) {
+  if (type == G_RX) {
     u[0] = u[3] = make_double2(c, 0.0);
     u[1] = u[2] = make_double2(0.0, -s);
   } else if (type == G_RZ) {
@@ -198,58 +219,60 @@ __device__ __forceinline__ void set_cosine(RotRec& r) {
   r.lo = 0.5 * r.c * ((1.0 - p) - pe);
 }
 
-// M (unitary) as scalar * diag(1, zo) * R * [exchange] * diag(1, zi); returns the scalar's
-// phase.  The larger entry of the first column is the pivot, so |t| <= 1.
-__device__ __forceinline__ double2 split_zyz(const double2 M[4], RotRec& r) {
-  const double na = cnorm2(M[0]), nc = cnorm2(M[2]);
+// A unitary with first column (p, q) and determinant det as scalar * diag(1, zo) * R * [exchange] * diag(1,
+// zi); returns the scalar's phase.  The larger entry of the first column is the pivot, so |t| <= 1.
+__device__ __forceinline__ double2 split_zyz(Q2 p, Q2 q, Q2 det, RotRec& r) {
+  const double2 pd = q_to(p), qd = q_to(q);
+  const double na = cnorm2(pd), nc = cnorm2(qd);
   const bool turn = nc > na;
-  const double2 piv = turn ? M[2] : M[0], oth = turn ? M[0] : M[2];
+  const Q2 piv = turn ? q : p;
   const double np = turn ? nc : na;
-  const double inp = fast_rcp(np);
-  const double2 q = cscale(cmulc(oth, piv), inp);  // f = 0: t zo, f = 1: -t / zo
-  const double t2 = cnorm2(q);
+  // other entry / pivot: f = 0: t zo, f = 1: -t / zo
+  const double2 x = q_to(q_mulc(turn ? p : q, piv));
+  const double x2 = cnorm2(x);
   // t below 1e-17 is an entry lost in the rounding of the others: any phase does
-  const double rt = t2 > 1e-34 ? fast_rsqrt(t2) : 0.0, t = t2 * rt;
+  const double rx = x2 > 1e-34 ? fast_rsqrt(x2) : 0.0;
+  r.t = x2 * rx * fast_rcp(np);
   double2 zo = make_double2(1.0, 0.0);
-  if (t2 > 1e-34) zo = cscale(turn ? make_double2(-q.x, q.y) : q, rt);
+  if (x2 > 1e-34) zo = cscale(turn ? make_double2(-x.x, x.y) : x, rx);
   zo = cunit(zo);
-  // turn = 0: zi = (d / a) / zo;  turn = 1: zi = -(b / c) zo
-  const double2 w = cscale(cmulc(turn ? M[1] : M[3], piv), inp);
-  double2 zi = turn ? cmul(make_double2(-w.x, -w.y), zo) : cmulc(w, zo);
-  zi = cunit(cunit(zi));
+  // the second column is (-conj q, conj p) det: its entry beside the pivot, over the pivot (f = 0: d / a, f
+  // = 1: b / c), is det conj(piv)^2 / np, negated for f = 1, where zi has another minus: zi = it / zo, or times zo
+  const Q2 w = q_mulc(q_mulc(det, piv), piv), zq = q_of(zo);
+  const double2 z = q_to(turn ? q_mul(w, zq) : q_mulc(w, zq));
+  const double2 zi = cunit(cscale(z, fast_rsqrt(cnorm2(z))));
   r.turn = turn;
-  r.t = t;
   // the quarter turn (x, y) -> (-y, x) as an exchange: its sign goes into zi
   r.zi = turn ? make_double2(-zi.x, -zi.y) : zi;
   r.zo = zo;
-  const double2 u = cscale(piv, fast_rsqrt(np));
-  return turn ? cmulc(u, zo) : u;
+  const Q2 u = turn ? q_mulc(piv, zq) : piv;
+  return cunit(cscale(q_to(u), fast_rsqrt(np)));
 }
 
 // A unitary with first column (p, q) and determinant det as W * Ry(atan t) * diag(1, zi) with W =
 // phase * Rx = [[w0, w1], [w1, w0]].  |t| <= 1 always.  The cosine is left to set_cosine.  On
-// return p, q, det are those of W.
-__device__ __forceinline__ void split_x(double2& p, double2& q, double2& det, RotRec& r) {
+// return p, q, det are those of W, made with t and zi as the record holds them: their roundings go no
+// further.
+__device__ __forceinline__ void split_x(Q2& p, Q2& q, Q2& det, RotRec& r) {
   // (p^2 - q^2) / det = e^{-2 i gamma} cos 2 beta, with zi = e^{2 i gamma}
-  const double2 pq = cadd(p, q), mq = csub(p, q);
-  const double2 d = cmulc(cmul(pq, mq), det);
+  const double2 d = q_to(q_mulc(q_mul(q_add(p, q), q_sub(p, q)), det));
   const double nd2 = cnorm2(d), rnd = nd2 > 1e-34 ? fast_rsqrt(nd2) : 0.0;
-  const double2 zi = nd2 > 1e-34 ? make_double2(d.x * rnd, -d.y * rnd) : make_double2(1.0, 0.0);
-  const double sb = fma(p.x, q.x, p.y * q.y);
-  const double t = 2.0 * sb * fast_rcp(fma(nd2, rnd, 1.0));
-  const double c = fast_rsqrt(fma(t, t, 1.0)), sn = t * c;
-  // W = A diag(1, conj zi) Ry(-beta); the second column of A is (-conj q, conj p) det
-  det = cmulc(det, zi);
-  const double2 b = cmulc(det, q);  // minus the upper entry of A diag(1, conj zi)
-  const double2 w0 = make_double2(fma(c, p.x, sn * b.x), fma(c, p.y, sn * b.y));
-  const double2 w1 = make_double2(fma(sn, p.x, -(c * b.x)), fma(sn, p.y, -(c * b.y)));
-  const double e = -0.5 * (fma(w0.x, w0.x, fma(w0.y, w0.y, -1.0)) + cnorm2(w1));
-  p = cgrow(w0, e);
-  q = cgrow(w1, e);
-  det = cunit(det);
+  r.zi = nd2 > 1e-34 ? cunit(make_double2(d.x * rnd, -d.y * rnd)) : make_double2(1.0, 0.0);
+  const double sb2 = 2.0 * q_to(q_sum(p.x, q.x, p.y, q.y)), den = fma(nd2, rnd, 1.0), inv = fast_rcp(den);
+  const double t0 = sb2 * inv;
+  r.t = fma(fma(-t0, den, sb2), inv, t0);
   r.turn = 0;
-  r.t = t;
-  r.zi = cunit(zi);
+  // cosine of t: one Newton step in units from the double
+  const long long t = q_of(r.t), c0 = q_of(fast_rsqrt(fma(r.t, r.t, 1.0)));
+  const long long c2 = q_mul(c0, c0), e = kQOne - c2 - q_mul(c2, q_mul(t, t));
+  const long long c = c0 + q_mul(c0, e) / 2, sn = q_mul(t, c);
+  // W = A diag(1, conj zi) Ry(-beta); the second column of A is (-conj q, conj p) det
+  det = q_mulc(det, q_of(r.zi));
+  det = q_add(det, q_scale(det, (kQOne - q_sum(det.x, det.x, det.y, det.y)) / 2));  // zi is a unit to 2^-53
+  const Q2 b = q_mulc(det, q);  // minus the upper entry of A diag(1, conj zi)
+  const Q2 w0 = {q_sum(c, p.x, sn, b.x), q_sum(c, p.y, sn, b.y)};
+  q = {q_diff(sn, p.x, c, b.x), q_diff(sn, p.y, c, b.y)};
+  p = w0;
 }
 
 // U3 = diag(1, phi) Ry(s, c) diag(1, lam), all three given as (cos, sin), times a phase: the
@@ -267,8 +290,13 @@ __device__ __forceinline__ double split_u3(double2 cs, double2 phi, double2 lam,
   return c < 0.0 ? -1.0 : 1.0;
 }
 
-// Matrix of a run (a lone U3: (cos, sin) of its three angles and phi lambda) from its CTA's
-// parameters.
+// Matrix of a run from its CTA's parameters: of a lone U3 (cos, sin) of its three angles and phi lambda; of
+// another gate by itself its entries; of several gates the product's entries in units (Q2), or kQBad for
+// the first where an angle is not finite.
+constexpr long long kQBad = (long long)0x8000000000000000ULL;
+__device__ __forceinline__ double2 q_bits(Q2 v) { return make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y)); }
+__device__ __forceinline__ Q2 q_of_bits(double2 v) { return {__double_as_longlong(v.x), __double_as_longlong(v.y)}; }
+
 __device__ __forceinline__ void run_matrix(const RotPlan& pl, const RotRun& run, const double2* sc,
                                            const double* theta, double2 M[4]) {
   Gate g = pl.gates[pl.members[run.first]];
@@ -278,14 +306,37 @@ __device__ __forceinline__ void run_matrix(const RotPlan& pl, const RotRun& run,
     M[3] = cmul(M[1], M[2]);
     return;
   }
-  gate_matrix(g.type, sc, soff, theta + g.pstart, M);
-  for (int k = 1; k < run.count; k++) {
-    double2 G[4];
-    if (soff >= 0) soff += gate_param_num(g.type);
-    g = pl.gates[pl.members[run.first + k]];
-    gate_matrix(g.type, sc, soff, theta + g.pstart, G);
-    matmul2(G, M);
+  if (run.count == 1) {
+    gate_matrix(g.type, param_sincos(sc, soff, theta + g.pstart, 0), M);
+    return;
   }
+  Q2 P[4] = {{kQOne, 0}, {0, 0}, {0, 0}, {kQOne, 0}};
+  bool finite = true;
+  for (int k = 0; k < run.count; k++) {
+    if (k > 0) {
+      if (soff >= 0) soff += gate_param_num(g.type);
+      g = pl.gates[pl.members[run.first + k]];
+    }
+    const double2 a = param_sincos(sc, soff, theta + g.pstart, 0);
+    finite = finite && isfinite(a.x);
+    Q2 G[4];
+    if (g.type == G_U3) {
+      const double2 ph = param_sincos(sc, soff, theta + g.pstart, 1), la = param_sincos(sc, soff, theta + g.pstart, 2);
+      finite = finite && isfinite(ph.x) && isfinite(la.x);
+      const Q2 c = q_of(a), f = q_of(ph), l = q_of(la);
+      G[0] = {c.x, 0};
+      G[1] = q_scale(l, -c.y);
+      G[2] = q_scale(f, c.y);
+      G[3] = q_scale(q_mul(f, l), c.x);
+    } else {
+      double2 u[4];
+      gate_matrix(g.type, a, u);
+      for (int j = 0; j < 4; j++) G[j] = q_of(u[j]);
+    }
+    q_matmul(G, P);
+  }
+  if (!finite) P[0].x = kQBad;
+  for (int j = 0; j < 4; j++) M[j] = q_bits(P[j]);
 }
 
 // Walks the chain that starts with run `first` (a run by itself: a chain of one), mat(j, M)
@@ -293,74 +344,85 @@ __device__ __forceinline__ void run_matrix(const RotPlan& pl, const RotRun& run,
 // the phase that the chain leaves.
 template <class Mat>
 __device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotRec* recs, Mat mat) {
-  const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
+  const double2 one = make_double2(1.0, 0.0);
+  const double nan = __longlong_as_double(0x7ff8000000000000LL);
   // the rotation pushed into the next run: diag(1, pz) times pphase (zpend), or a unitary given
-  // by its first column (wp, wq); wdet: its determinant
+  // by its first column (wp, wq) and its determinant wdet
   bool zpend = true;
-  double2 pz = one, pphase = one, wp = one, wq = zero, wdet = one, own = one;
+  double2 pz = one, pphase = one, own = one;
+  Q2 wp = {kQOne, 0}, wq = {0, 0}, wdet = {kQOne, 0};
+  bool finite = true;  // units hold no NaN: every record from the first that meets one on is marked
   for (int step = 0; step < kRotChain; step++) {
     const RotRun run = pl.runs[first + step];
     RotRec r = {0.0, 1.0, one, one, 0.0, 0.0};
     double2 M[4];
     mat(first + step, run, M);
+    Q2 Q[4];  // of several gates
+    if (run.count > 1) {
+      for (int k = 0; k < 4; k++) Q[k] = q_of_bits(M[k]);
+      finite = finite && Q[0].x != kQBad;
+    }
     if (run.kind == kOpCry) {
       r.t = M[2].x;
       r.c = M[0].x;
-    } else if (run.kind == kOpPhase) {  // diagonal
-      r.zi = cunit(cmulc(M[3], M[0]));
-      own = M[0];
-    } else if (!(run.kind & kOpZi)) {  // Ry or Rx by itself: M[0] = cos, M[2] = sin or -i sin
-      const double2 cs = make_double2(M[0].x, (run.kind & kOpX) ? -M[2].y : M[2].x);
-      const double sign = split_u3(cs, one, one, r);
-      r.zi = one;
-      // about X the quarter turn is -i times the exchange
-      own = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
+    } else if (!(run.kind & kOpRot) || !(run.kind & kOpZi)) {  // gates about one axis
+      if (run.count > 1) M[0] = q_to(Q[0]), M[2] = q_to(Q[2]), M[3] = q_to(Q[3]);
+      if (run.kind == kOpPhase) {  // diagonal
+        r.zi = cunit(cmulc(M[3], M[0]));
+        own = M[0];
+      } else {  // Ry or Rx: M[0] = cos, M[2] = sin or -i sin
+        const double2 cs = make_double2(M[0].x, (run.kind & kOpX) ? -M[2].y : M[2].x);
+        const double sign = split_u3(cs, one, one, r);
+        r.zi = one;
+        // about X the quarter turn is -i times the exchange
+        own = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
+      }
     } else if (run.lone_u3 && zpend && (run.push == kAxisNone || run.push == kAxisZ)) {
       const double2 lam = step ? cunit(cmul(M[2], pz)) : M[2];
       pphase = cscale(pphase, split_u3(M[0], M[1], lam, r));
       if (run.push == kAxisNone)
         own = pphase;
       else
-        pz = M[1], wdet = cmul(cmul(pphase, pphase), pz);
+        pz = M[1];
     } else {
       // A = M * pushed, by its first column (p, q) and its determinant
-      double2 p, q, d;
+      if (zpend) {
+        finite = finite && isfinite(pphase.x) && isfinite(pz.x);
+        wp = q_of(pphase);
+        wq = {0, 0};
+        wdet = q_mul(q_mul(wp, wp), q_of(pz));
+      }
+      Q2 p, q, d;
       if (run.lone_u3) {  // cos and sin, phi, lambda and phi lambda
-        const double2 y = zpend ? make_double2(0.0, 0.0) : cmul(M[2], wq);
-        const double2 u = zpend ? pphase : wp;
-        p = make_double2(fma(M[0].x, u.x, -(M[0].y * y.x)), fma(M[0].x, u.y, -(M[0].y * y.y)));
-        q = cmul(M[1], make_double2(fma(M[0].y, u.x, M[0].x * y.x), fma(M[0].y, u.y, M[0].x * y.y)));
-        d = cmul(M[3], wdet);
+        finite = finite && isfinite(M[0].x) && isfinite(M[3].x);
+        const Q2 cs = q_of(M[0]), phi = q_of(M[1]), lam = q_of(M[2]), y = q_mul(lam, wq);
+        p = {q_diff(cs.x, wp.x, cs.y, y.x), q_diff(cs.x, wp.y, cs.y, y.y)};
+        q = q_mul(phi, Q2{q_sum(cs.y, wp.x, cs.x, y.x), q_sum(cs.y, wp.y, cs.x, y.y)});
+        d = q_mul(q_mul(phi, lam), wdet);
       } else {
-        p = zpend ? cmul(M[0], pphase) : cadd(cmul(M[0], wp), cmul(M[1], wq));
-        q = zpend ? cmul(M[2], pphase) : cadd(cmul(M[2], wp), cmul(M[3], wq));
-        d = cmul(csub(cmul(M[0], M[3]), cmul(M[1], M[2])), wdet);
+        p = q_add(q_mul(Q[0], wp), q_mul(Q[1], wq));
+        q = q_add(q_mul(Q[2], wp), q_mul(Q[3], wq));
+        d = q_mul(q_sub(q_mul(Q[0], Q[3]), q_mul(Q[1], Q[2])), wdet);
       }
       if (run.push == kAxisNone || run.push == kAxisZ) {
-        // the second column of a unitary: (-conj q, conj p) det
-        const double2 A[4] = {p, cmulc(make_double2(-d.x, -d.y), q), q, cmulc(d, p)};
-        const double2 ph = split_zyz(A, r);
-        if (run.push == kAxisNone) {
-          own = ph;
-        } else {
-          zpend = true;
-          pphase = cunit(ph);
-          pz = r.zo;
-          wdet = cmul(cmul(pphase, pphase), pz);
-        }
+        const double2 ph = split_zyz(p, q, d, r);
+        zpend = true;
+        pphase = own = ph;
+        pz = r.zo;
       } else {
         // Y: with S = diag(1, i), S A S^dagger = Rx(-alpha) Ry(beta) diag(1, zi)
-        if (run.push == kAxisY) q = make_double2(-q.y, q.x);
+        if (run.push == kAxisY) q = {-q.y, q.x};
         split_x(p, q, d, r);
-        const double c2 = cnorm2(p) - cnorm2(q);
-        const double s2 = -2.0 * fma(p.x, q.y, -(p.y * q.x));  // sin of the full angle: -2 Im(conj(w0) w1)
+        const double c2 = q_to(q_sum(p.x, p.x, p.y, p.y) - q_sum(q.x, q.x, q.y, q.y));
+        const double s2 = -2.0 * q_to(q_diff(p.x, q.y, p.y, q.x));  // sin of the full angle: -2 Im(conj(w0) w1)
         zpend = false;
         wp = p;
-        wq = run.push == kAxisY ? make_double2(q.y, -q.x) : q;
+        wq = run.push == kAxisY ? Q2{q.y, -q.x} : q;
         wdet = d;
         r.zo = make_double2(c2, run.push == kAxisY ? -s2 : s2);
       }
     }
+    if (!finite) r.t = nan, r.zi = r.zo = make_double2(nan, nan);
     recs[run.rec] = r;
     if (run.push == kAxisNone) break;
   }

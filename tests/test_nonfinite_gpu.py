@@ -122,3 +122,37 @@ def test_nan_angle_of_a_controlled_rotation(sqg, n, names, batch):
     trace = np.trace(want[:5]).real
     for cost in (ev.cost_grad(th)[0], ev.cost_grad(th, checkpoint_interval=4)[0], ev.cost_grad(th, with_grad=False)[0]):
         same(cost[batch - 1:].cpu().numpy(), np.array([1.0 - trace / 5]), True)
+
+
+@pytest.mark.parametrize("batch", [1, 40])
+@pytest.mark.parametrize("which", range(9))
+@pytest.mark.parametrize("between", ["CZ", "CNOT", "CRY"])
+def test_nan_angle_anywhere_in_a_chain(sqg, between, which, batch):
+    """Runs of one and of several U3 whose rotations are pushed through two-qubit gates, one angle NaN:
+    matrix, state, cost and gradient are NaN, not a number that looks like a result."""
+    n = 6
+    c = sqg.Circuit(n)
+    for run in (1, 2, 1, 1):
+        for _ in range(run):
+            c.add_U3(0)
+        c.add_U3(1)
+        {"CZ": c.add_CZ, "CNOT": c.add_CNOT, "CRY": c.add_CRY}[between](0, 1)
+    for q in range(n):
+        c.add_RY(q)  # mixes every half that was left alone
+    rng = np.random.default_rng(which)
+    p = rng.uniform(0.3, 1.2, c.get_Parameter_Num())
+    u3 = [r[3] for r in c.gate_records() if r[0] == 7 and r[1] == 0]  # its angles start there
+    p[u3[which // 3 + which % 2] + which % 3] = np.nan
+    th = torch.from_numpy(np.repeat(p[None], batch, axis=0)).cuda()
+    T = np.linalg.qr(rng.standard_normal((1 << n, 1 << n)))[0].astype(np.complex128)
+    ev = sqg.CostEvaluator(c, T)
+    for kw in ({}, {"checkpoint_interval": 3}):
+        cost, grad = ev.cost_grad(th, **kw)
+        assert torch.isnan(cost).all() and torch.isnan(grad).any(dim=1).all()
+    assert torch.isnan(ev.cost_grad(th, with_grad=False)[0]).all()
+    m = torch.from_numpy(np.repeat(T[None], batch, axis=0)).cuda()
+    c.apply_to_device(th, m)
+    assert torch.isnan(m.real).flatten(1).any(dim=1).all()
+    v = torch.from_numpy(np.repeat(T[None, :, 0], batch, axis=0).copy()).cuda()
+    c.apply_state_device(th, v)
+    assert torch.isnan(v.real).any(dim=1).all()
