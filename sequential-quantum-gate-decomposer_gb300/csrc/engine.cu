@@ -446,6 +446,12 @@ int launch_plan(const sqg_circuit* c, const RotPlan& p, const double* theta, lon
   return cuda_status(cudaGetLastError(), "k_rot_plan");
 }
 
+// The plan of a launch of so many tiles: with short chains where it does not fill the device and waits for
+// them.
+const RotPlan& launch_plan_of(const sqg_circuit* c, long long tiles) {
+  return tiles < 3LL * device_sms() ? c->short_plan : c->plan;
+}
+
 struct EvalLayout {
   const RotPlan* rp;
   RotLayout rot;
@@ -459,7 +465,7 @@ EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckp
   EvalLayout l;
   l.plan = plan_tiles(c->N, cols, grad, B, even && grad && ckpt_interval == 0);
   if (ckpt_interval == 0) l.plan.threads = eval_threads(l.plan, c->N, B);
-  l.rp = (long long)B * l.plan.tiles < 3LL * device_sms() ? &c->short_plan : &c->plan;
+  l.rp = &launch_plan_of(c, (long long)B * l.plan.tiles);
   l.rot = rot_layout(*l.rp, B, 0);
   l.tr_off = l.rot.end;
   l.gr_off = align_up(l.tr_off + (size_t)B * l.plan.tiles * sizeof(double2), 256);
@@ -1199,7 +1205,8 @@ int sqg_apply(const sqg_circuit* c, const double* theta, int B, void* mtx, int c
     TilePlan pl = plan_tiles(c->N, cols, false);
     TileArgs a;
     memset(&a, 0, sizeof(a));
-    if ((st = launch_plan(c, c->plan, theta, c->P, B, rot_layout(c->plan, B, 0), ws, a, s))) return st;
+    const RotPlan& rp = launch_plan_of(c, (long long)B * pl.tiles);
+    if ((st = launch_plan(c, rp, theta, c->P, B, rot_layout(rp, B, 0), ws, a, s))) return st;
     a.mtx = (double2*)mtx;
     a.bstride = batch_stride;
     a.rstride = stride;
@@ -1250,7 +1257,8 @@ int sqg_apply_from_right(const sqg_circuit* c, const double* theta, void* mtx, i
   TilePlan pl = plan_tiles(c->N, rows, false);
   TileArgs a;
   memset(&a, 0, sizeof(a));
-  if ((st = launch_plan(c, c->plan, theta, c->P, 1, rot_layout(c->plan, 1, 0), (char*)workspace, a, s))) return st;
+  const RotPlan& rp = launch_plan_of(c, pl.tiles);
+  if ((st = launch_plan(c, rp, theta, c->P, 1, rot_layout(rp, 1, 0), (char*)workspace, a, s))) return st;
   a.mtx = (double2*)mtx;
   a.bstride = 0;
   a.rstride = stride;

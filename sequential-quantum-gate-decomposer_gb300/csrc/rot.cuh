@@ -56,7 +56,7 @@ struct RotOp {
 // One run (or CRY gate): its record, its gates members[first .. first + count), the axis it
 // pushes (kAxisNone: nothing) into the run right behind it in the chain order, whether the run
 // before it pushes into it, a copy of its operation's kind, coff and mask, and whether it is a
-// single U3.  soff: place of its first parameter in its CTA's parameter list, the parameters of its
+// single U3 with no other than Z rotations pushed into it and by it.  soff: place of its first parameter in its CTA's parameter list, the parameters of its
 // gates behind one another (-1: not listed).
 struct RotRun {
   int rec, first, count, push, pulled, kind, coff, mask, lone_u3, soff;
@@ -162,15 +162,6 @@ __device__ __forceinline__ Q2 q_mulc(Q2 a, Q2 b) {  // a * conj(b)
 __device__ __forceinline__ Q2 q_scale(Q2 a, long long s) { return {q_mul(a.x, s), q_mul(a.y, s)}; }
 __device__ __forceinline__ Q2 q_add(Q2 a, Q2 b) { return {a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ Q2 q_sub(Q2 a, Q2 b) { return {a.x - b.x, a.y - b.y}; }
-
-// M <- G M
-__device__ __forceinline__ void q_matmul(const Q2 G[4], Q2 M[4]) {
-  const Q2 a = M[0], b = M[1];
-  M[0] = q_add(q_mul(G[0], a), q_mul(G[1], M[2]));
-  M[1] = q_add(q_mul(G[0], b), q_mul(G[1], M[3]));
-  M[2] = q_add(q_mul(G[2], a), q_mul(G[3], M[2]));
-  M[3] = q_add(q_mul(G[2], b), q_mul(G[3], M[3]));
-}
 
 // (cos, sin) of every listed parameter of a CTA's runs, one per thread: a warp's FP64 instruction
 // costs the same for one lane as for 32.  sc: kRotParams entries of shared memory; the caller
@@ -290,23 +281,43 @@ __device__ __forceinline__ double split_u3(double2 cs, double2 phi, double2 lam,
   return c < 0.0 ? -1.0 : 1.0;
 }
 
-// Matrix of a run from its CTA's parameters: of a lone U3 (cos, sin) of its three angles and phi lambda; of
-// another gate by itself its entries; of several gates the product's entries in units (Q2), or kQBad for
-// the first where an angle is not finite.
+// M <- G M in units with G = diag(f0, f1) Ry diag(1, l), a form that every gate has: U3 by its angles, RX =
+// diag(1, -i) Ry diag(1, i), RZ = diag(c - i s, c + i s).  One form for all, so that the threads of a warp, each
+// with its own gates, stay together.
+__device__ __forceinline__ void q_gate(int type, double2 a, double2 phi, double2 lambda, Q2 M[4]) {
+  const Q2 one = {kQOne, 0}, cs = q_of(a);
+  const bool u3 = type == G_U3, rx = type == G_RX, rz = type == G_RZ;
+  const long long c = rz ? kQOne : cs.x, s = rz ? 0 : cs.y;
+  const Q2 l = u3 ? q_of(lambda) : rx ? Q2{0, kQOne} : one;
+  const Q2 f0 = rz ? Q2{cs.x, -cs.y} : one, f1 = u3 ? q_of(phi) : rx ? Q2{0, -kQOne} : rz ? cs : one;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const Q2 x = M[j], y = q_mul(l, M[2 + j]);
+    M[j] = q_mul(f0, Q2{q_diff(c, x.x, s, y.x), q_diff(c, x.y, s, y.y)});
+    M[2 + j] = q_mul(f1, Q2{q_sum(s, x.x, c, y.x), q_sum(s, x.y, c, y.y)});
+  }
+}
+
+// Matrix of a run from its CTA's parameters: of a lone U3 (cos, sin) of its three angles; of a rotation by
+// itself its entries; else entries in units (Q2), kQBad for the first where an angle is not finite.
 constexpr long long kQBad = (long long)0x8000000000000000ULL;
+__device__ __forceinline__ bool run_in_units(const RotRun& run) {
+  return run.count > 1 || ((run.kind & kOpRot) && (run.kind & kOpZi) && !run.lone_u3);
+}
 __device__ __forceinline__ double2 q_bits(Q2 v) { return make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y)); }
 __device__ __forceinline__ Q2 q_of_bits(double2 v) { return {__double_as_longlong(v.x), __double_as_longlong(v.y)}; }
 
 __device__ __forceinline__ void run_matrix(const RotPlan& pl, const RotRun& run, const double2* sc,
                                            const double* theta, double2 M[4]) {
+  const double2 one = make_double2(1.0, 0.0);
   Gate g = pl.gates[pl.members[run.first]];
   int soff = run.soff;
   if (run.lone_u3) {
     for (int k = 0; k < 3; k++) M[k] = param_sincos(sc, soff, theta + g.pstart, k);
-    M[3] = cmul(M[1], M[2]);
+    M[3] = one;
     return;
   }
-  if (run.count == 1) {
+  if (!run_in_units(run)) {
     gate_matrix(g.type, param_sincos(sc, soff, theta + g.pstart, 0), M);
     return;
   }
@@ -317,23 +328,15 @@ __device__ __forceinline__ void run_matrix(const RotPlan& pl, const RotRun& run,
       if (soff >= 0) soff += gate_param_num(g.type);
       g = pl.gates[pl.members[run.first + k]];
     }
-    const double2 a = param_sincos(sc, soff, theta + g.pstart, 0);
-    finite = finite && isfinite(a.x);
-    Q2 G[4];
+    const double* th = theta + g.pstart;
+    const double2 a = param_sincos(sc, soff, th, 0);
+    double2 ph = one, la = one;
     if (g.type == G_U3) {
-      const double2 ph = param_sincos(sc, soff, theta + g.pstart, 1), la = param_sincos(sc, soff, theta + g.pstart, 2);
-      finite = finite && isfinite(ph.x) && isfinite(la.x);
-      const Q2 c = q_of(a), f = q_of(ph), l = q_of(la);
-      G[0] = {c.x, 0};
-      G[1] = q_scale(l, -c.y);
-      G[2] = q_scale(f, c.y);
-      G[3] = q_scale(q_mul(f, l), c.x);
-    } else {
-      double2 u[4];
-      gate_matrix(g.type, a, u);
-      for (int j = 0; j < 4; j++) G[j] = q_of(u[j]);
+      ph = param_sincos(sc, soff, th, 1);
+      la = param_sincos(sc, soff, th, 2);
     }
-    q_matmul(G, P);
+    finite = finite && isfinite(a.x) && isfinite(ph.x) && isfinite(la.x);
+    q_gate(g.type, a, ph, la, P);
   }
   if (!finite) P[0].x = kQBad;
   for (int j = 0; j < 4; j++) M[j] = q_bits(P[j]);
@@ -357,8 +360,9 @@ __device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotR
     RotRec r = {0.0, 1.0, one, one, 0.0, 0.0};
     double2 M[4];
     mat(first + step, run, M);
-    Q2 Q[4];  // of several gates
-    if (run.count > 1) {
+    Q2 Q[4];
+    const bool units = run_in_units(run);
+    if (units) {
       for (int k = 0; k < 4; k++) Q[k] = q_of_bits(M[k]);
       finite = finite && Q[0].x != kQBad;
     }
@@ -366,7 +370,7 @@ __device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotR
       r.t = M[2].x;
       r.c = M[0].x;
     } else if (!(run.kind & kOpRot) || !(run.kind & kOpZi)) {  // gates about one axis
-      if (run.count > 1) M[0] = q_to(Q[0]), M[2] = q_to(Q[2]), M[3] = q_to(Q[3]);
+      if (units) M[0] = q_to(Q[0]), M[2] = q_to(Q[2]), M[3] = q_to(Q[3]);
       if (run.kind == kOpPhase) {  // diagonal
         r.zi = cunit(cmulc(M[3], M[0]));
         own = M[0];
@@ -377,7 +381,7 @@ __device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotR
         // about X the quarter turn is -i times the exchange
         own = r.turn && (run.kind & kOpX) ? make_double2(0.0, -sign) : make_double2(sign, 0.0);
       }
-    } else if (run.lone_u3 && zpend && (run.push == kAxisNone || run.push == kAxisZ)) {
+    } else if (run.lone_u3) {  // nothing but a phase pulled, nothing but a phase pushed
       const double2 lam = step ? cunit(cmul(M[2], pz)) : M[2];
       pphase = cscale(pphase, split_u3(M[0], M[1], lam, r));
       if (run.push == kAxisNone)
@@ -392,18 +396,8 @@ __device__ __forceinline__ double2 walk_chain(const RotPlan& pl, int first, RotR
         wq = {0, 0};
         wdet = q_mul(q_mul(wp, wp), q_of(pz));
       }
-      Q2 p, q, d;
-      if (run.lone_u3) {  // cos and sin, phi, lambda and phi lambda
-        finite = finite && isfinite(M[0].x) && isfinite(M[3].x);
-        const Q2 cs = q_of(M[0]), phi = q_of(M[1]), lam = q_of(M[2]), y = q_mul(lam, wq);
-        p = {q_diff(cs.x, wp.x, cs.y, y.x), q_diff(cs.x, wp.y, cs.y, y.y)};
-        q = q_mul(phi, Q2{q_sum(cs.y, wp.x, cs.x, y.x), q_sum(cs.y, wp.y, cs.x, y.y)});
-        d = q_mul(q_mul(phi, lam), wdet);
-      } else {
-        p = q_add(q_mul(Q[0], wp), q_mul(Q[1], wq));
-        q = q_add(q_mul(Q[2], wp), q_mul(Q[3], wq));
-        d = q_mul(q_sub(q_mul(Q[0], Q[3]), q_mul(Q[1], Q[2])), wdet);
-      }
+      Q2 p = q_add(q_mul(Q[0], wp), q_mul(Q[1], wq)), q = q_add(q_mul(Q[2], wp), q_mul(Q[3], wq));
+      Q2 d = q_mul(q_sub(q_mul(Q[0], Q[3]), q_mul(Q[1], Q[2])), wdet);
       if (run.push == kAxisNone || run.push == kAxisZ) {
         const double2 ph = split_zyz(p, q, d, r);
         zpend = true;
@@ -443,16 +437,17 @@ __device__ __forceinline__ bool finish_record(const RotRun& run, RotRec& r) {
 // CTA's runs is not finite, which sweeps in fixed point need to know and amplitudes that do not meet
 // that record must not notice (phase_factor).
 __device__ __forceinline__ void phase_product(double2 phase, bool finite, double2* out) {
-  __shared__ double2 ph[kRotThreads];
-  const int i = threadIdx.x;
-  ph[i] = phase;
+  __shared__ double2 ph[kRotThreads / 32];
+  const int warp = threadIdx.x >> 5;
+  for (int o = 16; o > 0; o >>= 1)
+    phase = cmul(phase, make_double2(__shfl_xor_sync(0xffffffffu, phase.x, o), __shfl_xor_sync(0xffffffffu, phase.y, o)));
+  if ((threadIdx.x & 31) == 0) ph[warp] = phase;
   finite = __syncthreads_and(finite);
-  for (int o = kRotThreads / 2; o > 0; o >>= 1) {
-    if (i < o) ph[i] = cmul(ph[i], ph[i + o]);
-    __syncthreads();
-  }
-  if (i == 0) *out = finite ? ph[0] : cadd(ph[0], ph[0]);
+  if (threadIdx.x > 0) return;
+  phase = cmul(cmul(ph[0], ph[1]), cmul(ph[2], ph[3]));
+  *out = finite ? phase : cadd(phase, phase);
 }
+static_assert(kRotThreads == 128, "phase_product multiplies four warps' products");
 
 // A phase as phase_product left it, and whether the records behind it are finite.  The larger component of
 // a phase is at most 1 and a few roundings, that of a doubled one at least 1.41.
@@ -488,9 +483,12 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
     run_matrix(pl, run, sc, theta, Ms[i]);
   }
   // Chains of two and more runs are few and take longest: they are dealt out over `deal` warps.  All
-  // four where the launch waits for one CTA (as few as possible wait for one another's branches),
-  // two, which hold the most there can be, where the FP64 pipe is shared by many CTAs and takes
-  // as long for a warp of two chains as for one of 32.
+  // four where the launch waits for one CTA (as few as possible wait for one another's branches), or the two
+  // or three that have no runs of their own, where the CTA has that few runs, so that chains do not wait
+  // for the runs by themselves (60 gates on five qubits applied to a matrix 83 -> 76 us; with one warp left over
+  // its chains would wait for one another: 98 U3 on seven qubits, gradient 205 -> 211 us).  Two, which hold
+  // the most there can be, where the FP64 pipe is shared by many CTAs and takes as long for a warp of two
+  // chains as for one of 32.
   const int warp = i >> 5, lane = i & 31;
   const bool head = i < n && !run.pulled && run.push != kAxisNone;
   const unsigned heads = __ballot_sync(0xffffffffu, head);
@@ -501,9 +499,12 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
     if (w < warp) rank += warp_heads[w];
     nheads += warp_heads[w];
   }
-  if (head) chain_of[(rank % deal) * 32 + rank / deal] = i;
+  int dealer = 0;  // the first warp
+  const int used = (n + 31) >> 5, idle = kRotThreads / 32 - used;
+  if (deal == kRotThreads / 32 && idle >= 2) dealer = used, deal = idle;
+  if (head) chain_of[(dealer + rank % deal) * 32 + rank / deal] = i;
   __syncthreads();
-  const bool walks = warp < deal && lane * deal + warp < nheads;
+  const bool walks = warp >= dealer && warp < dealer + deal && lane * deal + (warp - dealer) < nheads;
   double2 phase = make_double2(1.0, 0.0);
   auto mat = [&](int j, const RotRun&, double2 M[4]) {
     for (int k = 0; k < 4; k++) M[k] = Ms[j - base][k];

@@ -108,8 +108,7 @@ inline RotRuns find_rot_runs(int n, const std::vector<Gate>& gates) {
 inline RotPlanHost build_rot_plan(const RotRuns& rr, const std::vector<Gate>& gates, int max_chain) {
   const int L = (int)gates.size(), nruns = (int)rr.runs.size();
   struct Link {
-    int push = kAxisNone, next = -1, depth = 0;
-    bool pulled = false;
+    int push = kAxisNone, pulled = kAxisNone, next = -1, depth = 0;
   };
   std::vector<Link> links(nruns);
   for (int r = 0; r < nruns; r++) {
@@ -119,7 +118,7 @@ inline RotPlanHost build_rot_plan(const RotRuns& rr, const std::vector<Gate>& ga
     if (b.depth + 1 >= max_chain) continue;
     b.push = run.between;
     b.next = r;
-    links[r].pulled = true;
+    links[r].pulled = run.between;
     links[r].depth = b.depth + 1;
   }
   RotPlanHost pl;
@@ -135,13 +134,14 @@ inline RotPlanHost build_rot_plan(const RotRuns& rr, const std::vector<Gate>& ga
     pl.steps.push_back({kind, target, control, pl.noverlaps, mask, anchor});
     pl.noverlaps += (mask & 1) + (mask >> 1 & 1) + (mask >> 2);
   };
-  auto add_item = [&](int first, int count, int lone, int push, bool pulled) {
+  auto add_item = [&](int first, int count, int lone, int push, int pulled) {  // pulled: its axis
     const RotStep& op = pl.steps.back();
     auto member = [&](int k) { return lone >= 0 ? lone : rr.members[first + k]; };
     int np = 0;
     for (int k = 0; k < count; k++) np += gate_param_num(gates[member(k)].type);
-    const int lone_u3 = count == 1 && gates[member(0)].type == G_U3 ? 1 : 0;
-    items.push_back({{(int)pl.steps.size() - 1, first, count, push, pulled ? 1 : 0, op.kind, op.coff, op.mask, lone_u3, -1},
+    const bool z = (push == kAxisNone || push == kAxisZ) && (pulled == kAxisNone || pulled == kAxisZ);
+    const int lone_u3 = z && count == 1 && gates[member(0)].type == G_U3 ? 1 : 0;
+    items.push_back({{(int)pl.steps.size() - 1, first, count, push, pulled != kAxisNone ? 1 : 0, op.kind, op.coff, op.mask, lone_u3, -1},
                      lone, np, -1});
     return (int)items.size() - 1;
   };
@@ -150,7 +150,7 @@ inline RotPlanHost build_rot_plan(const RotRuns& rr, const std::vector<Gate>& ga
     if (gate_controlled(gt.type)) {
       const bool cry = gt.type == G_CRY;
       add_op(cry ? kOpCry : gt.type == G_CNOT ? kOpCnot : kOpCz, gt.target, gt.control, cry ? 2 : 0, g);
-      if (cry) add_item(0, 1, g, kAxisNone, false);
+      if (cry) add_item(0, 1, g, kAxisNone, kAxisNone);
       continue;
     }
     const RotRuns::Run& r = rr.runs[rr.run_of[g]];
@@ -168,7 +168,7 @@ inline RotPlanHost build_rot_plan(const RotRuns& rr, const std::vector<Gate>& ga
       while (m < end && rot_letter(gates[rr.members[m]].type) == axis) m++;
       const int kind = axis == kAxisZ ? kOpPhase : axis == kAxisX ? kOpRot | kOpX : kOpRot;
       add_op(kind, r.qubit, -1, 1 << (axis - 1), g);
-      add_item(m0, m - m0, -1, kAxisNone, false);
+      add_item(m0, m - m0, -1, kAxisNone, kAxisNone);
     }
   }
   for (int r = 0; r < nruns; r++)
