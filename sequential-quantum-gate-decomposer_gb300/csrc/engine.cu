@@ -949,21 +949,25 @@ static int cost_grad_args(const sqg_circuit* c, const double* theta, int B, cons
 }
 
 // Whether the tile kernels are faster than the environment-matrix evaluation where both can run.
-// The latter takes one CTA per vector, two per SM, and its time grows faster with the gates; the tiles
-// pay for the plan's numbers first.  Measured on GB300, environment matrix against tiles, us:
-// three qubits, 14 blocks 72 / 116 (one vector), 318 / 411 (3000); 30 blocks 313 / 332 (1024), 772 /
-// 666 (3000); 60 blocks 259 / 281 (one), 775 / 494 (700).
-// Four qubits, 6 blocks 89 / 84 (one), 91 / 121 (300), 194 / 208 (1024); 8 blocks 109 / 103, 113 / 137,
-// 241 / 235; 12 blocks 152 / 147 (64), 159 / 164 (300); 14 blocks 173 / 123, 181 / 179, 381 / 315; 40
-// blocks 1210 / 667 (1024).
-// Five qubits, one block 102 / 64 (one), 105 / 128 (300), 203 / 195 (700); two 138 / 142 (300); three 164 /
-// 74, 170 / 152, 329 / 241.
+// The latter takes one CTA per vector and its time grows faster with the gates, by a wave where its CTAs,
+// whose shared memory grows with them, no longer are all resident (two to three per SM); the tiles pay for the
+// plan's numbers first, which cost more from kRotBatch vectors on.  Each line lies where the tiles are not
+// slower on either side of it.  Measured on GB300 (152 SMs), gradient, us, environment matrix / tiles:
+// three qubits, 45 gates 73 / 118 (one vector), 320 / 425 (3000); 111 gates 180 / 243 (450), 331 / 335 (600), 344 /
+// 371 (700), 486 / 408 (920); 123 gates 197 / 256 (450), 359 / 346 (460), 364 / 351 (600), 535 / 428 (920); 138 gates
+// 223 / 277 (450), 408 / 373 (460); 153 gates 433 / 302 (310); 183 gates 266 / 289 (one), 278 / 417 (300).
+// Four qubits, 22 gates 90 / 94 (one), 90 / 94 (16); 25 gates 100 / 99 (one), 101 / 100 (16), 101 / 116 (32); 31 gates
+// 123 / 106 (26); 40 gates 154 / 146 (32), 160 / 163 (250), 161 / 167 (300); 43 gates 172 / 172 (250), 172 / 159 (304);
+// 28 gates 127 / 145 (340), 146 / 172 (500), 243 / 241 (1024); 34 gates 159 / 157 (340), 196 / 193 (500), 254 / 234
+// (800).
+// Five qubits, 8 gates 103 / 69 (one), 104 / 87 (76), 107 / 128 (300), 205 / 199 (700); 11 gates 139 / 114 (160), 139 /
+// 142 (304), 168 / 162 (340), 267 / 222 (700).
 static bool tiles_first(const sqg_circuit* c, int B) {
-  const bool waves = B > 2 * device_sms();  // more vectors than resident CTAs
+  const int sms = device_sms(), L = c->L;
   if (c->n >= 6) return true;
-  if (c->n == 5) return c->L >= 11 || 2 * B <= device_sms();
-  if (c->n == 4) return c->L >= (B <= 4 ? 24 : waves ? 28 : 40);
-  return c->n == 3 && waves && c->L >= 112;
+  if (c->n == 5) return L >= 11 || 2 * B <= sms;
+  if (c->n == 4) return L >= (B < kRotBatch ? 24 : B <= 2 * sms ? 43 : 34);
+  return c->n == 3 && ((L >= 112 && B > 5 * sms) || (L >= 120 && B > 3 * sms) || (L >= 144 && B > 2 * sms));
 }
 
 int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* target, int cols,
