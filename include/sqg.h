@@ -227,7 +227,8 @@ int sqg_decompose_batched(const sqg_circuit* circuit, const void* targets_dev, i
 
 /* One BFGS decomposition for any qbit_num the gradient supports (<= 12), run on the device as
  * a single CUDA graph launch: a conditional while-node whose body evaluates the cost and
- * gradient (the kernels of sqg_cost_grad) and then advances BFGS_Powell (Powell's Z update, the
+ * gradient (up to five qubits as sqg_decompose_batched, above gate by gate in FP64, so that the same call
+ * returns the same point) and then advances BFGS_Powell (Powell's Z update, the
  * reference line search, the restarts) on one CTA up to the next point to evaluate.  Replaces
  * the host loop of solve_layer_optimization_problem_BFGS (src-cpp/optimization_engines/
  * BFGS.cpp:42-152, src-cpp/common/BFGS_Powell.cpp:70-396).  Semantics and parameters as
@@ -300,7 +301,7 @@ int sqg_decompose_structures_adam(const sqg_circuit* circuit, const sqg_gate* ga
 
 /* One decomposition with SQUANDER's ADAM engine for any qbit_num the gradient supports
  * (<= 12), run on the device as a single CUDA graph launch: a conditional while-node whose
- * body evaluates the cost and gradient (the kernels of sqg_cost_grad) and then takes one
+ * body evaluates the cost and gradient (as sqg_decompose_bfgs_loop) and then takes one
  * pass of the engine loop on one CTA, with no host round trip between evaluations.  Replaces
  * the host loop of Optimization_Interface::solve_layer_optimization_problem_ADAM
  * (src-cpp/optimization_engines/ADAM.cpp:44-330), the optimizer

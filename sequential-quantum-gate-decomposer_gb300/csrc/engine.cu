@@ -6,15 +6,17 @@
 // Design (GB300-first, one GPU):
 //  * Column tiles.  Gates mix rows only, so every column of U^dagger is an independent
 //    state vector.  A CTA loads a tile of TC columns into shared memory (column-major:
-//    each column contiguous), applies ALL L gates there, and reads HBM once.  The whole
-//    circuit is fused, whatever qubits it touches (n <= 13 fits a column in 128 KB).
-//  * Adjoint gradient per column: psi = C u_j is uncomputed gate by gate with G^dagger
-//    while the co-state lambda (starting at e_{j+offset}) is propagated with G^dagger;
-//    for each parametric gate the 2x2 overlap R_ab = sum conj(lambda_a) psi_b is reduced
-//    over the tile and contracted with the derivative kernels.  O(L) passes in shared
-//    memory replace the reference's (P+1) dense derivative matrices.
-//  * FP64 is the binding resource on GB300, so the update rules (gates.cuh) minimise FP64
-//    instructions and everything else (index math, exchanges, sign flips) is integer work.
+//    each column contiguous), applies the whole circuit there, and reads HBM once, whatever
+//    qubits it touches (n <= 13 fits a column in 128 KB).
+//  * The circuit is applied as its rotation plan (rot.cuh): runs of single-qubit gates as one
+//    rotation, CNOTs as a change of places.
+//  * Adjoint gradient per column: psi = C u_j is undone operation by operation while the
+//    co-state lambda (starting at e_{j+offset}) is taken back with it; for each run two or three
+//    Pauli overlaps are summed over the tile, from which rotgrad.cuh makes the derivatives of its
+//    gates.  O(L) passes in shared memory replace the reference's (P+1) dense derivative matrices.
+//  * FP64 is the scarcest resource on GB300.  Cost and gradient, which are sums, are swept in 64-bit
+//    fixed point on the integer multiplier (fx.cuh); matrices and states that go back to the caller
+//    stay in FP64.
 //  * Deterministic reductions: per-tile partial traces go to the caller's workspace and
 //    are summed in a fixed order by a second kernel.
 #include <cuda.h>
@@ -132,8 +134,12 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_tile_forward(TileArgs a) {
   tile_forward_body<WRITE_BACK, TRACE, DIR>(a, blockIdx.y, blockIdx.x, smem);
 }
 
-// MINB: CTAs per SM that the registers are cut to.  Three where the launch fills the device with
-// tiles (the sweeps wait on the integer pipes' latencies), one where it does not (no spills).
+// MINB: CTAs per SM that the registers are cut to where the launch fills the device with tiles: the sweeps
+// wait on the integer pipes' latencies.  Three for real overlaps (80 registers, 196 bytes of them stored and
+// 240 loaded again), two for complex ones (three: 232 and 844 bytes).  One where it does not fill the device.
+// GB300, three against two: real, 8 qubits, 360 blocks, 64 vectors 40.1, 41.5 ms; 10 qubits, 6 vectors 17.5, 18.2 ms;
+// 4 qubits, 1024 vectors 725, 699 us; 6 qubits, 300 vectors 1.32, 1.30 ms; complex, 8 qubits 50.7, 50.1 ms; 9 qubits,
+// 300 gates of all kinds, 8 vectors 5.08, 4.89 ms.
 template <bool CPLX, int MINB>
 __global__ void __launch_bounds__(kMaxThreads, MINB) k_tile_adjoint(TileArgs a) {
   extern __shared__ double2 smem[];
@@ -1021,7 +1027,7 @@ int sqg_cost_grad(const sqg_circuit* c, const double* theta, int B, const void* 
   // the other variants multiply the derivative of the trace by the trace: complex overlaps
   const bool cplx = variant != SQG_FROBENIUS_NORM;
   const bool full = (long long)l.plan.tiles * B >= 3LL * device_sms();
-  auto adjoint = cplx ? (full ? k_tile_adjoint<true, 3> : k_tile_adjoint<true, 1>)
+  auto adjoint = cplx ? (full ? k_tile_adjoint<true, 2> : k_tile_adjoint<true, 1>)
                       : (full ? k_tile_adjoint<false, 3> : k_tile_adjoint<false, 1>);
   if ((st = set_smem(adjoint, l.plan.smem))) return st;
   adjoint<<<grid, l.plan.threads, l.plan.smem, s>>>(a);

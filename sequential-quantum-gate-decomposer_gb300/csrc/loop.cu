@@ -3,7 +3,7 @@
 // host round trip between evaluations.
 //
 // The graph holds a conditional WHILE node whose body is
-//   [cost + gradient at the parameters x: the engine's own kernels, sqg_cost_grad]
+//   [cost + gradient at the parameters x: loop_cost_grad, whose rounding the trajectory hangs on]
 //   -> [one CTA: the optimizer's work up to the next point to evaluate]
 // and the controller clears the loop condition once the decomposition is over.  The optimizer
 // state lives in the workspace between body executions.  Every body execution is one
@@ -50,7 +50,7 @@ struct LoopArgs {
 };
 
 // Workspace layout: state, cost, seven P-vectors, the two windows, then the scratch of
-// sqg_cost_grad; every part on a 256-byte boundary.
+// loop_cost_grad; every part on a 256-byte boundary.
 struct LoopLayout {
   size_t st, cost, vec[7], f0, dec, eval, end;
 };

@@ -1,8 +1,9 @@
 // Rotation plan of a circuit: the form in which the tile and state kernels apply it.
 //
-// What bounds these kernels is the number of FP64 instructions per amplitude pair (the FP64
-// pipe takes two lanes per clock and SM; every other pipe is nearly idle), so the plan rewrites
-// the gate list into operations with as few of them as the circuit allows:
+// What bounds these kernels is the number of products per amplitude pair: FP64 instructions where
+// amplitudes go back to the caller (the FP64 pipe takes two lanes per clock and SM; every other pipe is
+// nearly idle), fixed-point products (fx.cuh) for cost and gradient.  The plan rewrites the gate list into
+// operations with as few of them as the circuit allows:
 //  * A run of single-qubit gates on one qubit, with no two-qubit gate on that qubit between
 //    them, is one 2x2 unitary M.
 //  * M = scalar * diag(1, zo) * R * diag(1, zi) with R a rotation.  R is applied without its
@@ -19,10 +20,11 @@
 //    along the axis that the run pushes equals that of the next run and is not measured, and
 //    the derivatives of the run's gates follow from these three numbers, once per run
 //    (rot_grad_body) and not per amplitude.
-// Measured on GB300 against the gates as given (U3 14 instructions, merged runs 16): gradient at
-// 8 qubits, 360 blocks, 128 vectors 333 -> 182 ms; cost alone, 120 blocks, 200 vectors 41.5 ->
-// 25.3 ms; 2000 random gates on a 4096 x 4096 matrix 143 -> 99 ms; 829 gates on 24 qubits 128 ->
-// 86 ms.  The FP64 pipe is 91 % busy either way.
+// Measured on GB300 in FP64 against the gates as given (U3 14 instructions, merged runs 16): 2000 random gates
+// on a 4096 x 4096 matrix 143 -> 98 ms; 829 gates on 24 qubits 128 -> 87 ms, the FP64 pipe 92 % busy either way;
+// gradient at 8 qubits, 360 blocks, 128 vectors 333 -> 182 ms, and 77 ms with the sweeps in fixed point.
+// Error against long double, random circuits of 6 to 16 qubits and 200 to 2000 gates, as a multiple of that of
+// the gates as given: 0.94 in the mean at uniform angles (0.6 to 1.5), 0.6 and 0.7 at multiples of pi/4.
 // The numbers behind each operation depend on the parameters and are made per instance by
 // rot_plan_body; which operations there are depends on the gate list alone (build_rot_plan).
 #pragma once
@@ -90,9 +92,9 @@ struct RotPlan {
 
 constexpr int kRotThreads = 128;  // runs per CTA of the per-instance kernels; no chain straddles two
 constexpr int kRotParams = 512;  // parameters listed per CTA
-// Runs linked by pushed rotations.  Their numbers are made one after another, 4 us a run, and the
-// run that ends a chain costs 4 products more per pair and vector: 3 % at 16, 12 % at 4.  A launch
-// that does not fill the device waits for the chains: 46 U3 of one vector 52 us at 16, 29 us at 4.
+// Runs linked by pushed rotations.  Their numbers are made one after another, half a microsecond a run, and
+// the run that ends a chain costs 4 products more per pair and vector: 3 % at 16, 12 % at 4.  A launch
+// that does not fill the device waits for the chains: 46 U3 of one vector 36 us at 16, 30 us at 4.
 constexpr int kRotChain = 16, kRotShortChain = 4;
 constexpr int kRotChunk = 32;     // operations staged in shared memory together (a warp)
 // The cosines of a group of consecutive operations are multiplied in together.  In FP64 the scale costs no
