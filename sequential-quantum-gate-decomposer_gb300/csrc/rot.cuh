@@ -118,16 +118,18 @@ __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_dou
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double cnorm2(double2 a) { return fma(a.x, a.x, a.y * a.y); }
 // 1 / sqrt(x) and 1 / x for x in [2^-120, 2^120], to 1.5 and 1 times 2^-53 (relative): from the
-// single-precision value by two Newton steps.  The chains of rot_plan_body wait for every one of their
+// device's approximation of some 20 bits by two Newton steps.  The chains of rot_plan_body wait for every one of their
 // instructions, and the general functions take several times as many.
 __device__ __forceinline__ double fast_rsqrt(double x) {
-  double y = (double)rsqrtf((float)x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double h = -0.5 * x;
   y = fma(y, fma(h * y, y, 0.5), y);
   return fma(y, fma(h * y, y, 0.5), y);
 }
 __device__ __forceinline__ double fast_rcp(double x) {
-  double y = (double)__frcp_rn((float)x);
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   y = fma(y, fma(-x, y, 1.0), y);
   return fma(y, fma(-x, y, 1.0), y);
 }
@@ -225,7 +227,8 @@ __device__ __forceinline__ double2 split_zyz(Q2 p, Q2 q, Q2 det, RotRec& r) {
   const double x2 = cnorm2(x);
   // t below 1e-17 is an entry lost in the rounding of the others: any phase does
   const double rx = x2 > 1e-34 ? fast_rsqrt(x2) : 0.0;
-  r.t = x2 * rx * fast_rcp(np);
+  const double inv = fast_rcp(np), t = x2 * rx;
+  r.t = fma(fma(-t * inv, np, t), inv, t * inv);
   double2 zo = make_double2(1.0, 0.0);
   if (x2 > 1e-34) zo = cscale(turn ? make_double2(-x.x, x.y) : x, rx);
   zo = cunit(zo);
@@ -233,7 +236,7 @@ __device__ __forceinline__ double2 split_zyz(Q2 p, Q2 q, Q2 det, RotRec& r) {
   // = 1: b / c), is det conj(piv)^2 / np, negated for f = 1, where zi has another minus: zi = it / zo, or times zo
   const Q2 w = q_mulc(q_mulc(det, piv), piv), zq = q_of(zo);
   const double2 z = q_to(turn ? q_mul(w, zq) : q_mulc(w, zq));
-  const double2 zi = cunit(cscale(z, fast_rsqrt(cnorm2(z))));
+  const double2 zi = cunit(cscale(z, inv));  // |z| = |piv|^2
   r.turn = turn;
   // the quarter turn (x, y) -> (-y, x) as an exchange: its sign goes into zi
   r.zi = turn ? make_double2(-zi.x, -zi.y) : zi;
@@ -251,12 +254,13 @@ __device__ __forceinline__ void split_x(Q2& p, Q2& q, Q2& det, RotRec& r) {
   const double2 d = q_to(q_mulc(q_mul(q_add(p, q), q_sub(p, q)), det));
   const double nd2 = cnorm2(d), rnd = nd2 > 1e-34 ? fast_rsqrt(nd2) : 0.0;
   r.zi = nd2 > 1e-34 ? cunit(make_double2(d.x * rnd, -d.y * rnd)) : make_double2(1.0, 0.0);
-  const double sb2 = 2.0 * q_to(q_sum(p.x, q.x, p.y, q.y)), den = fma(nd2, rnd, 1.0), inv = fast_rcp(den);
-  const double t0 = sb2 * inv;
+  // tan beta = sin 2 beta / (1 + cos 2 beta), cos^2 beta = (1 + cos 2 beta) / 2
+  const double sb2 = 2.0 * q_to(q_sum(p.x, q.x, p.y, q.y)), den = fma(nd2, rnd, 1.0), root = fast_rsqrt(2.0 * den);
+  const double inv = 2.0 * root * root, t0 = sb2 * inv;
   r.t = fma(fma(-t0, den, sb2), inv, t0);
   r.turn = 0;
-  // cosine of t: one Newton step in units from the double
-  const long long t = q_of(r.t), c0 = q_of(fast_rsqrt(fma(r.t, r.t, 1.0)));
+  // the cosine of t as rounded: one Newton step in units from the double
+  const long long t = q_of(r.t), c0 = q_of(den * root);
   const long long c2 = q_mul(c0, c0), e = kQOne - c2 - q_mul(c2, q_mul(t, t));
   const long long c = c0 + q_mul(c0, e) / 2, sn = q_mul(t, c);
   // W = A diag(1, conj zi) Ry(-beta); the second column of A is (-conj q, conj p) det
@@ -485,17 +489,17 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
     run_matrix(pl, run, sc, theta, Ms[i]);
   }
   // Chains of two and more runs are few and take longest: they are dealt out over `deal` warps.  All
-  // four where the launch waits for one CTA (as few as possible wait for one another's branches), or the two
-  // or three that have no runs of their own, where the CTA has that few runs, so that chains do not wait
-  // for the runs by themselves (60 gates on five qubits applied to a matrix 83 -> 76 us; with one warp left over
-  // its chains would wait for one another: 98 U3 on seven qubits, gradient 205 -> 211 us).  Two, which hold
+  // four where the launch waits for one CTA (as few as possible wait for one another's branches); or, where runs
+  // by themselves take as long as a step of a chain, the warps that have no runs of their own, so that the few
+  // chains do not wait for those (60 gates of all kinds on five qubits applied to a matrix 83 -> 76 us).  Two, which hold
   // the most there can be, where the FP64 pipe is shared by many CTAs and takes as long for a warp of two
   // chains as for one of 32.
   const int warp = i >> 5, lane = i & 31;
   const bool head = i < n && !run.pulled && run.push != kAxisNone;
   const unsigned heads = __ballot_sync(0xffffffffu, head);
   if (lane == 0) warp_heads[warp] = __popc(heads);
-  __syncthreads();
+  const bool general = i < n && !run.pulled && !head && (run.kind & kOpRot) && (run.kind & kOpZi) && !run.lone_u3;
+  const bool long_runs = __syncthreads_or(general);
   int rank = __popc(heads & ((1u << lane) - 1)), nheads = 0;
   for (int w = 0; w < kRotThreads / 32; w++) {
     if (w < warp) rank += warp_heads[w];
@@ -503,7 +507,7 @@ __device__ __forceinline__ void rot_plan_body(const RotPlan& pl, int cta, const 
   }
   int dealer = 0;  // the first warp
   const int used = (n + 31) >> 5, idle = kRotThreads / 32 - used;
-  if (deal == kRotThreads / 32 && idle >= 2) dealer = used, deal = idle;
+  if (deal == kRotThreads / 32 && long_runs && nheads <= 2 * idle) dealer = used, deal = max(idle, 1);
   if (head) chain_of[(dealer + rank % deal) * 32 + rank / deal] = i;
   __syncthreads();
   const bool walks = warp >= dealer && warp < dealer + deal && lane * deal + (warp - dealer) < nheads;
