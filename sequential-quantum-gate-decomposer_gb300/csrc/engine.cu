@@ -452,11 +452,14 @@ int launch_plan(const sqg_circuit* c, const RotPlan& p, const double* theta, lon
   return cuda_status(cudaGetLastError(), "k_rot_plan");
 }
 
-// The plan of a launch of so many tiles: with short chains where it does not fill the device and waits for
-// them.
-const RotPlan& launch_plan_of(const sqg_circuit* c, long long tiles) {
-  return tiles < 3LL * device_sms() ? c->short_plan : c->plan;
+// The plan of a launch of so many tiles: with short chains where it waits for them.  Sweeps in fixed point do
+// while they do not fill the device (three tiles per SM), those in FP64 while an SM has no more than one tile:
+// GB300, chains of 16 against 4, 60 U3-CNOT blocks on 8 qubits, 75 tiles 751, 735 us; 38 gates on 9 qubits, 306
+// tiles 281, 292 us.
+const RotPlan& launch_plan_of(const sqg_circuit* c, long long tiles, int per_sm) {
+  return tiles < (long long)per_sm * device_sms() ? c->short_plan : c->plan;
 }
+constexpr int kShortPlanFx = 3, kShortPlanFp64 = 1;
 
 struct EvalLayout {
   const RotPlan* rp;
@@ -471,7 +474,7 @@ EvalLayout eval_layout(const sqg_circuit* c, int B, int cols, bool grad, int ckp
   EvalLayout l;
   l.plan = plan_tiles(c->N, cols, grad, B, even && grad && ckpt_interval == 0);
   if (ckpt_interval == 0) l.plan.threads = eval_threads(l.plan, c->N, B);
-  l.rp = &launch_plan_of(c, (long long)B * l.plan.tiles);
+  l.rp = &launch_plan_of(c, (long long)B * l.plan.tiles, kShortPlanFx);
   l.rot = rot_layout(*l.rp, B, 0);
   l.tr_off = l.rot.end;
   l.gr_off = align_up(l.tr_off + (size_t)B * l.plan.tiles * sizeof(double2), 256);
@@ -754,7 +757,9 @@ __global__ void __launch_bounds__(kStateThreads) k_state_block(StateArgs a) {
     double2 p = make_double2(1.0, 0.0);
     bool finite;  // no matter here
     for (int k = 0; k < a.nphase; k++) p = cmul(p, phase_factor(a.phases[(long long)b * a.nphase + k], finite));
-    for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = phase_mul(p, sv[end_place(ends, l)]);
+    with_phase(p, [&](auto mul) {
+      for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = mul(sv[end_place(ends, l)]);
+    });
   } else {
     for (int l = threadIdx.x; l < KK; l += blockDim.x) base[(l & lowmask) + hit[l >> a.low]] = sv[end_place(ends, l)];
   }
@@ -1215,7 +1220,7 @@ int sqg_apply(const sqg_circuit* c, const double* theta, int B, void* mtx, int c
     TilePlan pl = plan_tiles(c->N, cols, false);
     TileArgs a;
     memset(&a, 0, sizeof(a));
-    const RotPlan& rp = launch_plan_of(c, (long long)B * pl.tiles);
+    const RotPlan& rp = launch_plan_of(c, (long long)B * pl.tiles, kShortPlanFp64);
     if ((st = launch_plan(c, rp, theta, c->P, B, rot_layout(rp, B, 0), ws, a, s))) return st;
     a.mtx = (double2*)mtx;
     a.bstride = batch_stride;
@@ -1267,7 +1272,7 @@ int sqg_apply_from_right(const sqg_circuit* c, const double* theta, void* mtx, i
   TilePlan pl = plan_tiles(c->N, rows, false);
   TileArgs a;
   memset(&a, 0, sizeof(a));
-  const RotPlan& rp = launch_plan_of(c, pl.tiles);
+  const RotPlan& rp = launch_plan_of(c, pl.tiles, kShortPlanFp64);
   if ((st = launch_plan(c, rp, theta, c->P, 1, rot_layout(rp, 1, 0), (char*)workspace, a, s))) return st;
   a.mtx = (double2*)mtx;
   a.bstride = 0;

@@ -464,12 +464,34 @@ __device__ __forceinline__ double2 phase_factor(double2 p, bool& finite) {
   return cscale(p, 0.5);
 }
 
-// The common phase times an amplitude.  Phases of 1, -1, i and -i (none at all; rotations about X and Y, CRY)
-// move components as they are: an infinite one must not make NaN of the other.
+// The common phase of all amplitudes, times one of them.  Phases of 1, -1, i and -i (none at all; rotations
+// about X and Y, CRY) move components as they are: an infinite one must not make NaN of the other.  put(mul)
+// is called with the form that the phase has, so that the choice is not made per amplitude (a predicated
+// FP64 instruction takes the pipe as long as an executed one: 10 us for 1.2 million amplitudes).
+struct PhaseTurn {
+  bool swap;
+  unsigned fx, fy;  // sign bits of the components
+  __device__ __forceinline__ double2 operator()(double2 v) const {
+    return make_double2(flip_sign(swap ? v.y : v.x, fx), flip_sign(swap ? v.x : v.y, fy));
+  }
+};
+struct PhaseFactor {
+  double2 p;
+  __device__ __forceinline__ double2 operator()(double2 v) const { return cmul(p, v); }
+};
+template <class Put>
+__device__ __forceinline__ void with_phase(double2 p, Put put) {
+  if ((p.y == 0.0 && fabs(p.x) == 1.0) || (p.x == 0.0 && fabs(p.y) == 1.0)) {
+    const bool swap = p.x == 0.0;
+    const unsigned neg = (swap ? p.y : p.x) < 0.0 ? 0x80000000u : 0u;
+    put(PhaseTurn{swap, swap ? neg ^ 0x80000000u : neg, neg});
+  } else {
+    put(PhaseFactor{p});
+  }
+}
 __device__ __forceinline__ double2 phase_mul(double2 p, double2 v) {
-  if (p.y == 0.0) return p.x == 1.0 ? v : cscale(v, p.x);
-  if (p.x == 0.0) return make_double2(-p.y * v.y, p.y * v.x);
-  return cmul(p, v);
+  with_phase(p, [&](auto mul) { v = mul(v); });
+  return v;
 }
 
 // The numbers of all operations of the runs of one CTA, for one parameter vector, in one go:

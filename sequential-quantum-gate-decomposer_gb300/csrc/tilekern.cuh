@@ -64,17 +64,19 @@ __device__ __forceinline__ void store_tile(const double2* s, const TileArgs& a, 
                                            const int* ends) {
   double2* base = a.mtx + (long long)b * a.bstride;
   const int total = a.N * tc;
-  if (a.cstride == 1) {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int r = e / tc, c = e - r * tc;
-      base[(long long)r * a.rstride + v0 + c] = phase_mul(phase, s[c * a.N + end_place(ends, r)]);
+  with_phase(phase, [&](auto mul) {
+    if (a.cstride == 1) {
+      for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        int r = e / tc, c = e - r * tc;
+        base[(long long)r * a.rstride + v0 + c] = mul(s[c * a.N + end_place(ends, r)]);
+      }
+    } else {
+      for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        int c = e >> a.n, r = e & (a.N - 1);
+        base[(long long)(v0 + c) * a.rstride + r] = mul(s[c * a.N + r]);
+      }
     }
-  } else {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int c = e >> a.n, r = e & (a.N - 1);
-      base[(long long)(v0 + c) * a.rstride + r] = phase_mul(phase, s[c * a.N + r]);
-    }
-  }
+  });
 }
 
 // Operations are staged in shared memory kRotChunk at a time, so each CTA reads them from
