@@ -408,7 +408,7 @@ class Circuit:
         return -float(np.log(purity))
 
     def state_block_count(self):
-        """Fused passes over a state vector (blocks of the state-vector plan)."""
+        """Fused passes over one state vector (blocks of the plan that a batch of one takes)."""
         return _native.lib().sqg_state_block_count(self.native().handle)
 
     # ---- SQUANDER-compatible host API (numpy in, numpy out / in place) ---------------
